@@ -1,4 +1,5 @@
-"""ctypes binding of libb200tp.so (the C ABI declared in include/b200tp.h).
+"""ctypes binding of libb200tp.so (the C ABI declared in include/b200tp.h), and `native`, the torch binding over it
+(csrc/b2_torch.cpp) that the per-layer calls go through.
 
 There is no fallback: if the library has not been built, importing this module
 raises, and so does every layer that would have used it.
@@ -6,14 +7,17 @@ raises, and so does every layer that would have used it.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libb200tp.so")
+NATIVE_PATH = os.path.join(_HERE, "lib", "_b2torch.so")
 
-if not os.path.exists(LIB_PATH):
+if not (os.path.exists(LIB_PATH) and os.path.exists(NATIVE_PATH)):
     raise ImportError(
-        f"{LIB_PATH} is missing: build it with `python nano-vllm_b200/build.py` (nvcc, sm_100a). "
+        f"{LIB_PATH} or {NATIVE_PATH} is missing: build it with `python nano-vllm_b200/build.py` (nvcc, sm_100a). "
         "There is no CPU or PyTorch fallback for this path."
     )
 
@@ -109,3 +113,15 @@ def check(rc: int, what: str) -> None:
 
 def launch_count() -> int:
     return int(lib.b2_launch_count())
+
+
+def _load_native():
+    import torch  # noqa: F401  (its libraries must be in the process before the binding's)
+    loader = importlib.machinery.ExtensionFileLoader("_b2torch", NATIVE_PATH)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_b2torch", NATIVE_PATH, loader=loader))
+    loader.exec_module(module)
+    module.init(check)
+    return module
+
+
+native = _load_native()

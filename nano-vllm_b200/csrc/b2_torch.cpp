@@ -1,0 +1,300 @@
+// The step from torch tensors to the C ABI, in native code: checks dtypes and layouts, allocates the outputs, takes
+// the current stream and calls the library.  A layer of a short prompt or of a few decode rows lasts 50-100 us on the
+// GPU; the same step written in Python (per-argument attribute calls, ctypes conversion, a Stream object) cost 10-20 us
+// per call and four calls a layer, so the GPU waited for the host.  One call here is 2-4 us, launch included.
+//
+// Exceptions keep the Python wrappers' types: TypeError for a wrong dtype or device, ValueError for a shape that does
+// not fit, AssertionError for a violated layout contract; library errors go through _abi.check.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/Functions.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/DeviceGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/b200tp.h"
+
+namespace {
+
+PyObject* g_check = nullptr;  // _abi.check(rc, what): raises
+
+struct Raised {};  // a Python exception is set
+
+[[noreturn]] void raise(PyObject* type, const char* fmt, ...) {
+  va_list ap;
+  va_start(ap, fmt);
+  PyErr_FormatV(type, fmt, ap);
+  va_end(ap);
+  throw Raised{};
+}
+void expect(bool ok, const char* what) {
+  if (!ok) raise(PyExc_AssertionError, "%s", what);
+}
+void check(int rc, const char* what) {
+  if (rc == B2_OK) return;
+  PyObject* r = PyObject_CallFunction(g_check, "is", rc, what);
+  Py_XDECREF(r);
+  throw Raised{};
+}
+
+// ---- arguments -----------------------------------------------------------------
+const at::Tensor& tensor(PyObject* o, const char* what) {
+  if (!THPVariable_Check(o)) raise(PyExc_TypeError, "%s: expected a tensor, got %s", what, Py_TYPE(o)->tp_name);
+  return THPVariable_Unpack(o);
+}
+at::Tensor optional_tensor(PyObject* o, const char* what) { return o == Py_None ? at::Tensor() : tensor(o, what); }
+int64_t integer(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw Raised{};
+  return v;
+}
+float number(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw Raised{};
+  return static_cast<float>(v);
+}
+b2_ctx* context(PyObject* o) {
+  if (o == Py_None) return nullptr;
+  void* p = PyLong_AsVoidPtr(o);
+  if (p == nullptr && PyErr_Occurred()) throw Raised{};
+  return static_cast<b2_ctx*>(p);
+}
+void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+template <class T>
+const T* cptr(const at::Tensor& t) { return static_cast<const T*>(ptr(t)); }
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+// a CUDA bf16 tensor whose last dimension is contiguous
+at::Tensor bf16_rows(const at::Tensor& t, const char* what) {
+  if (t.scalar_type() != at::kBFloat16 || !t.is_cuda())
+    raise(PyExc_TypeError, "%s: expected a CUDA bf16 tensor, got %s on %s", what, c10::toString(t.scalar_type()), t.device().str().c_str());
+  return t.dim() > 0 && t.stride(-1) != 1 ? t.contiguous() : t;
+}
+// the same as rows a TMA map can describe: 2-D, 16-byte aligned base and row stride
+struct Rows {
+  at::Tensor t;
+  int64_t rows, cols, ld;
+};
+Rows matrix(const at::Tensor& x, const char* what) {
+  at::Tensor t = bf16_rows(x, what);
+  if (t.dim() != 2) t = t.reshape({-1, t.size(-1)});
+  if ((t.size(0) > 1 && t.stride(0) % 8 != 0) || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0) t = t.clone(at::MemoryFormat::Contiguous);
+  return {t, t.size(0), t.size(1), t.size(0) > 1 ? t.stride(0) : t.size(1)};
+}
+at::Tensor empty_rows(int64_t rows, int64_t cols, const at::Tensor& like) {
+  return at::detail::empty_cuda({rows, cols}, at::kBFloat16, like.device(), std::nullopt);
+}
+// out [rows, N] in the leading shape of x
+at::Tensor leading(const at::Tensor& out, const at::Tensor& x, int64_t n) {
+  if (x.dim() == 2) return out;
+  std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end() - 1);
+  shape.push_back(n);
+  return out.view(shape);
+}
+PyObject* wrap(const at::Tensor& t) { return THPVariable_Wrap(t); }
+PyObject* wrap(const at::Tensor& a, const at::Tensor& b) {
+  PyObject* p = PyTuple_New(2);
+  if (p == nullptr) throw Raised{};
+  PyTuple_SET_ITEM(p, 0, wrap(a));
+  PyTuple_SET_ITEM(p, 1, wrap(b));
+  return p;
+}
+
+using Args = PyObject* const*;
+
+// gemm(ctx, x, w, bias)
+PyObject* gemm(Args a) {
+  const at::Tensor& x = tensor(a[1], "gemm input");
+  const Rows in = matrix(x, "gemm input");
+  const at::Tensor w = bf16_rows(tensor(a[2], "gemm weight"), "gemm weight");
+  if (w.dim() != 2 || w.size(1) != in.cols) raise(PyExc_ValueError, "gemm: input has %lld features, weight has %lld", (long long)in.cols, (long long)w.size(-1));
+  const at::Tensor bias = optional_tensor(a[3], "gemm bias");
+  const int64_t n = w.size(0);
+  const at::Tensor out = empty_rows(in.rows, n, x);
+  if (in.rows)
+    check(b2_gemm(context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), out.data_ptr(), n, in.rows, n, in.cols, stream()), "b2_gemm");
+  return wrap(leading(out, x, n));
+}
+
+// gemm_silu_mul(ctx, x, w_pairs)
+PyObject* gemm_silu_mul(Args a) {
+  const at::Tensor& x = tensor(a[1], "gemm_silu_mul input");
+  const Rows in = matrix(x, "gemm_silu_mul input");
+  const at::Tensor& w = tensor(a[2], "gemm_silu_mul weight");
+  if (w.dim() != 2 || w.size(1) != in.cols || w.size(0) % 2) raise(PyExc_ValueError, "gemm_silu_mul: input has %lld features, paired weight has %lld rows of %lld", (long long)in.cols, (long long)w.size(0), (long long)w.size(-1));
+  const int64_t n = w.size(0) / 2;
+  const at::Tensor out = empty_rows(in.rows, n, x);
+  if (in.rows)
+    check(b2_gemm_silu_mul(context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), out.data_ptr(), n, in.rows, n, in.cols, stream()), "b2_gemm_silu_mul");
+  return wrap(leading(out, x, n));
+}
+
+struct Cache {
+  void *k = nullptr, *v = nullptr;
+  const int32_t* slots = nullptr;
+};
+Cache cache_of(const at::Tensor& k, const at::Tensor& v, const at::Tensor& slots, int64_t row) {
+  Cache c;
+  if (!k.defined() || k.numel() == 0) return c;
+  expect(k.stride(1) == row && slots.defined() && slots.scalar_type() == at::kInt, "k_cache rows must be contiguous and slot_mapping int32");
+  c.k = k.data_ptr();
+  c.v = v.data_ptr();
+  c.slots = slots.const_data_ptr<int32_t>();
+  return c;
+}
+
+// qkv_fused(ctx, x, w, bias, nq, nkv, head_dim, q_norm_w, k_norm_w, eps, positions, cos_sin, k_cache, v_cache, slot_mapping)
+PyObject* qkv_fused(Args a) {
+  const at::Tensor& x = tensor(a[1], "qkv input");
+  const Rows in = matrix(x, "qkv input");
+  const at::Tensor& w = tensor(a[2], "qkv weight");
+  const at::Tensor bias = optional_tensor(a[3], "qkv bias");
+  const int64_t nq = integer(a[4]), nkv = integer(a[5]), hd = integer(a[6]), n = w.size(0);
+  expect(n == (nq + 2 * nkv) * hd && w.size(1) == in.cols, "qkv_fused: weight shape");
+  const at::Tensor qw = optional_tensor(a[7], "q_norm_w"), kw = optional_tensor(a[8], "k_norm_w");
+  const at::Tensor& pos = tensor(a[10], "positions");
+  const at::Tensor& cs = tensor(a[11], "cos_sin");
+  expect(pos.scalar_type() == at::kLong && cs.scalar_type() == at::kFloat && cs.is_contiguous(), "positions must be int64, cos_sin contiguous fp32");
+  const at::Tensor kc = optional_tensor(a[12], "k_cache"), vc = optional_tensor(a[13], "v_cache"), sm = optional_tensor(a[14], "slot_mapping");
+  const Cache c = cache_of(kc, vc, sm, nkv * hd);
+  const at::Tensor out = empty_rows(in.rows, n, x);
+  if (in.rows)
+    check(b2_qkv_fused(context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), out.data_ptr(), n, in.rows, nq, nkv, hd, in.cols,
+                       ptr(qw), ptr(kw), number(a[9]), pos.const_data_ptr<int64_t>(), cs.const_data_ptr<float>(), c.k, c.v, c.slots, stream()), "b2_qkv_fused");
+  return wrap(out);
+}
+
+// rowpar_fused(ctx, x, w, bias, residual, norm_w, eps): None when the two-shot form serves this size
+PyObject* rowpar_fused(Args a) {
+  b2_ctx* ctx = context(a[0]);
+  const at::Tensor& x = tensor(a[1], "row-parallel input");
+  const Rows in = matrix(x, "row-parallel input");
+  const at::Tensor& w = tensor(a[2], "row-parallel weight");
+  const at::Tensor bias = optional_tensor(a[3], "bias"), norm_w = optional_tensor(a[5], "norm weight");
+  const int64_t n = w.size(0);
+  at::Tensor residual, res_out;
+  if (norm_w.defined()) {
+    residual = bf16_rows(tensor(a[4], "residual"), "residual").contiguous();
+    res_out = at::detail::empty_cuda(residual.sizes(), at::kBFloat16, residual.device(), std::nullopt);
+  }
+  if (in.rows) {
+    const int form = b2_rowpar_form(ctx, in.rows, n);
+    if (form < 0) check(-form, "b2_rowpar_form");
+    if (form == B2_FORM_TWOSHOT) Py_RETURN_NONE;
+  }
+  const at::Tensor out = empty_rows(in.rows, n, x);
+  if (in.rows)
+    check(b2_rowpar_fused(ctx, in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), in.rows, n, in.cols, ptr(residual), ptr(norm_w), number(a[6]),
+                          out.data_ptr(), ptr(res_out), stream()), "b2_rowpar_fused");
+  return norm_w.defined() ? wrap(out, res_out) : wrap(leading(out, x, n));
+}
+
+// rmsnorm(x, w, eps)
+PyObject* rmsnorm(Args a) {
+  at::Tensor x = bf16_rows(tensor(a[0], "rmsnorm input"), "rmsnorm input");
+  const at::Tensor& w = tensor(a[1], "rmsnorm weight");
+  const Rows in = matrix(x, "rmsnorm input");
+  const at::Tensor out = empty_rows(in.rows, in.cols, x);
+  check(b2_rmsnorm(in.t.data_ptr(), in.ld, w.data_ptr(), number(a[2]), in.rows, in.cols, out.data_ptr(), in.cols, stream()), "b2_rmsnorm");
+  return wrap(x.dim() == 2 ? out : out.view(x.sizes()));
+}
+
+// add_rmsnorm(x, residual, w, eps)
+PyObject* add_rmsnorm(Args a) {
+  const at::Tensor x = bf16_rows(tensor(a[0], "add_rmsnorm input"), "add_rmsnorm input").contiguous();
+  const at::Tensor r = bf16_rows(tensor(a[1], "residual"), "residual").contiguous();
+  const int64_t dim = x.size(-1), rows = x.numel() / dim;
+  const at::Tensor out = at::detail::empty_cuda(x.sizes(), at::kBFloat16, x.device(), std::nullopt);
+  const at::Tensor res_out = at::detail::empty_cuda(x.sizes(), at::kBFloat16, x.device(), std::nullopt);
+  check(b2_add_rmsnorm(x.data_ptr(), r.data_ptr(), tensor(a[2], "add_rmsnorm weight").data_ptr(), number(a[3]), rows, dim, out.data_ptr(), res_out.data_ptr(), stream()), "b2_add_rmsnorm");
+  return wrap(out, res_out);
+}
+
+// silu_and_mul(x)
+PyObject* silu_and_mul(Args a) {
+  const at::Tensor& x = tensor(a[0], "silu_and_mul input");
+  const Rows in = matrix(x, "silu_and_mul input");
+  const int64_t n = in.cols / 2;
+  const at::Tensor out = empty_rows(in.rows, n, x);
+  check(b2_silu_and_mul(in.t.data_ptr(), in.ld, in.rows, n, out.data_ptr(), stream()), "b2_silu_and_mul");
+  return wrap(leading(out, x, n));
+}
+
+// store_kvcache(key, value, k_cache, v_cache, slot_mapping)
+PyObject* store_kvcache(Args a) {
+  const at::Tensor &k = tensor(a[0], "key"), &v = tensor(a[1], "value"), &kc = tensor(a[2], "k_cache"), &vc = tensor(a[3], "v_cache"), &sm = tensor(a[4], "slot_mapping");
+  const int64_t n = k.size(0), hd = k.size(2), d = k.size(1) * hd;
+  // the reference's own preconditions (nanovllm/layers/attention.py:36-39)
+  expect(k.stride(-1) == 1 && v.stride(-1) == 1, "key and value must be contiguous in the last dimension");
+  expect(k.stride(1) == hd && v.stride(1) == hd, "heads must be contiguous");
+  expect(kc.stride(1) == d && vc.stride(1) == d, "cache rows must be contiguous");
+  expect(sm.numel() == n, "one slot per token");
+  expect(k.element_size() == 2 && kc.element_size() == 2 && sm.scalar_type() == at::kInt, "16-bit elements, int32 slots");
+  check(b2_store_kvcache(k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), kc.data_ptr(), vc.data_ptr(), sm.const_data_ptr<int32_t>(), n, d, stream()), "b2_store_kvcache");
+  Py_RETURN_NONE;
+}
+
+// qk_norm_rope_store(qkv, nq, nkv, head_dim, q_norm_w, k_norm_w, eps, positions, cos_sin, k_cache, v_cache, slot_mapping)
+PyObject* qk_norm_rope_store(Args a) {
+  const at::Tensor& qkv = tensor(a[0], "qkv");
+  expect(qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.scalar_type() == at::kBFloat16, "qkv must be a bf16 matrix with contiguous rows");
+  const int64_t nq = integer(a[1]), nkv = integer(a[2]), hd = integer(a[3]);
+  const at::Tensor qw = optional_tensor(a[4], "q_norm_w"), kw = optional_tensor(a[5], "k_norm_w");
+  const at::Tensor &pos = tensor(a[7], "positions"), &cs = tensor(a[8], "cos_sin");
+  expect(pos.scalar_type() == at::kLong && cs.scalar_type() == at::kFloat && cs.is_contiguous(), "positions must be int64, cos_sin contiguous fp32");
+  const at::Tensor kc = optional_tensor(a[9], "k_cache"), vc = optional_tensor(a[10], "v_cache"), sm = optional_tensor(a[11], "slot_mapping");
+  const Cache c = cache_of(kc, vc, sm, nkv * hd);
+  check(b2_qk_norm_rope_store(qkv.data_ptr(), qkv.stride(0), qkv.size(0), nq, nkv, hd, ptr(qw), ptr(kw), number(a[6]), pos.const_data_ptr<int64_t>(),
+                              cs.const_data_ptr<float>(), c.k, c.v, c.slots, stream()), "b2_qk_norm_rope_store");
+  Py_RETURN_NONE;
+}
+
+// embed(ctx, ids, w, vocab_start, vocab_end)
+PyObject* embed(Args a) {
+  at::Tensor ids = tensor(a[1], "token ids");
+  const at::Tensor& w = tensor(a[2], "embedding weight");
+  expect(ids.scalar_type() == at::kLong && ids.is_cuda(), "token ids must be CUDA int64");
+  ids = ids.contiguous();
+  const int64_t m = ids.numel(), h = w.size(1);
+  const at::Tensor out = at::detail::empty_cuda({m, h}, w.scalar_type(), w.device(), std::nullopt);
+  check(b2_embed(context(a[0]), ids.const_data_ptr<int64_t>(), w.data_ptr(), integer(a[3]), integer(a[4]), m, h, out.data_ptr(), stream()), "b2_embed");
+  if (ids.dim() == 1) return wrap(out);
+  std::vector<int64_t> shape(ids.sizes().begin(), ids.sizes().end());
+  shape.push_back(h);
+  return wrap(out.view(shape));
+}
+
+PyObject* init(Args a) {
+  Py_INCREF(a[0]);
+  Py_XDECREF(g_check);
+  g_check = a[0];
+  Py_RETURN_NONE;
+}
+
+template <PyObject* (*F)(Args), Py_ssize_t N>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != N) {
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", N, n);
+    return nullptr;
+  }
+  try {
+    return F(args);
+  } catch (const Raised&) {
+    return nullptr;
+  }
+  END_HANDLE_TH_ERRORS
+}
+
+#define B2_ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&entry<name, n>)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {B2_ENTRY(init, 1), B2_ENTRY(gemm, 4), B2_ENTRY(gemm_silu_mul, 3), B2_ENTRY(qkv_fused, 15), B2_ENTRY(rowpar_fused, 7),
+                         B2_ENTRY(rmsnorm, 3), B2_ENTRY(add_rmsnorm, 4), B2_ENTRY(silu_and_mul, 1), B2_ENTRY(store_kvcache, 5),
+                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(embed, 5), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_b2torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__b2torch(void) { return PyModule_Create(&module_def); }

@@ -31,6 +31,7 @@ class TPRuntime:
         torch.cuda.set_device(device)
         _abi.check(_abi.lib.b2_ctx_create(C.byref(cfg), C.byref(ctx)), "b2_ctx_create")
         self.ctx = ctx
+        self.handle = ctx.value  # the same as a plain integer, for the torch binding
         self.poisoned = False
         if world > 1:
             handle = (C.c_ubyte * _abi.HANDLE_BYTES)()
@@ -77,7 +78,7 @@ class TPRuntime:
             ops._LOGIT_VIEWS.clear()  # views of the buffer that is about to be freed
             torch.cuda.synchronize()
             _abi.lib.b2_ctx_destroy(self.ctx)
-            self.ctx = None
+            self.ctx = self.handle = None
 
 
 _RUNTIME: TPRuntime | None = None
