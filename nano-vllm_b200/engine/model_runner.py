@@ -12,6 +12,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass, field
 
+import numpy as np
 import torch
 import torch.distributed as dist
 
@@ -19,6 +20,8 @@ from ..layers.sampler import Sampler
 from ..models.qwen3 import Qwen3ForCausalLM
 from ..runtime import get_runtime, init_runtime, shutdown_runtime
 from ..utils.context import reset_context, set_context
+
+_TORCH_DTYPE = {np.dtype(np.int64): torch.int64, np.dtype(np.int32): torch.int32, np.dtype(np.float32): torch.float32}
 
 FUSED_SAMPLER_MAX_ROWS = 256  # b2_lm_head_sample takes one token tile of the feature-lane layout
 
@@ -74,6 +77,20 @@ def random_init_(model: torch.nn.Module, seed: int, tp_rank: int) -> None:
             p.data.copy_(torch.empty(p.shape, dtype=torch.float32, device=p.device).normal_(0, 0.02, generator=g))
 
 
+_ROW_INPUT_BYTES = 28
+
+
+def _row_inputs(buf: torch.Tensor) -> dict[str, torch.Tensor]:
+    """The per-row inputs of a decode step as views of one byte buffer of _ROW_INPUT_BYTES per row."""
+    n, out, at = buf.numel() // _ROW_INPUT_BYTES, {}, 0
+    for name, dtype in (("input_ids", torch.int64), ("positions", torch.int64), ("slot_mapping", torch.int32),
+                        ("context_lens", torch.int32), ("temperatures", torch.float32)):
+        size = n * dtype.itemsize
+        out[name] = buf[at:at + size].view(dtype)
+        at += size
+    return out
+
+
 class ModelRunner:
 
     def __init__(self, config: ModelConfig, *, max_num_seqs: int = 512, max_model_len: int = 4096, max_num_batched_tokens: int = 16384,
@@ -97,20 +114,19 @@ class ModelRunner:
                                     vocab=config.vocab_size, max_seqs=max_num_seqs, timeout_ms=timeout_ms)
         prev_dtype = torch.get_default_dtype()
         torch.set_default_dtype(torch.bfloat16)
-        torch.set_default_device(self.device)
         try:
-            self.model = Qwen3ForCausalLM(config)
-            if full_weights is not None:
-                self.model.load_full_weights(full_weights)
-            else:
-                random_init_(self.model, seed, self.rank)
-            self.sampler = Sampler()
-            self._allocate_kv_cache(num_kvcache_blocks, gpu_memory_utilization)
-            self.graphs: dict[int, torch.cuda.CUDAGraph] = {}
-            if not enforce_eager:
-                self._capture_graphs()
+            with self.device:  # (torch.set_default_device would leave a Python hook on every later torch call of the process)
+                self.model = Qwen3ForCausalLM(config)
+                if full_weights is not None:
+                    self.model.load_full_weights(full_weights)
+                else:
+                    random_init_(self.model, seed, self.rank)
+                self.sampler = Sampler()
+                self._allocate_kv_cache(num_kvcache_blocks, gpu_memory_utilization)
+                self.graphs: dict[int, torch.cuda.CUDAGraph] = {}
+                if not enforce_eager:
+                    self._capture_graphs()
         finally:
-            torch.set_default_device("cpu")
             torch.set_default_dtype(prev_dtype)
 
     # ---- teardown (reference :50-59) --------------------------------------
@@ -144,42 +160,66 @@ class ModelRunner:
     def _h2d(self, values, dtype):
         return torch.tensor(values, dtype=dtype, pin_memory=True).to(self.device, non_blocking=True)
 
-    def _block_tables(self, seqs: list[Seq]):
+    def _to_device(self, *arrays: np.ndarray) -> list[torch.Tensor]:
+        """The arrays on the device, sent as one pinned buffer in one copy (a copy costs the host and the stream a few
+        microseconds however small it is).  torch's pinned pool keeps the buffer until the copy has run."""
+        offsets, size = [], 0
+        for a in arrays:
+            offsets.append(size)
+            size += (a.nbytes + 15) & ~15
+        host = torch.empty(max(size, 16), dtype=torch.uint8, pin_memory=True)
+        raw = host.numpy()
+        for a, off in zip(arrays, offsets):
+            raw[off:off + a.nbytes] = a.reshape(-1).view(np.uint8)
+        dev = host.to(self.device, non_blocking=True)
+        return [dev[off:off + a.nbytes].view(_TORCH_DTYPE[a.dtype]).view(a.shape) for a, off in zip(arrays, offsets)]
+
+    def _block_tables(self, seqs: list[Seq]) -> np.ndarray:
         width = max(len(s.block_table) for s in seqs)
-        return self._h2d([s.block_table + [-1] * (width - len(s.block_table)) for s in seqs], torch.int32)
+        tables = np.full((len(seqs), width), -1, dtype=np.int32)
+        for row, s in zip(tables, seqs):
+            row[:len(s.block_table)] = s.block_table
+        return tables
 
     def prepare_prefill(self, seqs: list[Seq], num_new: list[int] | None = None):
         """Tokens [num_cached, num_cached + new) of each sequence are computed;
         their K/V go to the slots their block table assigns (reference :129-170)."""
-        ids, pos, slots, cu_q, cu_k = [], [], [], [0], [0]
-        max_q = max_k = 0
         bs = self.block_size
-        for i, s in enumerate(seqs):
-            start = s.num_cached_tokens
-            end = len(s) if num_new is None else start + num_new[i]
-            ids.extend(s.token_ids[start:end])
-            pos.extend(range(start, end))
-            cu_q.append(cu_q[-1] + end - start)
-            cu_k.append(cu_k[-1] + end)
-            max_q, max_k = max(max_q, end - start), max(max_k, end)
+        starts = [s.num_cached_tokens for s in seqs]
+        ends = [len(s) if num_new is None else a + num_new[i] for i, (s, a) in enumerate(zip(seqs, starts))]
+        news = [b - a for a, b in zip(starts, ends)]
+        total = sum(news)
+        ids, pos = np.empty(total, dtype=np.int64), np.empty(total, dtype=np.int64)
+        slots = np.empty(total, dtype=np.int32)
+        used, at = 0, 0  # tokens with a slot, tokens so far
+        for s, a, b, n in zip(seqs, starts, ends, news):
+            ids[at:at + n] = s.token_ids[a:b]
+            pos[at:at + n] = p = np.arange(a, b)
             if s.block_table:
-                slots.extend(s.block_table[p // bs] * bs + p % bs for p in range(start, end))
-        block_tables = self._block_tables(seqs) if cu_k[-1] > cu_q[-1] else None
-        ids_t, pos_t = self._h2d(ids, torch.int64), self._h2d(pos, torch.int64)
-        set_context(True, self._h2d(cu_q, torch.int32), self._h2d(cu_k, torch.int32), max_q, max_k,
-                    self._h2d(slots, torch.int32) if slots else None, None, block_tables)
+                slots[used:used + n] = np.asarray(s.block_table, dtype=np.int32)[p // bs] * bs + p % bs
+                used += n
+            at += n
+        cu_q, cu_k = np.zeros(len(seqs) + 1, dtype=np.int32), np.zeros(len(seqs) + 1, dtype=np.int32)
+        np.cumsum(news, out=cu_q[1:])
+        np.cumsum(ends, out=cu_k[1:])
+        arrays = [ids, pos, cu_q, cu_k, cu_q[1:] - 1, slots[:used]]
+        if cu_k[-1] > cu_q[-1]:
+            arrays.append(self._block_tables(seqs))
+        ids_t, pos_t, cu_q_t, cu_k_t, last_t, slots_t, *tables_t = self._to_device(*arrays)
+        set_context(True, cu_q_t, cu_k_t, max(news), max(ends), slots_t if used else None, None, tables_t[0] if tables_t else None,
+                    last_token_index=last_t)
         return ids_t, pos_t
 
     def prepare_decode(self, seqs: list[Seq]):
         """One new token per sequence: the last one of its list (reference :172-188)."""
         bs = self.block_size
-        ids = [s.token_ids[-1] for s in seqs]
-        pos = [len(s) - 1 for s in seqs]
-        slots = [s.block_table[(len(s) - 1) // bs] * bs + (len(s) - 1) % bs for s in seqs]
         lens = [len(s) for s in seqs]
-        set_context(False, slot_mapping=self._h2d(slots, torch.int32), context_lens=self._h2d(lens, torch.int32),
-                    block_tables=self._block_tables(seqs))
-        return self._h2d(ids, torch.int64), self._h2d(pos, torch.int64)
+        ids_t, pos_t, slots_t, lens_t, tables_t = self._to_device(
+            np.array([s.token_ids[-1] for s in seqs], dtype=np.int64), np.array([n - 1 for n in lens], dtype=np.int64),
+            np.array([s.block_table[(n - 1) // bs] * bs + (n - 1) % bs for s, n in zip(seqs, lens)], dtype=np.int32),
+            np.array(lens, dtype=np.int32), self._block_tables(seqs))
+        set_context(False, slot_mapping=slots_t, context_lens=lens_t, block_tables=tables_t)
+        return ids_t, pos_t
 
     # ---- forward ---------------------------------------------------------------
     @torch.inference_mode()
@@ -208,22 +248,24 @@ class ModelRunner:
 
     def _decode_staging(self):
         """Pinned host mirrors of the graphs' input buffers, allocated once: a decode step fills them with
-        numpy and issues one asynchronous copy per buffer straight into the graph's inputs (no per-step pinned
-        allocations, no device-to-device staging copies)."""
+        numpy and issues one asynchronous copy for all the per-row inputs straight into the graph's inputs (no per-step
+        pinned allocations, no device-to-device staging copies)."""
         if getattr(self, "_stage", None) is None:
             gv = self.graph_vars
-            self._stage = {k: torch.zeros(gv[k].shape, dtype=gv[k].dtype, pin_memory=True) for k in
-                           ("input_ids", "positions", "slot_mapping", "context_lens", "block_tables")}
-            self._stage_np = {k: v.numpy() for k, v in self._stage.items()}
+            self._stage = torch.zeros(gv["rows"].shape, dtype=torch.uint8, pin_memory=True)
+            self._stage_tables = torch.zeros(gv["block_tables"].shape, dtype=torch.int32, pin_memory=True)
+            self._stage_np = {k: v.numpy() for k, v in _row_inputs(self._stage).items()}
+            self._stage_np["block_tables"] = self._stage_tables.numpy()
             self._bt_rows = {}  # row of the staged block table -> the blocks last copied into the graph's table for it
-        return self._stage, self._stage_np
+        return self._stage_np
 
     @torch.inference_mode()
-    def _decode_graph_step(self, seqs: list[Seq]):
-        """prepare_decode + the graph replay of run_model in one go, for batches a captured graph covers."""
+    def _decode_graph_step(self, seqs: list[Seq], temperatures: list[float] | None):
+        """prepare_decode + the graph replay of run_model in one go, for batches a captured graph covers.  Returns the
+        hidden rows and the temperatures on the device (None for greedy decoding)."""
         n = len(seqs)
         bs = next(b for b in self.graph_bs if b >= n)
-        stage, np_ = self._decode_staging()
+        np_ = self._decode_staging()
         blk = self.block_size
         lens = [len(s) for s in seqs]
         np_["input_ids"][:n] = [s.token_ids[-1] for s in seqs]
@@ -232,6 +274,8 @@ class ModelRunner:
         np_["context_lens"][n:bs] = 0          # padded rows attend to nothing ...
         np_["slot_mapping"][:n] = [s.block_table[(l - 1) // blk] * blk + (l - 1) % blk for s, l in zip(seqs, lens)]
         np_["slot_mapping"][n:bs] = -1         # ... and store nothing
+        if temperatures is not None:
+            np_["temperatures"][:n] = temperatures
         # block tables change only when a sequence takes a new block (every 256 tokens) or the batch changes: rows are
         # rewritten, and the table copied, only then
         bt = np_["block_tables"]
@@ -240,42 +284,37 @@ class ModelRunner:
         for i, s in enumerate(seqs):
             t = s.block_table
             width = max(width, len(t))
-            key = tuple(t)
-            if rows.get(i) != key:
+            if rows.get(i) != t:
                 bt[i, :len(t)] = t
-                rows[i] = key
+                rows[i] = list(t)
                 dirty = True
         gv = self.graph_vars
-        for k in ("input_ids", "positions", "slot_mapping", "context_lens"):
-            gv[k][:bs].copy_(stage[k][:bs], non_blocking=True)
+        gv["rows"].copy_(self._stage, non_blocking=True)
         if dirty:
-            gv["block_tables"][:n, :width].copy_(stage["block_tables"][:n, :width], non_blocking=True)
+            gv["block_tables"][:n, :width].copy_(self._stage_tables[:n, :width], non_blocking=True)
         self.graphs[bs].replay()
         set_context(False)  # the LM head only needs to know this is not a prefill step
-        return gv["outputs"][:n]
+        return gv["outputs"][:n], gv["temperatures"][:n] if temperatures is not None else None
 
     @torch.inference_mode()
     def step(self, seqs: list[Seq], is_prefill: bool, temperatures: list[float] | None = None, num_new: list[int] | None = None):
         """One forward pass + sampling on rank 0; the chosen token ids are
         returned on every rank.  temperatures=None means greedy (argmax)."""
         if not is_prefill and not self.enforce_eager and len(seqs) <= self.graph_bs[-1]:
-            hidden = self._decode_graph_step(seqs)
+            hidden, temps = self._decode_graph_step(seqs, temperatures)
         else:
             ids, pos = self.prepare_prefill(seqs, num_new) if is_prefill else self.prepare_decode(seqs)
             hidden = self.run_hidden(ids, pos, is_prefill)
+            temps = None if temperatures is None else self._h2d(temperatures, torch.float32)
         if getattr(self, "_picked", None) is None or self._picked.numel() < len(seqs):
             self._picked = torch.zeros(max(len(seqs), self.max_num_seqs), dtype=torch.int64, device=self.device)
         picked = self._picked[:len(seqs)]  # one buffer for every step: rank 0's sampler fills it, the broadcast hands it to the others
         if self.fused_sampler and len(seqs) <= FUSED_SAMPLER_MAX_ROWS:
-            temps = None if temperatures is None else self._h2d(temperatures, torch.float32)
             self.model.sample_tokens(hidden, temps, self.sample_seed, out=picked)
         else:
             logits = self.model.compute_logits(hidden)
             if self.rank == 0:
-                if temperatures is None:
-                    picked = Sampler.greedy(logits)
-                else:
-                    picked = self.sampler(logits, self._h2d(temperatures, torch.float32))
+                picked = Sampler.greedy(logits) if temps is None else self.sampler(logits, temps)
         if self.world > 1:
             from .. import ops
             ops.broadcast_tokens(picked)  # rank 0's choice reaches every rank on the device
@@ -291,14 +330,14 @@ class ModelRunner:
         max_bs = min(self.max_num_seqs, 512)
         max_blocks = (self.max_model_len + self.block_size - 1) // self.block_size
         dev = self.device
+        rows = torch.zeros(max_bs * _ROW_INPUT_BYTES, dtype=torch.uint8, device=dev)
         gv = dict(
-            input_ids=torch.zeros(max_bs, dtype=torch.int64, device=dev),
-            positions=torch.zeros(max_bs, dtype=torch.int64, device=dev),
-            slot_mapping=torch.full((max_bs,), -1, dtype=torch.int32, device=dev),
-            context_lens=torch.zeros(max_bs, dtype=torch.int32, device=dev),
+            rows=rows,  # the per-row inputs below, side by side: one copy fills them all
+            **_row_inputs(rows),
             block_tables=torch.zeros(max_bs, max_blocks, dtype=torch.int32, device=dev),
             outputs=torch.zeros(max_bs, c.hidden_size, dtype=torch.bfloat16, device=dev),
         )
+        gv["slot_mapping"].fill_(-1)
         self.graph_bs = [b for b in (1, 2, 4, 8) if b <= max_bs] + list(range(16, max_bs + 1, 16))
         self.graph_pool = None
         for bs in reversed(self.graph_bs):

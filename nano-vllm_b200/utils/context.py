@@ -15,13 +15,16 @@ class Context:
 
     def __init__(self, is_prefill: bool = False, cu_seqlens_q: torch.Tensor | None = None, cu_seqlens_k: torch.Tensor | None = None,
                  max_seqlen_q: int = 0, max_seqlen_k: int = 0, slot_mapping: torch.Tensor | None = None,
-                 context_lens: torch.Tensor | None = None, block_tables: torch.Tensor | None = None):
+                 context_lens: torch.Tensor | None = None, block_tables: torch.Tensor | None = None,
+                 last_token_index: torch.Tensor | None = None):
         self.is_prefill = is_prefill
         self.cu_seqlens_q, self.cu_seqlens_k = cu_seqlens_q, cu_seqlens_k
         self.max_seqlen_q, self.max_seqlen_k = max_seqlen_q, max_seqlen_k
         self.slot_mapping, self.context_lens, self.block_tables = slot_mapping, context_lens, block_tables
-        # int32 index of the last token of every sequence (cu_seqlens_q[1:] - 1), built once per prefill step
-        self.last_token_index = (cu_seqlens_q[1:] - 1).to(torch.int32) if (is_prefill and cu_seqlens_q is not None) else None
+        # int32 index of the last token of every sequence (cu_seqlens_q[1:] - 1): from the caller, or built once per prefill step
+        if last_token_index is None and is_prefill and cu_seqlens_q is not None:
+            last_token_index = (cu_seqlens_q[1:] - 1).to(torch.int32)
+        self.last_token_index = last_token_index
 
 
 _current = Context()
@@ -32,9 +35,10 @@ def get_context() -> Context:
 
 
 def set_context(is_prefill, cu_seqlens_q=None, cu_seqlens_k=None, max_seqlen_q=0, max_seqlen_k=0, slot_mapping=None,
-                context_lens=None, block_tables=None) -> None:
+                context_lens=None, block_tables=None, last_token_index=None) -> None:
     global _current
-    _current = Context(is_prefill, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, slot_mapping, context_lens, block_tables)
+    _current = Context(is_prefill, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, slot_mapping, context_lens, block_tables,
+                       last_token_index)
 
 
 def reset_context() -> None:
