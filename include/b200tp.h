@@ -380,6 +380,24 @@ int b2_qk_norm_rope_store(void* qkv, int64_t ld_qkv, int M, int nq, int nkv, int
                           const int64_t* positions, const float* cos_sin,
                           void* k_cache, void* v_cache, const int32_t* slot_mapping, void* stream);
 
+/* ---- decode attention over the paged cache: what flash_attn_with_kvcache computes
+ *      for one query token per sequence (nanovllm/layers/attention.py:70-74) -------
+ * q [n_seqs, nq, head_dim] bf16 with row stride q_stride (a view of the qkv output);
+ * k_cache / v_cache [num_blocks, block_size, nkv, head_dim]; block_tables int32 with bt_width
+ * columns and row stride bt_stride; context_lens int32 (the new token included; 0 = a padded
+ * row, whose output is zero).  out [n_seqs, nq, head_dim] contiguous:
+ *   out = softmax(scale q K^T) V over the sequence's first context_lens tokens,
+ * fp32 scores and sums, probabilities rounded to bf16 for the second product.  Lengths and tables
+ * are read on the device, so a captured call serves any later batch of the same size; they are read while earlier
+ * b2_* kernels of the stream may still be running, so they must not be results of one, b2_advance_decode excepted.
+ * b2_paged_attention_supported says (1 / 0) whether the shape is served: head_dim 128, at most 8
+ * query heads per KV head, blocks of a multiple of 64 tokens, at most 1024 sequences. */
+int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
+                              int num_blocks, int block_size, const int32_t* block_tables, int64_t bt_stride, int bt_width,
+                              const int32_t* context_lens, int n_seqs, int nq, int nkv, int head_dim, float scale,
+                              void* out, void* stream);
+int b2_paged_attention_supported(int n_seqs, int nq, int nkv, int head_dim, int block_size);
+
 /* Greedy pick: out[i] = argmax_j logits[i, j] (first index on ties), int64.
  * The reference's Sampler (nanovllm/layers/sampler.py:7-12) at temperature -> 0. */
 int b2_argmax(const void* logits, int64_t ld, int B, int V, int64_t* out, void* stream);

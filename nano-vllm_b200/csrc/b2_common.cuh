@@ -51,6 +51,8 @@ struct B2Status {
 };
 
 #define B2_MAX_WORLD 8
+#define B2_ATTN_MAX_ITEMS 65536               // decode attention: (sequence, KV head) pairs of one call
+#define B2_ATTN_WS_FLOATS_PER_SM (2 * 2 * 1040)  // decode attention: two partial results per CTA, two CTAs per SM
 
 // ---------------------------------------------------------------------------
 // small PTX wrappers
@@ -389,6 +391,8 @@ struct b2_ctx {
   B2Status* status_dev;   // device alias of status_host
   __nv_bfloat16* gather_rows;  // [max_seqs][hidden] staging for the LM head
   unsigned long long* sample_keys;  // [max_seqs] fused sampler: this rank's best key per row, zero between calls
+  float* attn_ws;       // decode attention: partial results of items that span several CTAs
+  int* attn_counters;   // decode attention: arrivals per item, zero between launches
   unsigned long long* trace;   // [num_sms][8][2] phase stamps of the last GEMM launch
   bool trace_on;
 };

@@ -192,6 +192,9 @@ static int ctx_init(b2_ctx* c) {
     B2_CUDA(cudaMalloc(&c->sample_keys, static_cast<size_t>(c->cfg.max_seqs) * 8));
     B2_CUDA(cudaMemset(c->sample_keys, 0, static_cast<size_t>(c->cfg.max_seqs) * 8));
   }
+  B2_CUDA(cudaMalloc(&c->attn_ws, static_cast<size_t>(c->num_sms) * B2_ATTN_WS_FLOATS_PER_SM * sizeof(float)));
+  B2_CUDA(cudaMalloc(&c->attn_counters, B2_ATTN_MAX_ITEMS * sizeof(int)));
+  B2_CUDA(cudaMemset(c->attn_counters, 0, B2_ATTN_MAX_ITEMS * sizeof(int)));
   B2_CUDA(cudaMalloc(&c->trace, static_cast<size_t>(c->num_sms) * 16 * sizeof(unsigned long long)));
   B2_CUDA(cudaMemset(c->trace, 0, static_cast<size_t>(c->num_sms) * 16 * sizeof(unsigned long long)));
   c->trace_on = false;
@@ -233,6 +236,8 @@ int b2_ctx_destroy(b2_ctx* c) {
   cudaFree(c->splitk_ws);
   cudaFree(c->tile_counters);
   cudaFree(c->dstate);
+  cudaFree(c->attn_ws);
+  cudaFree(c->attn_counters);
   cudaFree(c->trace);
   if (c->gather_rows) cudaFree(c->gather_rows);
   if (c->sample_keys) cudaFree(c->sample_keys);
@@ -271,6 +276,7 @@ int b2_ctx_reset(b2_ctx* c) {
   B2_CUDA(cudaMemset(c->splitk_ws, 0, c->splitk_ws_bytes));
   B2_CUDA(cudaMemset(c->tile_counters, 0, static_cast<size_t>(c->tile_counter_cap) * 4 * sizeof(int)));
   B2_CUDA(cudaMemset(c->dstate, 0, sizeof(B2DeviceState)));
+  B2_CUDA(cudaMemset(c->attn_counters, 0, B2_ATTN_MAX_ITEMS * sizeof(int)));
   if (c->sample_keys) B2_CUDA(cudaMemset(c->sample_keys, 0, static_cast<size_t>(c->cfg.max_seqs) * 8));
   B2_CUDA(cudaDeviceSynchronize());
   c->status_host->code = 0;

@@ -449,14 +449,10 @@ __global__ void __launch_bounds__(256) broadcast_tokens_kernel(const BcastArgs a
 // A row whose next position has no block in its table (past the table's width, a -1 entry, or a slot beyond the
 // cache) is frozen: it stores nothing (slot -1) and its position and context length stay, so that a replay past
 // a sequence's capacity can never send the KV scatter outside the cache.
-__global__ void advance_decode_kernel(const int64_t* __restrict__ tokens, int64_t* __restrict__ input_ids,
-                                      int64_t* __restrict__ positions, int32_t* __restrict__ context_lens,
-                                      int32_t* __restrict__ slot_mapping, const int32_t* __restrict__ block_tables,
-                                      int64_t bt_stride, int bt_width, int block_size, int64_t num_slots, int n) {
-  b2::pdl_launch_dependents();
-  b2::pdl_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ void advance_row(int i, const int64_t* __restrict__ tokens, int64_t* __restrict__ input_ids,
+                                            int64_t* __restrict__ positions, int32_t* __restrict__ context_lens,
+                                            int32_t* __restrict__ slot_mapping, const int32_t* __restrict__ block_tables,
+                                            int64_t bt_stride, int bt_width, int block_size, int64_t num_slots) {
   input_ids[i] = tokens[i];
   const int64_t p = positions[i] + 1;
   const int64_t b = p / block_size;
@@ -470,6 +466,18 @@ __global__ void advance_decode_kernel(const int64_t* __restrict__ tokens, int64_
   positions[i] = p;
   context_lens[i] += 1;
   slot_mapping[i] = static_cast<int32_t>(slot);
+}
+
+__global__ void advance_decode_kernel(const int64_t* __restrict__ tokens, int64_t* __restrict__ input_ids,
+                                      int64_t* __restrict__ positions, int32_t* __restrict__ context_lens,
+                                      int32_t* __restrict__ slot_mapping, const int32_t* __restrict__ block_tables,
+                                      int64_t bt_stride, int bt_width, int block_size, int64_t num_slots, int n) {
+  b2::pdl_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) advance_row(i, tokens, input_ids, positions, context_lens, slot_mapping, block_tables, bt_stride, bt_width, block_size, num_slots);
+  // later kernels may read the new lengths ahead of their dependency wait: released only now
+  __threadfence();
+  b2::pdl_launch_dependents();
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

@@ -267,6 +267,22 @@ PyObject* embed(Args a) {
   return wrap(out.view(shape));
 }
 
+// paged_attention(ctx, q, k_cache, v_cache, context_lens, block_tables, scale): None when the kernel does not serve the shape
+PyObject* paged_attention(Args a) {
+  const at::Tensor &q = tensor(a[1], "q"), &kc = tensor(a[2], "k_cache"), &vc = tensor(a[3], "v_cache"), &lens = tensor(a[4], "context_lens"),
+                   &tables = tensor(a[5], "block_tables");
+  const int64_t n = q.size(0), nq = q.size(1), hd = q.size(2), nkv = kc.size(2), bs = kc.size(1);
+  if (!b2_paged_attention_supported(n, nq, nkv, hd, bs) || q.scalar_type() != at::kBFloat16 || q.stride(2) != 1 || q.stride(1) != hd || !kc.is_contiguous() ||
+      !vc.is_contiguous() || tables.stride(1) != 1)
+    Py_RETURN_NONE;
+  expect(lens.scalar_type() == at::kInt && tables.scalar_type() == at::kInt && kc.scalar_type() == at::kBFloat16, "int32 lengths and block tables, bf16 cache");
+  const at::Tensor out = at::detail::empty_cuda({n, nq, hd}, at::kBFloat16, q.device(), std::nullopt);
+  check(b2_paged_attention_decode(context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, kc.data_ptr(), vc.data_ptr(), kc.size(0), bs, tables.const_data_ptr<int32_t>(),
+                                  n > 1 ? tables.stride(0) : tables.size(1), tables.size(1), lens.const_data_ptr<int32_t>(), n, nq, nkv, hd, number(a[6]),
+                                  out.data_ptr(), stream()), "b2_paged_attention_decode");
+  return wrap(out);
+}
+
 PyObject* init(Args a) {
   Py_INCREF(a[0]);
   Py_XDECREF(g_check);
@@ -292,7 +308,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define B2_ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {B2_ENTRY(init, 1), B2_ENTRY(gemm, 4), B2_ENTRY(gemm_silu_mul, 3), B2_ENTRY(qkv_fused, 15), B2_ENTRY(rowpar_fused, 7),
                          B2_ENTRY(rmsnorm, 3), B2_ENTRY(add_rmsnorm, 4), B2_ENTRY(silu_and_mul, 1), B2_ENTRY(store_kvcache, 5),
-                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(embed, 5), {nullptr, nullptr, 0, nullptr}};
+                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(embed, 5), B2_ENTRY(paged_attention, 7), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_b2torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

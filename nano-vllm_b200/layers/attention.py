@@ -3,9 +3,10 @@
 `store_kvcache` has the signature and preconditions of
 nanovllm/layers/attention.py:33-40 (the Triton kernel at :10-30 is replaced by
 b2_store_kvcache: 16-byte vector copies, several tokens per CTA, bit-exact).
-`Attention` keeps the reference's interface (:43-75).  The attention
-arithmetic itself stays a library call, as in the reference: flash-attn's
-varlen kernel for prefill and its paged kv-cache kernel for decode.
+`Attention` keeps the reference's interface (:43-75).  Decode attention runs on
+b2_paged_attention_decode (flash-attn's paged kernel for the shapes it does not
+serve); prefill attention stays a library call, as in the reference: flash-attn's
+varlen kernel.
 """
 from __future__ import annotations
 
@@ -57,7 +58,8 @@ def _sdpa_paged(q, k_cache, v_cache, context_lens, block_tables, scale, q_lens=N
 
 
 class Attention(nn.Module):
-    # "flash_attn" (the reference's library call) or "sdpa" (plain PyTorch, for tests on small shapes when flash-attn cannot run)
+    # "flash_attn" (own decode kernel, the reference's library call otherwise) or "sdpa" (plain PyTorch, for tests on small
+    # shapes when flash-attn cannot run)
     backend = "flash_attn"
 
     def __init__(self, num_heads, head_dim, scale, num_kv_heads):
@@ -85,6 +87,10 @@ class Attention(nn.Module):
                     return torch.cat(outs)
                 return _sdpa_paged(q, k_cache, v_cache, k_lens, ctx.block_tables, self.scale, q_lens)
             return _sdpa_paged(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
+        if not ctx.is_prefill:
+            o = ops.paged_attention(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
+            if o is not None:
+                return o
         if flash_attn_varlen_func is None:
             raise RuntimeError("flash-attn is not importable; set Attention.backend = 'sdpa' for small test shapes")
         if ctx.is_prefill:
