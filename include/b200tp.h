@@ -100,7 +100,8 @@ int b2_ctx_reset(b2_ctx* ctx);
  * enabled, every CTA of those kernels records 8 (SM clock, global ns) stamps:
  * 0 set-up done, 1 first operand tile landed, 2 last MMA issued, 3 earlier
  * kernels complete (dependency wait passed), 4 epilogue done, 5 GEMM part
- * left, 6 reduce phase done, 7 kernel entry.  If
+ * left (GEMMs of more than 64 tokens: accumulator complete), 6 reduce phase
+ * done (or: CTA about to leave), 7 kernel entry.  If
  * host_out is non-NULL the call synchronises the device, copies
  * min(max_ctas, SM count) * 16 uint64 stamps of the most recent launch and
  * clears them.  Not for use during graph capture. */
@@ -390,8 +391,8 @@ int b2_qk_norm_rope_store(void* qkv, int64_t ld_qkv, int M, int nq, int nkv, int
  * fp32 scores and sums, probabilities rounded to bf16 for the second product.  Lengths and tables
  * are read on the device, so a captured call serves any later batch of the same size; they are read while earlier
  * b2_* kernels of the stream may still be running, so they must not be results of one, b2_advance_decode excepted.
- * b2_paged_attention_supported says (1 / 0) whether the shape is served: head_dim 128, at most 8
- * query heads per KV head, blocks of a multiple of 64 tokens, at most 1024 sequences. */
+ * b2_paged_attention_supported says (1 / 0) whether the shape is served: head_dim 128, one or
+ * two query heads per KV head, blocks of a multiple of 64 tokens, at most 1024 sequences. */
 int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
                               int num_blocks, int block_size, const int32_t* block_tables, int64_t bt_stride, int bt_width,
                               const int32_t* context_lens, int n_seqs, int nq, int nkv, int head_dim, float scale,

@@ -315,6 +315,15 @@ __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w 
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
+// silu(gate) * up on bf16-rounded inputs, with the reference's roundings (nanovllm/layers/activation.py:8-11, eager):
+// the activation is rounded to bf16 before the product, the product once more by the caller's pack
+__device__ __forceinline__ float silu_mul(float gate, float up) { return bf16_round(gate / (1.0f + expf(-gate))) * up; }
+// 8 bf16 = 4 (gate, up) pairs -> 4 bf16
+__device__ __forceinline__ uint2 silu_mul_pairs(const uint4& w) {
+  return make_uint2(pack_bf16(silu_mul(bf16_lo(w.x), bf16_hi(w.x)), silu_mul(bf16_lo(w.y), bf16_hi(w.y))),
+                    pack_bf16(silu_mul(bf16_lo(w.z), bf16_hi(w.z)), silu_mul(bf16_lo(w.w), bf16_hi(w.w))));
+}
+
 // replace a -0.0 half (the sentinel) by +0.0 in a packed pair
 __device__ __forceinline__ uint32_t scrub_sentinel(uint32_t w) {
   if ((w & 0xFFFFu) == B2_SENTINEL16) w &= 0xFFFF0000u;
@@ -404,6 +413,25 @@ void count_launch();
 bool pdl_enabled();  // false when the environment has B2_PDL=0
 int encode_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld_elems,
                    uint32_t box_inner, uint32_t box_rows);
+
+// What a GEMM's store epilogue does with the accumulator (b2_gemm, b2_gemm_silu_mul, b2_qkv_fused).
+struct StoreEpilogue {
+  uint16_t* C = nullptr;
+  int64_t ldc = 0;
+  const uint16_t* bias = nullptr;
+  int silu_pairs = 0;
+  int qkv_fused = 0, nq = 0, nkv = 0;
+  const int64_t* positions = nullptr;
+  const float* cos_sin = nullptr;
+  const uint16_t* q_norm_w = nullptr;
+  const uint16_t* k_norm_w = nullptr;
+  float qk_eps = 0.f;
+  uint16_t* k_cache = nullptr;
+  uint16_t* v_cache = nullptr;
+  const int32_t* slots = nullptr;
+};
+// b2_gemm_tile.cu: the GEMM for more than 64 tokens on CTA pairs
+int launch_tile_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K, const StoreEpilogue& e, cudaStream_t stream);
 }  // namespace b2
 
 #define B2_CUDA(call)                                            \

@@ -279,17 +279,6 @@ __host__ __device__ __forceinline__ int owned_rows3(int M, int world, int rank) 
 // (row of the P tile) q*32 + lane and columns c*32 .. c*32+31 (rows of the Q
 // tile).
 // ---------------------------------------------------------------------------
-// silu(gate) * up on bf16-rounded inputs, with the reference's roundings (nanovllm/layers/activation.py:8-11, eager):
-// the activation is rounded to bf16 before the product, the product once more by the caller's pack
-__device__ __forceinline__ float silu_mul(float gate, float up) {
-  return b2::bf16_round(gate / (1.0f + expf(-gate))) * up;
-}
-// 8 bf16 = 4 (gate, up) pairs -> 4 bf16
-__device__ __forceinline__ uint2 silu_mul_pairs(const uint4& w) {
-  return make_uint2(b2::pack_bf16(silu_mul(b2::bf16_lo(w.x), b2::bf16_hi(w.x)), silu_mul(b2::bf16_lo(w.y), b2::bf16_hi(w.y))),
-                    b2::pack_bf16(silu_mul(b2::bf16_lo(w.z), b2::bf16_hi(w.z)), silu_mul(b2::bf16_lo(w.w), b2::bf16_hi(w.w))));
-}
-
 // NC columns (tokens token0 ..) of one feature per lane, features = consecutive lanes.
 // Lanes 2i and 2i+1 hold features f and f+1 of the same tokens.  They swap
 // halves so that each lane stores a packed (f, f+1) pair: the even lane for
@@ -313,7 +302,7 @@ __device__ __forceinline__ void emit_feature_lanes(const GemmArgs& a, float (&v)
     if (token < a.M && fbase < a.N) {
       if (EPI == EPI_STORE) {
         if (a.silu_pairs) {  // w = (gate, up) of feature pair fbase / 2
-          const float act = silu_mul(b2::bf16_lo(w), b2::bf16_hi(w));
+          const float act = b2::silu_mul(b2::bf16_lo(w), b2::bf16_hi(w));
           a.C[token * a.ldc + (fbase >> 1)] = static_cast<uint16_t>(b2::pack_bf16(act, 0.f) & 0xFFFF);
         } else {
           *reinterpret_cast<uint32_t*>(a.C + token * a.ldc + fbase) = w;
@@ -380,7 +369,7 @@ __device__ __forceinline__ void flush_rows(const GemmArgs& a, unsigned char* wbu
     if (piece < npieces && token < a.M && feature < a.N) {
       const uint4 w = *reinterpret_cast<const uint4*>(wbuf + row * STAGE_ROW_BYTES + ((piece ^ (row & 15)) << 4));
       if (EPI == EPI_STORE) {
-        if (a.silu_pairs) *reinterpret_cast<uint2*>(a.C + token * a.ldc + (feature >> 1)) = silu_mul_pairs(w);
+        if (a.silu_pairs) *reinterpret_cast<uint2*>(a.C + token * a.ldc + (feature >> 1)) = b2::silu_mul_pairs(w);
         else *reinterpret_cast<uint4*>(a.C + token * a.ldc + feature) = w;
       } else if (EPI == EPI_PUSH2) {
         int lrow;
@@ -1349,7 +1338,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
       if (token < a.M && feat < a.N) {
         uint4 w = *reinterpret_cast<const uint4*>(out_buf + lt * (BM * 2) + piece * 16);
         if (EPI == EPI_STORE) {
-          if (a.silu_pairs) *reinterpret_cast<uint2*>(a.C + token * a.ldc + (feat >> 1)) = silu_mul_pairs(w);
+          if (a.silu_pairs) *reinterpret_cast<uint2*>(a.C + token * a.ldc + (feat >> 1)) = b2::silu_mul_pairs(w);
           else *reinterpret_cast<uint4*>(a.C + token * a.ldc + feat) = w;
         } else if (EPI == EPI_PUSH3) {
           w.x = b2::scrub_sentinel(w.x); w.y = b2::scrub_sentinel(w.y);
@@ -1819,6 +1808,28 @@ int plan_gemm(int epi, int M, int N, int K, int num_sms, int min_grid, int reduc
 template <int EPI>
 int launch_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K, GemmArgs& args,
                 int min_grid, cudaStream_t stream) {
+  if constexpr (EPI == EPI_STORE) {
+    if (M > 64) {  // more than a decode step's tokens: CTA pairs over tiles of up to 256 tokens, see b2_gemm_tile.cu
+      b2::StoreEpilogue e;
+      e.C = args.C;
+      e.ldc = args.ldc;
+      e.bias = args.bias;
+      e.silu_pairs = args.silu_pairs;
+      e.qkv_fused = args.qkv_fused;
+      e.nq = args.nq;
+      e.nkv = args.nkv;
+      e.positions = args.positions;
+      e.cos_sin = args.cos_sin;
+      e.q_norm_w = args.q_norm_w;
+      e.k_norm_w = args.k_norm_w;
+      e.qk_eps = args.qk_eps;
+      e.k_cache = args.k_cache;
+      e.v_cache = args.v_cache;
+      e.slots = args.slots;
+      g_last_gemm_path = 2;
+      return b2::launch_tile_gemm(ctx, A, lda, W, ldw, M, N, K, e, stream);
+    }
+  }
   const int reducers = 0;  // no CTAs are set aside for the reduce phase: every CTA reduces after its GEMM work
   GemmPlan plan;
   const int prc = plan_gemm(EPI, M, N, K, ctx->num_sms, min_grid, reducers, ctx->tile_counter_cap, true,
@@ -1854,7 +1865,7 @@ int launch_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t 
   if (rc != B2_OK) return rc;
 
   g_last_gemm_path = 0;
-  if constexpr (EPI == EPI_STORE || EPI == EPI_PUSH2) {
+  if constexpr (EPI == EPI_PUSH2) {
     // CTA pairs (tcgen05.mma.cta_group::2) for many-token problems: 1.1-1.2x the stream-K kernel from 512 tokens on
     if (pair_path_enabled() && !swap && bn >= 128 && M >= 512 && ctx->num_sms >= 2) {
       CUtensorMap tmQh;
@@ -1882,16 +1893,16 @@ int launch_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t 
     }
   } else if constexpr (EPI != EPI_PUSH2) {
     if (swap) {
-      switch (bn) {
-        case 32: return launch_inst<32, true, EPI>(tmP, tmQ, args, grid, stream);
-        case 64: return launch_inst<64, true, EPI>(tmP, tmQ, args, grid, stream);
-        case 128: return launch_inst<128, true, EPI>(tmP, tmQ, args, grid, stream);
-        default: return launch_inst<256, true, EPI>(tmP, tmQ, args, grid, stream);
+      if (bn == 32) return launch_inst<32, true, EPI>(tmP, tmQ, args, grid, stream);
+      if (bn == 64) return launch_inst<64, true, EPI>(tmP, tmQ, args, grid, stream);
+      if constexpr (EPI != EPI_STORE) {
+        if (bn == 128) return launch_inst<128, true, EPI>(tmP, tmQ, args, grid, stream);
+        return launch_inst<256, true, EPI>(tmP, tmQ, args, grid, stream);
       }
     }
   }
-  if constexpr (EPI == EPI_SAMPLE) {
-    return B2_ERR_SHAPE;  // the fused sampler exists in the feature-lane layout only (at most 256 token rows)
+  if constexpr (EPI == EPI_SAMPLE || EPI == EPI_STORE) {
+    return B2_ERR_SHAPE;  // feature-lane layout only: the fused sampler takes at most 256 token rows, the store epilogue 64 here
   } else {
     switch (bn) {
       case 64: return launch_inst<64, false, EPI>(tmP, tmQ, args, grid, stream);
@@ -2152,8 +2163,8 @@ int b2_qkv_fused(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t
   }
   rc = launch_gemm<EPI_STORE>(ctx, A, lda, W, ldw, M, N, K, args, 0, static_cast<cudaStream_t>(stream));
   if (rc != B2_OK) return rc;
-  if (args.qkv_fused && g_last_gemm_path == 1) return B2_OK;
-  // many tokens (or 64-wide heads): the projection ran on the stream-K kernel; finish the heads in a second launch
+  if (args.qkv_fused && g_last_gemm_path != 0) return B2_OK;  // the cluster and the tile kernel finish the heads themselves
+  // 64-wide heads, or a decode batch whose projection ran on the stream-K kernel: finish the heads in a second launch
   return b2_qk_norm_rope_store(qkv, ld_qkv, M, nq, nkv, head_dim, q_norm_w, k_norm_w, eps, positions, cos_sin, k_cache, v_cache, slot_mapping,
                                stream);
 }
