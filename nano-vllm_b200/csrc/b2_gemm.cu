@@ -428,50 +428,128 @@ __host__ __device__ __forceinline__ unsigned long long sample_key(uint32_t score
   return (static_cast<unsigned long long>(ord) << 32) | (0xFFFFFFFFu - vocab_id);
 }
 
-// One 32-token chunk of one vocabulary entry per lane (feature-lane layout).  The 32 x 32 keys of the warp are
-// reduced over the lanes by a halving exchange (31 shuffles of a key instead of 32 x 5): afterwards lane l holds
-// the best key of token token0 + l among the warp's 32 vocabulary entries, and merges it into the CTA's table.
-__device__ __forceinline__ void sample_feature_lanes(const GemmArgs& a, float (&v)[32], int feature, int token0, int lane,
-                                                     unsigned int call, unsigned long long* cta_best) {
+// Scores that can still win wait here for their logarithms: a warp evaluates 32 of them at a time.
+struct SampleQueue {
+  uint4 entry[384];                           // token row, vocabulary entry, bf16-rounded logit, random bits
+  __align__(16) float limit[32], inv_t[32];   // of the chunk's token rows
+};
+__device__ __forceinline__ void sample_flush(const GemmArgs& a, SampleQueue* queue, int n, int lane, unsigned long long* cta_best) {
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
+    const uint4 e = queue->entry[i];
+    float z = __uint_as_float(e.z);
+    if (a.temperatures != nullptr) z = z / __ldg(a.temperatures + e.x) + gumbel_from_bits(e.w);
+    atomicMax(cta_best + e.x, sample_key(__float_as_uint(z), static_cast<uint32_t>(a.vocab_offset) + e.y));
+  }
+  __syncwarp();
+}
+
+// All token rows of one vocabulary entry per lane (feature-lane layout): group g of the tile's columns, tokens 8 g .. 8 g + 7,
+// comes from load(g), requested one group ahead.
+// Bound: the instructions per score, of which the two logarithms, the division and the exchange between the lanes were nine
+// tenths, and their fetching: unrolled over 32 tokens the code streamed from the instruction cache's outer level (577 us for 256
+// rows of 1024 features, whose weights take 48 us to read).  A score is z / T - log(-log u) with 1 - u = (c + 1/2) 2^-23 and c
+// the complement of the 23 random bits, and -log(-log u) <= -log(1 - u) <= (clz(c) - 8) log 2.  So a few integer operations
+// bound it from above, and only what reaches the best score its row has in this CTA so far is queued for the exact evaluation
+// - a handful per row (NaN included: it wins).  While a row has no score yet the bound from below takes its place: for u >= 1/2,
+// -log u <= 2 log 2 (1 - u), hence -log(-log u) >= (clz(c) - 9) log 2 - 0.3267.
+template <class Load>
+__device__ __forceinline__ void sample_feature_lanes(const GemmArgs& a, Load&& load, int feature, int lane, unsigned int call,
+                                                     unsigned long long* cta_best, SampleQueue* queue) {
   const bool live = feature < a.N;
   const uint32_t vocab_id = static_cast<uint32_t>(a.vocab_offset + feature);
   const float bias = (a.bias != nullptr && live) ? __uint_as_float(static_cast<uint32_t>(a.bias[feature]) << 16) : 0.f;
-  unsigned long long k[32];
+  const bool noisy = a.temperatures != nullptr;
+  const int groups = (a.M + 7) >> 3;
+  int count = 0;
+  bool fresh = false;
+  float next[8];
+  load(0, next);
+#pragma unroll 1
+  for (int g = 0; g < groups; ++g) {
+    const int j0 = (g & 3) * 8;
+    if (j0 == 0) {
+      // rows 8 g + l, by lane l, for all lanes: the best score here (-inf: none yet, +inf: no such row), the inverse temperature
+      const int token = g * 8 + lane;
+      float best = INFINITY, inv_t = 1.f;
+      if (token < a.M) {
+        const uint32_t ord = static_cast<uint32_t>(*reinterpret_cast<volatile unsigned long long*>(cta_best + token) >> 32);
+        best = ord == 0u ? -INFINITY : __uint_as_float((ord & 0x80000000u) ? ord ^ 0x80000000u : ~ord);
+        if (noisy) inv_t = 1.f / __ldg(a.temperatures + token);
+      }
+      __syncwarp();
+      queue->limit[lane] = best;
+      queue->inv_t[lane] = inv_t;
+      fresh = __any_sync(0xffffffffu, best == -INFINITY);
+      __syncwarp();
+    }
+    uint32_t r[2][4];  // two generators side by side: one warp per scheduler has nothing else to fill their latency with
 #pragma unroll
-  for (int j0 = 0; j0 < 32; j0 += 4) {
-    uint32_t r[4] = {vocab_id, static_cast<uint32_t>(token0 + j0) >> 2, call, SAMPLE_TAG};
-    if (a.temperatures != nullptr) philox4x32_10(r, static_cast<uint32_t>(a.seed), static_cast<uint32_t>(a.seed >> 32));
+    for (int h = 0; h < 2; ++h) {
+      r[h][0] = vocab_id;
+      r[h][1] = static_cast<uint32_t>(2 * g + h);
+      r[h][2] = call;
+      r[h][3] = SAMPLE_TAG;
+      if (noisy) philox4x32_10(r[h], static_cast<uint32_t>(a.seed), static_cast<uint32_t>(a.seed >> 32));
+    }
+    float limit[8], it[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int token = token0 + j0 + i;
-      float z = b2::bf16_round(v[j0 + i] + bias);  // the logit as the unfused path stores it
-      if (a.temperatures != nullptr && token < a.M) z = z / __ldg(a.temperatures + token) + gumbel_from_bits(r[i]);
-      k[j0 + i] = (live && token < a.M) ? sample_key(__float_as_uint(z), vocab_id) : 0ull;
+    for (int h = 0; h < 2; ++h) {
+      const float4 l4 = *reinterpret_cast<const float4*>(queue->limit + j0 + 4 * h), t4 = *reinterpret_cast<const float4*>(queue->inv_t + j0 + 4 * h);
+      limit[4 * h] = l4.x; limit[4 * h + 1] = l4.y; limit[4 * h + 2] = l4.z; limit[4 * h + 3] = l4.w;
+      it[4 * h] = t4.x; it[4 * h + 1] = t4.y; it[4 * h + 2] = t4.z; it[4 * h + 3] = t4.w;
+    }
+    float z[8], upper[8], lower[8];
+    b2::tc_wait_ld(next);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) z[i] = b2::bf16_round(next[i] + bias);  // the logit as the unfused path stores it
+    if (g + 1 < groups) load(g + 1, next);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      upper[i] = lower[i] = z[i];
+      if (noisy) {
+        const uint32_t bits = r[i >> 2][i & 3];
+        const float zt = z[i] * it[i], n = static_cast<float>(__clz(~bits >> 9));
+        const float slack = fmaf(fabsf(zt), 1e-6f, 1e-3f);  // covers the roundings of both sides
+        upper[i] = zt + slack + fmaf(n, 0.6931473f, -8.f * 0.6931471f);
+        lower[i] = (bits >> 31) ? zt - slack + fmaf(n, 0.6931471f, -9.f * 0.6931473f - 0.3268f) : -INFINITY;
+      }
+    }
+    if (fresh) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (limit[i] == -INFINITY) {  // (the same in all lanes)
+          const int o = __float_as_int(live ? lower[i] : -INFINITY);
+          const int m = __reduce_max_sync(0xffffffffu, o >= 0 ? o : o ^ 0x7fffffff);  // order-preserving as a signed integer
+          limit[i] = __int_as_float(m >= 0 ? m : m ^ 0x7fffffff);
+        }
+    }
+    uint32_t may = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) may |= (live && !(upper[i] < limit[i]) && g * 8 + i < a.M) ? 1u << i : 0u;
+    if (__any_sync(0xffffffffu, may != 0u)) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool in = (may >> i) & 1u;
+        const uint32_t who = __ballot_sync(0xffffffffu, in);
+        if (in) queue->entry[count + __popc(who & ((1u << lane) - 1))] = make_uint4(g * 8 + i, feature, __float_as_uint(z[i]), r[i >> 2][i & 3]);
+        count += __popc(who);
+      }
+      if (count > 128) {  // room for 8 x 32 more
+        sample_flush(a, queue, count, lane, cta_best);
+        count = 0;
+      }
     }
   }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    const bool upper = (lane & o) != 0;
-#pragma unroll
-    for (int j = 0; j < o; ++j) {
-      const unsigned long long send = upper ? k[j] : k[j + o];
-      const unsigned long long keep = upper ? k[j + o] : k[j];
-      const unsigned long long recv = __shfl_xor_sync(0xffffffffu, send, o);
-      k[j] = keep > recv ? keep : recv;
-    }
-  }
-  if (k[0] != 0ull) atomicMax(cta_best + token0 + lane, k[0]);
+  if (count > 0) sample_flush(a, queue, count, lane, cta_best);
 }
 
 // One 32-column chunk c of a tile leaves the registers.  Feature-lane layout (SWAP): stored at once.
 // Token-row layout: parked in the warp's staging buffer; every fourth chunk (and the tile's last) flushes.
 template <int BN, bool SWAP, int EPI>
 __device__ __forceinline__ void emit_chunk(const GemmArgs& a, float (&v)[32], int p_row, int q_tile0, int c, int lane, unsigned int parity,
-                                           unsigned char* wbuf, unsigned int sample_call, unsigned long long* cta_best) {
-  if constexpr (EPI == EPI_SAMPLE) {
-    static_assert(SWAP, "the fused sampler needs the feature-lane layout");
-    sample_feature_lanes(a, v, p_row, q_tile0 + c * 32, lane, sample_call, cta_best);
-  } else if (SWAP) {
+                                           unsigned char* wbuf) {
+  if (SWAP) {
     emit_feature_lanes<32, EPI>(a, v, p_row, q_tile0 + c * 32, lane, parity);
   } else {
     stage_row_chunk(a, wbuf, lane, c & 3, v, q_tile0 + c * 32, is_push(EPI));
@@ -791,16 +869,21 @@ __device__ __forceinline__ void fused_tail(const GemmArgs& a, unsigned int parit
   }
 }
 
-// The CTA's table of best keys per token row (fused sampler only; other epilogues carry no such array)
+// The CTA's table of best keys per token row and the warps' queues (fused sampler only; other epilogues carry no such arrays)
 template <int EPI>
 struct SampleTable {
   __device__ static __forceinline__ unsigned long long* get() { return nullptr; }
+  __device__ static __forceinline__ SampleQueue* queues() { return nullptr; }
 };
 template <>
 struct SampleTable<EPI_SAMPLE> {
   __device__ static __forceinline__ unsigned long long* get() {
     __shared__ unsigned long long table[256];
     return table;
+  }
+  __device__ static __forceinline__ SampleQueue* queues() {
+    __shared__ SampleQueue queue[4];
+    return queue;
   }
 };
 
@@ -850,6 +933,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
     *abort_flag = 0;
     b2::mbar_fence_init();
   }
+  SampleQueue* const queues = SampleTable<EPI>::queues();
   if constexpr (EPI == EPI_SAMPLE)
     for (int t = threadIdx.x; t < 256; t += NUM_THREADS) cta_best[t] = 0ull;
   if (warp == 1 && has_gemm) {
@@ -969,15 +1053,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
         const int p_row = tp * BM + q * 32 + lane;
         const bool whole = (s.kb0 == 0 && s.kb1 == KB);
         if (whole) {
+          if constexpr (EPI == EPI_SAMPLE) {
+            sample_feature_lanes(a, [&](int g, float (&v)[8]) { b2::tmem_ld_32x8(taddr + g * 8, v); }, p_row, lane, sample_call, cta_best, queues + q);
+          } else {
 #pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
-            uint32_t r[32];
-            b2::tmem_ld_32x32(taddr + c * 32, r);
-            b2::tc_wait_ld();
-            float v[32];
+            for (int c = 0; c < BN / 32; ++c) {
+              uint32_t r[32];
+              b2::tmem_ld_32x32(taddr + c * 32, r);
+              b2::tc_wait_ld();
+              float v[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            emit_chunk<BN, SWAP, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf, sample_call, cta_best);
+              for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+              emit_chunk<BN, SWAP, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf);
+            }
           }
         } else {
           // This CTA holds only part of the tile's K range.  Every contributor adds its part into the
@@ -1006,6 +1094,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
           if (old == c_last - c_first) {
             __threadfence();
             if (lane == 0) a.counters[s.tile * 4 + q] = 0;
+            if constexpr (EPI == EPI_SAMPLE) {
+              sample_feature_lanes(
+                  a,
+                  [&](int g, float (&v)[8]) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                      float* p = slot + (2 * g + h) * 128;
+                      asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4 * h]), "=f"(v[4 * h + 1]), "=f"(v[4 * h + 2]), "=f"(v[4 * h + 3]) : "l"(p) : "memory");
+                      *reinterpret_cast<float4*>(p) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                  },
+                  p_row, lane, sample_call, cta_best, queues + q);
+              // (columns past the last token have only had zeros added)
+            } else {
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
               float v[32];
@@ -1017,7 +1119,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
               }
 #pragma unroll
               for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(slot + (c * 8 + j) * 128) = make_float4(0.f, 0.f, 0.f, 0.f);
-              emit_chunk<BN, SWAP, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf, sample_call, cta_best);
+              emit_chunk<BN, SWAP, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf);
+            }
             }
           }
         }
@@ -1578,7 +1681,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-        emit_chunk<BN, false, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf, 0u, nullptr);
+        emit_chunk<BN, false, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf);
       }
       b2::tc_fence_before();
       __syncwarp();

@@ -431,7 +431,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     }
     // this chunk's sums as bf16 pairs of tokens: out[i] = features lane / 4 + 0, 8, 16, 24 of group g + i
     auto finish = [&](int g, uint32_t (&out)[4][4]) {
-      b2::tc_wait_ld();
+      b2::tc_wait_ld(acc);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float v[8];

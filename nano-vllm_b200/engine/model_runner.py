@@ -309,8 +309,11 @@ class ModelRunner:
         if getattr(self, "_picked", None) is None or self._picked.numel() < len(seqs):
             self._picked = torch.zeros(max(len(seqs), self.max_num_seqs), dtype=torch.int64, device=self.device)
         picked = self._picked[:len(seqs)]  # one buffer for every step: rank 0's sampler fills it, the broadcast hands it to the others
-        if self.fused_sampler and len(seqs) <= FUSED_SAMPLER_MAX_ROWS:
-            self.model.sample_tokens(hidden, temps, self.sample_seed, out=picked)
+        if self.fused_sampler and (len(seqs) <= FUSED_SAMPLER_MAX_ROWS or self.world == 1):
+            # (several ranks exchange once per call, so they take one call or the unfused path)
+            for i in range(0, len(seqs), FUSED_SAMPLER_MAX_ROWS):
+                rows = slice(i, i + FUSED_SAMPLER_MAX_ROWS)
+                self.model.sample_tokens(hidden, None if temps is None else temps[rows], self.sample_seed, out=picked[rows], rows=rows)
         else:
             logits = self.model.compute_logits(hidden)
             if self.rank == 0:

@@ -47,9 +47,13 @@ class ParallelLMHead(VocabParallelEmbedding):
         ctx = get_context()
         return ops.lm_head(x, self.weight, ctx.last_token_index if ctx.is_prefill else None)
 
-    def forward_sample(self, x: torch.Tensor, temperatures: torch.Tensor | None, seed: int, out: torch.Tensor | None = None):
+    def forward_sample(self, x: torch.Tensor, temperatures: torch.Tensor | None, seed: int, out: torch.Tensor | None = None,
+                       rows: slice = slice(None)):
         """forward() followed by Sampler.forward (nanovllm/layers/sampler.py:7-12; greedy when temperatures is
         None) without materialising the logits: every rank scans its vocabulary slice in the GEMM epilogue and
-        only the best (score, id) per row reaches rank 0.  Returns int64 token ids, valid on rank 0."""
+        only the best (score, id) per row reaches rank 0.  `rows` of the batch (sequences): at most 256 of them; temperatures
+        and out belong to those.  Returns int64 token ids, valid on rank 0."""
         ctx = get_context()
-        return ops.lm_head_sample(x, self.weight, ctx.last_token_index if ctx.is_prefill else None, temperatures, seed, out)
+        if ctx.is_prefill:
+            return ops.lm_head_sample(x, self.weight, ctx.last_token_index[rows], temperatures, seed, out)
+        return ops.lm_head_sample(x[rows], self.weight, None, temperatures, seed, out)
