@@ -399,6 +399,22 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
                               void* out, void* stream);
 int b2_paged_attention_supported(int n_seqs, int nq, int nkv, int head_dim, int block_size);
 
+/* ---- causal prefill attention: what flash_attn_varlen_func computes
+ *      (nanovllm/layers/attention.py:64-69) ------------------------------------------
+ * q [tokens, nq, head_dim] bf16 (row stride q_stride).  Sequence b has query rows
+ * cu_q[b] .. cu_q[b+1] and cu_k[b+1] - cu_k[b] keys, of which its queries are the last; query i sees the keys up to its
+ * own position.  block_tables NULL: k and v are matrices of kv_rows rows (row stride kv_stride; views of the qkv output),
+ * sequence b's keys in rows cu_k[b] .. ; else k and v are the caches, kv_rows = blocks * block_size slots, and
+ * block_tables (bt_width columns, row stride bt_stride) says where.  max_q: the most query rows of a sequence.
+ * out [tokens, nq, head_dim] contiguous.  fp32 scores and sums, probabilities rounded to bf16 for the second product.
+ * b2_prefill_attention_supported says (1 / 0) whether the shape is served: head_dim 128, two query heads per KV head, blocks
+ * of a multiple of 128 tokens (block_size 0: no block table). */
+int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, int64_t kv_rows,
+                         const int32_t* block_tables, int64_t bt_stride, int bt_width, int block_size, const int32_t* cu_q,
+                         const int32_t* cu_k, int n_seqs, int max_q, int tokens, int nq, int nkv, int head_dim, float scale,
+                         void* out, void* stream);
+int b2_prefill_attention_supported(int nq, int nkv, int head_dim, int block_size);
+
 /* Greedy pick: out[i] = argmax_j logits[i, j] (first index on ties), int64.
  * The reference's Sampler (nanovllm/layers/sampler.py:7-12) at temperature -> 0. */
 int b2_argmax(const void* logits, int64_t ld, int B, int V, int64_t* out, void* stream);

@@ -79,6 +79,8 @@ SIGNATURES = {
     "b2_qk_norm_rope_store": [_p, _i64, _i, _i, _i, _i, _p, _p, _f, _p, _p, _p, _p, _p, _p],
     "b2_paged_attention_decode": [_p, _p, _i64, _p, _p, _i, _i, _p, _i64, _i, _p, _i, _i, _i, _i, _f, _p, _p],
     "b2_paged_attention_supported": [_i, _i, _i, _i, _i],
+    "b2_prefill_attention": [_p, _p, _i64, _p, _p, _i64, _i64, _p, _i64, _i, _i, _p, _p, _i, _i, _i, _i, _i, _i, _f, _p, _p],
+    "b2_prefill_attention_supported": [_i, _i, _i, _i],
     "b2_argmax": [_p, _i64, _i, _i, _p, _p],
     "b2_broadcast_tokens": [_p, _p, _i, _p],
     "b2_advance_decode": [_p, _p, _p, _p, _p, _p, _i64, _i, _i, _i64, _i, _p],

@@ -1,4 +1,4 @@
-// Decode attention over the paged KV cache: one new query token per sequence, grouped-query heads.
+// Attention with grouped-query heads: decode (one new query token per sequence over the paged KV cache) and causal prefill.
 #include <algorithm>
 #include <atomic>
 
@@ -66,6 +66,12 @@ __device__ __forceinline__ void mma_rows8(float& c0, float& c1, uint32_t a0, uin
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, d2, d3}, {%2, %3, %4, %3}, {%5, %6}, {%0, %1, %7, %7};\n\t}"
       : "+f"(c0), "+f"(c1)
       : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
+}
+// 2^x; results below the normal range are as good as zero here
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 __device__ __forceinline__ void consumers_meet() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
@@ -262,7 +268,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            p[i][e] = exp2f(s[i][e] - m);
+            p[i][e] = ex2(s[i][e] - m);
             l += p[i][e];
           }
         const uint32_t p0 = b2::pack_bf16(p[0][0], p[0][1]), p1 = b2::pack_bf16(p[1][0], p[1][1]);
@@ -422,6 +428,296 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   if (*abort_flag && tid == 0) b2::report_timeout(a.status, *abort_flag);
 }
 
+// ---------------------------------------------------------------------------
+// prefill_attention_kernel
+//
+// Causal attention of many query tokens per sequence over keys and values in rows of a matrix (the qkv output) or in the paged
+// cache.  Bound: the exponentials and the tensor pipe, which take about the same time per block (16 exponentials and 8192
+// multiply-adds per clock and SM).
+//
+// A CTA takes 128 query tokens of one sequence for the two heads that share a KV head: both heads' scores come from the same
+// K block, and while the tensor cores work for one head, four warps turn the other's scores into probabilities.
+//   warp 0      TMA: Q of both heads once, then K and V blocks of 128 tokens, two of each in flight
+//   warp 1      tcgen05.mma: S = Q K^T (128 x 128, fp32, tensor memory), O += P V with P read from tensor memory
+//   warps 2..9  one thread per query row and head: running maximum and sum, P = exp2(...) rounded to bf16 over S
+// Tensor memory: S of the two heads, then O of the two heads, 128 columns each.  O is rescaled only when a row's maximum has
+// grown by more than 2^8 since its scale was set: fp32 and bf16 have the range, so the result is the same.
+// ---------------------------------------------------------------------------
+constexpr int PF_ROWS = 128, PF_KEYS = 128, PF_THREADS = 320;
+constexpr uint32_t PF_TILE = 128 * 128 * 2;                     // 128 rows of 128 bf16, as two 64-wide swizzled halves
+constexpr uint32_t PF_SMEM = 1024 + 2 * PF_TILE + 4 * PF_TILE;  // alignment, Q, two K and two V blocks
+constexpr uint64_t PF_LIMIT_NS = 1000000000ull;
+
+struct PrefillArgs {
+  const int32_t *cu_q, *cu_k, *tables;  // tables: null = keys and values are rows cu_k[b] .. of the matrices
+  int64_t bt_stride;
+  int bt_width, block_size, kv_rows, nq, nkv;
+  uint16_t* out;
+  float scale_log2;
+  B2Status* status;
+};
+
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d), "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]),
+      "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// V as the second operand, [tokens][dimensions] with the dimensions contiguous: MN-major, 128-byte swizzle.  8 tokens are 1024
+// bytes apart (stride offset), the two halves of 64 dimensions PF_TILE / 2 (leading offset).
+__device__ __forceinline__ uint64_t umma_smem_desc_mn(uint32_t addr) {
+  return static_cast<uint64_t>((addr & 0x3FFFF) >> 4) | (static_cast<uint64_t>((PF_TILE / 2) >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+         (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
+}
+
+__global__ void __launch_bounds__(PF_THREADS, 1)
+prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const PrefillArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const uint32_t s_q = b2::smem_u32(smem), s_k = s_q + 2 * PF_TILE, s_v = s_k + 2 * PF_TILE;
+  __shared__ __align__(8) uint64_t s_bars[15];
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_abort;
+  volatile int* abort_flag = &s_abort;
+  const uint32_t bars = b2::smem_u32(s_bars);
+  const uint32_t q_full = bars, k_full = bars + 8, k_empty = bars + 24, v_full = bars + 40, v_empty = bars + 56, s_full = bars + 72, p_full = bars + 88,
+                 o_done = bars + 104;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    b2::tma_prefetch_desc(&tmQ);
+    b2::tma_prefetch_desc(&tmK);
+    b2::tma_prefetch_desc(&tmV);
+    b2::mbar_init(q_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      b2::mbar_init(k_full + i * 8, 1);
+      b2::mbar_init(k_empty + i * 8, 1);
+      b2::mbar_init(v_full + i * 8, 1);
+      b2::mbar_init(v_empty + i * 8, 1);
+      b2::mbar_init(s_full + i * 8, 1);
+      b2::mbar_init(p_full + i * 8, 4);
+      b2::mbar_init(o_done + i * 8, 1);
+    }
+    s_abort = 0;
+    b2::mbar_fence_init();
+  }
+  if (warp == 1) {
+    b2::tmem_alloc(b2::smem_u32(&s_tmem), 512);
+    b2::tmem_relinquish();
+  }
+  b2::tc_fence_before();
+  __syncthreads();
+  b2::tc_fence_after();
+  const uint32_t tmem = s_tmem;
+  b2::pdl_launch_dependents();
+  b2::pdl_wait();
+
+  // sequence, pair of heads, tile of 128 query tokens (the long rows of the causal triangle first)
+  const int b = blockIdx.z, pairs_per_kv = a.nq / a.nkv / 2;
+  const int head = blockIdx.y * 2, kv_head = blockIdx.y / pairs_per_kv;
+  const int q0 = __ldg(a.cu_q + b), q_len = __ldg(a.cu_q + b + 1) - q0;
+  const int k0 = __ldg(a.cu_k + b), kv_len = __ldg(a.cu_k + b + 1) - k0;
+  const int t0 = (gridDim.x - 1 - blockIdx.x) * PF_ROWS;
+  const int shift = kv_len - q_len;  // position of the first query token
+  const int n = t0 < q_len && kv_len > 0 ? max(1, (min(kv_len, shift + min(q_len, t0 + PF_ROWS)) + PF_KEYS - 1) / PF_KEYS) : 0;  // key blocks
+
+  if (warp == 0) {
+    if (lane == 0 && n > 0) {
+      b2::mbar_arrive_expect_tx(q_full, 2 * PF_TILE);
+      for (int h = 0; h < 2; ++h)
+        for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_q + h * PF_TILE + i * (PF_TILE / 2), &tmQ, q_full, (head + h) * 128 + i * 64, q0 + t0, b2::kEvictFirst);
+      const int x = kv_head * 128;
+      for (int j = 0; j < n; ++j) {
+        const int st = j & 1;
+        const uint32_t ph = ((j >> 1) & 1) ^ 1;
+        int y = k0 + j * PF_KEYS;
+        if (a.tables != nullptr) {
+          const int tok = j * PF_KEYS, blk = tok / a.block_size;
+          y = max(0, __ldg(a.tables + static_cast<int64_t>(b) * a.bt_stride + min(blk, a.bt_width - 1))) * a.block_size + tok - blk * a.block_size;
+          y = min(y, a.kv_rows - 1);  // (a bad table entry must not lead outside the cache)
+        }
+        if (!b2::mbar_wait(k_empty + st * 8, ph, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) break;
+        b2::mbar_arrive_expect_tx(k_full + st * 8, PF_TILE);
+        for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_k + st * PF_TILE + i * (PF_TILE / 2), &tmK, k_full + st * 8, x + i * 64, y, b2::kEvictLast);
+        if (!b2::mbar_wait(v_empty + st * 8, ph, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) break;
+        b2::mbar_arrive_expect_tx(v_full + st * 8, PF_TILE);
+        for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_v + st * PF_TILE + i * (PF_TILE / 2), &tmV, v_full + st * 8, x + i * 64, y, b2::kEvictLast);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && n > 0) {
+      constexpr uint32_t idesc_s = b2::umma_idesc_bf16(PF_KEYS);
+      constexpr uint32_t idesc_o = b2::umma_idesc_bf16(128) | (1u << 16);  // second operand MN-major
+      auto wait = [&](uint32_t bar, uint32_t phase, int code) {
+        const bool ok = b2::mbar_wait(bar, phase, abort_flag, PF_LIMIT_NS, code);
+        b2::tc_fence_after();
+        return ok;
+      };
+      auto scores = [&](int h, int st) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          b2::umma_bf16(tmem + h * 128, b2::umma_smem_desc(s_q + h * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3),
+                        b2::umma_smem_desc(s_k + st * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
+        b2::umma_commit(s_full + h * 8);
+      };
+      bool ok = wait(q_full, 0, B2_WAIT_SMEM_FULL) && wait(k_full, 0, B2_WAIT_SMEM_FULL);
+      if (ok) {
+        scores(0, 0);
+        scores(1, 0);
+        b2::umma_commit(k_empty);
+      }
+      for (int j = 0; ok && j < n; ++j) {
+        const int st = j & 1, nx = (j + 1) & 1;
+        ok = wait(v_full + st * 8, (j >> 1) & 1, B2_WAIT_SMEM_FULL);
+        for (int h = 0; ok && h < 2; ++h) {
+          ok = wait(p_full + h * 8, j & 1, B2_WAIT_TMEM_EMPTY);
+          if (!ok) break;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)  // 16 tokens: 8 columns of P, 2048 bytes of V
+            umma_bf16_ts(tmem + 256 + h * 128, tmem + h * 128 + k * 8, umma_smem_desc_mn(s_v + st * PF_TILE + k * 2048), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+          b2::umma_commit(o_done + h * 8);
+        }
+        if (!ok) break;
+        b2::umma_commit(v_empty + st * 8);
+        if (j + 1 < n) {
+          ok = wait(k_full + nx * 8, ((j + 1) >> 1) & 1, B2_WAIT_SMEM_FULL);
+          for (int h = 0; ok && h < 2; ++h) {
+            ok = wait(o_done + h * 8, j & 1, B2_WAIT_TMEM_FULL);  // P of this block has been read: its columns may take the next scores
+            if (ok) scores(h, nx);
+          }
+          if (ok) b2::umma_commit(k_empty + nx * 8);
+        }
+      }
+    }
+  } else if (n > 0) {
+    const int h = warp >= 6 ? 1 : 0, q = warp & 3, row = q * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
+    const uint32_t t_s = tmem + h * 128 + lanes, t_o = tmem + 256 + h * 128 + lanes;
+    const int pos = shift + t0 + row;  // the last key this row sees
+    float m = -INFINITY, l = 0.f;      // m: the maximum the row's scale is set to, in units of scores
+    bool ok = true;
+    for (int j = 0; ok && j < n; ++j) {
+      ok = b2::mbar_wait(s_full + h * 8, j & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_TMEM_FULL);
+      b2::tc_fence_after();
+      const int last = min(pos, kv_len - 1) - j * PF_KEYS;  // keys 0 .. last of the block count
+      const bool masked = __any_sync(0xffffffffu, last < PF_KEYS - 1);
+      float mx = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t r[32];
+        b2::tmem_ld_32x32(t_s + c * 32, r);
+        b2::tc_wait_ld();
+        if (masked) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) mx = fmaxf(mx, c * 32 + e <= last ? __uint_as_float(r[e]) : -INFINITY);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(r[e]));
+        }
+      }
+      // a new scale for the rows whose maximum has outgrown the old one; the first block sets it
+      const bool grow = mx > m && (m == -INFINITY || (mx - m) * a.scale_log2 > 8.f);
+      if (__any_sync(0xffffffffu, grow)) {
+        const float f = grow ? (m == -INFINITY ? 0.f : exp2f((m - mx) * a.scale_log2)) : 1.f;
+        if (grow) m = mx;
+        l *= f;
+        if (j > 0) {  // (the previous block's product is complete: its scores' successor has been computed after it)
+#pragma unroll 1
+          for (int c = 0; c < 8; ++c) {
+            uint32_t r[16];
+            b2::tmem_ld_32x16(t_o + c * 16, r);
+            b2::tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * f);
+            tmem_st_32x16(t_o + c * 16, r);
+          }
+        }
+      }
+      const float ref = m == -INFINITY ? 0.f : m * a.scale_log2;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t r[32], p[16];
+        b2::tmem_ld_32x32(t_s + c * 32, r);
+        b2::tc_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          float x = ex2(fmaf(__uint_as_float(r[e]), a.scale_log2, -ref)), y = ex2(fmaf(__uint_as_float(r[e + 1]), a.scale_log2, -ref));
+          if (masked) {
+            if (c * 32 + e > last) x = 0.f;
+            if (c * 32 + e + 1 > last) y = 0.f;
+          }
+          l += x + y;
+          p[e >> 1] = b2::pack_bf16(x, y);
+        }
+        tmem_st_32x16(t_s + c * 16, p);  // columns this row has read already
+      }
+      if (h == 0 && a.tables != nullptr && (j + 1) * PF_KEYS > kv_len) {
+        // rows of the cache past the context's end may hold anything: they count as zero
+        ok = b2::mbar_wait(v_full + (j & 1) * 8, (j >> 1) & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_FULL) && ok;
+        if (j * PF_KEYS + row >= kv_len) {
+          unsigned char* v = smem + (s_v - s_q) + (j & 1) * PF_TILE + row * 128;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) *reinterpret_cast<uint4*>(v + (i >> 3) * (PF_TILE / 2) + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      tc_wait_st();
+      b2::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) b2::mbar_arrive(p_full + h * 8);
+    }
+    ok = b2::mbar_wait(o_done + h * 8, (n - 1) & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_TMEM_FULL) && ok;
+    b2::tc_fence_after();
+    if (ok && !*abort_flag) {
+      // rows leave through this head's part of the Q buffer (its last product is complete): whole 256-byte rows
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      unsigned char* mine = smem + h * PF_TILE + q * 32 * 256;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t r[32];
+        b2::tmem_ld_32x32(t_o + c * 32, r);
+        b2::tc_wait_ld();
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) w[e] = b2::pack_bf16(__uint_as_float(r[g * 8 + 2 * e]) * inv, __uint_as_float(r[g * 8 + 2 * e + 1]) * inv);
+          const int piece = c * 4 + g;
+          *reinterpret_cast<uint4*>(mine + lane * 256 + ((piece ^ (lane & 15)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      __syncwarp();
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i) {
+        const int r = i * 2 + (lane >> 4), piece = lane & 15, t = t0 + q * 32 + r;
+        if (t < q_len)
+          *reinterpret_cast<uint4*>(a.out + (static_cast<int64_t>(q0 + t) * a.nq + head + h) * 128 + piece * 8) =
+              *reinterpret_cast<const uint4*>(mine + r * 256 + ((piece ^ (r & 15)) << 4));
+      }
+    }
+  }
+
+  __syncwarp();
+  b2::tc_fence_before();
+  __syncthreads();
+  b2::tc_fence_after();
+  const int aborted = *abort_flag;
+  if (aborted) {
+    for (int i = 0; i < 100; ++i) __nanosleep(2000);  // copies in flight land before the CTA leaves
+    if (threadIdx.x == 0) b2::report_timeout(a.status, aborted);
+  }
+  if (warp == 1) b2::tmem_dealloc(tmem, 512);
+}
+
+
 // dynamic shared memory, and the deepest ring with which two CTAs fit an SM (228 KB, 1 KB of it reserved per CTA)
 size_t attention_smem(int n_seqs, int group, int& stages) {
   const size_t rest = 1024 + static_cast<size_t>(ATT_WARPS) * group * ATT_HD * sizeof(float) + (2 * static_cast<size_t>(n_seqs) + 1) * sizeof(int);
@@ -438,6 +734,7 @@ int configure_once() {
   if (!done[dev].load(std::memory_order_acquire)) {
     B2_CUDA(cudaFuncSetAttribute(paged_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  113 * 1024));
+    B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     done[dev].store(true, std::memory_order_release);
   }
   return B2_OK;
@@ -491,6 +788,45 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   const int crc = configure_once();
   if (crc != B2_OK) return crc;
   B2_CUDA(b2_launch(paged_decode_kernel, dim3(grid), dim3(ATT_THREADS), smem, static_cast<cudaStream_t>(stream), maps[0], maps[1], maps[2], maps[3], a));
+  return B2_OK;
+}
+
+int b2_prefill_attention_supported(int nq, int nkv, int head_dim, int block_size) {
+  return nkv > 0 && nq == 2 * nkv && head_dim == 128 && (block_size <= 0 || block_size % PF_KEYS == 0);
+}
+
+int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, int64_t kv_rows,
+                         const int32_t* block_tables, int64_t bt_stride, int bt_width, int block_size, const int32_t* cu_q, const int32_t* cu_k,
+                         int n_seqs, int max_q, int tokens, int nq, int nkv, int head_dim, float scale, void* out, void* stream) {
+  if (ctx == nullptr || n_seqs < 0 || tokens < 0 || nq <= 0 || nkv <= 0 || max_q < 0) return B2_ERR_ARG;
+  if (n_seqs == 0 || tokens == 0 || max_q == 0) return B2_OK;
+  if (!b2_prefill_attention_supported(nq, nkv, head_dim, block_tables != nullptr ? block_size : 0) || n_seqs > 65535 || kv_rows > (1 << 30)) return B2_ERR_UNSUPPORTED;
+  if (!q || !k || !v || !cu_q || !cu_k || !out || kv_rows <= 0) return B2_ERR_ARG;
+  if (block_tables != nullptr && (bt_width <= 0 || bt_stride < bt_width || block_size <= 0)) return B2_ERR_ARG;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15) return B2_ERR_ARG;
+  if (q_stride % 8 != 0 || kv_stride % 8 != 0 || q_stride < static_cast<int64_t>(nq) * head_dim || kv_stride < static_cast<int64_t>(nkv) * head_dim) return B2_ERR_ARG;
+  const int crc = configure_once();
+  if (crc != B2_OK) return crc;
+  CUtensorMap tmQ, tmK, tmV;
+  int rc = b2::encode_tmap_2d(&tmQ, q, static_cast<uint64_t>(nq) * head_dim, tokens, q_stride, 64, PF_ROWS);
+  if (rc == B2_OK) rc = b2::encode_tmap_2d(&tmK, k, static_cast<uint64_t>(nkv) * head_dim, kv_rows, kv_stride, 64, PF_KEYS);
+  if (rc == B2_OK) rc = b2::encode_tmap_2d(&tmV, v, static_cast<uint64_t>(nkv) * head_dim, kv_rows, kv_stride, 64, PF_KEYS);
+  if (rc != B2_OK) return rc;
+  PrefillArgs a{};
+  a.cu_q = cu_q;
+  a.cu_k = cu_k;
+  a.tables = block_tables;
+  a.bt_stride = bt_stride;
+  a.bt_width = bt_width;
+  a.block_size = block_size;
+  a.kv_rows = static_cast<int>(kv_rows);
+  a.nq = nq;
+  a.nkv = nkv;
+  a.out = static_cast<uint16_t*>(out);
+  a.scale_log2 = scale * 1.4426950408889634f;
+  a.status = ctx->status_dev;
+  B2_CUDA(b2_launch(prefill_attention_kernel, dim3((max_q + PF_ROWS - 1) / PF_ROWS, nq / 2, n_seqs), dim3(PF_THREADS), PF_SMEM, static_cast<cudaStream_t>(stream),
+                    tmQ, tmK, tmV, a));
   return B2_OK;
 }
 

@@ -283,6 +283,27 @@ PyObject* paged_attention(Args a) {
   return wrap(out);
 }
 
+// prefill_attention(ctx, q, k, v, cu_q, cu_k, max_q, block_tables, scale): None when the kernel does not serve the shape.
+// k, v: [rows, nkv, head_dim], or the caches when block_tables is given
+PyObject* prefill_attention(Args a) {
+  const at::Tensor &q = tensor(a[1], "q"), &k = tensor(a[2], "k"), &v = tensor(a[3], "v"), &cu_q = tensor(a[4], "cu_seqlens_q"), &cu_k = tensor(a[5], "cu_seqlens_k");
+  const at::Tensor tables = optional_tensor(a[7], "block_tables");
+  const bool paged = tables.defined();
+  const int64_t n = q.size(0), nq = q.size(1), hd = q.size(2), nkv = k.size(-2), bs = paged ? k.size(1) : 0;
+  if (!b2_prefill_attention_supported(nq, nkv, hd, bs) || q.scalar_type() != at::kBFloat16 || k.scalar_type() != at::kBFloat16 || q.stride(2) != 1 || q.stride(1) != hd ||
+      k.stride(-1) != 1 || k.stride(-2) != hd || v.strides() != k.strides() || k.dim() != (paged ? 4 : 3) || (paged && (!k.is_contiguous() || tables.stride(1) != 1)))
+    Py_RETURN_NONE;
+  expect(cu_q.scalar_type() == at::kInt && cu_k.scalar_type() == at::kInt && (!paged || tables.scalar_type() == at::kInt), "int32 lengths and block tables");
+  const at::Tensor out = at::detail::empty_cuda({n, nq, hd}, at::kBFloat16, q.device(), std::nullopt);
+  const int64_t n_seqs = cu_q.numel() - 1, rows = paged ? k.size(0) * bs : k.size(0);
+  if (n)
+    check(b2_prefill_attention(context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, k.data_ptr(), v.data_ptr(), paged || rows == 1 ? nkv * hd : k.stride(0), rows,
+                               paged ? tables.const_data_ptr<int32_t>() : nullptr, paged ? (n_seqs > 1 ? tables.stride(0) : tables.size(1)) : 0, paged ? tables.size(1) : 0, bs,
+                               cu_q.const_data_ptr<int32_t>(), cu_k.const_data_ptr<int32_t>(), n_seqs, integer(a[6]), n, nq, nkv, hd, number(a[8]), out.data_ptr(), stream()),
+          "b2_prefill_attention");
+  return wrap(out);
+}
+
 PyObject* init(Args a) {
   Py_INCREF(a[0]);
   Py_XDECREF(g_check);
@@ -308,7 +329,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define B2_ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {B2_ENTRY(init, 1), B2_ENTRY(gemm, 4), B2_ENTRY(gemm_silu_mul, 3), B2_ENTRY(qkv_fused, 15), B2_ENTRY(rowpar_fused, 7),
                          B2_ENTRY(rmsnorm, 3), B2_ENTRY(add_rmsnorm, 4), B2_ENTRY(silu_and_mul, 1), B2_ENTRY(store_kvcache, 5),
-                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(embed, 5), B2_ENTRY(paged_attention, 7), {nullptr, nullptr, 0, nullptr}};
+                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(embed, 5), B2_ENTRY(paged_attention, 7), B2_ENTRY(prefill_attention, 9), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_b2torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -4,9 +4,9 @@
 nanovllm/layers/attention.py:33-40 (the Triton kernel at :10-30 is replaced by
 b2_store_kvcache: 16-byte vector copies, several tokens per CTA, bit-exact).
 `Attention` keeps the reference's interface (:43-75).  Decode attention runs on
-b2_paged_attention_decode (flash-attn's paged kernel for the shapes it does not
-serve); prefill attention stays a library call, as in the reference: flash-attn's
-varlen kernel.
+b2_paged_attention_decode and prefill attention on b2_prefill_attention; the
+shapes they do not serve stay a library call, as in the reference: flash-attn's
+paged and varlen kernels.
 """
 from __future__ import annotations
 
@@ -58,7 +58,7 @@ def _sdpa_paged(q, k_cache, v_cache, context_lens, block_tables, scale, q_lens=N
 
 
 class Attention(nn.Module):
-    # "flash_attn" (own decode kernel, the reference's library call otherwise) or "sdpa" (plain PyTorch, for tests on small
+    # "flash_attn" (own kernels, the reference's library call for what they do not serve) or "sdpa" (plain PyTorch, for tests on small
     # shapes when flash-attn cannot run)
     backend = "flash_attn"
 
@@ -87,10 +87,14 @@ class Attention(nn.Module):
                     return torch.cat(outs)
                 return _sdpa_paged(q, k_cache, v_cache, k_lens, ctx.block_tables, self.scale, q_lens)
             return _sdpa_paged(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
-        if not ctx.is_prefill:
+        if ctx.is_prefill:
+            cached = ctx.block_tables is not None  # prefix cache / chunked prefill: read K/V from the cache
+            o = ops.prefill_attention(q, k_cache if cached else k, v_cache if cached else v, ctx.cu_seqlens_q, ctx.cu_seqlens_k, ctx.max_seqlen_q,
+                                      ctx.block_tables, self.scale)
+        else:
             o = ops.paged_attention(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
-            if o is not None:
-                return o
+        if o is not None:
+            return o
         if flash_attn_varlen_func is None:
             raise RuntimeError("flash-attn is not importable; set Attention.backend = 'sdpa' for small test shapes")
         if ctx.is_prefill:

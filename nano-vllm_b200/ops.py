@@ -127,6 +127,14 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     return _native.paged_attention(get_runtime().handle, q, k_cache, v_cache, context_lens, block_tables, scale)
 
 
+def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.Tensor, max_seqlen_q: int,
+                      block_tables: torch.Tensor | None, scale: float) -> torch.Tensor | None:
+    """Causal attention of q [tokens, nq, head_dim] over k, v [tokens, nkv, head_dim], or over the paged caches when
+    block_tables is given.  None when the kernel does not serve the shape (it takes head_dim 128 and two query heads per
+    KV head)."""
+    return _native.prefill_attention(get_runtime().handle, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, block_tables, scale)
+
+
 class _DevicePtr:
     """Minimal __cuda_array_interface__ carrier so torch can view library-owned memory."""
 

@@ -1,4 +1,4 @@
-"""Decode attention over the paged cache against plain PyTorch attention in fp32."""
+"""Attention - decode over the paged cache, causal prefill over rows and over the cache - against plain PyTorch in fp32."""
 import pytest
 import torch
 
@@ -59,3 +59,49 @@ def test_paged_attention_declines_other_shapes(rt):
     kc = torch.zeros(1, 256, 1, 128, dtype=torch.bfloat16, device=DEV)
     lens, tables = torch.ones(1, dtype=torch.int32, device=DEV), torch.zeros(1, 1, dtype=torch.int32, device=DEV)
     assert ops.paged_attention(torch.zeros(1, 3, 128, dtype=torch.bfloat16, device=DEV), kc, kc, lens, tables, 1.0) is None
+
+
+# (new tokens, cached tokens) per sequence: edges of the 128-token tiles and key blocks, a prefix, several blocks, one token
+PREFILL = [([(1, 0)], False), ([(127, 0), (128, 0), (129, 0)], False), ([(117, 0)], False), ([(300, 0), (5, 0), (1000, 0)], False),
+           ([(100, 512), (130, 256), (1, 255), (256, 1)], True), ([(900, 1100)], True)]
+
+
+@pytest.mark.parametrize("seqs,paged", PREFILL)
+def test_prefill_attention_against_fp32(rt, seqs, paged):
+    from nanovllm_b200 import ops
+    nq, nkv, hd, bs, scale = 16, 8, 128, 256, 128 ** -0.5
+    g = torch.Generator().manual_seed(sum(a + b for a, b in seqs))
+    tokens = sum(a for a, _ in seqs)
+    qkv = torch.randn(tokens, (nq + 2 * nkv) * hd, generator=g).bfloat16()
+    need = [-(-(a + b) // bs) for a, b in seqs]
+    free = torch.randperm(sum(need), generator=g).tolist()
+    tables = torch.full((len(seqs), max(need) + 1), -1, dtype=torch.int32)
+    kc, vc = (torch.full((sum(need), bs, nkv, hd), float("nan")).bfloat16() for _ in range(2))
+    ref, at = torch.zeros(tokens, nq, hd), 0
+    for i, (new, old) in enumerate(seqs):
+        tables[i, :need[i]] = torch.tensor([free.pop() for _ in range(need[i])], dtype=torch.int32)
+        rows = qkv[at:at + new]
+        k, v = (rows[:, (nq + j * nkv) * hd:(nq + (j + 1) * nkv) * hd].view(new, nkv, hd) for j in (0, 1))
+        if paged:
+            k, v = (torch.cat((torch.randn(old, nkv, hd, generator=g).bfloat16(), x)) for x in (k, v))
+            for p in range(old + new):
+                blk = int(tables[i, p // bs])
+                kc[blk, p % bs], vc[blk, p % bs] = k[p], v[p]
+        q = rows[:, :nq * hd].float().view(new, nq, hd)
+        kf, vf = (x.float().repeat_interleave(nq // nkv, 1) for x in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q, kf) * scale
+        s.masked_fill_(torch.arange(old + new) > (torch.arange(new) + old).unsqueeze(1), float("-inf"))
+        ref[at:at + new] = torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), vf)
+        at += new
+    cu = torch.tensor([0] + [a for a, _ in seqs]).cumsum(0).to(torch.int32).to(DEV)
+    cu_k = torch.tensor([0] + [a + b for a, b in seqs]).cumsum(0).to(torch.int32).to(DEV)
+    x = qkv.to(DEV)
+    q, k, v = (x[:, a * hd:b * hd].view(tokens, b - a, hd) for a, b in ((0, nq), (nq, nq + nkv), (nq + nkv, nq + 2 * nkv)))
+    max_q = max(a for a, _ in seqs)
+    if paged:
+        got = ops.prefill_attention(q, kc.to(DEV), vc.to(DEV), cu, cu_k, max_q, tables.to(DEV), scale)
+    else:
+        got = ops.prefill_attention(q, k, v, cu, cu_k, max_q, None, scale)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(got, ref, f"prefill attention {seqs}")
