@@ -98,6 +98,7 @@ struct GemmArgs {
   uint16_t* v_cache;
   const int32_t* slots;
   int silu_pairs;  // 1: features come in (gate, up) pairs; store silu(gate) * up, one value per pair, at column feature / 2
+  int ring_stages;  // cluster kernel: stages of its operand ring
   // stream-K combine
   float* ws;
   int* counters;
@@ -798,10 +799,10 @@ __device__ __forceinline__ void fused_tail(const GemmArgs& a, unsigned int parit
     // Every partial row of this CTA is on its way: from here on the CTA only waits for data, so the next kernel's CTAs
     // may take the SMs that are free.  (Released at set-up instead, they could occupy SMs before all CTAs of this
     // grid are resident, while the resident ones spin on rows the missing ones have yet to produce.)
-// Row-owner form: every rank waits for every other rank inside the same launch, so a store to a peer that lingers in
+    // Row-owner form: every rank waits for every other rank inside the same launch, so a store to a peer that lingers in
     // a write buffer until the kernel ends would never leave: push the partial rows out before waiting for anything.
     if (EPI == EPI_PUSH3) __threadfence_system();
-        if (threadIdx.x == 0) b2::pdl_launch_dependents();
+    if (threadIdx.x == 0) b2::pdl_launch_dependents();
     if (!aborted) {
       if (EPI == EPI_PUSH) {
         switch (a.world) {
@@ -1164,28 +1165,42 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
 // in its own shared memory, sums them after one cluster barrier, and writes its share of the output
 // as whole 256-byte token rows.  No global-memory round trip and no atomics on the critical path.
 // Feature-lane layout only (weights on the 128-row MMA side); up to 256 tokens as token tiles of BN <= 64, one cluster each.
+// Bound by latency: a launch streams 0.5-12 MB of weights, so set-up, one DRAM round trip, the cluster barriers and the exchange
+// are most of it.  The shared memory is therefore laid out for the tokens that a launch has (a fixed layout took a whole SM and
+// kept the next kernel out of it), only groups that hold tokens are exchanged, and nothing in the exchange divides by S:
+// 0.6B widths at one token qkv 5.3 -> 4.7 us, gate/up 6.1 -> 5.7; 8B widths down at 64 tokens 25.9 -> 24.9.
 // ---------------------------------------------------------------------------
 template <int BN>
 struct CfgCluster {
   static constexpr uint32_t P_BYTES = BM * BK * 2;
   static constexpr uint32_t Q_BYTES = BN * BK * 2;
   static constexpr uint32_t STAGE_BYTES = P_BYTES + Q_BYTES;
-  static constexpr int GROUPS = BN / 4;                                 // 4-column groups of the accumulator
-  static constexpr uint32_t RED_BYTES = (GROUPS + 8) * BM * 16;         // [source CTA][local group][feature][4] fp32
-  static constexpr uint32_t OUT_BYTES = BN * BM * 2;                    // [token][feature] bf16 staging of the output
-  static constexpr int STAGES_RAW = (200704 - RED_BYTES - OUT_BYTES) / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
   static constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
-  static constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + RED_BYTES + OUT_BYTES;
-  static_assert(STAGES >= 3, "too little shared memory left for the operand pipeline");
-  static_assert(SMEM_BYTES <= 232448, "more shared memory than an SM has");
+  static constexpr int MAX_STAGES = 12;
+  static constexpr uint32_t EXTRA = 1024 + 256;     // alignment, barriers
+  // The K split is chosen for CTAs that have an SM to themselves (this much shared memory), whatever a launch then takes: the
+  // order of the sums, and so the result, does not depend on how few tokens there are.
+  static constexpr uint32_t PLAN_BYTES = 200000;
+  static constexpr uint32_t ALL = 227 * 1024 - 256; // (static shared memory: a few words)
+  // 4-column groups of the accumulator that hold tokens, most of them any CTA of a cluster of S owns
+  __host__ __device__ static constexpr int live_groups(int M) { return ((M < BN ? M : BN) + 3) / 4; }
+  __host__ __device__ static constexpr int owned_groups(int M, int S) { return (live_groups(M) + S - 1) / S; }
+  __host__ __device__ static constexpr uint32_t red_bytes(int M, int S) { return S * owned_groups(M, S) * BM * 16; }  // [source CTA][local group][feature][4] fp32
+  __host__ __device__ static constexpr uint32_t out_bytes(int M, int S) { return owned_groups(M, S) * 4 * BM * 2; }   // [token][feature] bf16 staging of the output
+  // A few tokens and a short K range need half an SM or less; two CTAs then fit, so that a kernel's set-up and its first ring of
+  // weights run under the previous kernel's tail.  A long stream of weights takes all the ring it can get.
+  static int stages(int M, int S, int kblocks) {
+    const int room = static_cast<int>((ALL - EXTRA - red_bytes(M, S) - out_bytes(M, S)) / STAGE_BYTES);
+    return std::min({MAX_STAGES, room, (kblocks + S - 1) / S});
+  }
+  static uint32_t smem_bytes(int M, int S, int stages) { return stages * STAGE_BYTES + EXTRA + red_bytes(M, S) + out_bytes(M, S); }
 };
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(NUM_THREADS, EPI == EPI_STORE ? 2 : 1)  // (the reduce phase of 8 ranks wants its registers)
 gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ, const GemmArgs a) {
   using C = CfgCluster<BN>;
-  constexpr int STAGES = C::STAGES;
+  const int STAGES = a.ring_stages;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw_addr = b2::smem_u32(smem_raw);
   unsigned char* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -1197,7 +1212,6 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   unsigned char* red_buf = smem + STAGES * C::STAGE_BYTES + 256;
-  unsigned char* out_buf = red_buf + C::RED_BYTES;
   __shared__ float red[NUM_THREADS / 32];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1212,7 +1226,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
   const int kb_base = KB / S, kb_rem = KB % S;
   const int kb0 = crank * kb_base + min(crank, kb_rem);
   const int n_units = kb_base + (crank < kb_rem ? 1 : 0);
-  const int GL = (C::GROUPS + S - 1) / S;  // most groups any CTA of the cluster owns
+  const int groups = C::live_groups(a.M - tok0);
+  const int GL = C::owned_groups(a.M, S);  // most groups any CTA of a cluster owns
+  unsigned char* out_buf = red_buf + C::red_bytes(a.M, S);
 
   if (threadIdx.x == 0) {
     stamp(a, 7);
@@ -1234,7 +1250,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
   __syncthreads();
   b2::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (threadIdx.x == 0 && !is_push(EPI)) b2::pdl_launch_dependents();  // fused row-parallel calls: later, see fused_tail
+  if (threadIdx.x == 0 && !is_push(EPI)) b2::pdl_launch_dependents();
   if (threadIdx.x == 0) stamp(a, 0);
   unsigned int parity = 0;
   // fused qkv heads: rotary factors and cache slots of the first rows this warp will finish, fetched while the
@@ -1306,7 +1322,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
         const int token = tok0 + (((lt >> 2) * S + crank) << 2) + (lt & 3);
         pre_slot[i] = -1;
         pre_cs[i][0] = pre_cs[i][1] = pre_cs[i][2] = pre_cs[i][3] = 0.f;
-        if (token < a.M && (lt >> 2) * S + crank < C::GROUPS) {
+        if (token < a.M && (lt >> 2) * S + crank < groups) {
           if (a.k_cache != nullptr && tile >= a.nq) pre_slot[i] = __ldg(a.slots + token);
           if (rotated) {
             const float* cs = a.cos_sin + __ldg(a.positions + token) * 128;
@@ -1320,17 +1336,22 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
       b2::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
       const uint32_t red_local = b2::smem_u32(red_buf);
+      int owner = 0;  // of group g = c * 8 + j: g mod S, its place there g / S
+      uint32_t local = red_local + (crank * GL * BM + f) * 16;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = 0; c * 8 < groups; ++c) {
         uint32_t r[32];
         b2::tmem_ld_32x32(taddr + c * 32, r);
         b2::tc_wait_ld();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int g = c * 8 + j, owner = g % S, gl = g / S;
-          const uint32_t local = red_local + ((crank * GL + gl) * BM + f) * 16;
-          b2::st_cluster_v4(b2::map_to_cta(local, owner), __uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                            __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+          if (c * 8 + j < groups)
+            b2::st_cluster_v4(b2::map_to_cta(local, owner), __uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                              __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+          if (++owner == S) {
+            owner = 0;
+            local += BM * 16;
+          }
         }
       }
     }
@@ -1352,7 +1373,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
     int owned = 0;
     for (int gl = 0; gl < GL; ++gl) {
       const int g = gl * S + crank;
-      if (g >= C::GROUPS) break;
+      if (g >= groups) break;
       float4 sum = make_float4(bias, bias, bias, bias);
       for (int src = 0; src < S; ++src) {
         const float4 t = *reinterpret_cast<const float4*>(red_buf + ((src * GL + gl) * BM + f) * 16);
@@ -1584,7 +1605,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
   b2::cluster_wait();
   b2::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (threadIdx.x == 0 && !is_push(EPI)) b2::pdl_launch_dependents();  // fused row-parallel calls: later, see fused_tail
+  if (threadIdx.x == 0 && !is_push(EPI)) b2::pdl_launch_dependents();
   if (threadIdx.x == 0) stamp(a, 0);
   unsigned int parity = 0;
 
@@ -1729,16 +1750,17 @@ template <int BN, int EPI>
 int configure_cluster_kernel() {
   static PerDeviceOnce configured;
   return configured.ensure([&]() -> int {
-    B2_CUDA(cudaFuncSetAttribute(gemm_cluster_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, CfgCluster<BN>::SMEM_BYTES));
+    B2_CUDA(cudaFuncSetAttribute(gemm_cluster_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, CfgCluster<BN>::ALL));
     return B2_OK;
   });
 }
 
 template <int BN, int EPI>
-int launch_cluster_inst(const CUtensorMap& tmP, const CUtensorMap& tmQ, const GemmArgs& args, int tiles, int S, cudaStream_t stream) {
+int launch_cluster_inst(const CUtensorMap& tmP, const CUtensorMap& tmQ, GemmArgs& args, int tiles, int S, cudaStream_t stream) {
   const int crc = configure_cluster_kernel<BN, EPI>();
   if (crc != B2_OK) return crc;
-  B2_CUDA(b2_launch_cluster(gemm_cluster_kernel<BN, EPI>, dim3(tiles * S), dim3(NUM_THREADS), CfgCluster<BN>::SMEM_BYTES, stream,
+  args.ring_stages = CfgCluster<BN>::stages(args.M, S, args.kblocks);
+  B2_CUDA(b2_launch_cluster(gemm_cluster_kernel<BN, EPI>, dim3(tiles * S), dim3(NUM_THREADS), CfgCluster<BN>::smem_bytes(args.M, S, args.ring_stages), stream,
                             static_cast<unsigned>(S), tmP, tmQ, args));
   return B2_OK;
 }
@@ -1786,7 +1808,7 @@ int max_resident_clusters(int S) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S * 64);
   cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = CfgCluster<BN>::SMEM_BYTES;
+  cfg.dynamicSmemBytes = CfgCluster<BN>::PLAN_BYTES;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = S;

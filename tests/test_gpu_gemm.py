@@ -306,3 +306,18 @@ def test_pair_kernel():
     env.pop("B2_PAIR", None)
     res = subprocess.run([sys.executable, "-c", PAIR_SCRIPT % {"root": root}], env=env, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-4000:]
+
+
+@pytest.mark.parametrize("n,k", [(1024, 3072), (4096, 4096), (1048, 456)])
+@pytest.mark.parametrize("m", [1, 4, 5, 31, 33, 61, 64])
+def test_few_tokens_layout(ops, rt, m, n, k):
+    """The cluster kernel lays its shared memory out by the 4-token groups that hold tokens: sizes around their edges; the sums do not
+    depend on how many other tokens there are."""
+    x, w = _case(64, n, k, n + k)
+    x, w = x.to(DEV), w.to(DEV)
+    got, full = ops.gemm(x[:m], w), ops.gemm(x[-64:], w)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(got, (x[:m].double() @ w.double().t()).float(), f"few tokens {m}x{n}x{k}", abs_tol=2e-2)
+    if m > 32:  # (one token tile size)
+        assert torch.equal(got, full[:m])
