@@ -627,7 +627,7 @@ struct TilePlan {
 // Geometry of one problem (host arithmetic only; resident(split, bytes) = clusters of 2 * split CTAs with that much shared
 // memory the device holds at once).  The candidates' times are estimated, in nanoseconds, from what the parts were measured
 // to take on this part, and the fastest is taken:
-//   weights from DRAM at 6.4 TB/s; operands into an SM at 85 B/ns (from L2 or DRAM), and a turn of the ring takes the loaded
+//   weights from DRAM at 6.4 TB/s; operands into an SM at 82 B/ns (from L2 or DRAM), and a turn of the ring takes the loaded
 //   DRAM latency of 1.6 us; 2 clocks of the tensor pipe per token column and K block of a pair; the exchange of a split tile
 //   at 20 B/ns per SM (SM-to-SM network; stores and bulk copies alike) plus two cluster barriers; 0.6 us per 32 tokens stored
 //   by four warps (an SM sends about 14 bytes per clock).
@@ -646,12 +646,14 @@ int plan_tile_gemm(int M, int N, int K, int num_sms, int tile_cap, Resident&& re
     const int tiles_t = (M + bn - 1) / bn;
     const int64_t tiles = static_cast<int64_t>(tiles_f) * tiles_t;
     const int stage = W_BYTES + bn * BK, groups = bn / 8;
-    for (int s = 1; s <= (cut ? MAX_SPLIT : 1); ++s) {
+    for (int v = 0; v <= (cut ? MAX_SPLIT : 1); ++v) {  // 0: whole tiles, two CTAs per SM, one tile each
+      const int s = std::max(v, 1);
       const int64_t work = tiles * s;  // pairs launched
+      if (v == 0 && (work <= pairs || work > 2 * pairs)) continue;
       if (s > 1 && (kblocks < 2 * s || work > 2 * pairs)) break;
       const int most = (groups + s - 1) / s, kb = (kblocks + s - 1) / s;
       const uint32_t red = s > 1 ? static_cast<uint32_t>(s - 1) * most * 4096 : 0;
-      const bool multi = s == 1 && (work > pairs || kb * stage > static_cast<int>(SMEM_HALF - SMEM_EXTRA));
+      const bool multi = v == 1 && (work > pairs || kb * stage > static_cast<int>(SMEM_HALF - SMEM_EXTRA));
       // all of an SM's shared memory where no second CTA comes and the ring would use it
       const bool deep = multi || (work <= pairs && kb * stage > static_cast<int>(SMEM_HALF - SMEM_EXTRA));
       const uint32_t limit = deep ? SMEM_ALL : SMEM_HALF;
@@ -663,7 +665,7 @@ int plan_tile_gemm(int M, int N, int K, int num_sms, int tile_cap, Resident&& re
       if (ring + SMEM_EXTRA > limit) continue;
       if (s > 1 && resident(s, ring + SMEM_EXTRA) < tiles) continue;  // (two waves of a split tile never pay)
       const double t_mem = 2.0 * N * K / 6400.0;
-      const double t_kb = std::max({stage / 85.0, 1600.0 / stages, (std::max(bn, 64) * 2 + 40) / 1.9});
+      const double t_kb = std::max({stage / 82.0, (v == 0 ? 800.0 : 1600.0) / stages, (std::max(bn, 64) * 2 + 40) / 1.9});
       const double t_out = (multi ? 300.0 : 600.0) * ((groups + 4 * s - 1) / (4 * s)) + (s > 1 ? 1500.0 + (s - 1) * most * 4096 / 20.0 : 0.0);
       int64_t rounds = work / pairs, ranged = work % pairs;  // MULTI
       double cost;
@@ -677,7 +679,9 @@ int plan_tile_gemm(int M, int N, int K, int num_sms, int tile_cap, Resident&& re
         }
         cost = std::max(t_mem, ranged > 0 ? in_ranges : whole) + t_out;
       } else {
-        cost = std::max(t_mem, static_cast<double>((2 * work + num_sms - 1) / num_sms) * kb * t_kb) + t_out;
+        // (two CTAs of an SM overlap each other's latencies: measured 95 B/ns where one alone gets 80; 777 tokens x 6144 x 4096
+        // as 168 whole tiles on 148 SMs 57 -> 41 us)
+        cost = std::max(t_mem, static_cast<double>((2 * work + num_sms - 1) / num_sms) * kb * (v == 0 ? 0.85 : 1.0) * t_kb) + t_out + (v == 0 ? t_out : 0.0);
       }
       if (cost < best) {
         best = cost;

@@ -20,9 +20,10 @@ def rt(pkg):
 
 
 # one token past the decode kernels; edges of 32-, 64- and 256-token tiles; features that end inside a CTA's half; few K blocks; a
-# split over 2..4 pairs; ranges of K blocks (long K, tiles that do not fill the pairs); whole rounds with a remainder
+# split over 2..4 pairs; ranges of K blocks (long K, tiles that do not fill the pairs); whole tiles, two CTAs per SM; whole rounds with
+# a remainder
 SHAPES = [(65, 256, 64), (96, 128, 128), (97, 1032, 520), (128, 1024, 2048), (160, 4096, 4096), (255, 136, 1024), (256, 4096, 4096), (257, 512, 1024),
-          (391, 5120, 25600), (511, 6144, 4096), (512, 4096, 520), (777, 5120, 8192), (1500, 24576, 512)]
+          (391, 5120, 25600), (511, 6144, 4096), (512, 4096, 520), (777, 5120, 8192), (777, 6144, 4096), (1500, 24576, 512)]
 
 
 @pytest.mark.parametrize("m,n,k", SHAPES)
