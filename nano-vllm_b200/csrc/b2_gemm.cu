@@ -1931,10 +1931,29 @@ int plan_gemm(int epi, int M, int N, int K, int num_sms, int min_grid, int reduc
 }
 
 template <int EPI>
+int resident_clusters_of(int bn, int S) {
+  if constexpr (EPI == EPI_PUSH2 || EPI == EPI_SAMPLE) return 0;
+  else return bn == 32 ? max_resident_clusters<32, EPI>(S) : max_resident_clusters<64, EPI>(S);
+}
+
+// 65..256 tokens, nothing to exchange with peers: whether the decode kernel serves them better, as token tiles of 64 with their K range split over a
+// cluster.  It reads the weights once per token tile and its epilogue finishes 64 tokens alone, so this holds while there is room
+// to split every tile and each CTA's share of K is short (launch, set-up and the exchange are then most of either kernel): widths
+// of the 0.6B model, 119 tokens, qkv 11.2 -> 9.3 us; fused with the norm, which is a launch of its own behind the many-token
+// kernel, o 11.1 -> 9.9 and down 12.6 -> 10.6.  Where a share is longer it loses: 32 K blocks each, 65 tokens x 4096 x 4096,
+// 17.0 -> 17.8 us; unsplit tiles, 160 tokens x 4096 x 1024, 11.7 -> 15.7.
+template <int EPI>
+bool short_clusters(const b2_ctx* ctx, int M, int N, int K) {
+  GemmPlan p;
+  if (M <= 64 || M > 256 || plan_gemm(EPI, M, N, K, ctx->num_sms, 0, 0, ctx->tile_counter_cap, true, resident_clusters_of<EPI>, p) != B2_OK) return false;
+  return p.cluster_split >= 2 && (p.kblocks + p.cluster_split - 1) / p.cluster_split <= 12;
+}
+
+template <int EPI>
 int launch_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K, GemmArgs& args,
                 int min_grid, cudaStream_t stream) {
   if constexpr (EPI == EPI_STORE) {
-    if (M > 64) {  // more than a decode step's tokens: CTA pairs over tiles of up to 256 tokens, see b2_gemm_tile.cu
+    if (M > 64 && !short_clusters<EPI>(ctx, M, N, K)) {  // CTA pairs over tiles of up to 256 tokens, see b2_gemm_tile.cu
       b2::StoreEpilogue e;
       e.C = args.C;
       e.ldc = args.ldc;
@@ -1958,10 +1977,7 @@ int launch_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t 
   const int reducers = 0;  // no CTAs are set aside for the reduce phase: every CTA reduces after its GEMM work
   GemmPlan plan;
   const int prc = plan_gemm(EPI, M, N, K, ctx->num_sms, min_grid, reducers, ctx->tile_counter_cap, true,
-                            [](int bn, int S) {
-                              if constexpr (EPI == EPI_PUSH2 || EPI == EPI_SAMPLE) return 0;
-                              else return bn == 32 ? max_resident_clusters<32, EPI>(S) : max_resident_clusters<64, EPI>(S);
-                            },
+                            resident_clusters_of<EPI>,
                             plan, (ctx->whole_tiles && (EPI == EPI_PUSH2 || EPI == EPI_PUSH3)) ? PLAN_WHOLE_TILES : 0);
   if (prc != B2_OK) return prc;
   const bool swap = plan.swap != 0;
@@ -2415,10 +2431,10 @@ int b2_rowpar_fused(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int6
   if (bias != nullptr && !aligned16(bias)) return B2_ERR_ARG;
   const int chunk = ctx->cfg.oneshot_tokens;
   const int world = ctx->cfg.world;
-  if (world == 1 && M > 64 && ctx->rowpar_form == B2_FORM_AUTO) {
-    // One rank, many tokens: nothing crosses a link, so the block is the plain GEMM (CTA pairs from 512 tokens on)
-    // followed by the HBM-bound add + RMSNorm kernel in place - two launches, both near their rooflines, instead of
-    // one whose reduce phase walks the rows one CTA at a time.
+  if (world == 1 && M > 64 && ctx->rowpar_form == B2_FORM_AUTO && !(M <= chunk && short_clusters<EPI_PUSH>(ctx, M, N, Kr))) {
+    // One rank, many tokens: nothing crosses a link, so the block is the plain GEMM on CTA pairs followed by the HBM-bound
+    // add + RMSNorm kernel in place - two launches, both near their rooflines, instead of one whose reduce phase walks the
+    // rows one CTA at a time.
     GemmArgs args{};
     args.C = static_cast<uint16_t*>(normed_out);
     args.ldc = N;

@@ -321,3 +321,22 @@ def test_few_tokens_layout(ops, rt, m, n, k):
     assert_close_bf16(got, (x[:m].double() @ w.double().t()).float(), f"few tokens {m}x{n}x{k}", abs_tol=2e-2)
     if m > 32:  # (one token tile size)
         assert torch.equal(got, full[:m])
+
+
+@pytest.mark.parametrize("m,n,k,path", [(65, 4096, 1024, 1), (128, 1024, 3072, 1), (129, 1032, 1544, 1), (256, 1024, 3072, 1), (256, 1024, 3136, 2), (129, 4096, 1024, 2)])
+def test_up_to_256_tokens_on_clusters(ops, rt, m, n, k, path):
+    """65..256 tokens run on the cluster kernel while its K split leaves each CTA a short share, on the CTA-pair kernel above that;
+    fused with residual + norm likewise."""
+    from nanovllm_b200 import _abi
+    xs, ws, residual, norm_w = O.rowpar_case(m, k, n, 1, seed=m + k + 2)
+    x, w = xs[0].to(DEV), ws[0].to(DEV)
+    y = ops.gemm(x, w)
+    assert _abi.lib.b2_last_gemm_kernel() == path
+    normed, new_res = ops.rowpar_fused(x, w, None, residual.to(DEV), norm_w.to(DEV), 1e-6)
+    assert _abi.lib.b2_last_gemm_kernel() == path
+    torch.cuda.synchronize()
+    rt.check_status()
+    exact_n, exact_s = O.fused_row_parallel_norm_exact(xs, ws, residual, norm_w, 1e-6)
+    assert_close_bf16(y, xs[0].float() @ ws[0].float().t(), f"gemm {m}x{k}x{n}")
+    assert_close_bf16(new_res, exact_s, f"residual {m}x{k}x{n}")
+    assert_close_bf16(normed, exact_n, f"normed {m}x{k}x{n}")
