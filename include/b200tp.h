@@ -119,8 +119,10 @@ int64_t b2_launch_count(void);
  *      (nanovllm/layers/embed_head.py:61) -----------------------------------
  * C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]), bf16 in, fp32 accumulate, bf16 out.
  * lda/ldw/ldc are row strides in elements (multiples of 8); K a multiple of 8.
- * tcgen05 tensor-core kernel fed by TMA; the work is split along K over the
- * SMs (stream-K) when there are fewer output tiles than SMs.  W is treated as
+ * tcgen05 tensor-core kernels fed by TMA: up to 64 tokens the K range is split
+ * over clusters or over all SMs (stream-K), more tokens run on CTA pairs (or,
+ * up to 256, as 64-token tiles on clusters).  From 512 tokens on every output
+ * is one unbroken sum over K.  W is treated as
  * a constant: the kernel may start fetching it while the previous b2_* kernel
  * on the stream is still running, so W must not be the output of a b2_* call
  * that immediately precedes this one (A, bias and C have no such rule). */
@@ -134,9 +136,9 @@ int b2_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw,
  * qkv[M, (nq + 2 nkv) head_dim] = A W^T (+ bias); then, per token and head:
  * q and k heads are RMS-normalised (weights may both be NULL) and rotated,
  * k and v heads are also written to the paged cache (k_cache may be NULL).
- * Arguments as b2_gemm and b2_qk_norm_rope_store.  For up to 64 tokens and
- * head_dim 128 everything happens in the GEMM's epilogue (one launch);
- * otherwise the projection and the head kernel run as two launches. */
+ * Arguments as b2_gemm and b2_qk_norm_rope_store.  With head_dim 128
+ * everything happens in the GEMM's epilogue (one launch; the stream-K kernel
+ * excepted); otherwise the projection and the head kernel run as two launches. */
 int b2_qkv_fused(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw, const void* bias, void* qkv,
                  int64_t ld_qkv, int M, int nq, int nkv, int head_dim, int K, const void* q_norm_w,
                  const void* k_norm_w, float eps, const int64_t* positions, const float* cos_sin, void* k_cache,
@@ -211,7 +213,8 @@ int b2_gemm_static_scratch(const void* A, int64_t lda, const void* W, int64_t ld
  *              -0.0 in an output of this form is stored as +0.0.
  * On one rank with more than 64 tokens nothing crosses a link and the call
  * runs as the plain GEMM followed by the add + RMSNorm kernel in place (two
- * launches), unless a form is forced. */
+ * launches), unless a form is forced or up to 256 tokens fit the cluster
+ * kernel with a short K range per CTA (one launch). */
 int b2_rowpar_fused(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw, const void* bias,
                     int M, int N, int Kr, const void* residual_in, const void* norm_w, float eps,
                     void* normed_out, void* residual_out, void* stream);
@@ -435,7 +438,8 @@ typedef struct b2_gemm_plan {
   int cluster_split; /* > 0: cluster kernel, K split this many ways; 0: stream-K */
 } b2_gemm_plan;
 
-/* epilogue: 0 = b2_gemm / b2_lm_head / b2_gemm_silu_mul / b2_qkv_fused,
+/* epilogue: 0 = b2_gemm / b2_lm_head / b2_gemm_silu_mul / b2_qkv_fused (up to 64 tokens; above that the plan is only
+ * followed where it is a cluster plan with a short K range, and the CTA-pair kernel serves the rest),
  * 1 = b2_rowpar_fused (one-shot form), 2 = b2_rowpar_fused_twoshot, 3 = b2_lm_head_sample,
  * 4 = b2_rowpar_fused (row-owner form).  resident_clusters: NULL
  * (cluster kernel not considered) or int[18]: entry [S] for 32-token tiles and
@@ -459,7 +463,7 @@ int b2_plan_cta_units(const b2_gemm_plan* plan, int cta, int* units, int cap);
 int b2_plan_tile_contributors(const b2_gemm_plan* plan, int tile, int* first_cta, int* last_cta);
 
 /* Which kernel the calling thread's most recent GEMM-shaped call launched: 0 = persistent stream-K kernel,
- * 1 = cluster split-K kernel, 2 = CTA-pair kernel (problems of at least 512 tokens). */
+ * 1 = cluster split-K kernel, 2 = CTA-pair kernel (store GEMMs of more than 64 tokens, the two-shot form from 512). */
 int b2_last_gemm_kernel(void);
 
 /* Two-shot row ownership: the rank that reduces token row `token` (blocks of

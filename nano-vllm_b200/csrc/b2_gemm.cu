@@ -1,11 +1,13 @@
 // bf16 GEMMs for sm_100a: TMA-fed shared-memory pipeline, tcgen05.mma with fp32
 // accumulators in tensor memory, warp-specialised (1 TMA thread, 1 MMA thread,
-// 4 epilogue warps).  Two kernels share the operand convention and epilogues:
+// 4 epilogue warps).  Two kernels share the operand convention and epilogues (store
+// GEMMs of more tokens than these serve are in b2_gemm_tile.cu):
 //
 //   gemm_kernel          persistent over a stream-K partition of the work (any size)
 //   gemm_cluster_kernel  one thread-block cluster per output tile, K split over the
 //                        cluster, parts combined through distributed shared memory
-//                        (decode sizes: at most 64 tokens and one wave of tiles)
+//                        (decode sizes: at most 64 tokens and one wave of tiles; up to 256
+//                        as token tiles of 64 where the K split stays short)
 //
 // D[p, q] = sum_k P[p, k] * Q[q, k]; both operands are K-major (row-major with
 // K contiguous).  P tiles have 128 rows (the MMA M dimension = 128 TMEM
@@ -1777,8 +1779,8 @@ int launch_pair_inst(const CUtensorMap& tmP, const CUtensorMap& tmQ, const GemmA
   return B2_OK;
 }
 
-// The CTA-pair kernel serves many-token problems (at least 512 tokens, tiles of 128 or 256 features); B2_PAIR=0 in
-// the environment sends them to the stream-K kernel instead (for comparison).
+// The CTA-pair kernel serves the two-shot form (at least 512 tokens, tiles of 128 or 256 features); B2_PAIR=0 in the
+// environment sends it to the stream-K kernel instead (for comparison).
 bool pair_path_enabled() {
   static const bool on = [] {
     const char* e = getenv("B2_PAIR");
