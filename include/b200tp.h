@@ -384,6 +384,16 @@ int b2_qk_norm_rope_store(void* qkv, int64_t ld_qkv, int M, int nq, int nkv, int
                           const int64_t* positions, const float* cos_sin,
                           void* k_cache, void* v_cache, const int32_t* slot_mapping, void* stream);
 
+/* The head norm and the rotation on their own, for callers that keep the
+ * reference's separate steps.  x: token t's head h at x + t ldx + h dim (dim
+ * <= 256, a multiple of 8), out likewise with ldo. */
+int b2_head_rmsnorm(const void* x, int64_t ldx, int heads, const void* w, float eps, int tokens, int dim, void* out,
+                    int64_t ldo, void* stream);
+/* q [M, nq heads], k [M, nkv heads] with row strides ldq / ldk (heads of a row contiguous), rotated into
+ * the contiguous q_out and k_out; the other arguments as b2_qk_norm_rope_store. */
+int b2_rope(const void* q, int64_t ldq, const void* k, int64_t ldk, int M, int nq, int nkv, int head_dim,
+            const int64_t* positions, const float* cos_sin, void* q_out, void* k_out, void* stream);
+
 /* ---- decode attention over the paged cache: what flash_attn_with_kvcache computes
  *      for one query token per sequence (nanovllm/layers/attention.py:70-74) -------
  * q [n_seqs, nq, head_dim] bf16 with row stride q_stride (a view of the qkv output);

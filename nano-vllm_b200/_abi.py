@@ -68,6 +68,8 @@ SIGNATURES = {
     "b2_rowpar_form": [_p, _i, _i],
     "b2_rowpar_fused_twoshot": [_p, _p, _i64, _p, _i64, _p, _i, _i, _i, _p, _p, _f, C.POINTER(_p), _p, _p],
     "b2_rmsnorm": [_p, _i64, _p, _f, _i, _i, _p, _i64, _p],
+    "b2_head_rmsnorm": [_p, _i64, _i, _p, _f, _i, _i, _p, _i64, _p],
+    "b2_rope": [_p, _i64, _p, _i64, _i, _i, _i, _i, _p, _p, _p, _p, _p],
     "b2_add_rmsnorm": [_p, _p, _p, _f, _i, _i, _p, _p, _p],
     "b2_store_kvcache": [_p, _i64, _p, _i64, _p, _p, _p, _i, _i, _p],
     "b2_embed": [_p, _p, _p, _i64, _i64, _i, _i, _p, _p],

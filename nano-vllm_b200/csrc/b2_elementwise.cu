@@ -119,6 +119,38 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* __restrict
   }
 }
 
+// RMSNorm of short rows, the heads of q or k: token t's head h starts at x + t * ldx + h * dim, so the heads are read where the
+// projection left them.  Bound: HBM (2 dim 2 bytes per head).  One 16-byte vector per thread, LANES threads per head: rmsnorm_kernel
+// would give a head of 128 a whole warp, half of it idle.
+// With rope_kernel it saves six copies of q and k per layer: 391 tokens of the original layer code, 239 -> 221 us.
+template <int LANES>
+__global__ void __launch_bounds__(256) head_rmsnorm_kernel(const uint16_t* __restrict__ x, int64_t ldx, int heads, const uint16_t* __restrict__ w,
+                                                           float eps, int tokens, int dim, uint16_t* __restrict__ out, int64_t ldo) {
+  b2::pdl_launch_dependents();
+  b2::pdl_wait();
+  const int64_t row = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / LANES;
+  const int v = threadIdx.x % LANES;
+  const int64_t token = row / heads;
+  const int64_t head = row - token * heads;
+  const bool active = token < tokens && v < (dim >> 3);
+  float f[8];
+  float ss = 0.f;
+  if (active) {
+    unpack8(ldg_v4(x + token * ldx + head * dim + v * 8), f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+  }
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (!active) return;
+  const float rstd = rsqrtf(ss / static_cast<float>(dim) + eps);
+  float wv[8], y[8];
+  unpack8(ldg_v4(w + v * 8), wv);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) y[e] = bf16_round(f[e] * rstd) * wv[e];
+  stg_v4(out + token * ldo + head * dim + v * 8, pack8(y));
+}
+
 // ---------------------------------------------------------------------------
 // SiLU(gate) * up
 // ---------------------------------------------------------------------------
@@ -233,6 +265,41 @@ __global__ void __launch_bounds__(256) qk_norm_rope_store_kernel(uint16_t* __res
       k_cache[cache_off + HALF + lane] = b;
     }
   }
+}
+
+// neox rotation of q and k heads into new tensors.  Bound: HBM (4 head_dim bytes per head; the factors of a token stay in L2).
+// A thread rotates 8 element pairs: 16-byte vectors of both halves of a head.
+__global__ void __launch_bounds__(256) rope_kernel(const uint16_t* __restrict__ q, int64_t ldq, const uint16_t* __restrict__ k, int64_t ldk, int M,
+                                                   int nq, int nkv, int half, const int64_t* __restrict__ positions,
+                                                   const float* __restrict__ cos_sin, uint16_t* __restrict__ q_out, uint16_t* __restrict__ k_out) {
+  b2::pdl_launch_dependents();
+  b2::pdl_wait();
+  const int per_head = half >> 3, heads = nq + nkv, per_token = heads * per_head;
+  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t token = i / per_token;
+  if (token >= M) return;
+  const int in_token = static_cast<int>(i - token * per_token);
+  const int head = in_token / per_head, v = (in_token - head * per_head) * 8;
+  const bool is_q = head < nq;
+  const int h = is_q ? head : head - nq, hd = 2 * half;
+  const uint16_t* src = (is_q ? q + token * ldq : k + token * ldk) + static_cast<int64_t>(h) * hd + v;
+  uint16_t* dst = (is_q ? q_out + token * nq * hd : k_out + token * nkv * hd) + static_cast<int64_t>(h) * hd + v;
+  const float* cs = cos_sin + __ldg(positions + token) * hd + v;
+  float x1[8], x2[8], c[8], s[8], y1[8], y2[8];
+  unpack8(ldg_v4(src), x1);
+  unpack8(ldg_v4(src + half), x2);
+#pragma unroll
+  for (int e = 0; e < 8; e += 4) {
+    *reinterpret_cast<float4*>(c + e) = __ldg(reinterpret_cast<const float4*>(cs + e));
+    *reinterpret_cast<float4*>(s + e) = __ldg(reinterpret_cast<const float4*>(cs + half + e));
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {  // separate roundings of the products, as in qk_norm_rope_store_kernel
+    y1[e] = __fsub_rn(__fmul_rn(x1[e], c[e]), __fmul_rn(x2[e], s[e]));
+    y2[e] = __fadd_rn(__fmul_rn(x2[e], c[e]), __fmul_rn(x1[e], s[e]));
+  }
+  stg_v4(dst, pack8(y1));
+  stg_v4(dst + half, pack8(y2));
 }
 
 // ---------------------------------------------------------------------------
@@ -531,7 +598,35 @@ static int launch_rmsnorm(bool add, const void* x, int64_t ldx, const void* res,
   return B2_OK;
 }
 
+int b2_head_rmsnorm(const void* x, int64_t ldx, int heads, const void* w, float eps, int tokens, int dim, void* out, int64_t ldo, void* stream) {
+  if (tokens < 0 || heads <= 0 || dim <= 0 || dim % 8 != 0 || dim > 256) return B2_ERR_ARG;
+  if (tokens == 0) return B2_OK;
+  if (!x || !w || !out || !aligned16(x) || !aligned16(w) || !aligned16(out) || ldx % 8 != 0 || ldo % 8 != 0) return B2_ERR_ARG;
+  const int lanes = dim <= 128 ? 16 : 32;
+  const int64_t grid = (static_cast<int64_t>(tokens) * heads * lanes + 255) / 256;
+  if (grid > 0x7fffffff) return B2_ERR_SHAPE;
+  B2_CUDA(b2_launch(lanes == 16 ? head_rmsnorm_kernel<16> : head_rmsnorm_kernel<32>, dim3(static_cast<unsigned>(grid)), dim3(256), 0,
+                    static_cast<cudaStream_t>(stream), static_cast<const uint16_t*>(x), ldx, heads, static_cast<const uint16_t*>(w), eps, tokens, dim,
+                    static_cast<uint16_t*>(out), ldo));
+  return B2_OK;
+}
+
+int b2_rope(const void* q, int64_t ldq, const void* k, int64_t ldk, int M, int nq, int nkv, int head_dim, const int64_t* positions,
+            const float* cos_sin, void* q_out, void* k_out, void* stream) {
+  if (M < 0 || nq <= 0 || nkv <= 0 || (head_dim != 128 && head_dim != 64)) return B2_ERR_ARG;
+  if (M == 0) return B2_OK;
+  if (!q || !k || !positions || !cos_sin || !q_out || !k_out) return B2_ERR_ARG;
+  if (!aligned16(q) || !aligned16(k) || !aligned16(cos_sin) || !aligned16(q_out) || !aligned16(k_out) || ldq % 8 != 0 || ldk % 8 != 0) return B2_ERR_ARG;
+  const int64_t grid = (static_cast<int64_t>(M) * (nq + nkv) * (head_dim / 16) + 255) / 256;
+  if (grid > 0x7fffffff) return B2_ERR_SHAPE;
+  B2_CUDA(b2_launch(rope_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<const uint16_t*>(q), ldq,
+                    static_cast<const uint16_t*>(k), ldk, M, nq, nkv, head_dim / 2, positions, cos_sin, static_cast<uint16_t*>(q_out),
+                    static_cast<uint16_t*>(k_out)));
+  return B2_OK;
+}
+
 int b2_rmsnorm(const void* x, int64_t ldx, const void* w, float eps, int rows, int dim, void* out, int64_t ldo, void* stream) {
+  if (dim <= 256) return b2_head_rmsnorm(x, ldx, 1, w, eps, rows, dim, out, ldo, stream);
   return launch_rmsnorm(false, x, ldx, nullptr, w, eps, rows, dim, out, ldo, nullptr, stream);
 }
 

@@ -94,6 +94,10 @@ at::Tensor leading(const at::Tensor& out, const at::Tensor& x, int64_t n) {
   shape.push_back(n);
   return out.view(shape);
 }
+// [tokens, heads, head_dim] whose heads lie one after the other in each token's row, in 16-byte vectors
+bool heads_in_rows(const at::Tensor& t) {
+  return t.stride(2) == 1 && (t.size(1) == 1 || t.stride(1) == t.size(2)) && t.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+}
 PyObject* wrap(const at::Tensor& t) { return THPVariable_Wrap(t); }
 PyObject* wrap(const at::Tensor& a, const at::Tensor& b) {
   PyObject* p = PyTuple_New(2);
@@ -196,6 +200,12 @@ PyObject* rowpar_fused(Args a) {
 PyObject* rmsnorm(Args a) {
   at::Tensor x = bf16_rows(tensor(a[0], "rmsnorm input"), "rmsnorm input");
   const at::Tensor& w = tensor(a[1], "rmsnorm weight");
+  const int64_t dim = x.dim() > 0 ? x.size(-1) : 0;
+  if (x.dim() == 3 && dim <= 256 && heads_in_rows(x)) {  // heads of q or k, read from the rows of the projection
+    const at::Tensor out = at::detail::empty_cuda(x.sizes(), at::kBFloat16, x.device(), std::nullopt);
+    check(b2_head_rmsnorm(x.data_ptr(), x.stride(0), x.size(1), w.data_ptr(), number(a[2]), x.size(0), dim, out.data_ptr(), x.size(1) * dim, stream()), "b2_rmsnorm");
+    return wrap(out);
+  }
   const Rows in = matrix(x, "rmsnorm input");
   const at::Tensor out = empty_rows(in.rows, in.cols, x);
   check(b2_rmsnorm(in.t.data_ptr(), in.ld, w.data_ptr(), number(a[2]), in.rows, in.cols, out.data_ptr(), in.cols, stream()), "b2_rmsnorm");
@@ -250,6 +260,33 @@ PyObject* qk_norm_rope_store(Args a) {
   check(b2_qk_norm_rope_store(qkv.data_ptr(), qkv.stride(0), qkv.size(0), nq, nkv, hd, ptr(qw), ptr(kw), number(a[6]), pos.const_data_ptr<int64_t>(),
                               cs.const_data_ptr<float>(), c.k, c.v, c.slots, stream()), "b2_qk_norm_rope_store");
   Py_RETURN_NONE;
+}
+
+// rope(positions, q, k, cos_sin, head_dim): rotated copies; q, k [tokens, heads, head_dim], or flattened over the heads
+PyObject* rope(Args a) {
+  at::Tensor pos = tensor(a[0], "positions");
+  const at::Tensor& cs = tensor(a[3], "cos_sin");
+  const int64_t hd = integer(a[4]), t = pos.numel();
+  expect(cs.scalar_type() == at::kFloat && cs.is_contiguous(), "cos_sin must be contiguous fp32");
+  if (pos.scalar_type() != at::kLong) pos = pos.to(at::kLong);
+  pos = pos.contiguous();
+  at::Tensor in[2];
+  int64_t heads[2], ld[2];
+  for (int i = 0; i < 2; ++i) {
+    at::Tensor x = tensor(a[1 + i], i == 0 ? "query" : "key");
+    if (x.scalar_type() != at::kBFloat16) x = x.to(at::kBFloat16);
+    if (x.dim() != 3 || x.size(0) != t || x.size(2) != hd) x = x.reshape({t, t > 0 ? x.numel() / (t * hd) : 1, hd});
+    if (!x.is_cuda()) raise(PyExc_TypeError, "rotary embedding: expected CUDA tensors");
+    if (!heads_in_rows(x)) x = x.clone(at::MemoryFormat::Contiguous);
+    heads[i] = x.size(1);
+    ld[i] = t > 1 ? x.stride(0) : heads[i] * hd;
+    in[i] = x;
+  }
+  const at::Tensor qo = at::detail::empty_cuda(tensor(a[1], "query").sizes(), at::kBFloat16, in[0].device(), std::nullopt);
+  const at::Tensor ko = at::detail::empty_cuda(tensor(a[2], "key").sizes(), at::kBFloat16, in[1].device(), std::nullopt);
+  check(b2_rope(in[0].data_ptr(), ld[0], in[1].data_ptr(), ld[1], t, heads[0], heads[1], hd, pos.const_data_ptr<int64_t>(), cs.const_data_ptr<float>(),
+                qo.data_ptr(), ko.data_ptr(), stream()), "b2_rope");
+  return wrap(qo, ko);
 }
 
 // embed(ctx, ids, w, vocab_start, vocab_end)
@@ -329,7 +366,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define B2_ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {B2_ENTRY(init, 1), B2_ENTRY(gemm, 4), B2_ENTRY(gemm_silu_mul, 3), B2_ENTRY(qkv_fused, 15), B2_ENTRY(rowpar_fused, 7),
                          B2_ENTRY(rmsnorm, 3), B2_ENTRY(add_rmsnorm, 4), B2_ENTRY(silu_and_mul, 1), B2_ENTRY(store_kvcache, 5),
-                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(embed, 5), B2_ENTRY(paged_attention, 7), B2_ENTRY(prefill_attention, 9), {nullptr, nullptr, 0, nullptr}};
+                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(rope, 5), B2_ENTRY(embed, 5), B2_ENTRY(paged_attention, 7), B2_ENTRY(prefill_attention, 9), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_b2torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -3,8 +3,8 @@
 The decoder layer does not call `forward`: its rotation runs inside the qkv
 projection's epilogue (or the q/k-norm + RoPE + KV-scatter kernel) on the same
 cos||sin table.  `forward(positions, query, key)` keeps the reference's class
-usable on its own (:37-48): it runs that kernel with the head norm and the
-KV scatter switched off.
+usable on its own (:37-48): it reads q and k where
+the projection left them and writes rotated copies.
 """
 from __future__ import annotations
 
@@ -31,16 +31,7 @@ class RotaryEmbedding(nn.Module):
     def forward(self, positions: torch.Tensor, query: torch.Tensor, key: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
         """query [T, heads, head_size], key [T, kv_heads, head_size] (or flattened over the heads); returns rotated
         copies, fp32 arithmetic and one rounding to bf16, as the reference's apply_rotary_emb (:6-14)."""
-        hd = self.head_size
-        t = positions.numel()
-        q2, k2 = query.reshape(t, -1), key.reshape(t, -1)
-        nq, nkv = q2.shape[1] // hd, k2.shape[1] // hd
-        # the kernel works in place on a [T, (nq + 2 nkv) hd] row (q heads, k heads, v heads): the v part stays unused
-        buf = torch.empty(t, (nq + 2 * nkv) * hd, dtype=torch.bfloat16, device=query.device)
-        buf[:, :nq * hd] = q2
-        buf[:, nq * hd:(nq + nkv) * hd] = k2
-        ops.qk_norm_rope_store(buf, nq, nkv, hd, None, None, 0.0, positions.reshape(-1).to(torch.int64), self.cos_sin_cache, None, None, None)
-        return buf[:, :nq * hd].reshape(query.shape), buf[:, nq * hd:(nq + nkv) * hd].reshape(key.shape)
+        return ops.rope(positions, query, key, self.cos_sin_cache, self.head_size)
 
 
 @lru_cache(1)

@@ -116,6 +116,11 @@ def qk_norm_rope_store(qkv: torch.Tensor, nq: int, nkv: int, head_dim: int, q_no
     _native.qk_norm_rope_store(qkv, nq, nkv, head_dim, q_norm_w, k_norm_w, eps, positions, cos_sin, k_cache, v_cache, slot_mapping)
 
 
+def rope(positions: torch.Tensor, q: torch.Tensor, k: torch.Tensor, cos_sin: torch.Tensor, head_dim: int) -> tuple[torch.Tensor, torch.Tensor]:
+    """Rotated copies of q [tokens, heads, head_dim] and k (or flattened over the heads)."""
+    return _native.rope(positions, q, k, cos_sin, head_dim)
+
+
 def embed(ids: torch.Tensor, w: torch.Tensor, vocab_start: int, vocab_end: int, world: int) -> torch.Tensor:
     return _native.embed(get_runtime().handle if world > 1 else None, ids, w, vocab_start, vocab_end)
 

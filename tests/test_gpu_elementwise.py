@@ -195,3 +195,29 @@ def test_argmax(ops):
     assert got[3].item() == 77
     small = torch.randn(5, 1000, generator=g).bfloat16()
     assert torch.equal(ops.argmax(small.to(DEV)).cpu(), small.float().argmax(-1))
+
+
+@pytest.mark.parametrize("t,nq,nkv,hd", [(1, 16, 8, 128), (7, 3, 1, 64), (391, 32, 8, 128)])
+def test_head_norm_and_rotation_of_projection_views(ops, t, nq, nkv, hd):
+    """q and k norm and rotary embedding on views of the projection's rows (and on rows no vector can read) against the fused head kernel."""
+    g = torch.Generator(device=DEV).manual_seed(t)
+    qkv = torch.randn(t, (nq + 2 * nkv) * hd, device=DEV, generator=g).bfloat16()
+    odd = torch.empty(t, qkv.shape[1] + 3, dtype=torch.bfloat16, device=DEV)[:, 3:].copy_(qkv)
+    qw, kw = ((torch.rand(hd, device=DEV, generator=g) + 0.5).bfloat16() for _ in range(2))
+    pos = torch.randint(0, 512, (t,), device=DEV, generator=g)
+    table = O.rope_cache(hd, 512, 1e6).to(DEV)
+    fused = qkv.clone()
+    ops.qk_norm_rope_store(fused, nq, nkv, hd, qw, kw, 1e-6, pos, table, None, None, None)
+    ref = fused.split([nq * hd, nkv * hd, nkv * hd], dim=-1)
+    for rows in (qkv, odd):
+        before = rows.clone()
+        q, k, _ = rows.split([nq * hd, nkv * hd, nkv * hd], dim=-1)
+        q, k = ops.rmsnorm(q.view(t, nq, hd), qw, 1e-6), ops.rmsnorm(k.view(t, nkv, hd), kw, 1e-6)
+        for a, b in (ops.rope(pos, q, k, table, hd), ops.rope(pos.int(), q.view(t, -1), k.view(t, -1), table, hd)):
+            assert ulp_mismatch_fraction(a.reshape(t, -1), ref[0], 1) < 1e-3 and ulp_mismatch_fraction(b.reshape(t, -1), ref[1], 1) < 1e-3
+        q, k, _ = rows.split([nq * hd, nkv * hd, nkv * hd], dim=-1)
+        a, b = ops.rope(pos, q.view(t, nq, hd), k.view(t, nkv, hd), table, hd)
+        plain = qkv.clone()
+        ops.qk_norm_rope_store(plain, nq, nkv, hd, None, None, 0.0, pos, table, None, None, None)
+        assert torch.equal(torch.cat([a.reshape(t, -1), b.reshape(t, -1)], -1), plain[:, :(nq + nkv) * hd])
+        assert torch.equal(rows, before)
