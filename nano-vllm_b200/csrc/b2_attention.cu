@@ -22,7 +22,9 @@ namespace {
 // Work split: the tiles of the whole batch, in the order (sequence, head, position), are dealt in contiguous equal ranges
 // to the CTAs - the contexts' lengths are read on the device, so a captured graph stays balanced for any batch.  A
 // (sequence, head) that spans several CTAs is combined by whichever of them finishes last; a CTA holds at most two such
-// parts and settles both at its end.
+// parts and settles both at its end.  Settling takes 3-4 us (a fence, an atomic and the parts' way through L2), as long as
+// walking 8 tiles: where every (sequence, head) can have a CTA of its own and the longest is no further than that above
+// the even share, they are dealt whole.  One sequence of 300 tokens 5.9 -> 4.8 us, 37 of 40..700 tokens 16.5 -> 13.1.
 // ---------------------------------------------------------------------------
 constexpr int ATT_WARPS = 4, ATT_THREADS = (ATT_WARPS + 1) * 32;  // the last warp is the producer
 constexpr int ATT_TILE = 64;          // tokens per tile
@@ -38,6 +40,7 @@ constexpr int ATT_HALF_BYTES = ATT_TILE * 128;          // 64 tokens x 64 dimens
 constexpr int ATT_STAGE_BYTES = 4 * ATT_HALF_BYTES;     // K dimensions 0..63, 64..127, V the same
 constexpr int ATT_SLOT = ATT_ROWS * ATT_HD + 2 * ATT_ROWS;  // floats of one partial result: O, then the maxima and sums
 constexpr int ATT_MAX_SEQS = 1024;
+constexpr int ATT_COMBINE_TILES = 8;  // what combining the parts of an item costs, in tiles
 static_assert(ATT_CTAS_PER_SM * 2 * ATT_SLOT == B2_ATTN_WS_FLOATS_PER_SM, "the context allocates two slots per CTA");
 
 struct AttnArgs {
@@ -113,7 +116,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   int* s_len = first_tile + a.n_seqs + 1;
   __shared__ float s_m[ATT_WARPS][ATT_ROWS], s_l[ATT_WARPS][ATT_ROWS];
   __shared__ __align__(8) uint64_t s_bars[2 * ATT_MAX_STAGES];
-  __shared__ int s_abort, s_last[2];
+  __shared__ int s_abort, s_last[2], s_most;
   volatile int* abort_flag = &s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t bar_full = b2::smem_u32(s_bars), bar_empty = bar_full + ATT_MAX_STAGES * 8;
@@ -134,7 +137,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   const int max_len = a.bt_width * a.block_size;
   if (warp == 0) {
     const int per = (a.n_seqs + 31) / 32, s0 = lane * per;
-    int mine = 0;
+    int mine = 0, most = 0;
 #pragma unroll 4
     for (int i = 0; i < per; ++i)
       if (s0 + i < a.n_seqs) {
@@ -143,7 +146,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         s_len[s0 + i] = len;
         first_tile[s0 + i + 1] = t;
         mine += t;
+        most = max(most, t);
       }
+    most = __reduce_max_sync(0xffffffffu, most);
     int incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -151,17 +156,28 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       if (lane >= o) incl += up;
     }
     int at = incl - mine;
-    if (lane == 0) first_tile[0] = 0;
+    if (lane == 0) {
+      first_tile[0] = 0;
+      s_most = most;
+    }
     for (int i = 0; i < per; ++i)
       if (s0 + i < a.n_seqs) first_tile[s0 + i + 1] = at += first_tile[s0 + i + 1];
   }
   __syncthreads();
   const int total = first_tile[a.n_seqs] * a.nkv;
-  const int ctas = min(static_cast<int>(gridDim.x), total);
-  const int cta = blockIdx.x;
+  // (parts of an item are fewer, and no CTA has more tiles, when as many CTAs as need be take the same number of them)
+  const int cta = blockIdx.x, items = a.n_seqs * a.nkv, cap = static_cast<int>(gridDim.x);
+  const int per = (total + cap - 1) / cap;
+  const int spread = per <= 8 ? (total + per - 1) / per : cap;
+  const bool by_item = items <= cap && s_most <= total / spread + ATT_COMBINE_TILES;
+  const int ctas = by_item ? items : spread;
   if (cta >= ctas) return;
   const int base = total / ctas, rem = total % ctas;
-  auto begin_of = [&](int i) { return i * base + min(i, rem); };
+  auto begin_of = [&](int i) {
+    if (!by_item) return i * base + min(i, rem);
+    const int b = i / a.nkv, first = first_tile[b];
+    return b == a.n_seqs ? total : first * a.nkv + (i - b * a.nkv) * (first_tile[b + 1] - first);
+  };
   auto cta_of = [&](int t) { const int big = rem * (base + 1); return t < big ? t / (base + 1) : rem + (t - big) / base; };
   AttnWalk walk(first_tile, a.n_seqs, a.nkv, begin_of(cta), begin_of(cta + 1));
   int stage = 0;
