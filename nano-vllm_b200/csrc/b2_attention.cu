@@ -116,7 +116,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   int* s_len = first_tile + a.n_seqs + 1;
   __shared__ float s_m[ATT_WARPS][ATT_ROWS], s_l[ATT_WARPS][ATT_ROWS];
   __shared__ __align__(8) uint64_t s_bars[2 * ATT_MAX_STAGES];
-  __shared__ int s_abort, s_last[2], s_most;
+  __shared__ int s_abort, s_last[2], s_most, s_live;
   volatile int* abort_flag = &s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t bar_full = b2::smem_u32(s_bars), bar_empty = bar_full + ATT_MAX_STAGES * 8;
@@ -137,18 +137,20 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   const int max_len = a.bt_width * a.block_size;
   if (warp == 0) {
     const int per = (a.n_seqs + 31) / 32, s0 = lane * per;
-    int mine = 0, most = 0;
+    int mine = 0, most = 0, live = 0;
 #pragma unroll 4
     for (int i = 0; i < per; ++i)
       if (s0 + i < a.n_seqs) {
         const int len = max(0, min(__ldg(a.lens + s0 + i), max_len));
-        const int t = max(1, (len + ATT_TILE - 1) / ATT_TILE);  // a padded row has one tile too: its output is zero
+        const int t = (len + ATT_TILE - 1) / ATT_TILE;
         s_len[s0 + i] = len;
         first_tile[s0 + i + 1] = t;
         mine += t;
         most = max(most, t);
+        if (t > 0) live = s0 + i + 1;
       }
     most = __reduce_max_sync(0xffffffffu, most);
+    live = __reduce_max_sync(0xffffffffu, live);
     int incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -159,14 +161,24 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     if (lane == 0) {
       first_tile[0] = 0;
       s_most = most;
+      s_live = live;
     }
     for (int i = 0; i < per; ++i)
       if (s0 + i < a.n_seqs) first_tile[s0 + i + 1] = at += first_tile[s0 + i + 1];
   }
   __syncthreads();
+  // rows without a context (a graph's padded ones) have no tiles; their output is zero
+  if (warp < ATT_WARPS)
+    for (int b = blockIdx.x; b < a.n_seqs; b += gridDim.x)
+      if (s_len[b] == 0) {
+        b2::pdl_wait();
+        const int row = a.nkv * a.group * ATT_HD;
+        for (int i = tid * 8; i < row; i += ATT_WARPS * 32 * 8) *reinterpret_cast<uint4*>(a.out + static_cast<int64_t>(b) * row + i) = make_uint4(0, 0, 0, 0);
+      }
   const int total = first_tile[a.n_seqs] * a.nkv;
+  if (total == 0) return;
   // (parts of an item are fewer, and no CTA has more tiles, when as many CTAs as need be take the same number of them)
-  const int cta = blockIdx.x, items = a.n_seqs * a.nkv, cap = static_cast<int>(gridDim.x);
+  const int cta = blockIdx.x, items = s_live * a.nkv, cap = static_cast<int>(gridDim.x);
   const int per = (total + cap - 1) / cap;
   const int spread = per <= 8 ? (total + per - 1) / per : cap;
   const bool by_item = items <= cap && s_most <= total / spread + ATT_COMBINE_TILES;
@@ -176,7 +188,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   auto begin_of = [&](int i) {
     if (!by_item) return i * base + min(i, rem);
     const int b = i / a.nkv, first = first_tile[b];
-    return b == a.n_seqs ? total : first * a.nkv + (i - b * a.nkv) * (first_tile[b + 1] - first);
+    return b >= s_live ? total : first * a.nkv + (i - b * a.nkv) * (first_tile[b + 1] - first);
   };
   auto cta_of = [&](int t) { const int big = rem * (base + 1); return t < big ? t / (base + 1) : rem + (t - big) / base; };
   AttnWalk walk(first_tile, a.n_seqs, a.nkv, begin_of(cta), begin_of(cta + 1));
@@ -209,7 +221,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             b2::tma_load_2d(dst + 2 * ATT_HALF_BYTES, &tmV, fb, x, y, b2::kEvictFirst);
             b2::tma_load_2d(dst + 3 * ATT_HALF_BYTES, &tmV, fb, x + 64, y, b2::kEvictFirst);
           } else {
-            const int groups = (left + 15) >> 4;  // none for a padded row
+            const int groups = (left + 15) >> 4;
             b2::mbar_arrive_expect_tx(fb, groups * (ATT_STAGE_BYTES / 4));
             for (int i = 0; i < groups; ++i) {
               const uint32_t d = dst + i * 16 * 128;

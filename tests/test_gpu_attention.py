@@ -22,7 +22,9 @@ def rt(pkg):
 CASES = [((1,), 16, 8), ((63, 64, 65, 0, 15, 16, 17), 16, 8), ((255, 256, 257, 0), 16, 8), ((4096,), 2, 1), ((4000, 3), 8, 8), ((300,), 8, 8),
          (tuple(range(1, 620, 7)), 8, 4), ((700,) * 130, 2, 1),
          # dealt whole or cut: the longest item just within and just past the limit, as many items as CTAs and one sequence more, equal counts
-         ((576,), 16, 8), ((577,), 16, 8), (tuple(range(40, 706, 18)), 16, 8), (tuple(range(40, 724, 18)), 16, 8), ((3000,), 16, 8)]
+         ((576,), 16, 8), ((577,), 16, 8), (tuple(range(40, 706, 18)), 16, 8), (tuple(range(40, 724, 18)), 16, 8), ((3000,), 16, 8),
+         # rows without a context at the end, between others, alone
+         (tuple(range(40, 706, 18)) + (0,) * 11, 16, 8), ((0, 300, 0, 0, 900, 0), 16, 8), ((0, 0), 16, 8), ((700,) * 60 + (0,) * 4, 8, 8)]
 
 
 @pytest.mark.parametrize("lens,nq,nkv", CASES)
