@@ -653,6 +653,11 @@ int b2_qk_norm_rope_store(void* qkv, int64_t ld_qkv, int M, int nq, int nkv, int
   if (!qkv || !positions || !cos_sin || ld_qkv < static_cast<int64_t>(nq + 2 * nkv) * head_dim || ld_qkv % 8 != 0) return B2_ERR_ARG;
   if ((q_norm_w == nullptr) != (k_norm_w == nullptr)) return B2_ERR_ARG;
   if (k_cache != nullptr && (!v_cache || !slot_mapping)) return B2_ERR_ARG;
+  // the widest accesses of a lane: 2 elements of a q or k head's halves and 4 of a V row, half of that where head_dim is 64
+  const auto on = [](const void* p, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
+  const uintptr_t unit = head_dim / 32;
+  if (!on(qkv, k_cache != nullptr ? 2 * unit : unit) || !on(k_cache, unit) || !on(v_cache, 2 * unit) || !on(cos_sin, 4) || !on(q_norm_w, 2) || !on(k_norm_w, 2))
+    return B2_ERR_ARG;
   const int64_t warps = static_cast<int64_t>(M) * (nq + 2 * nkv);
   const int grid = static_cast<int>((warps + 7) / 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream);

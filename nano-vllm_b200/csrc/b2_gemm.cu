@@ -2291,7 +2291,8 @@ int b2_qkv_fused(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t
   args.C = static_cast<uint16_t*>(qkv);
   args.ldc = ld_qkv;
   args.bias = static_cast<const uint16_t*>(bias);
-  if (head_dim == 128) {  // one head per 128-feature tile: the cluster kernel can finish the heads itself
+  // one head per 128-feature tile: the GEMM can finish the heads itself (of more than 64 tokens in 16-byte vectors)
+  if (head_dim == 128 && (M <= 64 || (aligned16(q_norm_w) && aligned16(k_norm_w) && aligned16(cos_sin) && aligned16(k_cache) && aligned16(v_cache)))) {
     args.qkv_fused = 1;
     args.nq = nq;
     args.nkv = nkv;

@@ -91,6 +91,22 @@ __device__ __forceinline__ void quad_meets(int part) {
   if (part == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
   else asm volatile("bar.sync 2, 128;" ::: "memory");
 }
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  f[0] = b2::bf16_lo(v.x); f[1] = b2::bf16_hi(v.x); f[2] = b2::bf16_lo(v.y); f[3] = b2::bf16_hi(v.y);
+  f[4] = b2::bf16_lo(v.z); f[5] = b2::bf16_hi(v.z); f[6] = b2::bf16_lo(v.w); f[7] = b2::bf16_hi(v.w);
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(b2::pack_bf16(f[0], f[1]), b2::pack_bf16(f[2], f[3]), b2::pack_bf16(f[4], f[5]), b2::pack_bf16(f[6], f[7]));
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 v = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// bf16(bf16(x * rstd) * w)
+__device__ __forceinline__ uint4 normed(const float (&x)[8], float rstd, const uint4& w) {
+  return make_uint4(mul_bf16x2(b2::pack_bf16(x[0] * rstd, x[1] * rstd), w.x), mul_bf16x2(b2::pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
+                    mul_bf16x2(b2::pack_bf16(x[4] * rstd, x[5] * rstd), w.z), mul_bf16x2(b2::pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
+}
 // token t of a staging buffer of head rows: 16 pieces of 16 bytes, piece index XORed with the token so that neither the
 // transposing stores nor the row reads meet in a bank
 __device__ __forceinline__ uint32_t staged(int token, int piece) { return token * (FM * 2) + ((piece ^ (token & 7)) << 4); }
@@ -498,34 +514,36 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
     } else {
       // qkv projection: this CTA's 128 features are one head.  q: norm and rotation; k: the same, and into the cache; v: into
-      // the cache.  Four warps share a staging buffer of whole head rows; a warp finishes every fourth token's row, lane l
-      // holding dimensions (2l, 2l + 1) of both halves, four rows at a time so that their reductions overlap.  Arithmetic and
-      // roundings are those of qk_norm_rope_store_kernel.
+      // the cache.  Four warps share a staging buffer of whole head rows; a warp finishes four tokens' rows at a time, 8 lanes a
+      // row with 8 dimensions of either half each, so that every access is a 16-byte vector and a norm takes three exchanges (a
+      // row per warp in 4-byte accesses was bound by its memory instructions and exchanges: 97 -> 77 us at 8000 tokens x 4096 x 1024, plain stores 54).
+      // Arithmetic, order of the sums and roundings are those of qk_norm_rope_store_kernel: a lane's four partial sums are what
+      // four of its lanes hold.
       const bool rotated = head < a.nq + a.nkv;
-      float nw[4] = {1.f, 1.f, 1.f, 1.f};
+      const int row4 = lane >> 3, pc = lane & 7;
+      uint4 nw1 = make_uint4(0, 0, 0, 0), nw2 = nw1;
       const uint16_t* norm = rotated ? (head < a.nq ? a.q_norm_w : a.k_norm_w) : nullptr;
       uint16_t* cache = nullptr;
       if (head >= a.nq && a.k_cache != nullptr) cache = rotated ? a.k_cache + (head - a.nq) * FM : a.v_cache + (head - a.nq - a.nkv) * FM;
       if (norm != nullptr) {
-        const uint32_t w1 = *reinterpret_cast<const uint32_t*>(norm + lane * 2), w2 = *reinterpret_cast<const uint32_t*>(norm + 64 + lane * 2);
-        nw[0] = b2::bf16_lo(w1); nw[1] = b2::bf16_hi(w1); nw[2] = b2::bf16_lo(w2); nw[3] = b2::bf16_hi(w2);
+        nw1 = *reinterpret_cast<const uint4*>(norm + pc * 8);
+        nw2 = *reinterpret_cast<const uint4*>(norm + 64 + pc * 8);
       }
       const int own = (g1 - g0) * 8;
-      float2 cs[4], sn[4];  // rotary factors and cache slots of the next four rows travel while these four are finished
-      int slot[4];
-      auto ahead = [&](int row0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = min(row0 + 4 * i, own - 1);
-          if (cache != nullptr) slot[i] = __ldg(a.slots + min(tok0 + g0 * 8 + row, a.M - 1));
-          if (rotated) {
-            const float* f = a.cos_sin + static_cast<int64_t>(s_pos[row]) * FM + lane * 2;
-            cs[i] = __ldg(reinterpret_cast<const float2*>(f));
-            sn[i] = __ldg(reinterpret_cast<const float2*>(f + 64));
-          }
+      float4 factors[4];  // rotary factors (cosines, sines) and cache slot of the next row travel while this one is finished
+      int slot = -1;
+      auto ahead = [&](int row) {
+        row = min(row, own - 1);
+        if (cache != nullptr) slot = __ldg(a.slots + min(tok0 + g0 * 8 + row, a.M - 1));
+        if (rotated) {
+          const float4* f = reinterpret_cast<const float4*>(a.cos_sin + static_cast<int64_t>(s_pos[row]) * FM + pc * 8);
+          factors[0] = __ldg(f);
+          factors[1] = __ldg(f + 1);
+          factors[2] = __ldg(f + 16);
+          factors[3] = __ldg(f + 17);
         }
       };
-      if (first_g < g1) ahead((first_g - g0) * 8 + qw);
+      if (first_g < g1) ahead((first_g - g0) * 8 + qw * 4 + row4);
       for (int g = first_g; g < g1; g += STEP) {
         uint32_t out[4][4];
         finish(g, out);
@@ -538,55 +556,47 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const int live = ok ? min(own, a.M - tok0 - g0 * 8) - (g - g0) * 8 : 0;
 #pragma unroll
         for (int i0 = 0; i0 < 32; i0 += 16) {
-          float x[4][4];
-          uint32_t lo[4], hi[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int lt = qw + i0 + 4 * i;
-            lo[i] = *reinterpret_cast<const uint32_t*>(stg + staged(lt, lane >> 2) + (lane & 3) * 4);
-            hi[i] = *reinterpret_cast<const uint32_t*>(stg + staged(lt, 8 + (lane >> 2)) + (lane & 3) * 4);
-            x[i][0] = b2::bf16_lo(lo[i]); x[i][1] = b2::bf16_hi(lo[i]); x[i][2] = b2::bf16_lo(hi[i]); x[i][3] = b2::bf16_hi(hi[i]);
-          }
+          const int lt = i0 + qw * 4 + row4;
+          uint4 lo = *reinterpret_cast<const uint4*>(stg + staged(lt, pc)), hi = *reinterpret_cast<const uint4*>(stg + staged(lt, 8 + pc));
           if (rotated) {
+            float x1[8], x2[8];
+            unpack8(lo, x1);
+            unpack8(hi, x2);
             if (norm != nullptr) {
               float ss[4];
 #pragma unroll
-              for (int i = 0; i < 4; ++i) ss[i] = (x[i][0] * x[i][0] + x[i][2] * x[i][2]) + (x[i][1] * x[i][1] + x[i][3] * x[i][3]);
+              for (int k = 0; k < 4; ++k) ss[k] = (x1[2 * k] * x1[2 * k] + x2[2 * k] * x2[2 * k]) + (x1[2 * k + 1] * x1[2 * k + 1] + x2[2 * k + 1] * x2[2 * k + 1]);
 #pragma unroll
-              for (int o = 16; o > 0; o >>= 1)
+              for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float rstd = rsqrtf(ss[i] / 128.0f + a.qk_eps);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) x[i][e] = b2::bf16_round(b2::bf16_round(x[i][e] * rstd) * nw[e]);
-              }
+                for (int k = 0; k < 4; ++k) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
+              const float rstd = rsqrtf(((ss[0] + ss[2]) + (ss[1] + ss[3])) / 128.0f + a.qk_eps);
+              // (a product of two bf16 values has one rounding to bf16 either way)
+              lo = normed(x1, rstd, nw1);
+              hi = normed(x2, rstd, nw2);
+              unpack8(lo, x1);
+              unpack8(hi, x2);
             }
+            const float* c = reinterpret_cast<const float*>(factors);
+            float y1[8], y2[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float2 c = cs[i], n = sn[i];
-              // separate roundings of the products, as the eager reference computes them
-              lo[i] = b2::pack_bf16(__fsub_rn(__fmul_rn(x[i][0], c.x), __fmul_rn(x[i][2], n.x)), __fsub_rn(__fmul_rn(x[i][1], c.y), __fmul_rn(x[i][3], n.y)));
-              hi[i] = b2::pack_bf16(__fadd_rn(__fmul_rn(x[i][2], c.x), __fmul_rn(x[i][0], n.x)), __fadd_rn(__fmul_rn(x[i][3], c.y), __fmul_rn(x[i][1], n.y)));
+            for (int e = 0; e < 8; ++e) {  // separate roundings of the products, as the eager reference computes them
+              y1[e] = __fsub_rn(__fmul_rn(x1[e], c[e]), __fmul_rn(x2[e], c[8 + e]));
+              y2[e] = __fadd_rn(__fmul_rn(x2[e], c[e]), __fmul_rn(x1[e], c[8 + e]));
             }
+            lo = pack8(y1);
+            hi = pack8(y2);
           }
-          int to_slot[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) to_slot[i] = cache != nullptr ? slot[i] : -1;
-          ahead((g - g0 + (i0 == 0 ? 0 : STEP)) * 8 + (i0 ^ 16) + qw);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int lt = qw + i0 + 4 * i;
-            if (lt < live) {
-              uint16_t* dst = a.C + static_cast<int64_t>(tok0 + g * 8 + lt) * a.ldc + f0 + lane * 2;
-              *reinterpret_cast<uint32_t*>(dst) = lo[i];
-              *reinterpret_cast<uint32_t*>(dst + 64) = hi[i];
-              if (to_slot[i] >= 0) {
-                uint16_t* to = cache + static_cast<int64_t>(to_slot[i]) * a.nkv * FM + lane * 2;
-                *reinterpret_cast<uint32_t*>(to) = lo[i];
-                *reinterpret_cast<uint32_t*>(to + 64) = hi[i];
-              }
+          const int to_slot = cache != nullptr ? slot : -1;
+          ahead((g - g0 + (i0 == 0 ? 0 : STEP)) * 8 + (i0 ^ 16) + qw * 4 + row4);
+          if (lt < live) {
+            uint16_t* dst = a.C + static_cast<int64_t>(tok0 + g * 8 + lt) * a.ldc + f0 + pc * 8;
+            *reinterpret_cast<uint4*>(dst) = lo;
+            *reinterpret_cast<uint4*>(dst + 64) = hi;
+            if (to_slot >= 0) {
+              uint16_t* to = cache + static_cast<int64_t>(to_slot) * a.nkv * FM + pc * 8;
+              *reinterpret_cast<uint4*>(to) = lo;
+              *reinterpret_cast<uint4*>(to + 64) = hi;
             }
           }
         }

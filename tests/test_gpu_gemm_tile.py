@@ -78,3 +78,30 @@ def test_silu_epilogue(rt, m):
     rt.check_status()
     ref = O.silu_and_mul(torch.cat([O.linear(x, w[0::2]), O.linear(x, w[1::2])], dim=-1))
     assert ulp_mismatch_fraction(got, ref, 2) < 2e-2
+
+
+@pytest.mark.parametrize("m", [65, 300, 513])
+def test_qkv_with_operands_off_the_16_byte_grid(rt, m):
+    """Norm weights, rotary table and caches that no 16-byte vector can read: the heads are finished by the head kernel."""
+    from nanovllm_b200 import ops
+    nq, nkv, hd, k = 4, 2, 128, 512
+    g = torch.Generator(device=DEV).manual_seed(m)
+    x = torch.empty(m, k, device=DEV).normal_(generator=g).bfloat16()
+    w = torch.empty((nq + 2 * nkv) * hd, k, device=DEV).normal_(0, 0.05, generator=g).bfloat16()
+    pos = torch.randint(0, 512, (m,), device=DEV, generator=g)
+    slots = torch.randperm(768, device=DEV, generator=g)[:m].to(torch.int32)
+    tables = (O.rope_cache(hd, 512, 1e6).to(DEV), (torch.rand(2, hd, device=DEV, generator=g) + 0.5).bfloat16())
+    outs = []
+    for off in (0, 8):  # bytes
+
+        def shifted(t):
+            n = off // t.element_size()
+            return torch.empty(t.numel() + 8, dtype=t.dtype, device=DEV)[n:n + t.numel()].view(t.shape).copy_(t)
+
+        table, qw, kw = shifted(tables[0]), shifted(tables[1][0]), shifted(tables[1][1])
+        kc, vc = (shifted(torch.zeros(3, 256, nkv, hd, dtype=torch.bfloat16, device=DEV)) for _ in range(2))
+        outs.append((ops.qkv_fused(x, w, None, nq, nkv, hd, qw, kw, 1e-6, pos, table, kc, vc, slots), kc, vc))
+    torch.cuda.synchronize()
+    rt.check_status()
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
