@@ -214,3 +214,31 @@ def test_token_parity_qwen3_0_6b_shape(pkg, temperature):
         assert r["same"] >= 0.95 * r["n"], f"fewer than 95 % of the positions are identical: {r}"
     finally:
         runner.exit()
+
+
+@pytest.mark.parametrize("n", [256, 257, 270])
+def test_sampling_of_more_rows_than_one_call_takes(pkg, n):
+    """Prefill and decode of batches around the fused sampler's 256 rows: every row's greedy token has the row's largest logit."""
+    ensure_group()
+    from nanovllm_b200.engine.model_runner import ModelRunner, Seq, sequential_block_tables
+    _attention_backend()
+    runner = ModelRunner(_config(SHAPE), max_num_seqs=272, max_model_len=256, max_num_batched_tokens=1024, num_kvcache_blocks=272,
+                         oneshot_tokens=256, full_weights=O.init_full_weights(SHAPE, seed=31))
+    try:
+        g = torch.Generator().manual_seed(n)
+        tables = sequential_block_tables([256] * n, 256)
+        seqs = [Seq(torch.randint(0, SHAPE.vocab, (1 + i % 3,), generator=g).tolist(), bt) for i, bt in enumerate(tables)]
+        for is_prefill in (True, False):
+            tokens = torch.tensor(runner.step(seqs, is_prefill))
+            if is_prefill:
+                logits = runner.run_model(*runner.prepare_prefill(seqs), True)
+            else:
+                logits = runner.model.compute_logits(runner.graph_vars["outputs"][:n])
+            logits = logits[:n].float().cpu()
+            best = logits.max(-1).values
+            assert (logits.gather(1, tokens[:, None])[:, 0] >= best - 2e-2 - 1e-2 * best.abs()).all()
+            assert (tokens == logits.argmax(-1)).float().mean() > 0.9
+            for s, t in zip(seqs, tokens.tolist()):
+                s.token_ids.append(t)
+    finally:
+        runner.exit()
