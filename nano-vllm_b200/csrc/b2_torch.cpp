@@ -8,9 +8,12 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <algorithm>
+
 #include <ATen/Functions.h>
 #include <ATen/cuda/EmptyTensor.h>
-#include <c10/core/DeviceGuard.h>
+#include <c10/core/GradMode.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -304,15 +307,53 @@ PyObject* embed(Args a) {
   return wrap(out.view(shape));
 }
 
-// paged_attention(ctx, q, k_cache, v_cache, context_lens, block_tables, scale): None when the kernel does not serve the shape
+// ---- attention -----------------------------------------------------------------
+// The kernels read lengths, tables, keys and values through raw pointers.  What makes a call not theirs (head layout, strides,
+// alignment) is left to the caller's general path; what is wrong with it is an error here, before anything is launched.
+void same_device(const at::Tensor& t, const at::Tensor& q, const char* what) {
+  if (t.device() != q.device()) raise(PyExc_TypeError, "%s is on %s, the query on %s", what, t.device().str().c_str(), q.device().str().c_str());
+}
+void on_current_gpu(const at::Tensor& q, const char* what) {
+  if (!q.is_cuda() || q.device().index() != c10::cuda::current_device()) raise(PyExc_TypeError, "%s: expected a tensor on the current GPU, got %s", what, q.device().str().c_str());
+}
+void int32_vector(const at::Tensor& t, int64_t n, const char* what) {
+  if (t.dim() != 1 || t.size(0) != n) raise(PyExc_ValueError, "%s: expected %lld elements, got %lld in %lld dimensions", what, (long long)n, (long long)t.numel(), (long long)t.dim());
+  expect(t.scalar_type() == at::kInt && t.is_contiguous(), "lengths must be contiguous int32");
+}
+void block_table_rows(const at::Tensor& t, int64_t n) {
+  if (t.size(0) != n) raise(PyExc_ValueError, "block_tables: %lld rows for %lld sequences", (long long)t.size(0), (long long)n);
+  expect(t.scalar_type() == at::kInt, "int32 block tables");
+}
+void values_like_keys(const at::Tensor& k, const at::Tensor& v, int64_t hd) {
+  if (k.size(-1) != hd) raise(PyExc_ValueError, "keys have head dimension %lld, the query %lld", (long long)k.size(-1), (long long)hd);
+  if (v.sizes() != k.sizes()) raise(PyExc_ValueError, "keys and values differ in shape");
+  if (k.scalar_type() != at::kBFloat16 || v.scalar_type() != at::kBFloat16)
+    raise(PyExc_TypeError, "expected bf16 keys and values, got %s and %s", c10::toString(k.scalar_type()), c10::toString(v.scalar_type()));
+}
+bool on_16_bytes(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0; }
+// rows of `heads` heads side by side that the kernels' vector loads and tensor maps can address
+bool row_layout(const at::Tensor& t, int64_t heads, int64_t hd) {
+  return t.stride(-1) == 1 && t.stride(-2) == hd && on_16_bytes(t) && (t.size(0) <= 1 || (t.stride(0) % 8 == 0 && t.stride(0) >= heads * hd));
+}
+bool table_layout(const at::Tensor& t) { return t.dim() == 2 && t.size(1) > 0 && t.stride(1) == 1 && (t.size(0) <= 1 || t.stride(0) >= t.size(1)); }
+
+// paged_attention(ctx, q, k_cache, v_cache, context_lens, block_tables, scale): None when the kernel does not serve the call
 PyObject* paged_attention(Args a) {
   const at::Tensor &q = tensor(a[1], "q"), &kc = tensor(a[2], "k_cache"), &vc = tensor(a[3], "v_cache"), &lens = tensor(a[4], "context_lens"),
                    &tables = tensor(a[5], "block_tables");
+  if (q.dim() != 3 || kc.dim() != 4) Py_RETURN_NONE;
   const int64_t n = q.size(0), nq = q.size(1), hd = q.size(2), nkv = kc.size(2), bs = kc.size(1);
-  if (!b2_paged_attention_supported(n, nq, nkv, hd, bs) || q.scalar_type() != at::kBFloat16 || q.stride(2) != 1 || q.stride(1) != hd || !kc.is_contiguous() ||
-      !vc.is_contiguous() || tables.stride(1) != 1)
+  if (!b2_paged_attention_supported(n, nq, nkv, hd, bs) || q.scalar_type() != at::kBFloat16 || !row_layout(q, nq, hd) || kc.size(0) == 0 ||
+      !kc.is_contiguous() || !vc.is_contiguous() || !on_16_bytes(kc) || !on_16_bytes(vc) || !table_layout(tables))
     Py_RETURN_NONE;
-  expect(lens.scalar_type() == at::kInt && tables.scalar_type() == at::kInt && kc.scalar_type() == at::kBFloat16, "int32 lengths and block tables, bf16 cache");
+  values_like_keys(kc, vc, hd);
+  int32_vector(lens, n, "context_lens");
+  block_table_rows(tables, n);
+  on_current_gpu(q, "q");
+  same_device(kc, q, "k_cache");
+  same_device(vc, q, "v_cache");
+  same_device(lens, q, "context_lens");
+  same_device(tables, q, "block_tables");
   const at::Tensor out = at::detail::empty_cuda({n, nq, hd}, at::kBFloat16, q.device(), std::nullopt);
   check(b2_paged_attention_decode(context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, kc.data_ptr(), vc.data_ptr(), kc.size(0), bs, tables.const_data_ptr<int32_t>(),
                                   n > 1 ? tables.stride(0) : tables.size(1), tables.size(1), lens.const_data_ptr<int32_t>(), n, nq, nkv, hd, number(a[6]),
@@ -320,23 +361,36 @@ PyObject* paged_attention(Args a) {
   return wrap(out);
 }
 
-// prefill_attention(ctx, q, k, v, cu_q, cu_k, max_q, block_tables, scale): None when the kernel does not serve the shape.
+// prefill_attention(ctx, q, k, v, cu_q, cu_k, max_q, block_tables, scale): None when the kernel does not serve the call.
 // k, v: [rows, nkv, head_dim], or the caches when block_tables is given
 PyObject* prefill_attention(Args a) {
   const at::Tensor &q = tensor(a[1], "q"), &k = tensor(a[2], "k"), &v = tensor(a[3], "v"), &cu_q = tensor(a[4], "cu_seqlens_q"), &cu_k = tensor(a[5], "cu_seqlens_k");
   const at::Tensor tables = optional_tensor(a[7], "block_tables");
   const bool paged = tables.defined();
-  const int64_t n = q.size(0), nq = q.size(1), hd = q.size(2), nkv = k.size(-2), bs = paged ? k.size(1) : 0;
-  if (!b2_prefill_attention_supported(nq, nkv, hd, bs) || q.scalar_type() != at::kBFloat16 || k.scalar_type() != at::kBFloat16 || q.stride(2) != 1 || q.stride(1) != hd ||
-      k.stride(-1) != 1 || k.stride(-2) != hd || v.strides() != k.strides() || k.dim() != (paged ? 4 : 3) || (paged && (!k.is_contiguous() || tables.stride(1) != 1)))
+  if (q.dim() != 3 || k.dim() != (paged ? 4 : 3)) Py_RETURN_NONE;
+  const int64_t n = q.size(0), nq = q.size(1), hd = q.size(2), nkv = k.size(-2), bs = paged ? k.size(1) : 0, rows = paged ? k.size(0) * bs : k.size(0);
+  if (!b2_prefill_attention_supported(nq, nkv, hd, bs) || q.scalar_type() != at::kBFloat16 || k.scalar_type() != at::kBFloat16 || !row_layout(q, nq, hd) || rows == 0 ||
+      rows > (1 << 30) || cu_q.numel() > 65536 || v.strides() != k.strides() || !on_16_bytes(v))
     Py_RETURN_NONE;
-  expect(cu_q.scalar_type() == at::kInt && cu_k.scalar_type() == at::kInt && (!paged || tables.scalar_type() == at::kInt), "int32 lengths and block tables");
+  if (paged ? !k.is_contiguous() || !on_16_bytes(k) || !table_layout(tables) : !row_layout(k, nkv, hd)) Py_RETURN_NONE;
+  if (c10::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) Py_RETURN_NONE;  // (forward only)
+  const int64_t n_seqs = cu_q.numel() - 1, max_q = integer(a[6]);
+  values_like_keys(k, v, hd);
+  int32_vector(cu_q, std::max<int64_t>(1, n_seqs + 1), "cu_seqlens_q");
+  int32_vector(cu_k, n_seqs + 1, "cu_seqlens_k");
+  if (paged) block_table_rows(tables, n_seqs);
+  if (n > 0 && (n_seqs < 1 || max_q < 1)) raise(PyExc_ValueError, "%lld query tokens in %lld sequences of at most %lld", (long long)n, (long long)n_seqs, (long long)max_q);
+  on_current_gpu(q, "q");
+  same_device(k, q, "k");
+  same_device(v, q, "v");
+  same_device(cu_q, q, "cu_seqlens_q");
+  same_device(cu_k, q, "cu_seqlens_k");
+  if (paged) same_device(tables, q, "block_tables");
   const at::Tensor out = at::detail::empty_cuda({n, nq, hd}, at::kBFloat16, q.device(), std::nullopt);
-  const int64_t n_seqs = cu_q.numel() - 1, rows = paged ? k.size(0) * bs : k.size(0);
   if (n)
     check(b2_prefill_attention(context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, k.data_ptr(), v.data_ptr(), paged || rows == 1 ? nkv * hd : k.stride(0), rows,
                                paged ? tables.const_data_ptr<int32_t>() : nullptr, paged ? (n_seqs > 1 ? tables.stride(0) : tables.size(1)) : 0, paged ? tables.size(1) : 0, bs,
-                               cu_q.const_data_ptr<int32_t>(), cu_k.const_data_ptr<int32_t>(), n_seqs, integer(a[6]), n, nq, nkv, hd, number(a[8]), out.data_ptr(), stream()),
+                               cu_q.const_data_ptr<int32_t>(), cu_k.const_data_ptr<int32_t>(), n_seqs, max_q, n, nq, nkv, hd, number(a[8]), out.data_ptr(), stream()),
           "b2_prefill_attention");
   return wrap(out);
 }

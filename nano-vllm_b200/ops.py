@@ -128,15 +128,16 @@ def embed(ids: torch.Tensor, w: torch.Tensor, vocab_start: int, vocab_end: int, 
 def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, context_lens: torch.Tensor, block_tables: torch.Tensor,
                     scale: float) -> torch.Tensor | None:
     """Decode attention: one query token per sequence, q [n, nq, head_dim], over the paged cache.  None when the
-    kernel does not serve the shape (head_dim other than 128, more than 2 query heads per KV head)."""
+    kernel does not serve the call (head_dim other than 128, more than 2 query heads per KV head, a layout it cannot address);
+    operands that do not fit each other, or are not on one GPU, raise."""
     return _native.paged_attention(get_runtime().handle, q, k_cache, v_cache, context_lens, block_tables, scale)
 
 
 def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.Tensor, max_seqlen_q: int,
                       block_tables: torch.Tensor | None, scale: float) -> torch.Tensor | None:
     """Causal attention of q [tokens, nq, head_dim] over k, v [tokens, nkv, head_dim], or over the paged caches when
-    block_tables is given.  None when the kernel does not serve the shape (it takes head_dim 128 and two query heads per
-    KV head)."""
+    block_tables is given.  None when the kernel does not serve the call (it takes head_dim 128, two query heads per
+    KV head, forward only); operands that do not fit each other, or are not on one GPU, raise."""
     return _native.prefill_attention(get_runtime().handle, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, block_tables, scale)
 
 
