@@ -687,8 +687,9 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         }
         tmem_st_32x16(t_s + c * 16, p);  // columns this row has read already
       }
-      if (h == 0 && a.tables != nullptr && (j + 1) * PF_KEYS > kv_len) {
-        // rows of the cache past the context's end may hold anything: they count as zero
+      if (h == 0 && (j + 1) * PF_KEYS > kv_len) {
+        // Rows past the sequence's last key count as zero: in the cache they may hold anything, in a matrix they are the next
+        // sequence's, and a probability of zero times Inf or NaN is NaN.
         ok = b2::mbar_wait(v_full + (j & 1) * 8, (j >> 1) & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_FULL) && ok;
         if (j * PF_KEYS + row >= kv_len) {
           unsigned char* v = smem + (s_v - s_q) + (j & 1) * PF_TILE + row * 128;

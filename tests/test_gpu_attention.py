@@ -109,3 +109,22 @@ def test_prefill_attention_against_fp32(rt, seqs, paged):
     torch.cuda.synchronize()
     rt.check_status()
     assert_close_bf16(got, ref, f"prefill attention {seqs}")
+
+
+def test_prefill_does_not_see_the_next_sequence(rt):
+    """Rows past a sequence's last key are its neighbour's: their values, whatever they are, must not reach it."""
+    from nanovllm_b200 import ops
+    nq, nkv, hd = 4, 2, 128
+    g = torch.Generator(device=DEV).manual_seed(5)
+    lens = [100, 60, 129, 40]  # every one ends inside a block of 128 keys
+    t = sum(lens)
+    q, k, v = (torch.empty(t, h, hd, device=DEV).normal_(generator=g).bfloat16() for h in (nq, nkv, nkv))
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    clean = ops.prefill_attention(q, k, v, cu, cu, max(lens), None, hd ** -0.5)
+    k[100:160], v[100:160] = float("nan"), float("inf")  # the second sequence
+    q[289:], k[289:], v[289:] = float("inf"), float("-inf"), float("nan")  # and the fourth
+    got = ops.prefill_attention(q, k, v, cu, cu, max(lens), None, hd ** -0.5)
+    torch.cuda.synchronize()
+    rt.check_status()
+    for a, b in ((0, 100), (160, 289)):
+        assert torch.equal(got[a:b], clean[a:b])
