@@ -20,7 +20,7 @@ std::atomic<int64_t> g_launches{0};
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn g_encode = nullptr;
+std::atomic<EncodeTiledFn> g_encode{nullptr};
 
 __global__ void b2_fill_u32_kernel(uint32_t* p, size_t n, uint32_t v) {
   size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
@@ -54,7 +54,8 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 int encode_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld_elems,
                    uint32_t box_inner, uint32_t box_rows) {
-  if (g_encode == nullptr) {
+  EncodeTiledFn encode = g_encode.load(std::memory_order_acquire);
+  if (encode == nullptr) {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;
     cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
@@ -63,15 +64,16 @@ int encode_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t 
       snprintf(g_last_error, sizeof(g_last_error), "cuTensorMapEncodeTiled not available from the driver");
       return B2_ERR_CUDA;
     }
-    g_encode = reinterpret_cast<EncodeTiledFn>(fn);
+    encode = reinterpret_cast<EncodeTiledFn>(fn);
+    g_encode.store(encode, std::memory_order_release);
   }
   cuuint64_t dims[2] = {inner, rows};
   cuuint64_t strides[1] = {ld_elems * 2};  // bytes between rows
   cuuint32_t box[2] = {box_inner, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     snprintf(g_last_error, sizeof(g_last_error),
              "cuTensorMapEncodeTiled failed (%d): base=%p inner=%llu rows=%llu ld=%llu box=%ux%u", static_cast<int>(r), base,

@@ -43,6 +43,16 @@ void check(int rc, const char* what) {
   throw Raised{};
 }
 
+// One call of the library.  The GIL is released around it: a launch waits when the stream's queue is full, and other Python
+// threads have to go on meanwhile.  (Arguments are converted by the caller, with the GIL held; the library's error text is per thread.)
+template <class... P, class... A>
+void launch(const char* what, int (*f)(P...), A... args) {
+  PyThreadState* const state = PyEval_SaveThread();
+  const int rc = f(args...);
+  PyEval_RestoreThread(state);
+  check(rc, what);
+}
+
 // ---- arguments -----------------------------------------------------------------
 const at::Tensor& tensor(PyObject* o, const char* what) {
   if (!THPVariable_Check(o)) raise(PyExc_TypeError, "%s: expected a tensor, got %s", what, Py_TYPE(o)->tp_name);
@@ -122,7 +132,7 @@ PyObject* gemm(Args a) {
   const int64_t n = w.size(0);
   const at::Tensor out = empty_rows(in.rows, n, x);
   if (in.rows)
-    check(b2_gemm(context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), out.data_ptr(), n, in.rows, n, in.cols, stream()), "b2_gemm");
+    launch("b2_gemm", b2_gemm, context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), out.data_ptr(), n, in.rows, n, in.cols, stream());
   return wrap(leading(out, x, n));
 }
 
@@ -135,7 +145,7 @@ PyObject* gemm_silu_mul(Args a) {
   const int64_t n = w.size(0) / 2;
   const at::Tensor out = empty_rows(in.rows, n, x);
   if (in.rows)
-    check(b2_gemm_silu_mul(context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), out.data_ptr(), n, in.rows, n, in.cols, stream()), "b2_gemm_silu_mul");
+    launch("b2_gemm_silu_mul", b2_gemm_silu_mul, context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), out.data_ptr(), n, in.rows, n, in.cols, stream());
   return wrap(leading(out, x, n));
 }
 
@@ -169,8 +179,8 @@ PyObject* qkv_fused(Args a) {
   const Cache c = cache_of(kc, vc, sm, nkv * hd);
   const at::Tensor out = empty_rows(in.rows, n, x);
   if (in.rows)
-    check(b2_qkv_fused(context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), out.data_ptr(), n, in.rows, nq, nkv, hd, in.cols,
-                       ptr(qw), ptr(kw), number(a[9]), pos.const_data_ptr<int64_t>(), cs.const_data_ptr<float>(), c.k, c.v, c.slots, stream()), "b2_qkv_fused");
+    launch("b2_qkv_fused", b2_qkv_fused, context(a[0]), in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), out.data_ptr(), n, in.rows, nq, nkv, hd, in.cols,
+           ptr(qw), ptr(kw), number(a[9]), pos.const_data_ptr<int64_t>(), cs.const_data_ptr<float>(), c.k, c.v, c.slots, stream());
   return wrap(out);
 }
 
@@ -194,8 +204,8 @@ PyObject* rowpar_fused(Args a) {
   }
   const at::Tensor out = empty_rows(in.rows, n, x);
   if (in.rows)
-    check(b2_rowpar_fused(ctx, in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), in.rows, n, in.cols, ptr(residual), ptr(norm_w), number(a[6]),
-                          out.data_ptr(), ptr(res_out), stream()), "b2_rowpar_fused");
+    launch("b2_rowpar_fused", b2_rowpar_fused, ctx, in.t.data_ptr(), in.ld, w.data_ptr(), w.stride(0), ptr(bias), in.rows, n, in.cols, ptr(residual), ptr(norm_w),
+           number(a[6]), out.data_ptr(), ptr(res_out), stream());
   return norm_w.defined() ? wrap(out, res_out) : wrap(leading(out, x, n));
 }
 
@@ -206,12 +216,12 @@ PyObject* rmsnorm(Args a) {
   const int64_t dim = x.dim() > 0 ? x.size(-1) : 0;
   if (x.dim() == 3 && dim <= 256 && heads_in_rows(x)) {  // heads of q or k, read from the rows of the projection
     const at::Tensor out = at::detail::empty_cuda(x.sizes(), at::kBFloat16, x.device(), std::nullopt);
-    check(b2_head_rmsnorm(x.data_ptr(), x.stride(0), x.size(1), w.data_ptr(), number(a[2]), x.size(0), dim, out.data_ptr(), x.size(1) * dim, stream()), "b2_rmsnorm");
+    launch("b2_rmsnorm", b2_head_rmsnorm, x.data_ptr(), x.stride(0), x.size(1), w.data_ptr(), number(a[2]), x.size(0), dim, out.data_ptr(), x.size(1) * dim, stream());
     return wrap(out);
   }
   const Rows in = matrix(x, "rmsnorm input");
   const at::Tensor out = empty_rows(in.rows, in.cols, x);
-  check(b2_rmsnorm(in.t.data_ptr(), in.ld, w.data_ptr(), number(a[2]), in.rows, in.cols, out.data_ptr(), in.cols, stream()), "b2_rmsnorm");
+  launch("b2_rmsnorm", b2_rmsnorm, in.t.data_ptr(), in.ld, w.data_ptr(), number(a[2]), in.rows, in.cols, out.data_ptr(), in.cols, stream());
   return wrap(x.dim() == 2 ? out : out.view(x.sizes()));
 }
 
@@ -222,7 +232,7 @@ PyObject* add_rmsnorm(Args a) {
   const int64_t dim = x.size(-1), rows = x.numel() / dim;
   const at::Tensor out = at::detail::empty_cuda(x.sizes(), at::kBFloat16, x.device(), std::nullopt);
   const at::Tensor res_out = at::detail::empty_cuda(x.sizes(), at::kBFloat16, x.device(), std::nullopt);
-  check(b2_add_rmsnorm(x.data_ptr(), r.data_ptr(), tensor(a[2], "add_rmsnorm weight").data_ptr(), number(a[3]), rows, dim, out.data_ptr(), res_out.data_ptr(), stream()), "b2_add_rmsnorm");
+  launch("b2_add_rmsnorm", b2_add_rmsnorm, x.data_ptr(), r.data_ptr(), tensor(a[2], "add_rmsnorm weight").data_ptr(), number(a[3]), rows, dim, out.data_ptr(), res_out.data_ptr(), stream());
   return wrap(out, res_out);
 }
 
@@ -232,7 +242,7 @@ PyObject* silu_and_mul(Args a) {
   const Rows in = matrix(x, "silu_and_mul input");
   const int64_t n = in.cols / 2;
   const at::Tensor out = empty_rows(in.rows, n, x);
-  check(b2_silu_and_mul(in.t.data_ptr(), in.ld, in.rows, n, out.data_ptr(), stream()), "b2_silu_and_mul");
+  launch("b2_silu_and_mul", b2_silu_and_mul, in.t.data_ptr(), in.ld, in.rows, n, out.data_ptr(), stream());
   return wrap(leading(out, x, n));
 }
 
@@ -246,7 +256,7 @@ PyObject* store_kvcache(Args a) {
   expect(kc.stride(1) == d && vc.stride(1) == d, "cache rows must be contiguous");
   expect(sm.numel() == n, "one slot per token");
   expect(k.element_size() == 2 && kc.element_size() == 2 && sm.scalar_type() == at::kInt, "16-bit elements, int32 slots");
-  check(b2_store_kvcache(k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), kc.data_ptr(), vc.data_ptr(), sm.const_data_ptr<int32_t>(), n, d, stream()), "b2_store_kvcache");
+  launch("b2_store_kvcache", b2_store_kvcache, k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), kc.data_ptr(), vc.data_ptr(), sm.const_data_ptr<int32_t>(), n, d, stream());
   Py_RETURN_NONE;
 }
 
@@ -260,8 +270,8 @@ PyObject* qk_norm_rope_store(Args a) {
   expect(pos.scalar_type() == at::kLong && cs.scalar_type() == at::kFloat && cs.is_contiguous(), "positions must be int64, cos_sin contiguous fp32");
   const at::Tensor kc = optional_tensor(a[9], "k_cache"), vc = optional_tensor(a[10], "v_cache"), sm = optional_tensor(a[11], "slot_mapping");
   const Cache c = cache_of(kc, vc, sm, nkv * hd);
-  check(b2_qk_norm_rope_store(qkv.data_ptr(), qkv.stride(0), qkv.size(0), nq, nkv, hd, ptr(qw), ptr(kw), number(a[6]), pos.const_data_ptr<int64_t>(),
-                              cs.const_data_ptr<float>(), c.k, c.v, c.slots, stream()), "b2_qk_norm_rope_store");
+  launch("b2_qk_norm_rope_store", b2_qk_norm_rope_store, qkv.data_ptr(), qkv.stride(0), qkv.size(0), nq, nkv, hd, ptr(qw), ptr(kw), number(a[6]), pos.const_data_ptr<int64_t>(),
+         cs.const_data_ptr<float>(), c.k, c.v, c.slots, stream());
   Py_RETURN_NONE;
 }
 
@@ -287,8 +297,8 @@ PyObject* rope(Args a) {
   }
   const at::Tensor qo = at::detail::empty_cuda(tensor(a[1], "query").sizes(), at::kBFloat16, in[0].device(), std::nullopt);
   const at::Tensor ko = at::detail::empty_cuda(tensor(a[2], "key").sizes(), at::kBFloat16, in[1].device(), std::nullopt);
-  check(b2_rope(in[0].data_ptr(), ld[0], in[1].data_ptr(), ld[1], t, heads[0], heads[1], hd, pos.const_data_ptr<int64_t>(), cs.const_data_ptr<float>(),
-                qo.data_ptr(), ko.data_ptr(), stream()), "b2_rope");
+  launch("b2_rope", b2_rope, in[0].data_ptr(), ld[0], in[1].data_ptr(), ld[1], t, heads[0], heads[1], hd, pos.const_data_ptr<int64_t>(), cs.const_data_ptr<float>(),
+         qo.data_ptr(), ko.data_ptr(), stream());
   return wrap(qo, ko);
 }
 
@@ -300,7 +310,7 @@ PyObject* embed(Args a) {
   ids = ids.contiguous();
   const int64_t m = ids.numel(), h = w.size(1);
   const at::Tensor out = at::detail::empty_cuda({m, h}, w.scalar_type(), w.device(), std::nullopt);
-  check(b2_embed(context(a[0]), ids.const_data_ptr<int64_t>(), w.data_ptr(), integer(a[3]), integer(a[4]), m, h, out.data_ptr(), stream()), "b2_embed");
+  launch("b2_embed", b2_embed, context(a[0]), ids.const_data_ptr<int64_t>(), w.data_ptr(), integer(a[3]), integer(a[4]), m, h, out.data_ptr(), stream());
   if (ids.dim() == 1) return wrap(out);
   std::vector<int64_t> shape(ids.sizes().begin(), ids.sizes().end());
   shape.push_back(h);
@@ -355,9 +365,9 @@ PyObject* paged_attention(Args a) {
   same_device(lens, q, "context_lens");
   same_device(tables, q, "block_tables");
   const at::Tensor out = at::detail::empty_cuda({n, nq, hd}, at::kBFloat16, q.device(), std::nullopt);
-  check(b2_paged_attention_decode(context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, kc.data_ptr(), vc.data_ptr(), kc.size(0), bs, tables.const_data_ptr<int32_t>(),
-                                  n > 1 ? tables.stride(0) : tables.size(1), tables.size(1), lens.const_data_ptr<int32_t>(), n, nq, nkv, hd, number(a[6]),
-                                  out.data_ptr(), stream()), "b2_paged_attention_decode");
+  launch("b2_paged_attention_decode", b2_paged_attention_decode, context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, kc.data_ptr(), vc.data_ptr(), kc.size(0), bs,
+         tables.const_data_ptr<int32_t>(), n > 1 ? tables.stride(0) : tables.size(1), tables.size(1), lens.const_data_ptr<int32_t>(), n, nq, nkv, hd, number(a[6]),
+         out.data_ptr(), stream());
   return wrap(out);
 }
 
@@ -388,10 +398,9 @@ PyObject* prefill_attention(Args a) {
   if (paged) same_device(tables, q, "block_tables");
   const at::Tensor out = at::detail::empty_cuda({n, nq, hd}, at::kBFloat16, q.device(), std::nullopt);
   if (n)
-    check(b2_prefill_attention(context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, k.data_ptr(), v.data_ptr(), paged || rows == 1 ? nkv * hd : k.stride(0), rows,
-                               paged ? tables.const_data_ptr<int32_t>() : nullptr, paged ? (n_seqs > 1 ? tables.stride(0) : tables.size(1)) : 0, paged ? tables.size(1) : 0, bs,
-                               cu_q.const_data_ptr<int32_t>(), cu_k.const_data_ptr<int32_t>(), n_seqs, max_q, n, nq, nkv, hd, number(a[8]), out.data_ptr(), stream()),
-          "b2_prefill_attention");
+    launch("b2_prefill_attention", b2_prefill_attention, context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, k.data_ptr(), v.data_ptr(),
+           paged || rows == 1 ? nkv * hd : k.stride(0), rows, paged ? tables.const_data_ptr<int32_t>() : nullptr, paged ? (n_seqs > 1 ? tables.stride(0) : tables.size(1)) : 0, paged ? tables.size(1) : 0, bs,
+           cu_q.const_data_ptr<int32_t>(), cu_k.const_data_ptr<int32_t>(), n_seqs, max_q, n, nq, nkv, hd, number(a[8]), out.data_ptr(), stream());
   return wrap(out);
 }
 

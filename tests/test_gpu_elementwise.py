@@ -221,3 +221,35 @@ def test_head_norm_and_rotation_of_projection_views(ops, t, nq, nkv, hd):
         ops.qk_norm_rope_store(plain, nq, nkv, hd, None, None, 0.0, pos, table, None, None, None)
         assert torch.equal(torch.cat([a.reshape(t, -1), b.reshape(t, -1)], -1), plain[:, :(nq + nkv) * hd])
         assert torch.equal(rows, before)
+
+
+def test_other_threads_run_while_a_launch_waits(ops):
+    """A launch on a full stream waits for room; meanwhile the process's other Python threads go on."""
+    import threading
+    import time
+
+    x, w = torch.ones(4, 512, device=DEV).bfloat16(), torch.ones(512, device=DEV).bfloat16()
+    ops.rmsnorm(x, w, 1e-6)
+    torch.cuda.synchronize()
+    gaps, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    t = threading.Thread(target=tick)
+    t.start()
+    start = time.perf_counter()
+    torch.cuda._sleep(1_000_000_000)  # about half a second of GPU time
+    for _ in range(3000):             # more than a stream's queue holds
+        ops.rmsnorm(x, w, 1e-6)
+    issued = time.perf_counter() - start
+    torch.cuda.synchronize()
+    stop.set()
+    t.join()
+    assert issued > 0.2, "the queue never filled: nothing was shown"
+    assert max(gaps) < issued / 2, f"a thread stood still for {max(gaps):.2f} of {issued:.2f} s"
