@@ -453,7 +453,11 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       }
     }
   }
-  if (*abort_flag && tid == 0) b2::report_timeout(a.status, *abort_flag);
+  const int aborted = *abort_flag;
+  if (aborted) {
+    for (int i = 0; i < 100; ++i) __nanosleep(2000);  // copies in flight land before the CTA leaves
+    if (tid == 0) b2::report_timeout(a.status, aborted);
+  }
 }
 
 // ---------------------------------------------------------------------------
