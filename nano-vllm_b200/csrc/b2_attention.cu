@@ -698,7 +698,8 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         if (j * PF_KEYS + row >= kv_len) {
           unsigned char* v = smem + (s_v - s_q) + (j & 1) * PF_TILE + row * 128;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) *reinterpret_cast<uint4*>(v + (i >> 3) * (PF_TILE / 2) + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+          for (int i = 0; i < 16; ++i)  // (another piece of every row of eight, so that they do not meet in a bank)
+            *reinterpret_cast<uint4*>(v + (i >> 3) * (PF_TILE / 2) + ((i ^ row) & 7) * 16) = make_uint4(0, 0, 0, 0);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
