@@ -472,8 +472,10 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 //   warp 0      TMA: Q of both heads once, then K and V blocks of 128 tokens, two of each in flight
 //   warp 1      tcgen05.mma: S = Q K^T (128 x 128, fp32, tensor memory), O += P V with P read from tensor memory
 //   warps 2..9  one thread per query row and head: running maximum and sum, P = exp2(...) rounded to bf16 over S
-// Tensor memory: S of the two heads, then O of the two heads, 128 columns each.  O is rescaled only when a row's maximum has
-// grown by more than 2^8 since its scale was set: fp32 and bf16 have the range, so the result is the same.
+// Tensor memory: S of the two heads, then O of the two heads, 128 columns each.  O is rescaled whenever a row's maximum grows, so
+// that the largest probability is exactly 1.  (Rescaling only past a growth of 2^8 rounds it: against float64, scores of standard
+// deviation 3, 2048 tokens, the error was 2.13e-3 where flash-attn's is 1.76e-3, and is 1.77e-3 now; of that the output's own
+// rounding is 1.66e-3.  8192 tokens x 16 heads take 478 us instead of 446.)
 // ---------------------------------------------------------------------------
 constexpr int PF_ROWS = 128, PF_KEYS = 128, PF_THREADS = 320;
 constexpr uint32_t PF_TILE = 128 * 128 * 2;                     // 128 rows of 128 bf16, as two 64-wide swizzled halves
@@ -634,7 +636,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
     const uint32_t t_s = tmem + h * 128 + lanes, t_o = tmem + 256 + h * 128 + lanes;
     const int pos = shift + t0 + row;  // the last key this row sees
-    float m = -INFINITY, l = 0.f;      // m: the maximum the row's scale is set to, in units of scores
+    float m = -INFINITY, l = 0.f;      // the row's maximum, in units of scores, and its sum
     bool ok = true;
     for (int j = 0; ok && j < n; ++j) {
       ok = b2::mbar_wait(s_full + h * 8, j & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_TMEM_FULL);
@@ -655,21 +657,25 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(r[e]));
         }
       }
-      // a new scale for the rows whose maximum has outgrown the old one; the first block sets it
-      const bool grow = mx > m && (m == -INFINITY || (mx - m) * a.scale_log2 > 8.f);
+      const bool grow = mx > m;
       if (__any_sync(0xffffffffu, grow)) {
         const float f = grow ? (m == -INFINITY ? 0.f : exp2f((m - mx) * a.scale_log2)) : 1.f;
         if (grow) m = mx;
         l *= f;
         if (j > 0) {  // (the previous block's product is complete: its scores' successor has been computed after it)
-#pragma unroll 1
-          for (int c = 0; c < 8; ++c) {
-            uint32_t r[16];
-            b2::tmem_ld_32x16(t_o + c * 16, r);
+#pragma unroll
+          for (int c = 0; c < 4; c += 2) {
+            uint32_t r[2][32];
+            b2::tmem_ld_32x32(t_o + c * 32, r[0]);
+            b2::tmem_ld_32x32(t_o + c * 32 + 32, r[1]);
             b2::tc_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * f);
-            tmem_st_32x16(t_o + c * 16, r);
+            for (int i = 0; i < 4; ++i) {
+              uint32_t w[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(__uint_as_float(r[i >> 1][(i & 1) * 16 + e]) * f);
+              tmem_st_32x16(t_o + c * 32 + i * 16, w);
+            }
           }
         }
       }

@@ -128,3 +128,25 @@ def test_prefill_does_not_see_the_next_sequence(rt):
     rt.check_status()
     for a, b in ((0, 100), (160, 289)):
         assert torch.equal(got[a:b], clean[a:b])
+
+
+@pytest.mark.parametrize("std", [1.0, 4.0])
+def test_prefill_rounds_probabilities_against_the_row_maximum(rt, std):
+    """Probabilities are rounded to bf16 relative to their row's maximum, which is then exact: the error against float64 is that of
+    plain PyTorch doing the same, whether the scores are flat or peaked.  Bound: the maximum of an earlier block is not the row's,
+    which moves each rounding but not their size; over 1.5 million elements the two errors agree to a percent or two.  (A scale that
+    lags behind the maximum by up to 2^8 shows 1.2 times the error at the second setting.)"""
+    from nanovllm_b200 import ops
+    nq, nkv, hd, t = 8, 4, 128, 1500
+    g = torch.Generator(device=DEV).manual_seed(17)
+    q, k, v = (torch.empty(t, h, hd, device=DEV).normal_(0, s, generator=g).bfloat16() for h, s in ((nq, std), (nkv, 1.0), (nkv, 1.0)))
+    cu = torch.tensor([0, t], dtype=torch.int32, device=DEV)
+    got = ops.prefill_attention(q, k, v, cu, cu, t, None, hd ** -0.5)
+    kd, vd = (x.double().repeat_interleave(2, 1) for x in (k, v))
+    scores = torch.einsum("qhd,khd->hqk", q.double(), kd) * hd ** -0.5
+    scores.masked_fill_(torch.ones(t, t, dtype=torch.bool, device=DEV).triu(1), float("-inf"))
+    exact = torch.einsum("hqk,khd->qhd", torch.softmax(scores, -1), vd)
+    p = torch.exp(scores - scores.amax(-1, keepdim=True)).float()
+    plain = (torch.einsum("hqk,khd->qhd", p.bfloat16().double(), vd) / p.double().sum(-1).t().unsqueeze(-1)).bfloat16()
+    ours, bound = ((x.double() - exact).norm().item() for x in (got, plain))
+    assert ours <= 1.05 * bound, f"error {ours / exact.norm().item():.3e} against {bound / exact.norm().item():.3e}"
