@@ -213,8 +213,7 @@ int b2_gemm_static_scratch(const void* A, int64_t lda, const void* W, int64_t ld
  *              -0.0 in an output of this form is stored as +0.0.
  * On one rank with more than 64 tokens nothing crosses a link and the call
  * runs as the plain GEMM followed by the add + RMSNorm kernel in place (two
- * launches), unless a form is forced or up to 256 tokens fit the cluster
- * kernel with a short K range per CTA (one launch). */
+ * launches), unless a form is forced. */
 int b2_rowpar_fused(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw, const void* bias,
                     int M, int N, int Kr, const void* residual_in, const void* norm_w, float eps,
                     void* normed_out, void* residual_out, void* stream);

@@ -2434,10 +2434,11 @@ int b2_rowpar_fused(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int6
   if (bias != nullptr && !aligned16(bias)) return B2_ERR_ARG;
   const int chunk = ctx->cfg.oneshot_tokens;
   const int world = ctx->cfg.world;
-  if (world == 1 && M > 64 && ctx->rowpar_form == B2_FORM_AUTO && !(M <= chunk && short_clusters<EPI_PUSH>(ctx, M, N, Kr))) {
-    // One rank, many tokens: nothing crosses a link, so the block is the plain GEMM on CTA pairs followed by the HBM-bound
-    // add + RMSNorm kernel in place - two launches, both near their rooflines, instead of one whose reduce phase walks the
-    // rows one CTA at a time.
+  if (world == 1 && M > 64 && ctx->rowpar_form == B2_FORM_AUTO) {
+    // One rank, more tokens than a decode step has: nothing crosses a link, so the block is the plain GEMM followed by the
+    // HBM-bound add + RMSNorm kernel in place.  One fused launch would spare a few microseconds of launch, but its CTAs release
+    // the next kernel late, write the rows to the inbox and back, and walk them one CTA at a time: 256 tokens x 1024 x 2048
+    // 9.5 us as two launches, 11.2 fused; 128 x 1024 x 3072 9.3 and 10.9.
     GemmArgs args{};
     args.C = static_cast<uint16_t*>(normed_out);
     args.ldc = N;

@@ -340,3 +340,18 @@ def test_up_to_256_tokens_on_clusters(ops, rt, m, n, k, path):
     assert_close_bf16(y, xs[0].float() @ ws[0].float().t(), f"gemm {m}x{k}x{n}")
     assert_close_bf16(new_res, exact_s, f"residual {m}x{k}x{n}")
     assert_close_bf16(normed, exact_n, f"normed {m}x{k}x{n}")
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 1024, 2048), (128, 1024, 3072), (256, 1024, 2048), (257, 1024, 2048)])
+def test_one_rank_above_decode_sizes_is_gemm_then_norm(ops, rt, m, n, k):
+    """From 65 tokens on a row-parallel call on one rank is two launches, the GEMM and the add + RMSNorm, with their results."""
+    from nanovllm_b200 import _abi
+    xs, ws, residual, norm_w = O.rowpar_case(m, k, n, 1, seed=m + k)
+    x, w, r, nw = xs[0].to(DEV), ws[0].to(DEV), residual.to(DEV), norm_w.to(DEV)
+    before = _abi.launch_count()
+    normed, new_res = ops.rowpar_fused(x, w, None, r, nw, 1e-6)
+    assert _abi.launch_count() - before == 2
+    want_n, want_r = ops.add_rmsnorm(ops.gemm(x, w), r, nw, 1e-6)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert torch.equal(normed, want_n) and torch.equal(new_res, want_r)
