@@ -1938,24 +1938,34 @@ int resident_clusters_of(int bn, int S) {
   else return bn == 32 ? max_resident_clusters<32, EPI>(S) : max_resident_clusters<64, EPI>(S);
 }
 
-// 65..256 tokens, nothing to exchange with peers: whether the decode kernel serves them better, as token tiles of 64 with their K range split over a
-// cluster.  It reads the weights once per token tile and its epilogue finishes 64 tokens alone, so this holds while there is room
-// to split every tile and each CTA's share of K is short (launch, set-up and the exchange are then most of either kernel): widths
-// of the 0.6B model, 119 tokens, qkv 11.2 -> 9.3 us; fused with the norm, which is a launch of its own behind the many-token
-// kernel, o 11.1 -> 9.9 and down 12.6 -> 10.6.  Where a share is longer it loses: 32 K blocks each, 65 tokens x 4096 x 4096,
-// 17.0 -> 17.8 us; unsplit tiles, 160 tokens x 4096 x 1024, 11.7 -> 15.7.
-template <int EPI>
-bool short_clusters(const b2_ctx* ctx, int M, int N, int K) {
-  GemmPlan p;
-  if (M <= 64 || M > 256 || plan_gemm(EPI, M, N, K, ctx->num_sms, 0, 0, ctx->tile_counter_cap, true, resident_clusters_of<EPI>, p) != B2_OK) return false;
-  return p.cluster_split >= 2 && (p.kblocks + p.cluster_split - 1) / p.cluster_split <= 12;
+// A plain GEMM of 65..256 tokens: whether the decode kernel serves it better than the CTA pairs, as token tiles of 64 with their K
+// range split over a cluster.  It reads the weights once per token tile and its epilogue finishes 64 tokens alone, so this holds
+// while there is room to split every tile and each CTA's share of K is short (launch, set-up and the exchange are then most of
+// either kernel).  Microseconds on CTA pairs and on clusters, by K blocks per CTA:
+//   K split in 2, 128 CTAs:  128 tokens x 4096: 8 blocks 8.5 and 7.4, 16: 12.7 and 9.9, 24: 15.3 and 12.2, 32: 17.8 and 14.5; 66 tokens, 32: 14.4
+//                            and 14.0 (the planner offers no longer share)
+//   K split in 2, 96 CTAs:   66 tokens x 3072: 18 blocks 10.5 and 9.3, 24: 11.6 and 11.1, 32: 13.1 and 13.5
+//   K split in 4:            192 tokens x 1024: 8 blocks 9.4 and 6.8, 12: 10.9 and 7.8, 16: 12.4 and 8.8, 32: 17.6 and 13.0
+//   K split in 8:            96 tokens x 1024: 8 blocks 11.2 and 7.3, 12: 13.9 and 9.0, 24: 15.1 and 13.6, 28: 14.9 and 14.9
+//   unsplit:                 150 tokens x 4096 x 1024 9.5 and 10.0
+// So a split in two is taken up to a quarter of the CTAs' number.  Larger splits are taken to 12 blocks, the longest that any shape
+// of the 0.6B, 8B and 32B models has on one GPU; past that the table favours clusters up to 24, which is not used yet.
+bool short_clusters(const GemmPlan& p) {
+  const int share = (p.kblocks + std::max(1, p.cluster_split) - 1) / std::max(1, p.cluster_split);
+  return p.cluster_split >= 2 && share <= (p.cluster_split == 2 ? std::max(12, p.gemm_ctas / 4) : 12);
 }
 
 template <int EPI>
 int launch_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K, GemmArgs& args,
                 int min_grid, cudaStream_t stream) {
+  const int reducers = 0;  // no CTAs are set aside for the reduce phase: every CTA reduces after its GEMM work
+  GemmPlan plan;
+  int prc = B2_ERR_SHAPE;
+  if (EPI != EPI_STORE || M <= 256)
+    prc = plan_gemm(EPI, M, N, K, ctx->num_sms, min_grid, reducers, ctx->tile_counter_cap, true, resident_clusters_of<EPI>, plan,
+                    (ctx->whole_tiles && (EPI == EPI_PUSH2 || EPI == EPI_PUSH3)) ? PLAN_WHOLE_TILES : 0);
   if constexpr (EPI == EPI_STORE) {
-    if (M > 64 && !short_clusters<EPI>(ctx, M, N, K)) {  // CTA pairs over tiles of up to 256 tokens, see b2_gemm_tile.cu
+    if (M > 64 && (prc != B2_OK || !short_clusters(plan))) {  // CTA pairs over tiles of up to 256 tokens, see b2_gemm_tile.cu
       b2::StoreEpilogue e;
       e.C = args.C;
       e.ldc = args.ldc;
@@ -1976,11 +1986,6 @@ int launch_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int64_t 
       return b2::launch_tile_gemm(ctx, A, lda, W, ldw, M, N, K, e, stream);
     }
   }
-  const int reducers = 0;  // no CTAs are set aside for the reduce phase: every CTA reduces after its GEMM work
-  GemmPlan plan;
-  const int prc = plan_gemm(EPI, M, N, K, ctx->num_sms, min_grid, reducers, ctx->tile_counter_cap, true,
-                            resident_clusters_of<EPI>,
-                            plan, (ctx->whole_tiles && (EPI == EPI_PUSH2 || EPI == EPI_PUSH3)) ? PLAN_WHOLE_TILES : 0);
   if (prc != B2_OK) return prc;
   const bool swap = plan.swap != 0;
   const int bn = plan.bn;

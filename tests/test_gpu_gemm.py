@@ -355,3 +355,15 @@ def test_one_rank_above_decode_sizes_is_gemm_then_norm(ops, rt, m, n, k):
     torch.cuda.synchronize()
     rt.check_status()
     assert torch.equal(normed, want_n) and torch.equal(new_res, want_r)
+
+
+@pytest.mark.parametrize("m,n,k,path", [(65, 4096, 4096, 1), (128, 4096, 4096, 1), (128, 4096, 4160, 2), (96, 3072, 3072, 1), (96, 3072, 3136, 2), (129, 4096, 4096, 2)])
+def test_k_split_in_two_up_to_a_quarter_of_the_ctas(ops, rt, m, n, k, path):
+    """Clusters of two: 128 of them take shares of 32 K blocks, 96 shares of 24; longer ones run on the CTA pairs."""
+    from nanovllm_b200 import _abi
+    xs, ws, _, _ = O.rowpar_case(m, k, n, 1, seed=m + k)
+    y = ops.gemm(xs[0].to(DEV), ws[0].to(DEV))
+    assert _abi.lib.b2_last_gemm_kernel() == path
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(y, xs[0].float() @ ws[0].float().t(), f"gemm {m}x{k}x{n}")
