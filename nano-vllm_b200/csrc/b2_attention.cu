@@ -12,12 +12,11 @@ namespace {
 // Bound: HBM.  Every K and V row of every context is read once (512 bytes per token and KV head) and used for the
 // G = nq / nkv query heads of its group; nothing else of size moves.
 //
-// One warp brings the tiles (64 tokens of one (sequence, KV head): 16 KB of K, 16 KB of V) into a 3-stage ring by TMA (2
-// stages where 8 heads share a KV head) and runs ahead over the borders between heads and sequences, so that two CTAs per
-// SM keep up to 190 KB in flight; four warps
-// take 16 tokens each from a landed tile (ldmatrix, mma.sync.m16n8k16 with the 8 upper rows empty: the tensor pipe is idle
-// most of the time anyway) and keep their own running maximum and sum.  The rows of a context's last tile come in
-// groups of 16, so that little is read past its end.
+// One warp brings the tiles (64 tokens of one (sequence, KV head): 16 KB of K, 16 KB of V) into a 3-stage ring by TMA and runs
+// ahead over the borders between heads and sequences, so that two CTAs per SM keep up to 190 KB in flight; four warps take 16
+// tokens each from a landed tile (ldmatrix, mma.sync.m16n8k16 with the rows past the group's heads empty: the tensor pipe is
+// idle most of the time anyway) and keep their own running maximum and sum.  The rows of a context's last tile come in groups of
+// 16, so that little is read past its end.
 //
 // Work split: the tiles of the whole batch, in the order (sequence, head, position), are dealt in contiguous equal ranges
 // to the CTAs - the contexts' lengths are read on the device, so a captured graph stays balanced for any batch.  A
@@ -29,16 +28,18 @@ namespace {
 constexpr int ATT_WARPS = 4, ATT_THREADS = (ATT_WARPS + 1) * 32;  // the last warp is the producer
 constexpr int ATT_TILE = 64;          // tokens per tile
 constexpr int ATT_HD = 128;           // head dimension
-constexpr int ATT_ROWS = 8;           // query heads of a group the fragments have room for
-// Served: groups of one and two heads.  (The kernel is faster than flash-attn's for 4 and 8 heads too: 53 us against 71 at 64
-// contexts of 1056 tokens.  But its last bits differ, and over the 36 layers of a 4096-wide model, every one of which rounds
-// to bf16 some ten times, that grows to 3 % of the hidden state; such models keep the results they had.)
+// Query heads per KV head: one and two are served.  Not because more would be slower or less exact - with room for them the
+// kernel took 53 us against flash-attn's 71 at 64 contexts of 1056 tokens and 4 heads, and its relative error against float64 is
+// the smaller one: 2.12e-3 against 2.23e-3 for 4 and for 8 heads, 1.69e-3 against 1.77e-3 where scores have standard deviation 3
+// (the output's own rounding is 1.66e-3 of each; with 2 heads 2.10e-3 against 2.23e-3) - but because the two round differently,
+// which over the 36 layers of a 4096-wide model grows to 3 % of the hidden state: the models with wider groups keep the results
+// they had.
 constexpr int ATT_MAX_GROUP = 2;
 constexpr int ATT_CTAS_PER_SM = 2;
-constexpr int ATT_MAX_STAGES = 3;
+constexpr int ATT_STAGES = 3;
 constexpr int ATT_HALF_BYTES = ATT_TILE * 128;          // 64 tokens x 64 dimensions: one swizzled box
 constexpr int ATT_STAGE_BYTES = 4 * ATT_HALF_BYTES;     // K dimensions 0..63, 64..127, V the same
-constexpr int ATT_SLOT = ATT_ROWS * ATT_HD + 2 * ATT_ROWS;  // floats of one partial result: O, then the maxima and sums
+constexpr int ATT_SLOT = ATT_MAX_GROUP * ATT_HD + 2 * ATT_MAX_GROUP;  // floats of one partial result: O, then the maxima and sums
 constexpr int ATT_MAX_SEQS = 1024;
 constexpr int ATT_COMBINE_TILES = 8;  // what combining the parts of an item costs, in tiles
 static_assert(ATT_CTAS_PER_SM * 2 * ATT_SLOT == B2_ATTN_WS_FLOATS_PER_SM, "the context allocates two slots per CTA");
@@ -53,7 +54,7 @@ struct AttnArgs {
   float* ws;       // [2 * CTAs][ATT_SLOT]
   int* counters;   // [sequences * KV heads], zero between launches
   B2Status* status;
-  int bt_width, block_size, num_blocks, n_seqs, nkv, group, stages;
+  int bt_width, block_size, num_blocks, n_seqs, nkv, group;
   float scale_log2;  // softmax scale * log2(e)
 };
 
@@ -111,19 +112,19 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                     const __grid_constant__ CUtensorMap tmV16, const AttnArgs a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  float* s_o = reinterpret_cast<float*>(smem + a.stages * ATT_STAGE_BYTES);  // [warp][head of the group][ATT_HD]
+  float* s_o = reinterpret_cast<float*>(smem + ATT_STAGES * ATT_STAGE_BYTES);  // [warp][head of the group][ATT_HD]
   int* first_tile = reinterpret_cast<int*>(s_o + ATT_WARPS * a.group * ATT_HD);
   int* s_len = first_tile + a.n_seqs + 1;
-  __shared__ float s_m[ATT_WARPS][ATT_ROWS], s_l[ATT_WARPS][ATT_ROWS];
-  __shared__ __align__(8) uint64_t s_bars[2 * ATT_MAX_STAGES];
+  __shared__ float s_m[ATT_WARPS][ATT_MAX_GROUP], s_l[ATT_WARPS][ATT_MAX_GROUP];
+  __shared__ __align__(8) uint64_t s_bars[2 * ATT_STAGES];
   __shared__ int s_abort, s_last[2], s_most, s_live;
   volatile int* abort_flag = &s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t bar_full = b2::smem_u32(s_bars), bar_empty = bar_full + ATT_MAX_STAGES * 8;
+  const uint32_t bar_full = b2::smem_u32(s_bars), bar_empty = bar_full + ATT_STAGES * 8;
   if (tid == 0) {
     b2::tma_prefetch_desc(&tmK);
     b2::tma_prefetch_desc(&tmV);
-    for (int i = 0; i < a.stages; ++i) {
+    for (int i = 0; i < ATT_STAGES; ++i) {
       b2::mbar_init(bar_full + i * 8, 1);
       b2::mbar_init(bar_empty + i * 8, ATT_WARPS);
     }
@@ -231,7 +232,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
               b2::tma_load_2d(d + 3 * ATT_HALF_BYTES, &tmV16, fb, x + 64, y + i * 16, b2::kEvictFirst);
             }
           }
-          if (++stage == a.stages) { stage = 0; phase ^= 1; }
+          if (++stage == ATT_STAGES) { stage = 0; phase ^= 1; }
         }
       }
     }
@@ -317,18 +318,18 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       }
       __syncwarp();
       if (lane == 0) b2::mbar_arrive(bar_empty + stage * 8);
-      if (++stage == a.stages) { stage = 0; phase ^= 1; }
+      if (++stage == ATT_STAGES) { stage = 0; phase ^= 1; }
     }
 
     // ---- the four warps' parts meet in shared memory ----
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     consumers_meet();  // the previous segment's parts have been read
-    if (c == 0) {
-      s_m[warp][g] = m;
-      s_l[warp][g] = l;
-    }
     if (g < a.group) {
+      if (c == 0) {
+        s_m[warp][g] = m;
+        s_l[warp][g] = l;
+      }
 #pragma unroll
       for (int j = 0; j < 16; ++j) *reinterpret_cast<float2*>(s_o + (warp * a.group + g) * ATT_HD + j * 8 + c * 2) = make_float2(o[j][0], o[j][1]);
     }
@@ -357,8 +358,8 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       } else {
         *reinterpret_cast<float4*>(slot + r * ATT_HD + d) = acc;
         if (d == 0) {
-          slot[ATT_ROWS * ATT_HD + r] = mx;
-          slot[ATT_ROWS * ATT_HD + ATT_ROWS + r] = sum;
+          slot[ATT_MAX_GROUP * ATT_HD + r] = mx;
+          slot[ATT_MAX_GROUP * ATT_HD + ATT_MAX_GROUP + r] = sum;
         }
       }
     }
@@ -400,8 +401,8 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             if (k < n) {
-              pm[k] = b2::ld_cg_f32(part(k) + ATT_ROWS * ATT_HD + r);
-              ps[k] = b2::ld_cg_f32(part(k) + ATT_ROWS * ATT_HD + ATT_ROWS + r);
+              pm[k] = b2::ld_cg_f32(part(k) + ATT_MAX_GROUP * ATT_HD + r);
+              ps[k] = b2::ld_cg_f32(part(k) + ATT_MAX_GROUP * ATT_HD + ATT_MAX_GROUP + r);
               x[k] = b2::ld_cg_v4(part(k) + r * ATT_HD + d);
             }
 #pragma unroll
@@ -425,13 +426,13 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       consumers_meet();
       for (int r = warp; r < a.group; r += ATT_WARPS) {
         float mx = -INFINITY, sum = 0.f;
-        for (int k = lane; k < n; k += 32) mx = fmaxf(mx, b2::ld_cg_f32(part(k) + ATT_ROWS * ATT_HD + r));
+        for (int k = lane; k < n; k += 32) mx = fmaxf(mx, b2::ld_cg_f32(part(k) + ATT_MAX_GROUP * ATT_HD + r));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
         for (int k = lane; k < n; k += 32) {
-          const float f = mx == -INFINITY ? 0.f : exp2f(b2::ld_cg_f32(part(k) + ATT_ROWS * ATT_HD + r) - mx);
+          const float f = mx == -INFINITY ? 0.f : exp2f(b2::ld_cg_f32(part(k) + ATT_MAX_GROUP * ATT_HD + r) - mx);
           s_o[r * (ATT_WARPS * ATT_HD) + k] = f;
-          sum += f * b2::ld_cg_f32(part(k) + ATT_ROWS * ATT_HD + ATT_ROWS + r);
+          sum += f * b2::ld_cg_f32(part(k) + ATT_MAX_GROUP * ATT_HD + ATT_MAX_GROUP + r);
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
@@ -485,7 +486,7 @@ constexpr uint64_t PF_LIMIT_NS = 1000000000ull;
 struct PrefillArgs {
   const int32_t *cu_q, *cu_k, *tables;  // tables: null = keys and values are rows cu_k[b] .. of the matrices
   int64_t bt_stride;
-  int bt_width, block_size, kv_rows, nq, nkv;
+  int bt_width, block_size, kv_rows, nq;
   uint16_t* out;
   float scale_log2;
   B2Status* status;
@@ -555,8 +556,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   b2::pdl_wait();
 
   // sequence, pair of heads, tile of 128 query tokens (the long rows of the causal triangle first)
-  const int b = blockIdx.z, pairs_per_kv = a.nq / a.nkv / 2;
-  const int head = blockIdx.y * 2, kv_head = blockIdx.y / pairs_per_kv;
+  const int b = blockIdx.z, kv_head = blockIdx.y, head = kv_head * 2;
   const int q0 = __ldg(a.cu_q + b), q_len = __ldg(a.cu_q + b + 1) - q0;
   const int k0 = __ldg(a.cu_k + b), kv_len = __ldg(a.cu_k + b + 1) - k0;
   const int t0 = (gridDim.x - 1 - blockIdx.x) * PF_ROWS;
@@ -757,13 +757,11 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   if (warp == 1) b2::tmem_dealloc(tmem, 512);
 }
 
-
-// dynamic shared memory, and the deepest ring with which two CTAs fit an SM (228 KB, 1 KB of it reserved per CTA)
-size_t attention_smem(int n_seqs, int group, int& stages) {
-  const size_t rest = 1024 + static_cast<size_t>(ATT_WARPS) * group * ATT_HD * sizeof(float) + (2 * static_cast<size_t>(n_seqs) + 1) * sizeof(int);
-  stages = rest + ATT_MAX_STAGES * ATT_STAGE_BYTES + 512 <= 113 * 1024 ? ATT_MAX_STAGES : 2;
-  return rest + stages * ATT_STAGE_BYTES;
+constexpr size_t ATT_SMEM_LIMIT = 113 * 1024;  // two CTAs per SM (228 KB, 1 KB of it reserved per CTA)
+constexpr size_t attention_smem(int n_seqs, int group) {
+  return 1024 + ATT_STAGES * ATT_STAGE_BYTES + static_cast<size_t>(ATT_WARPS) * group * ATT_HD * sizeof(float) + (2 * static_cast<size_t>(n_seqs) + 1) * sizeof(int);
 }
+static_assert(attention_smem(ATT_MAX_SEQS, ATT_MAX_GROUP) + 512 <= ATT_SMEM_LIMIT, "the ring, the warps' parts and the batch fit (512: static)");
 
 // the opt-in to more than 48 KB of dynamic shared memory belongs to a device, not to the process
 int configure_once() {
@@ -772,8 +770,7 @@ int configure_once() {
   B2_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return b2::set_error(B2_ERR_UNSUPPORTED, "device ordinal %d not supported", dev);
   if (!done[dev].load(std::memory_order_acquire)) {
-    B2_CUDA(cudaFuncSetAttribute(paged_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 113 * 1024));
+    B2_CUDA(cudaFuncSetAttribute(paged_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM_LIMIT));
     B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     done[dev].store(true, std::memory_order_release);
   }
@@ -824,7 +821,7 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   }
   const int64_t most = static_cast<int64_t>(n_seqs) * nkv * ((static_cast<int64_t>(bt_width) * block_size + ATT_TILE - 1) / ATT_TILE);
   const int grid = static_cast<int>(std::min<int64_t>(most, static_cast<int64_t>(ctx->num_sms) * ATT_CTAS_PER_SM));
-  const size_t smem = attention_smem(n_seqs, a.group, a.stages);
+  const size_t smem = attention_smem(n_seqs, a.group);
   const int crc = configure_once();
   if (crc != B2_OK) return crc;
   B2_CUDA(b2_launch(paged_decode_kernel, dim3(grid), dim3(ATT_THREADS), smem, static_cast<cudaStream_t>(stream), maps[0], maps[1], maps[2], maps[3], a));
@@ -861,11 +858,10 @@ int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const voi
   a.block_size = block_size;
   a.kv_rows = static_cast<int>(kv_rows);
   a.nq = nq;
-  a.nkv = nkv;
   a.out = static_cast<uint16_t*>(out);
   a.scale_log2 = scale * 1.4426950408889634f;
   a.status = ctx->status_dev;
-  B2_CUDA(b2_launch(prefill_attention_kernel, dim3((max_q + PF_ROWS - 1) / PF_ROWS, nq / 2, n_seqs), dim3(PF_THREADS), PF_SMEM, static_cast<cudaStream_t>(stream),
+  B2_CUDA(b2_launch(prefill_attention_kernel, dim3((max_q + PF_ROWS - 1) / PF_ROWS, nkv, n_seqs), dim3(PF_THREADS), PF_SMEM, static_cast<cudaStream_t>(stream),
                     tmQ, tmK, tmV, a));
   return B2_OK;
 }

@@ -52,7 +52,7 @@ struct B2Status {
 
 #define B2_MAX_WORLD 8
 #define B2_ATTN_MAX_ITEMS 65536               // decode attention: (sequence, KV head) pairs of one call
-#define B2_ATTN_WS_FLOATS_PER_SM (2 * 2 * 1040)  // decode attention: two partial results per CTA, two CTAs per SM
+#define B2_ATTN_WS_FLOATS_PER_SM (2 * 2 * 260)  // decode attention: two partial results per CTA, two CTAs per SM
 
 // ---------------------------------------------------------------------------
 // small PTX wrappers
