@@ -471,6 +471,30 @@ int b2_plan_cta_units(const b2_gemm_plan* plan, int cta, int* units, int cap);
  * last - first + 1 arrivals. */
 int b2_plan_tile_contributors(const b2_gemm_plan* plan, int tile, int* first_cta, int* last_cta);
 
+/* The same for the kernel of CTA pairs over tiles of 256 features x up to 256 tokens, which serves the store GEMMs
+ * (b2_gemm, b2_gemm_silu_mul, b2_qkv_fused, b2_rowpar_fused on one rank) of more than 64 tokens that no cluster plan takes. */
+typedef struct b2_tile_plan {
+  int bn;               /* token columns of a tile                                                       */
+  int tiles_f, tiles_t; /* feature tiles, token tiles                                                    */
+  int kblocks;          /* 64-wide K blocks per tile                                                     */
+  int split;            /* pairs of a cluster that share a tile's K range (1: none)                      */
+  int group;            /* token tiles visited together                                                  */
+  int stages;           /* of the operand ring                                                           */
+  int multi;            /* 1: one CTA per SM walks several tiles; 0: one tile, or a share of one, per pair */
+  int rounds, ranged;   /* multi: whole tiles per pair, tiles after those that are dealt out by K blocks */
+  int grid;             /* CTAs launched, two per pair                                                   */
+  int out_off, bar_off, smem; /* shared memory: output staging, barriers, bytes in all                   */
+} b2_tile_plan;
+/* resident_clusters: NULL (no tile is split over a cluster) or int[10]: entry [S] with half of an SM's shared memory per
+ * CTA, [5 + S] with all of it = clusters of 2 S CTAs the device holds at once. */
+int b2_plan_tile_gemm(int M, int N, int K, int num_sms, const int* resident_clusters, b2_tile_plan* plan);
+/* What pair `pair` of the grid computes, in order, as triples (tile, first K block, past the last) written to
+ * segments[3 * cap].  Returns their number (which may exceed cap), or a negative error code. */
+int b2_plan_tile_segments(const b2_tile_plan* plan, int pair, int* segments, int cap);
+/* The pairs between which the K blocks of a tile that is dealt out by K blocks lie: its counter expects
+ * last - first + 1 arrivals and its sum is kept in the first one's workspace slot. */
+int b2_plan_tile_holders(const b2_tile_plan* plan, int tile, int* first_pair, int* last_pair);
+
 /* Which kernel the calling thread's most recent GEMM-shaped call launched: 0 = persistent stream-K kernel,
  * 1 = cluster split-K kernel, 2 = CTA-pair kernel (store GEMMs of more than 64 tokens, the two-shot form from 512). */
 int b2_last_gemm_kernel(void);

@@ -48,6 +48,12 @@ class GemmPlan(C.Structure):
     _fields_ = [(n, C.c_int) for n in ("swap", "bn", "tiles_p", "tiles_q", "kblocks", "gemm_ctas", "round_robin", "grid", "cluster_split")]
 
 
+class TilePlan(C.Structure):
+    """b2_tile_plan: the same for the CTA-pair kernel of more than 64 tokens."""
+    _fields_ = [(n, C.c_int) for n in ("bn", "tiles_f", "tiles_t", "kblocks", "split", "group", "stages", "multi", "rounds", "ranged", "grid",
+                                       "out_off", "bar_off", "smem")]
+
+
 _p, _i, _i64, _f = C.c_void_p, C.c_int, C.c_int64, C.c_float
 
 SIGNATURES = {
@@ -91,6 +97,9 @@ SIGNATURES = {
     "b2_plan_gemm_opts": [_i, _i, _i, _i, _i, C.POINTER(_i), _i, C.POINTER(GemmPlan)],
     "b2_plan_cta_units": [C.POINTER(GemmPlan), _i, C.POINTER(_i), _i],
     "b2_plan_tile_contributors": [C.POINTER(GemmPlan), _i, C.POINTER(_i), C.POINTER(_i)],
+    "b2_plan_tile_gemm": [_i, _i, _i, _i, C.POINTER(_i), C.POINTER(TilePlan)],
+    "b2_plan_tile_segments": [C.POINTER(TilePlan), _i, C.POINTER(_i), _i],
+    "b2_plan_tile_holders": [C.POINTER(TilePlan), _i, C.POINTER(_i), C.POINTER(_i)],
     "b2_last_gemm_kernel": [],
     "b2_row_owner": [_i, _i, C.POINTER(_i)],
     "b2_owned_rows": [_i, _i, _i],

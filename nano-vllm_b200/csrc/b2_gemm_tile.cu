@@ -119,12 +119,22 @@ __device__ __forceinline__ void stamp(const TileArgs& a, int slot) {
   }
 }
 
+// The remaining tiles' K blocks (of a split tile: its own) in one range per pair, the first `rem` of them one block longer.
+struct Ranges {
+  int len, rem;
+  __host__ __device__ __forceinline__ Ranges(int units, int pairs) : len(units / pairs), rem(units % pairs) {}
+  __host__ __device__ __forceinline__ int begin(int pair) const { return pair * len + (pair < rem ? pair : rem); }
+  __host__ __device__ __forceinline__ int holder(int unit) const {
+    const int big = rem * (len + 1);
+    return unit < big ? unit / (len + 1) : rem + (unit - big) / len;
+  }
+};
 // What a pair works through: `rounds` whole tiles, then its range of the remaining tiles' K blocks, tile by tile.  (The
 // single instance: its share of the one tile.)
 struct Walk {
   int pairs, pair, rounds, whole, kblocks, t, u, u1;  // whole: tiles dealt out whole; u: position in the remaining tiles' K blocks
   int tile, k0, k1;
-  __device__ __forceinline__ bool next() {
+  __host__ __device__ __forceinline__ bool next() {
     if (pair + t * pairs < whole) {
       tile = pair + t * pairs;
       k0 = 0;
@@ -136,11 +146,25 @@ struct Walk {
     tile = u / kblocks;
     k0 = u - tile * kblocks;
     tile += rounds * pairs;
-    k1 = min(kblocks, k0 + u1 - u);
+    k1 = k0 + u1 - u < kblocks ? k0 + u1 - u : kblocks;
     u += k1 - k0;
     return true;
   }
 };
+// grid_pair: of `pairs` in the grid; cluster_pair: of the `split` that share a tile (single instance)
+template <bool MULTI>
+__host__ __device__ __forceinline__ Walk first_walk(const Ranges& r, int pairs, int grid_pair, int cluster_pair, int kblocks, int rounds, int ranged, int tiles) {
+  Walk w;
+  w.pairs = pairs;
+  w.pair = grid_pair;
+  w.kblocks = kblocks;
+  w.t = 0;
+  w.rounds = MULTI ? rounds : 0;
+  w.whole = MULTI ? (ranged > 0 ? rounds * pairs : tiles) : 0;
+  w.u = r.begin(MULTI ? grid_pair : cluster_pair);
+  w.u1 = r.begin((MULTI ? grid_pair : cluster_pair) + 1);
+  return w;
+}
 __device__ __forceinline__ void ld_cg_f4(uint32_t* r, const float* p) {
   asm volatile("ld.global.cg.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
 }
@@ -177,20 +201,9 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     f0 = ft * 2 * FM + side * FM;
     tok0 = (first_t + in_grp - ft * width) * a.bn;
   };
-  Walk first;
-  first.pairs = gridDim.x / 2;
-  first.pair = blockIdx.x / 2;
-  first.kblocks = a.kblocks;
-  first.t = 0;
-  // the remaining tiles' K blocks in ranges of part_len, the first part_rem of them one longer (single: the tile's among its pairs)
-  const int parts = MULTI ? first.pairs : S, part_no = MULTI ? first.pair : pair;
-  const int units = MULTI ? a.ranged * a.kblocks : a.kblocks;
-  const int part_len = units / parts, part_rem = units % parts;
-  auto part_begin = [&](int i) { return i * part_len + min(i, part_rem); };
-  first.rounds = MULTI ? a.rounds : 0;
-  first.whole = MULTI ? (a.ranged > 0 ? a.rounds * first.pairs : a.tilesF * a.tilesT) : 0;
-  first.u = part_begin(part_no);
-  first.u1 = part_begin(part_no + 1);
+  const int pairs = gridDim.x / 2;
+  const Ranges ranges(MULTI ? a.ranged * a.kblocks : a.kblocks, MULTI ? pairs : S);
+  const Walk first = first_walk<MULTI>(ranges, pairs, blockIdx.x / 2, pair, a.kblocks, a.rounds, a.ranged, a.tilesF * a.tilesT);
   auto next = [&](Walk& w) {
     const bool any = w.next();
     if (!MULTI) w.tile = blockIdx.x / (2 * S);
@@ -388,9 +401,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     float* sums = nullptr;   // where its fp32 sum lies, if not in tensor memory
     if (MULTI && w.k1 - w.k0 < a.kblocks) {
       // Part of the tile's K range: added into the slot of the first pair that holds some of it.
-      const int u = (w.tile - first.rounds * first.pairs) * a.kblocks, big = part_rem * (part_len + 1);
-      auto holder = [&](int i) { return i < big ? i / (part_len + 1) : part_rem + (i - big) / part_len; };
-      const int p0 = holder(u), p1 = holder(u + a.kblocks - 1);
+      const int u = (w.tile - first.rounds * pairs) * a.kblocks;
+      const int p0 = ranges.holder(u), p1 = ranges.holder(u + a.kblocks - 1);
       float* slot = a.ws + static_cast<size_t>(p0 * 2 + side) * (FM * 256) + q * (32 * 256) + lane * 4;
       for (int g = first_g; g < g1; g += STEP) {
         tmem_ld_16x256_x4(taddr + g * 8, acc[0]);
@@ -629,10 +641,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   if (threadIdx.x == 0) stamp(a, 6);
 }
 
-struct TilePlan {
-  int bn, tiles_f, tiles_t, kblocks, split, group, stages, multi, rounds, ranged;
-  uint32_t out_off, bar_off, smem;
-};
+using TilePlan = b2_tile_plan;
 
 // Geometry of one problem (host arithmetic only; resident(split, bytes) = clusters of 2 * split CTAs with that much shared
 // memory the device holds at once).  The candidates' times are estimated, in nanoseconds, from what the parts were measured
@@ -677,7 +686,7 @@ int plan_tile_gemm(int M, int N, int K, int num_sms, int tile_cap, Resident&& re
       const double t_mem = 2.0 * N * K / 6400.0;
       const double t_kb = std::max({stage / 82.0, (v == 0 ? 800.0 : 1600.0) / stages, (std::max(bn, 64) * 2 + 40) / 1.9});
       const double t_out = (multi ? 300.0 : 600.0) * ((groups + 4 * s - 1) / (4 * s)) + (s > 1 ? 1500.0 + (s - 1) * most * 4096 / 20.0 : 0.0);
-      int64_t rounds = work / pairs, ranged = work % pairs;  // MULTI
+      int64_t rounds = multi ? work / pairs : 0, ranged = multi ? work % pairs : 0;
       double cost;
       if (multi) {
         // the rest as one more round, or in ranges of K blocks: two parts per pair into L2 at 26 B/ns, one tile back
@@ -695,7 +704,9 @@ int plan_tile_gemm(int M, int N, int K, int num_sms, int tile_cap, Resident&& re
       }
       if (cost < best) {
         best = cost;
-        *p = TilePlan{bn, tiles_f, tiles_t, kblocks, s, std::min(tiles_t, 16), stages, multi ? 1 : 0, static_cast<int>(rounds), static_cast<int>(ranged), out_off, ring, ring + SMEM_EXTRA};
+        const int64_t grid = multi ? (ranged > 0 ? pairs : std::min<int64_t>(tiles, pairs)) * 2 : work * 2;
+        *p = TilePlan{bn, tiles_f, tiles_t, kblocks, s, std::min(tiles_t, 16), stages, multi ? 1 : 0, static_cast<int>(rounds), static_cast<int>(ranged),
+                      static_cast<int>(grid), static_cast<int>(out_off), static_cast<int>(ring), static_cast<int>(ring + SMEM_EXTRA)};
       }
     }
   }
@@ -784,10 +795,44 @@ int launch_tile_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int
   rc = encode_tmap_2d(&tmX, A, K, M, lda, BK, p.bn / 2);
   if (rc != B2_OK) return rc;
   if (p.multi)
-    B2_CUDA(b2_launch_cluster(gemm_tile_kernel<true>, dim3(p.ranged > 0 ? ctx->num_sms & ~1 : std::min(p.tiles_f * p.tiles_t * 2, ctx->num_sms & ~1)), dim3(Shape<true>::THREADS), p.smem, stream, 2u, tmW, tmX, a));
+    B2_CUDA(b2_launch_cluster(gemm_tile_kernel<true>, dim3(p.grid), dim3(Shape<true>::THREADS), p.smem, stream, 2u, tmW, tmX, a));
   else
-    B2_CUDA(b2_launch_cluster(gemm_tile_kernel<false>, dim3(p.tiles_f * p.tiles_t * 2 * p.split), dim3(Shape<false>::THREADS), p.smem, stream, 2u * p.split, tmW, tmX, a));
+    B2_CUDA(b2_launch_cluster(gemm_tile_kernel<false>, dim3(p.grid), dim3(Shape<false>::THREADS), p.smem, stream, 2u * p.split, tmW, tmX, a));
   return B2_OK;
 }
 
 }  // namespace b2
+
+// ---------------------------------------------------------------------------
+// The planner as data, for tests that run without a GPU (no CUDA call here).
+// ---------------------------------------------------------------------------
+extern "C" int b2_plan_tile_gemm(int M, int N, int K, int num_sms, const int* resident_clusters, b2_tile_plan* plan) {
+  if (plan == nullptr) return B2_ERR_ARG;
+  return plan_tile_gemm(M, N, K, num_sms, 1 << 18, [&](int split, uint32_t smem) { return resident_clusters != nullptr ? resident_clusters[(smem > SMEM_HALF ? MAX_SPLIT + 1 : 0) + split] : 0; }, plan);
+}
+
+extern "C" int b2_plan_tile_segments(const b2_tile_plan* plan, int pair, int* segments, int cap) {
+  if (plan == nullptr || plan->grid <= 0 || pair < 0 || pair >= plan->grid / 2 || cap < 0 || (cap > 0 && segments == nullptr)) return -B2_ERR_ARG;
+  const int pairs = plan->grid / 2, tiles = plan->tiles_f * plan->tiles_t;
+  const Ranges r(plan->multi ? plan->ranged * plan->kblocks : plan->kblocks, plan->multi ? pairs : plan->split);
+  Walk w = plan->multi ? first_walk<true>(r, pairs, pair, 0, plan->kblocks, plan->rounds, plan->ranged, tiles)
+                       : first_walk<false>(r, pairs, pair, pair % plan->split, plan->kblocks, 0, 0, tiles);
+  int n = 0;
+  for (; w.next(); ++n)
+    if (n < cap) {
+      segments[3 * n] = plan->multi ? w.tile : pair / plan->split;
+      segments[3 * n + 1] = w.k0;
+      segments[3 * n + 2] = w.k1;
+    }
+  return n;
+}
+
+extern "C" int b2_plan_tile_holders(const b2_tile_plan* plan, int tile, int* first_pair, int* last_pair) {
+  if (plan == nullptr || first_pair == nullptr || last_pair == nullptr || !plan->multi || plan->ranged <= 0 || plan->grid <= 0) return B2_ERR_ARG;
+  const int pairs = plan->grid / 2, u = (tile - plan->rounds * pairs) * plan->kblocks;
+  if (u < 0 || tile >= plan->tiles_f * plan->tiles_t) return B2_ERR_ARG;
+  const Ranges r(plan->ranged * plan->kblocks, pairs);
+  *first_pair = r.holder(u);
+  *last_pair = r.holder(u + plan->kblocks - 1);
+  return B2_OK;
+}
