@@ -18,7 +18,7 @@ def rt(pkg):
 
 
 # tile edges (63, 64, 65; 16-row groups), block edges (255..257), padded rows (0), one context over many CTAs, a batch whose
-# work ends inside a CTA's range, every group size
+# work ends inside a CTA's range, one and two query heads per KV head
 CASES = [((1,), 16, 8), ((63, 64, 65, 0, 15, 16, 17), 16, 8), ((255, 256, 257, 0), 16, 8), ((4096,), 2, 1), ((4000, 3), 8, 8), ((300,), 8, 8),
          (tuple(range(1, 620, 7)), 8, 4), ((700,) * 130, 2, 1),
          # dealt whole or cut: the longest item just within and just past the limit, as many items as CTAs and one sequence more, equal counts
@@ -150,3 +150,33 @@ def test_prefill_rounds_probabilities_against_the_row_maximum(rt, std):
     plain = (torch.einsum("hqk,khd->qhd", p.bfloat16().double(), vd) / p.double().sum(-1).t().unsqueeze(-1)).bfloat16()
     ours, bound = ((x.double() - exact).norm().item() for x in (got, plain))
     assert ours <= 1.05 * bound, f"error {ours / exact.norm().item():.3e} against {bound / exact.norm().item():.3e}"
+
+
+@pytest.mark.parametrize("nq,nkv", [(2, 1), (8, 4), (32, 16)])
+@pytest.mark.parametrize("slope", [0.0, 0.05, -0.05])
+def test_prefill_rescales_as_maxima_grow(rt, nq, nkv, slope):
+    """Scores that rise or fall along the keys, by 2^9 from one block of 128 keys to the next: with the rise every block's maximum
+    outgrows all earlier ones and the sum so far is scaled away, with the fall the first block outweighs the rest.  Both query
+    heads of a KV head, in several head layouts, get their own scale."""
+    from nanovllm_b200 import ops
+    hd, lens = 128, [700, 129, 64]
+    t = sum(lens)
+    g = torch.Generator().manual_seed(nq)
+    q, k, v = (torch.randn(t, h, hd, generator=g).bfloat16().float() for h in (nq, nkv, nkv))
+    if slope:  # dimension 0 carries the trend, half as steep for the second head of a pair
+        q[..., 0] = torch.tensor([16.0, 8.0]).repeat(nq // 2)
+        at = torch.cat([torch.arange(n) for n in lens])
+        k[..., 0] = (at * slope * hd ** 0.5 / 16.0).unsqueeze(1)
+    q, k, v = (x.bfloat16() for x in (q, k, v))
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    ref = torch.zeros(t, nq, hd)
+    for a, b in zip(cu[:-1].tolist(), cu[1:].tolist()):
+        kf, vf = (x[a:b].double().repeat_interleave(2, 1) for x in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q[a:b].double(), kf) * hd ** -0.5
+        s.masked_fill_(torch.ones(b - a, b - a, dtype=torch.bool).triu(1), float("-inf"))
+        ref[a:b] = torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), vf).float()
+    cu = cu.to(DEV)
+    got = ops.prefill_attention(q.to(DEV), k.to(DEV), v.to(DEV), cu, cu, max(lens), None, hd ** -0.5)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(got, ref, f"prefill {nq}/{nkv} heads, slope {slope}")
