@@ -121,7 +121,7 @@ int64_t b2_launch_count(void);
  * lda/ldw/ldc are row strides in elements (multiples of 8); K a multiple of 8.
  * tcgen05 tensor-core kernels fed by TMA: up to 64 tokens the K range is split
  * over clusters or over all SMs (stream-K), more tokens run on CTA pairs (or,
- * up to 256, as 64-token tiles on clusters).  From 512 tokens on every output
+ * up to 256 and where K is split, as 64-token tiles on clusters).  From 512 tokens on every output
  * is one unbroken sum over K.  W is treated as
  * a constant: the kernel may start fetching it while the previous b2_* kernel
  * on the stream is still running, so W must not be the output of a b2_* call
@@ -403,6 +403,7 @@ int b2_rope(const void* q, int64_t ldq, const void* k, int64_t ldk, int M, int n
  * fp32 scores and sums, probabilities rounded to bf16 for the second product.  Lengths and tables
  * are read on the device, so a captured call serves any later batch of the same size; they are read while earlier
  * b2_* kernels of the stream may still be running, so they must not be results of one, b2_advance_decode excepted.
+ * Calls of one context must be stream-ordered: they share its workspace for partial results.
  * b2_paged_attention_supported says (1 / 0) whether the shape is served: head_dim 128, one or
  * two query heads per KV head, blocks of a multiple of 64 tokens, at most 1024 sequences. */
 int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,

@@ -7,7 +7,7 @@
 //   gemm_cluster_kernel  one thread-block cluster per output tile, K split over the
 //                        cluster, parts combined through distributed shared memory
 //                        (decode sizes: at most 64 tokens and one wave of tiles; up to 256
-//                        as token tiles of 64 where the K split stays short)
+//                        as token tiles of 64 where K is split and a CTA's share stays short)
 //
 // D[p, q] = sum_k P[p, k] * Q[q, k]; both operands are K-major (row-major with
 // K contiguous).  P tiles have 128 rows (the MMA M dimension = 128 TMEM
@@ -1112,18 +1112,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
               // (columns past the last token have only had zeros added)
             } else {
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-              float v[32];
+              for (int c = 0; c < BN / 32; ++c) {
+                float v[32];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                float4 t;
-                asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "l"(slot + (c * 8 + j) * 128) : "memory");
-                v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
+                for (int j = 0; j < 8; ++j) {
+                  float4 t;
+                  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "l"(slot + (c * 8 + j) * 128) : "memory");
+                  v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(slot + (c * 8 + j) * 128) = make_float4(0.f, 0.f, 0.f, 0.f);
+                emit_chunk<BN, SWAP, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf);
               }
-#pragma unroll
-              for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(slot + (c * 8 + j) * 128) = make_float4(0.f, 0.f, 0.f, 0.f);
-              emit_chunk<BN, SWAP, EPI>(a, v, p_row, tq * BN, c, lane, parity, wbuf);
-            }
             }
           }
         }
@@ -1916,7 +1916,8 @@ int plan_gemm(int epi, int M, int N, int K, int num_sms, int min_grid, int reduc
     const int64_t pairs = static_cast<int64_t>(p.tilesP) * tq64;
     int split = 0;
     if (pairs <= num_sms) split = pick_cluster_split(64, static_cast<int>(pairs), p.kblocks, num_sms, resident);
-    // a plain GEMM's CTAs wait for nobody, so its tiles need not be resident together: up to 4 waves of unsplit tiles
+    // a plain GEMM's CTAs wait for nobody, so its tiles need not be resident together: up to 4 waves of unsplit tiles (b2_plan_gemm
+    // shows such a plan; launch_gemm prefers the CTA pairs to it, see short_clusters)
     else if (epi == EPI_STORE && pairs <= 4 * static_cast<int64_t>(num_sms) && p.kblocks <= 48 && resident(64, 1) > 0) split = 1;
     {
       // (only while a CTA's share of K stays short: with a long K range and no room to split it, stream-K over all SMs wins)

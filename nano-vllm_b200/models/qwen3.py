@@ -57,7 +57,8 @@ class Qwen3Attention(nn.Module):
         """Everything up to (not including) o_proj: returns [T, q_size]."""
         ctx = get_context()
         have_cache = self.attn.k_cache.numel() > 0
-        # projection, q/k head norm, RoPE and the K/V scatter: one launch for decode-sized batches, two otherwise
+        # projection, q/k head norm, RoPE and the K/V scatter: one launch (two for 64-wide heads and where a decode batch's projection
+        # has too many tiles for the cluster kernel)
         qkv = ops.qkv_fused(hidden_states, self.qkv_proj.weight, self.qkv_proj.bias, self.num_heads, self.num_kv_heads, self.head_dim,
                             None if self.qkv_bias else self.q_norm.weight, None if self.qkv_bias else self.k_norm.weight,
                             self.rms_norm_eps, positions, self.rotary_emb.cos_sin_cache,

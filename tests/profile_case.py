@@ -11,6 +11,10 @@ cases:
   oproj_decode    fused row-parallel launch, M=64, N=4096, Kr=4096 (Qwen3-8B o_proj at TP=1), 8 weight copies
   gemm_prefill    GEMM M=4096, N=4096, K=4096
   gemm_mid        GEMM M=256, N=4096, K=1024 (Qwen3-0.6B qkv at a 256-sequence decode step), 40 weight copies
+  qkv_prefill     qkv projection M=2048, N=4096, K=1024 with the head work in its epilogue (Qwen3-0.6B prefill), 24 weight copies
+  silu_mid        gate/up + SiLU*mul, M=256, N=24576, K=4096, 2 weight copies
+  attn_decode     decode attention, 64 contexts of 300..1371 tokens, 16 query / 8 KV heads, paged cache in shuffled blocks
+  attn_prefill    causal prefill attention, 8 sequences of 2048 tokens, 16 query / 8 KV heads
   rowpar_decode   fused row-parallel launch, M=64, N=4096, Kr=12288 (Qwen3-8B down_proj at TP=1)
   rowpar_prefill  fused row-parallel launch, M=1024, N=5120, Kr=1024
   store_kvcache   paged-KV scatter, 16384 tokens x D=1024
@@ -54,12 +58,12 @@ def main():
         m, n, k, copies = {"gemm_decode": (64, 24576, 4096, 4), "gemm_prefill": (4096, 4096, 4096, 2), "gemm_mid": (256, 4096, 1024, 40)}[a.case]
         x, ws = rnd(m, k), [rnd(n, k, scale=0.02) for _ in range(copies)]
         call = lambda i: ops.gemm(x, ws[i % copies])
-    elif a.case == "silu_decode":
-        m, i, k, copies = 64, 12288, 4096, 4
+    elif a.case in ("silu_decode", "silu_mid"):
+        m, i, k, copies = {"silu_decode": (64, 12288, 4096, 4), "silu_mid": (256, 12288, 4096, 2)}[a.case]
         x, ws = rnd(m, k), [rnd(2 * i, k, scale=0.02) for _ in range(copies)]
         call = lambda j: ops.gemm_silu_mul(x, ws[j % copies])
-    elif a.case == "qkv_decode":
-        m, nq, nkv, k, copies = 64, 32, 8, 4096, 8
+    elif a.case in ("qkv_decode", "qkv_prefill"):
+        m, nq, nkv, k, copies = {"qkv_decode": (64, 32, 8, 4096, 8), "qkv_prefill": (2048, 16, 8, 1024, 24)}[a.case]
         x, ws = rnd(m, k), [rnd((nq + 2 * nkv) * 128, k, scale=0.02) for _ in range(copies)]
         qw, kw = rnd(128), rnd(128)
         pos = torch.randint(0, 2048, (m,), device=dev)
@@ -71,6 +75,20 @@ def main():
         vc = torch.zeros_like(kc)
         slots = torch.randperm(16 * 256, device=dev)[:m].to(torch.int32)
         call = lambda j: ops.qkv_fused(x, ws[j % copies], None, nq, nkv, 128, qw, kw, 1e-6, pos, cos_sin, kc, vc, slots)
+    elif a.case == "attn_decode":
+        lens = [300 + 17 * i for i in range(64)]
+        need = [-(-n // 256) for n in lens]
+        order = torch.randperm(sum(need), device=dev, generator=g).to(torch.int32)
+        tables = torch.zeros(64, max(need), dtype=torch.int32, device=dev)
+        for i, n in enumerate(need):
+            tables[i, :n] = order[sum(need[:i]):sum(need[:i]) + n]
+        kc, vc, q = rnd(sum(need), 256, 8, 128), rnd(sum(need), 256, 8, 128), rnd(64, 16, 128)
+        context_lens = torch.tensor(lens, dtype=torch.int32, device=dev)
+        call = lambda i: ops.paged_attention(q, kc, vc, context_lens, tables, 128 ** -0.5)
+    elif a.case == "attn_prefill":
+        q, k, v = rnd(16384, 16, 128), rnd(16384, 8, 128), rnd(16384, 8, 128)
+        cu = torch.arange(0, 16385, 2048, dtype=torch.int32, device=dev)
+        call = lambda i: ops.prefill_attention(q, k, v, cu, cu, 2048, None, 128 ** -0.5)
     elif a.case in ("rowpar_decode", "rowpar_prefill", "oproj_decode"):
         m, n, k, copies = {"rowpar_decode": (64, 4096, 12288, 4), "rowpar_prefill": (1024, 5120, 1024, 8), "oproj_decode": (64, 4096, 4096, 8)}[a.case]
         x, ws, res, nw = rnd(m, k), [rnd(n, k, scale=0.02) for _ in range(copies)], rnd(m, n), rnd(n)
