@@ -743,6 +743,9 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
               *reinterpret_cast<const uint4*>(mine + r * 256 + ((piece ^ (r & 15)) << 4));
       }
     }
+  } else if (t0 < q_len) {  // queries of a sequence without keys: nothing to attend to
+    for (int i = threadIdx.x - 64; i < min(PF_ROWS, q_len - t0) * 32; i += PF_THREADS - 64)
+      *reinterpret_cast<uint4*>(a.out + (static_cast<int64_t>(q0 + t0 + (i >> 5)) * a.nq + head) * 128 + (i & 31) * 8) = make_uint4(0, 0, 0, 0);
   }
 
   __syncwarp();

@@ -180,3 +180,18 @@ def test_prefill_rescales_as_maxima_grow(rt, nq, nkv, slope):
     torch.cuda.synchronize()
     rt.check_status()
     assert_close_bf16(got, ref, f"prefill {nq}/{nkv} heads, slope {slope}")
+
+
+def test_prefill_of_a_sequence_without_keys_is_zero(rt):
+    from nanovllm_b200 import ops
+    nq, nkv, hd = 4, 2, 128
+    q = torch.randn(210, nq, hd, generator=torch.Generator().manual_seed(1)).bfloat16().to(DEV)
+    cache = torch.randn(2, 1, 256, nkv, hd, generator=torch.Generator().manual_seed(2)).bfloat16().to(DEV)
+    cu_q = torch.tensor([0, 5, 205, 210], dtype=torch.int32, device=DEV)
+    cu_k = torch.tensor([0, 5, 5, 12], dtype=torch.int32, device=DEV)
+    tables = torch.zeros(3, 1, dtype=torch.int32, device=DEV)
+    torch.full((210, nq, hd), 7.0, dtype=torch.bfloat16, device=DEV)  # what the allocator hands out next is not zero already
+    got = ops.prefill_attention(q, cache[0], cache[1], cu_q, cu_k, 200, tables, hd ** -0.5)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert (got[5:205] == 0).all() and (got[:5] != 0).any() and (got[205:] != 0).any()
