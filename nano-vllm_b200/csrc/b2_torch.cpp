@@ -45,11 +45,16 @@ void check(int rc, const char* what) {
 
 // One call of the library.  The GIL is released around it: a launch waits when the stream's queue is full, and other Python
 // threads have to go on meanwhile.  (Arguments are converted by the caller, with the GIL held; the library's error text is per thread.)
+struct Unlocked {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
 template <class... P, class... A>
 void launch(const char* what, int (*f)(P...), A... args) {
-  PyThreadState* const state = PyEval_SaveThread();
-  const int rc = f(args...);
-  PyEval_RestoreThread(state);
+  const int rc = [&] {
+    const Unlocked unlocked;
+    return f(args...);
+  }();
   check(rc, what);
 }
 
@@ -399,8 +404,9 @@ PyObject* prefill_attention(Args a) {
   const at::Tensor out = at::detail::empty_cuda({n, nq, hd}, at::kBFloat16, q.device(), std::nullopt);
   if (n)
     launch("b2_prefill_attention", b2_prefill_attention, context(a[0]), q.data_ptr(), n > 1 ? q.stride(0) : nq * hd, k.data_ptr(), v.data_ptr(),
-           paged || rows == 1 ? nkv * hd : k.stride(0), rows, paged ? tables.const_data_ptr<int32_t>() : nullptr, paged ? (n_seqs > 1 ? tables.stride(0) : tables.size(1)) : 0, paged ? tables.size(1) : 0, bs,
-           cu_q.const_data_ptr<int32_t>(), cu_k.const_data_ptr<int32_t>(), n_seqs, max_q, n, nq, nkv, hd, number(a[8]), out.data_ptr(), stream());
+           paged || rows == 1 ? nkv * hd : k.stride(0), rows, paged ? tables.const_data_ptr<int32_t>() : nullptr,
+           paged ? (n_seqs > 1 ? tables.stride(0) : tables.size(1)) : 0, paged ? tables.size(1) : 0, bs, cu_q.const_data_ptr<int32_t>(),
+           cu_k.const_data_ptr<int32_t>(), n_seqs, max_q, n, nq, nkv, hd, number(a[8]), out.data_ptr(), stream());
   return wrap(out);
 }
 
