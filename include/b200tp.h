@@ -412,6 +412,29 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
                               void* out, void* stream);
 int b2_paged_attention_supported(int n_seqs, int nq, int nkv, int head_dim, int block_size);
 
+/* ---- the decoder layers of one decode step in one launch (one rank) -------------------
+ * What the calls of a layer compute, for all layers: norm, qkv projection with q/k head norm, rotation and cache scatter,
+ * attention over the paged cache, o projection + residual, norm, gate/up + SiLU * mul, down projection + residual
+ * (nanovllm/models/qwen3.py:146-159), and the norm after the last one.  x [rows][hidden] bf16: the embedded tokens;
+ * positions int64, context_lens / slot_mapping int32 [rows], block_tables as for b2_paged_attention_decode; out
+ * [rows][hidden].  Rows after the last one with a context are padding: their output is zero and nothing is stored for them.
+ * Weights are [out][in] contiguous, gate and up rows interleaved; q_norm and k_norm may be null together.
+ * Partial sums, norms' inputs and the residual's sums are fp32.  The launch is cooperative (one CTA per SM).
+ * b2_decode_stack_workspace: bytes of device memory a call needs (16-byte aligned, contents irrelevant), or 0 where the
+ * shape is not served: one rank, head_dim 128, at most two query heads per KV head, at most 16 rows, blocks of a power of two
+ * of at least 16 tokens, 1024 hidden features, nq * 128 and inter multiples of 1024 up to 3072: a layer that fits the SMs' shared memory. */
+typedef struct b2_stack_layer {
+  const void *qkv_w, *o_w, *gate_up_w, *down_w, *in_norm, *post_norm, *q_norm, *k_norm;
+  void *k_cache, *v_cache; /* [num_blocks][block_size][nkv][head_dim] */
+} b2_stack_layer;
+int64_t b2_decode_stack_workspace(b2_ctx* ctx, int rows, int layers, int hidden, int nq, int nkv, int head_dim, int inter,
+                                  int block_size);
+int b2_decode_stack(b2_ctx* ctx, const b2_stack_layer* layers, int n_layers, const void* final_norm, int hidden, int nq,
+                    int nkv, int head_dim, int inter, float eps, float qk_eps, float scale, const float* cos_sin, const void* x,
+                    int rows, const int64_t* positions, const int32_t* context_lens, const int32_t* slot_mapping,
+                    const int32_t* block_tables, int64_t bt_stride, int bt_width, int block_size, int num_blocks, void* out,
+                    void* workspace, int64_t workspace_bytes, void* stream);
+
 /* ---- causal prefill attention: what flash_attn_varlen_func computes
  *      (nanovllm/layers/attention.py:64-69) ------------------------------------------
  * q [tokens, nq, head_dim] bf16 (row stride q_stride).  Sequence b has query rows

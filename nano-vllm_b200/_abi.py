@@ -32,7 +32,8 @@ _ERR_NAMES = {1: "bad argument", 2: "shape outside what the context was created 
 WAIT_NAMES = {0: "none", 1: "GEMM: TMA stage never filled", 2: "GEMM: stage never freed", 3: "GEMM: accumulator never completed",
               4: "GEMM: accumulator never drained", 5: "fused row-parallel: partial rows never arrived",
               6: "embedding: owner row never arrived", 7: "LM head: a peer's logits never arrived",
-              8: "token broadcast: rank 0's tokens never arrived", 9: "two-shot row-parallel: rows owned by other ranks never arrived"}
+              8: "token broadcast: rank 0's tokens never arrived", 9: "two-shot row-parallel: rows owned by other ranks never arrived",
+              10: "decode step in one launch: another CTA's results never arrived"}
 
 
 class Config(C.Structure):
@@ -89,6 +90,8 @@ SIGNATURES = {
     "b2_paged_attention_supported": [_i, _i, _i, _i, _i],
     "b2_prefill_attention": [_p, _p, _i64, _p, _p, _i64, _i64, _p, _i64, _i, _i, _p, _p, _i, _i, _i, _i, _i, _i, _f, _p, _p],
     "b2_prefill_attention_supported": [_i, _i, _i, _i],
+    "b2_decode_stack_workspace": [_p, _i, _i, _i, _i, _i, _i, _i, _i],
+    "b2_decode_stack": [_p, _p, _i, _p, _i, _i, _i, _i, _i, _f, _f, _f, _p, _p, _i, _p, _p, _p, _p, _i64, _i, _i, _i, _p, _p, _i64, _p],
     "b2_argmax": [_p, _i64, _i, _i, _p, _p],
     "b2_broadcast_tokens": [_p, _p, _i, _p],
     "b2_advance_decode": [_p, _p, _p, _p, _p, _p, _i64, _i, _i, _i64, _i, _p],
@@ -112,7 +115,7 @@ for _name, _args in SIGNATURES.items():
     _fn.restype = _i
 lib.b2_last_error.restype = C.c_char_p
 lib.b2_last_error.argtypes = []
-lib.b2_launch_count.restype = _i64
+lib.b2_launch_count.restype = lib.b2_decode_stack_workspace.restype = _i64
 lib.b2_launch_count.argtypes = []
 
 EXPORTED = list(SIGNATURES) + ["b2_last_error", "b2_launch_count"]

@@ -17,7 +17,7 @@ LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libb200tp.so")
 BINDING = os.path.join(LIBDIR, "_b2torch.so")
 BINDING_SOURCE = "b2_torch.cpp"
-SOURCES = ["b2_ctx.cu", "b2_elementwise.cu", "b2_attention.cu", "b2_gemm_tile.cu", "b2_gemm.cu"]
+SOURCES = ["b2_ctx.cu", "b2_elementwise.cu", "b2_attention.cu", "b2_stack.cu", "b2_gemm_tile.cu", "b2_gemm.cu"]
 HEADERS = ["b2_common.cuh", os.path.join("..", "..", "include", "b200tp.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17"]
 

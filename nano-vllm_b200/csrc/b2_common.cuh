@@ -22,7 +22,8 @@ enum : int {
   B2_WAIT_EMBED = 6,        // embedding waiting for the owner rank's row
   B2_WAIT_LOGITS = 7,       // rank 0 waiting for peers' logits slices
   B2_WAIT_TOKENS = 8,       // a rank waiting for rank 0's sampled tokens
-  B2_WAIT_ROWS = 9          // two-shot: waiting for the other owners' finished rows
+  B2_WAIT_ROWS = 9,         // two-shot: waiting for the other owners' finished rows
+  B2_WAIT_STACK = 10        // decode step in one launch: waiting for what the other CTAs hand over
 };
 
 // The bf16 bit pattern that marks "not written yet" in data-as-flag buffers:

@@ -410,6 +410,67 @@ PyObject* prefill_attention(Args a) {
   return wrap(out);
 }
 
+// ---- the decoder layers of a decode step -----------------------------------------------------
+// a contiguous bf16 tensor on the query's device that the kernel's 16-byte accesses can address
+bool plain(const at::Tensor& t, const at::Tensor& x, at::IntArrayRef shape) {
+  return t.scalar_type() == at::kBFloat16 && t.device() == x.device() && t.sizes() == shape && t.is_contiguous() && on_16_bytes(t);
+}
+
+// decode_stack(ctx, x, positions, layers, final_norm, nq, nkv, head_dim, inter, eps, qk_eps, scale, cos_sin, context_lens,
+//              slot_mapping, block_tables): None when the kernel does not serve the call.
+// layers: per layer (qkv_w, o_w, gate_up_w in pairs, down_w, in_norm, post_norm, q_norm, k_norm, k_cache, v_cache)
+PyObject* decode_stack(Args a) {
+  b2_ctx* ctx = context(a[0]);
+  const at::Tensor &x = tensor(a[1], "decode input"), &pos = tensor(a[2], "positions"), &final_norm = tensor(a[4], "final norm"), &cs = tensor(a[12], "cos_sin"),
+                   &lens = tensor(a[13], "context_lens"), &slots = tensor(a[14], "slot_mapping"), &tables = tensor(a[15], "block_tables");
+  if (!PyList_Check(a[3])) raise(PyExc_TypeError, "decode_stack: layers must be a list");
+  const Py_ssize_t n_layers = PyList_GET_SIZE(a[3]);
+  const int64_t nq = integer(a[5]), nkv = integer(a[6]), hd = integer(a[7]), inter = integer(a[8]);
+  if (x.dim() != 2 || n_layers < 1) Py_RETURN_NONE;
+  const int64_t n = x.size(0), h = x.size(1);
+  std::vector<b2_stack_layer> layers(n_layers);
+  int64_t blocks = 0, bs = 0;
+  for (Py_ssize_t i = 0; i < n_layers; ++i) {
+    PyObject* l = PyList_GET_ITEM(a[3], i);
+    if (!PyTuple_Check(l) || PyTuple_GET_SIZE(l) != 10) raise(PyExc_TypeError, "decode_stack: a layer is a tuple of 10");
+    at::Tensor w[10];
+    for (int k = 0; k < 10; ++k) w[k] = optional_tensor(PyTuple_GET_ITEM(l, k), "decode_stack layer");
+    if (!w[8].defined() || !w[9].defined() || w[8].dim() != 4) Py_RETURN_NONE;
+    if (i == 0) {
+      blocks = w[8].size(0);
+      bs = w[8].size(1);
+    }
+    const int64_t q = nq * hd, rows = (nq + 2 * nkv) * hd;
+    if (!plain(w[0], x, {rows, h}) || !plain(w[1], x, {h, q}) || !plain(w[2], x, {2 * inter, h}) || !plain(w[3], x, {h, inter}) || !plain(w[4], x, {h}) ||
+        !plain(w[5], x, {h}) || w[6].defined() != w[7].defined() || (w[6].defined() && (!plain(w[6], x, {hd}) || !plain(w[7], x, {hd}))) ||
+        !plain(w[8], x, {blocks, bs, nkv, hd}) || !plain(w[9], x, {blocks, bs, nkv, hd}))
+      Py_RETURN_NONE;
+    layers[i] = {ptr(w[0]), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(w[4]), ptr(w[5]), ptr(w[6]), ptr(w[7]), ptr(w[8]), ptr(w[9])};
+  }
+  if (n == 0 || blocks == 0 || !plain(x, x, {n, h}) || !plain(final_norm, x, {h}) || !table_layout(tables) || tables.scalar_type() != at::kInt || !cs.is_contiguous() ||
+      cs.scalar_type() != at::kFloat || cs.size(-1) != hd || pos.scalar_type() != at::kLong || !pos.is_contiguous() || pos.numel() != n)
+    Py_RETURN_NONE;
+  const int64_t bytes = b2_decode_stack_workspace(ctx, n, n_layers, h, nq, nkv, hd, inter, bs);
+  if (bytes == 0) Py_RETURN_NONE;
+  on_current_gpu(x, "decode input");
+  int32_vector(lens, n, "context_lens");
+  int32_vector(slots, n, "slot_mapping");
+  block_table_rows(tables, n);
+  for (const at::Tensor* t : {&pos, &cs, &lens, &slots, &tables}) same_device(*t, x, "an operand of the decode step");
+  const at::Tensor out = empty_rows(n, h, x), ws = at::detail::empty_cuda({bytes}, at::kByte, x.device(), std::nullopt);
+  const float eps = number(a[9]), qk_eps = number(a[10]), scale = number(a[11]);
+  void* const on_stream = stream();
+  const int rc = [&] {
+    const Unlocked unlocked;
+    return b2_decode_stack(ctx, layers.data(), n_layers, final_norm.data_ptr(), h, nq, nkv, hd, inter, eps, qk_eps, scale, cs.const_data_ptr<float>(), x.data_ptr(), n,
+                           pos.const_data_ptr<int64_t>(), lens.const_data_ptr<int32_t>(), slots.const_data_ptr<int32_t>(), tables.const_data_ptr<int32_t>(),
+                           n > 1 ? tables.stride(0) : tables.size(1), tables.size(1), bs, blocks, out.data_ptr(), ws.data_ptr(), bytes, on_stream);
+  }();
+  if (rc == B2_ERR_UNSUPPORTED) Py_RETURN_NONE;  // (the CTAs cannot all be resident)
+  check(rc, "b2_decode_stack");
+  return wrap(out);
+}
+
 PyObject* init(Args a) {
   Py_INCREF(a[0]);
   Py_XDECREF(g_check);
@@ -435,7 +496,8 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define B2_ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {B2_ENTRY(init, 1), B2_ENTRY(gemm, 4), B2_ENTRY(gemm_silu_mul, 3), B2_ENTRY(qkv_fused, 15), B2_ENTRY(rowpar_fused, 7),
                          B2_ENTRY(rmsnorm, 3), B2_ENTRY(add_rmsnorm, 4), B2_ENTRY(silu_and_mul, 1), B2_ENTRY(store_kvcache, 5),
-                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(rope, 5), B2_ENTRY(embed, 5), B2_ENTRY(paged_attention, 7), B2_ENTRY(prefill_attention, 9), {nullptr, nullptr, 0, nullptr}};
+                         B2_ENTRY(qk_norm_rope_store, 12), B2_ENTRY(rope, 5), B2_ENTRY(embed, 5), B2_ENTRY(paged_attention, 7), B2_ENTRY(prefill_attention, 9),
+                         B2_ENTRY(decode_stack, 16), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_b2torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -125,6 +125,9 @@ class Qwen3Model(nn.Module):
 
     def forward(self, input_ids: torch.Tensor, positions: torch.Tensor) -> torch.Tensor:
         residual = self.embed_tokens(input_ids)
+        normed = self._decode_in_one_launch(residual, positions)
+        if normed is not None:
+            return normed
         # layer 0 has no residual yet: plain norm, the embedding becomes the residual (reference :152-153)
         normed = self.layers[0].input_layernorm(residual)
         n = len(self.layers)
@@ -132,6 +135,44 @@ class Qwen3Model(nn.Module):
             next_norm = self.layers[i + 1].input_layernorm if i + 1 < n else self.norm
             normed, residual = layer(positions, normed, residual, next_norm)
         return normed
+
+
+    def _decode_in_one_launch(self, embedded: torch.Tensor, positions: torch.Tensor) -> torch.Tensor | None:
+        """All layers of a decode step through ops.decode_stack; None where that does not apply: the layers then run one by one.
+        It computes what the stock layers compute, so every layer must be one, without hooks of its own."""
+        ctx = get_context()
+        if ctx.is_prefill or ctx.context_lens is None or ctx.slot_mapping is None or ctx.block_tables is None or Attention.backend != "flash_attn":
+            return None
+        first = self.layers[0]
+        layers = []
+        for layer in self.layers:
+            if not _is_stock(layer):
+                return None
+            attn, mlp = layer.self_attn, layer.mlp
+            if attn.qkv_bias or attn.rotary_emb.cos_sin_cache is not first.self_attn.rotary_emb.cos_sin_cache:
+                return None
+            if (layer.input_layernorm.eps, layer.post_attention_layernorm.eps, attn.rms_norm_eps) != (self.norm.eps, self.norm.eps, first.self_attn.rms_norm_eps):
+                return None
+            layers.append((attn.qkv_proj.weight, attn.o_proj.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight, layer.input_layernorm.weight,
+                           layer.post_attention_layernorm.weight, attn.q_norm.weight, attn.k_norm.weight, attn.attn.k_cache, attn.attn.v_cache))
+        attn = first.self_attn
+        return ops.decode_stack(embedded, positions, layers, self.norm.weight, attn.num_heads, attn.num_kv_heads, attn.head_dim,
+                                first.mlp.down_proj.weight.shape[1], self.norm.eps, attn.rms_norm_eps, attn.attn.scale,
+                                attn.rotary_emb.cos_sin_cache, ctx.context_lens, ctx.slot_mapping, ctx.block_tables)
+
+
+def _is_stock(layer: nn.Module) -> bool:
+    """A decoder layer made of this file's modules, whose calls nothing listens to."""
+    if type(layer) is not Qwen3DecoderLayer or type(layer.self_attn) is not Qwen3Attention or type(layer.mlp) is not Qwen3MLP:
+        return False
+    attn, mlp = layer.self_attn, layer.mlp
+    if type(attn.attn) is not Attention or type(attn.o_proj) is not RowParallelLinear or type(mlp.down_proj) is not RowParallelLinear:
+        return False
+    if type(mlp.gate_up_proj) is not MergedColumnParallelLinear or not mlp.gate_up_proj.paired or attn.o_proj.bias is not None or mlp.down_proj.bias is not None:
+        return False
+    if attn.qkv_proj.bias is not None or type(layer.input_layernorm) is not RMSNorm or type(layer.post_attention_layernorm) is not RMSNorm:
+        return False
+    return not any(m._forward_hooks or m._forward_pre_hooks for m in (layer, layer.input_layernorm))
 
 
 class Qwen3ForCausalLM(nn.Module):
