@@ -16,6 +16,11 @@
 // the main loop every pair hands the accumulator columns that others own to them through distributed shared memory (the ring
 // is free by then), adds what it received to its own and stores its share.
 //
+// The TMA and the MMA warp walk with all their lanes and elect a thread to issue.  The instructions take descriptors, coordinates and barriers
+// from uniform registers; in code that one lane runs alone the compiler moves every operand there anew, and a K block took 585 clocks of
+// issue whatever its width (the tensor pipe wants 128 at 64 tokens, 512 at 256).  It is 310 at 64 and 333 at 160 tokens now: 391 tokens
+// x 6144 x 4096 28.8 -> 21.4 us, 777 x 24576 x 4096 150 -> 130, 256 x 4096 x 1024 10.6 -> 8.0.
+//
 // The accumulator has features in lanes and tokens in columns.  It leaves tensor memory in the 16x256b shape, whose
 // fragments are those of stmatrix: a transposing stmatrix puts 8 features of one token next to each other, and rows of
 // 32 features per warp (64 bytes), or of 128 (one attention head) per four warps, go out of shared memory.
@@ -243,46 +248,53 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   if (threadIdx.x == 0) stamp(a, 0);
 
   if (warp == 0) {
-    // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0) {
-      const uint32_t full0 = b2::map_to_cta(bar_full, cr & ~1);  // the even CTA's "full" barriers, as a cluster address
-      const int x_half = side * (a.bn >> 1);
-      Walk w = first;
-      int f0 = 0, tok0 = 0, pre = 0;
-      if (next(w)) {
-        place(w.tile, f0, tok0);
-        pre = min(w.k1 - w.k0, STAGES);
-      } else {
-        w.k0 = w.k1 = 0;
-      }
+    // ---------------- TMA producer (both CTAs): the whole warp walks, one thread issues ----------------
+    const uint32_t full0 = b2::map_to_cta(bar_full, cr & ~1);  // the even CTA's "full" barriers, as a cluster address
+    const int x_half = side * (a.bn >> 1);
+    Walk w = first;
+    int f0 = 0, tok0 = 0, pre = 0;
+    if (next(w)) {
+      place(w.tile, f0, tok0);
+      pre = min(w.k1 - w.k0, STAGES);
+    } else {
+      w.k0 = w.k1 = 0;
+    }
+    if (b2::elect_one()) {
       for (int i = 0; i < pre; ++i) {  // weights depend on no earlier kernel
         if (side == 0) b2::mbar_arrive_expect_tx(bar_full + i * 8, 2 * stage_bytes);
         b2::tma_load_2d_pair(smem_base + i * stage_bytes, &tmW, full0 + i * 8, (w.k0 + i) * BK, f0, b2::kEvictNormal);
       }
-      b2::pdl_wait();
-      stamp(a, 3);
+    }
+    __syncwarp();
+    b2::pdl_wait();
+    if (lane == 0) stamp(a, 3);
+    if (b2::elect_one()) {
       for (int i = 0; i < pre; ++i) b2::tma_load_2d_pair(smem_base + i * stage_bytes + W_BYTES, &tmX, full0 + i * 8, (w.k0 + i) * BK, tok0 + x_half, b2::kEvictNormal);
-      int stage = pre == STAGES ? 0 : pre;
-      uint32_t phase = pre == STAGES ? 1 : 0;
-      int kb = w.k0 + pre;
-      for (;;) {
-        if (kb == w.k1) {
-          if (!next(w)) break;
-          place(w.tile, f0, tok0);
-          kb = w.k0;
-        }
-        if (!b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) break;
-        if (side == 0) b2::mbar_arrive_expect_tx(bar_full + stage * 8, 2 * stage_bytes);
+    }
+    __syncwarp();
+    int stage = pre == STAGES ? 0 : pre;
+    uint32_t phase = pre == STAGES ? 1 : 0;
+    int kb = w.k0 + pre;
+    for (;;) {
+      if (kb == w.k1) {
+        if (!next(w)) break;
+        place(w.tile, f0, tok0);
+        kb = w.k0;
+      }
+      if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_EMPTY))) break;
+      if (b2::elect_one()) {
         const uint32_t dst = smem_base + stage * stage_bytes;
+        if (side == 0) b2::mbar_arrive_expect_tx(bar_full + stage * 8, 2 * stage_bytes);
         b2::tma_load_2d_pair(dst, &tmW, full0 + stage * 8, kb * BK, f0, b2::kEvictNormal);
         b2::tma_load_2d_pair(dst + W_BYTES, &tmX, full0 + stage * 8, kb * BK, tok0 + x_half, b2::kEvictNormal);
-        ++kb;
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      __syncwarp();
+      ++kb;
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (even CTA of each pair) ----------------
-    if (lane == 0 && side == 0) {
+    // ---------------- MMA issuer (even CTA of each pair): the whole warp walks, one thread issues ----------------
+    if (side == 0) {
       const uint32_t idesc = b2::umma_idesc_bf16_pair(a.bn);
       const uint16_t both = static_cast<uint16_t>(3u << (cr & ~1));
       b2::pdl_wait();  // the pipeline's time limit must not include the wait for earlier kernels
@@ -293,24 +305,48 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       for (int t = 0; ok && next(w); ++t) {
         const int acc = t % T::ACC;
         if (MULTI && t >= T::ACC) {
-          if (!b2::mbar_wait(bar_drained + acc * 8, ((t / T::ACC) & 1) ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_TMEM_EMPTY)) break;
+          if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_drained + acc * 8, ((t / T::ACC) & 1) ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_TMEM_EMPTY))) break;
           b2::tc_fence_after();
         }
         const uint32_t d = tmem_base + acc * acc_cols;
-        for (int i = 0; i < w.k1 - w.k0; ++i) {
-          if (!b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_FULL)) { ok = false; break; }
-          if (t == 0 && i == 0) stamp(a, 1);
+        // Two stages a turn where the second has landed too: a turn's wait, vote and addresses take longer (about 350 clocks) than the
+        // four instructions of a stage
+        const int n = w.k1 - w.k0;
+        for (int i = 0; i < n;) {
+          if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_FULL))) { ok = false; break; }
+          if (t == 0 && i == 0 && lane == 0) stamp(a, 1);
+          const int next_stage = stage + 1 == STAGES ? 0 : stage + 1;
+          const uint32_t next_phase = phase ^ (next_stage == 0 ? 1u : 0u);
+          const bool two = i + 1 < n && __all_sync(0xffffffffu, b2::mbar_test(bar_full + next_stage * 8, next_phase));
           b2::tc_fence_after();
-          const uint64_t dw = b2::umma_smem_desc(smem_base + stage * stage_bytes);
-          const uint64_t dx = b2::umma_smem_desc(smem_base + stage * stage_bytes + W_BYTES);
+          if (b2::elect_one()) {
+            const uint32_t at = smem_base + stage * stage_bytes;
+            const uint64_t dw = b2::umma_smem_desc(at), dx = b2::umma_smem_desc(at + W_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) b2::umma_bf16_pair(d, dw + 2 * k, dx + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-          b2::umma_commit_pair(bar_empty + stage * 8, both);
+            for (int k = 0; k < BK / 16; ++k) b2::umma_bf16_pair(d, dw + 2 * k, dx + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+            b2::umma_commit_pair(bar_empty + stage * 8, both);
+            if (two) {
+              const uint32_t at2 = smem_base + next_stage * stage_bytes;
+              const uint64_t dw2 = b2::umma_smem_desc(at2), dx2 = b2::umma_smem_desc(at2 + W_BYTES);
+#pragma unroll
+              for (int k = 0; k < BK / 16; ++k) b2::umma_bf16_pair(d, dw2 + 2 * k, dx2 + 2 * k, idesc, 1u);
+              b2::umma_commit_pair(bar_empty + next_stage * 8, both);
+            }
+          }
+          __syncwarp();
+          if (two) {
+            i += 2;
+            stage = next_stage;
+            phase = next_phase;
+          } else {
+            ++i;
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) b2::umma_commit_pair(bar_done + acc * 8, both);
+        if (ok && b2::elect_one()) b2::umma_commit_pair(bar_done + acc * 8, both);
+        __syncwarp();
       }
-      stamp(a, 2);
+      if (lane == 0) stamp(a, 2);
     }
   }
 
