@@ -957,69 +957,76 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
 
   if (has_gemm) {
     if (warp == 0) {
-      // ---------------- TMA producer ----------------
-      if (lane == 0) {
-        const uint64_t polP = SWAP ? b2::kEvictFirst : b2::kEvictNormal;
-        const uint64_t polQ = SWAP ? b2::kEvictLast : b2::kEvictNormal;
-        const int n_units = work.n_units;
-        const int pre = n_units < STAGES ? n_units : STAGES;
-        // The weight tiles of the first stages depend on no earlier kernel: fetch them before the
-        // dependency wait, so that they are in flight (or landed) when the activations become valid.
-        Cursor cw = cursor_begin(work, a.tilesQ);
-        for (int i = 0; i < pre; ++i) {
+      // ---------------- TMA producer: the whole warp walks, one thread issues (as in b2_gemm_tile.cu) ----------------
+      const uint64_t polP = SWAP ? b2::kEvictFirst : b2::kEvictNormal;
+      const uint64_t polQ = SWAP ? b2::kEvictLast : b2::kEvictNormal;
+      const int n_units = work.n_units;
+      const int pre = n_units < STAGES ? n_units : STAGES;
+      // The weight tiles of the first stages depend on no earlier kernel: fetch them before the
+      // dependency wait, so that they are in flight (or landed) when the activations become valid.
+      Cursor cw = cursor_begin(work, a.tilesQ);
+      for (int i = 0; i < pre; ++i) {
+        if (b2::elect_one()) {
           const uint32_t fb = bar_full + i * 8;
           b2::mbar_arrive_expect_tx(fb, C::STAGE_BYTES);
           const uint32_t dst = smem_base + i * C::STAGE_BYTES;
           if (SWAP) b2::tma_load_2d(dst, &tmP, fb, cw.kb * BK, cw.tp * BM, polP);
           else b2::tma_load_2d(dst + C::P_BYTES, &tmQ, fb, cw.kb * BK, cw.tq * BN, polQ);
-          cursor_next(work, a.tilesQ, cw);
         }
-        b2::pdl_wait();
-        stamp(a, 3);
-        Cursor cx = cursor_begin(work, a.tilesQ);
-        for (int i = 0; i < pre; ++i) {
+        __syncwarp();
+        cursor_next(work, a.tilesQ, cw);
+      }
+      b2::pdl_wait();
+      if (lane == 0) stamp(a, 3);
+      Cursor cx = cursor_begin(work, a.tilesQ);
+      for (int i = 0; i < pre; ++i) {
+        if (b2::elect_one()) {
           const uint32_t fb = bar_full + i * 8;
           const uint32_t dst = smem_base + i * C::STAGE_BYTES;
           if (SWAP) b2::tma_load_2d(dst + C::P_BYTES, &tmQ, fb, cx.kb * BK, cx.tq * BN, polQ);
           else b2::tma_load_2d(dst, &tmP, fb, cx.kb * BK, cx.tp * BM, polP);
-          cursor_next(work, a.tilesQ, cx);
         }
-        int stage = pre == STAGES ? 0 : pre;
-        uint32_t phase = pre == STAGES ? 1 : 0;
-        for (int i = pre; i < n_units; ++i) {  // cx now stands at unit `pre`
-          if (!b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) break;
+        __syncwarp();
+        cursor_next(work, a.tilesQ, cx);
+      }
+      int stage = pre == STAGES ? 0 : pre;
+      uint32_t phase = pre == STAGES ? 1 : 0;
+      for (int i = pre; i < n_units; ++i) {  // cx now stands at unit `pre`
+        if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_EMPTY))) break;
+        if (b2::elect_one()) {
           const uint32_t fb = bar_full + stage * 8;
           b2::mbar_arrive_expect_tx(fb, C::STAGE_BYTES);
           const uint32_t dst = smem_base + stage * C::STAGE_BYTES;
           b2::tma_load_2d(dst, &tmP, fb, cx.kb * BK, cx.tp * BM, polP);
           b2::tma_load_2d(dst + C::P_BYTES, &tmQ, fb, cx.kb * BK, cx.tq * BN, polQ);
-          cursor_next(work, a.tilesQ, cx);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        cursor_next(work, a.tilesQ, cx);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     } else if (warp == 1) {
-      // ---------------- MMA issuer ----------------
-      if (lane == 0) {
-        constexpr uint32_t idesc = b2::umma_idesc_bf16(BN);
-        // The first stage cannot fill before the earlier kernels have completed (the activations are fetched after the
-        // producer's dependency wait): wait for them here, so that the pipeline's time limit measures the pipeline
-        // alone and not an earlier kernel that is itself waiting for a peer.
-        b2::pdl_wait();
-        int stage = 0;
-        uint32_t phase = 0;
-        int u = 0, seg = 0;
-        Seg s;
-        bool ok = true;
-        while (ok && next_seg(work, u, s)) {
-          const int acc = seg % ACC;
-          const uint32_t use = static_cast<uint32_t>(seg / ACC);  // how often this accumulator was used before
-          if (!b2::mbar_wait(bar_tempty + acc * 8, (use & 1) ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_TMEM_EMPTY)) break;
+      // ---------------- MMA issuer: likewise ----------------
+      constexpr uint32_t idesc = b2::umma_idesc_bf16(BN);
+      // The first stage cannot fill before the earlier kernels have completed (the activations are fetched after the
+      // producer's dependency wait): wait for them here, so that the pipeline's time limit measures the pipeline
+      // alone and not an earlier kernel that is itself waiting for a peer.
+      b2::pdl_wait();
+      int stage = 0;
+      uint32_t phase = 0;
+      int u = 0, seg = 0;
+      Seg s;
+      bool ok = true;
+      while (ok && next_seg(work, u, s)) {
+        const int acc = seg % ACC;
+        const uint32_t use = static_cast<uint32_t>(seg / ACC);  // how often this accumulator was used before
+        if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_tempty + acc * 8, (use & 1) ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_TMEM_EMPTY))) break;
+        b2::tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        for (int kb = s.kb0; kb < s.kb1; ++kb) {
+          if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_FULL))) { ok = false; break; }
+          if (seg == 0 && kb == s.kb0 && lane == 0) stamp(a, 1);
           b2::tc_fence_after();
-          const uint32_t d_tmem = tmem_base + acc * BN;
-          for (int kb = s.kb0; kb < s.kb1; ++kb) {
-            if (!b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_FULL)) { ok = false; break; }
-            if (seg == 0 && kb == s.kb0) stamp(a, 1);
-            b2::tc_fence_after();
+          if (b2::elect_one()) {
             const uint32_t sp = smem_base + stage * C::STAGE_BYTES;
             const uint64_t dp = b2::umma_smem_desc(sp);
             const uint64_t dq = b2::umma_smem_desc(sp + C::P_BYTES);
@@ -1029,14 +1036,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
               b2::umma_bf16(d_tmem, dp + 2 * k, dq + 2 * k, idesc, (kb > s.kb0 || k > 0) ? 1u : 0u);
             }
             b2::umma_commit(bar_empty + stage * 8);  // stage reusable once these MMAs have read it
-            if (++stage == STAGES) { stage = 0; phase ^= 1; }
           }
-          if (!ok) break;
-          b2::umma_commit(bar_tfull + acc * 8);
-          ++seg;
+          __syncwarp();
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        stamp(a, 2);
+        if (!ok) break;
+        if (b2::elect_one()) b2::umma_commit(bar_tfull + acc * 8);
+        __syncwarp();
+        ++seg;
       }
+      if (lane == 0) stamp(a, 2);
     } else {
       // ---------------- epilogue warps ----------------
       const int q = warp & 3;  // TMEM lane quadrant this warp may read
@@ -1170,7 +1179,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
 // Bound by latency: a launch streams 0.5-12 MB of weights, so set-up, one DRAM round trip, the cluster barriers and the exchange
 // are most of it.  The shared memory is therefore laid out for the tokens that a launch has (a fixed layout took a whole SM and
 // kept the next kernel out of it), only groups that hold tokens are exchanged, and nothing in the exchange divides by S:
-// 0.6B widths at one token qkv 5.3 -> 4.7 us, gate/up 6.1 -> 5.7; 8B widths down at 64 tokens 25.9 -> 24.9.
+// 0.6B widths at one token qkv 5.3 -> 4.7 us, gate/up 6.1 -> 5.7; 8B widths down at 64 tokens 25.9 -> 24.9.  A CTA's few K blocks are a
+// chain, so what issuing one takes counts (an elected thread of a uniform warp, see b2_gemm_tile.cu): 8B widths at 5 tokens qkv
+// 13.3 -> 11.8 us, o with its norm 12.0 -> 10.8, gate/up (stream-K kernel) 36.1 -> 34.2; at 64 tokens qkv 16.5 -> 14.9.
 // ---------------------------------------------------------------------------
 template <int BN>
 struct CfgCluster {
@@ -1263,53 +1274,75 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
   int pre_slot[PRE_ROWS];
 
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      const int pre = n_units < STAGES ? n_units : STAGES;
+    // ---------------- TMA producer: the whole warp walks, one thread issues (as in b2_gemm_tile.cu) ----------------
+    const int pre = n_units < STAGES ? n_units : STAGES;
+    if (b2::elect_one()) {
       for (int i = 0; i < pre; ++i) {  // weights do not depend on earlier kernels
         const uint32_t fb = bar_full + i * 8;
         b2::mbar_arrive_expect_tx(fb, C::STAGE_BYTES);
         b2::tma_load_2d(smem_base + i * C::STAGE_BYTES, &tmP, fb, (kb0 + i) * BK, tile * BM, b2::kEvictFirst);
       }
-      b2::pdl_wait();
-      stamp(a, 3);
+    }
+    __syncwarp();
+    b2::pdl_wait();
+    if (lane == 0) stamp(a, 3);
+    if (b2::elect_one()) {
       for (int i = 0; i < pre; ++i)
         b2::tma_load_2d(smem_base + i * C::STAGE_BYTES + C::P_BYTES, &tmQ, bar_full + i * 8, (kb0 + i) * BK, tok0, b2::kEvictLast);
-      int stage = pre == STAGES ? 0 : pre;
-      uint32_t phase = pre == STAGES ? 1 : 0;
-      for (int i = pre; i < n_units; ++i) {
-        if (!b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) break;
+    }
+    __syncwarp();
+    int stage = pre == STAGES ? 0 : pre;
+    uint32_t phase = pre == STAGES ? 1 : 0;
+    for (int i = pre; i < n_units; ++i) {
+      if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_EMPTY))) break;
+      if (b2::elect_one()) {
         const uint32_t fb = bar_full + stage * 8;
         b2::mbar_arrive_expect_tx(fb, C::STAGE_BYTES);
         const uint32_t dst = smem_base + stage * C::STAGE_BYTES;
         b2::tma_load_2d(dst, &tmP, fb, (kb0 + i) * BK, tile * BM, b2::kEvictFirst);
         b2::tma_load_2d(dst + C::P_BYTES, &tmQ, fb, (kb0 + i) * BK, tok0, b2::kEvictLast);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      __syncwarp();
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = b2::umma_idesc_bf16(BN);
-      b2::pdl_wait();  // the pipeline's time limit must not include the wait for earlier kernels
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int i = 0; i < n_units; ++i) {
-        if (!b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_FULL)) { ok = false; break; }
-        if (i == 0) stamp(a, 1);
-        b2::tc_fence_after();
-        const uint32_t sp = smem_base + stage * C::STAGE_BYTES;
-        const uint64_t dp = b2::umma_smem_desc(sp);
-        const uint64_t dq = b2::umma_smem_desc(sp + C::P_BYTES);
+    // ---------------- MMA issuer: likewise; two stages a turn where the second has landed too ----------------
+    constexpr uint32_t idesc = b2::umma_idesc_bf16(BN);
+    b2::pdl_wait();  // the pipeline's time limit must not include the wait for earlier kernels
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    auto multiply = [&](int st, bool first) {
+      const uint32_t sp = smem_base + st * C::STAGE_BYTES;
+      const uint64_t dp = b2::umma_smem_desc(sp);
+      const uint64_t dq = b2::umma_smem_desc(sp + C::P_BYTES);
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) b2::umma_bf16(tmem_base, dp + 2 * k, dq + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-        b2::umma_commit(bar_empty + stage * 8);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      for (int k = 0; k < BK / UMMA_K; ++k) b2::umma_bf16(tmem_base, dp + 2 * k, dq + 2 * k, idesc, (!first || k > 0) ? 1u : 0u);
+      b2::umma_commit(bar_empty + st * 8);
+    };
+    for (int i = 0; i < n_units;) {
+      if (!__all_sync(0xffffffffu, b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, PIPE_LIMIT_NS, B2_WAIT_SMEM_FULL))) { ok = false; break; }
+      if (i == 0 && lane == 0) stamp(a, 1);
+      const int next_stage = stage + 1 == STAGES ? 0 : stage + 1;
+      const uint32_t next_phase = phase ^ (next_stage == 0 ? 1u : 0u);
+      const bool two = i + 1 < n_units && __all_sync(0xffffffffu, b2::mbar_test(bar_full + next_stage * 8, next_phase));
+      b2::tc_fence_after();
+      if (b2::elect_one()) {
+        multiply(stage, i == 0);
+        if (two) multiply(next_stage, false);
       }
-      if (ok) b2::umma_commit(bar_tfull);
-      stamp(a, 2);
+      __syncwarp();
+      if (two) {
+        ++i;
+        stage = next_stage;
+        phase = next_phase;
+      }
+      ++i;
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
+    if (ok && b2::elect_one()) b2::umma_commit(bar_tfull);
+    __syncwarp();
+    if (lane == 0) stamp(a, 2);
   } else {
     // ---------------- epilogue, first half: hand every group of the accumulator to the CTA that owns it ----------------
     const int q = warp & 3;
