@@ -466,7 +466,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 //
 // Causal attention of many query tokens per sequence over keys and values in rows of a matrix (the qkv output) or in the paged
 // cache.  Bound: the exponentials and the tensor pipe, which take about the same time per block (16 exponentials and 4096
-// multiply-adds per clock and SM); one sequence of 8192 tokens, 16 heads, 478 us = 575 TFLOP/s.
+// multiply-adds per clock and SM); one sequence of 8192 tokens, 16 heads, 458 us = 601 TFLOP/s.
 //
 // A CTA takes 128 query tokens of one sequence for the two heads that share a KV head: both heads' scores come from the same
 // K block, and while the tensor cores work for one head, four warps turn the other's scores into probabilities.
@@ -476,7 +476,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 // Tensor memory: S of the two heads, then O of the two heads, 128 columns each.  O is rescaled whenever a row's maximum grows, so
 // that the largest probability is exactly 1.  (Rescaling only past a growth of 2^8 rounds it: against float64, scores of standard
 // deviation 3, 2048 tokens, the error was 2.13e-3 where flash-attn's is 1.76e-3, and is 1.77e-3 now; of that the output's own
-// rounding is 1.66e-3.  8192 tokens x 16 heads take 478 us instead of 446.)
+// rounding is 1.66e-3.  8192 tokens x 16 heads took 478 us instead of 446; 458 since the TMA and MMA warps walk whole, see b2_gemm_tile.cu.)
 // ---------------------------------------------------------------------------
 constexpr int PF_ROWS = 128, PF_KEYS = 128, PF_THREADS = 320;
 constexpr uint32_t PF_TILE = 128 * 128 * 2;                     // 128 rows of 128 bf16, as two 64-wide swizzled halves
@@ -564,11 +564,16 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   const int n = t0 < q_len && kv_len > 0 ? max(1, (min(kv_len, shift + min(q_len, t0 + PF_ROWS)) + PF_KEYS - 1) / PF_KEYS) : 0;  // key blocks
 
   if (warp == 0) {
-    if (lane == 0 && n > 0) {
-      b2::mbar_arrive_expect_tx(q_full, 2 * PF_TILE);
-      for (int h = 0; h < 2; ++h)
-        for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_q + h * PF_TILE + i * (PF_TILE / 2), &tmQ, q_full, (head + h) * 128 + i * 64, q0 + t0, b2::kEvictFirst);
+    // (the whole warp walks and one thread issues, here and in the next warp: operands then stay in uniform registers)
+    if (n > 0) {
+      if (b2::elect_one()) {
+        b2::mbar_arrive_expect_tx(q_full, 2 * PF_TILE);
+        for (int h = 0; h < 2; ++h)
+          for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_q + h * PF_TILE + i * (PF_TILE / 2), &tmQ, q_full, (head + h) * 128 + i * 64, q0 + t0, b2::kEvictFirst);
+      }
+      __syncwarp();
       const int x = kv_head * 128;
+      auto free = [&](uint32_t bar, uint32_t phase) { return __all_sync(0xffffffffu, b2::mbar_wait(bar, phase, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) != 0; };
       for (int j = 0; j < n; ++j) {
         const int st = j & 1;
         const uint32_t ph = ((j >> 1) & 1) ^ 1;
@@ -578,35 +583,44 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           y = max(0, __ldg(a.tables + static_cast<int64_t>(b) * a.bt_stride + min(blk, a.bt_width - 1))) * a.block_size + tok - blk * a.block_size;
           y = min(y, a.kv_rows - 1);  // (a bad table entry must not lead outside the cache)
         }
-        if (!b2::mbar_wait(k_empty + st * 8, ph, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) break;
-        b2::mbar_arrive_expect_tx(k_full + st * 8, PF_TILE);
-        for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_k + st * PF_TILE + i * (PF_TILE / 2), &tmK, k_full + st * 8, x + i * 64, y, b2::kEvictLast);
-        if (!b2::mbar_wait(v_empty + st * 8, ph, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) break;
-        b2::mbar_arrive_expect_tx(v_full + st * 8, PF_TILE);
-        for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_v + st * PF_TILE + i * (PF_TILE / 2), &tmV, v_full + st * 8, x + i * 64, y, b2::kEvictLast);
+        if (!free(k_empty + st * 8, ph)) break;
+        if (b2::elect_one()) {
+          b2::mbar_arrive_expect_tx(k_full + st * 8, PF_TILE);
+          for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_k + st * PF_TILE + i * (PF_TILE / 2), &tmK, k_full + st * 8, x + i * 64, y, b2::kEvictLast);
+        }
+        __syncwarp();
+        if (!free(v_empty + st * 8, ph)) break;
+        if (b2::elect_one()) {
+          b2::mbar_arrive_expect_tx(v_full + st * 8, PF_TILE);
+          for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_v + st * PF_TILE + i * (PF_TILE / 2), &tmV, v_full + st * 8, x + i * 64, y, b2::kEvictLast);
+        }
+        __syncwarp();
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (n > 0) {
       constexpr uint32_t idesc_s = b2::umma_idesc_bf16(PF_KEYS);
       constexpr uint32_t idesc_o = b2::umma_idesc_bf16(128) | (1u << 16);  // second operand MN-major
       auto wait = [&](uint32_t bar, uint32_t phase, int code) {
-        const bool ok = b2::mbar_wait(bar, phase, abort_flag, PF_LIMIT_NS, code);
+        const bool ok = __all_sync(0xffffffffu, b2::mbar_wait(bar, phase, abort_flag, PF_LIMIT_NS, code)) != 0;
         b2::tc_fence_after();
         return ok;
       };
-      auto scores = [&](int h, int st) {
+      auto scores = [&](int h, int st, bool last_of_block) {
+        if (b2::elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          b2::umma_bf16(tmem + h * 128, b2::umma_smem_desc(s_q + h * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3),
-                        b2::umma_smem_desc(s_k + st * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
-        b2::umma_commit(s_full + h * 8);
+          for (int k = 0; k < 8; ++k)
+            b2::umma_bf16(tmem + h * 128, b2::umma_smem_desc(s_q + h * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3),
+                          b2::umma_smem_desc(s_k + st * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
+          b2::umma_commit(s_full + h * 8);
+          if (last_of_block) b2::umma_commit(k_empty + st * 8);
+        }
+        __syncwarp();
       };
       bool ok = wait(q_full, 0, B2_WAIT_SMEM_FULL) && wait(k_full, 0, B2_WAIT_SMEM_FULL);
       if (ok) {
-        scores(0, 0);
-        scores(1, 0);
-        b2::umma_commit(k_empty);
+        scores(0, 0, false);
+        scores(1, 0, true);
       }
       for (int j = 0; ok && j < n; ++j) {
         const int st = j & 1, nx = (j + 1) & 1;
@@ -614,20 +628,22 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         for (int h = 0; ok && h < 2; ++h) {
           ok = wait(p_full + h * 8, j & 1, B2_WAIT_TMEM_EMPTY);
           if (!ok) break;
+          if (b2::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k)  // 16 tokens: 8 columns of P, 2048 bytes of V
-            umma_bf16_ts(tmem + 256 + h * 128, tmem + h * 128 + k * 8, umma_smem_desc_mn(s_v + st * PF_TILE + k * 2048), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-          b2::umma_commit(o_done + h * 8);
+            for (int k = 0; k < 8; ++k)  // 16 tokens: 8 columns of P, 2048 bytes of V
+              umma_bf16_ts(tmem + 256 + h * 128, tmem + h * 128 + k * 8, umma_smem_desc_mn(s_v + st * PF_TILE + k * 2048), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+            b2::umma_commit(o_done + h * 8);
+            if (h == 1) b2::umma_commit(v_empty + st * 8);
+          }
+          __syncwarp();
         }
         if (!ok) break;
-        b2::umma_commit(v_empty + st * 8);
         if (j + 1 < n) {
           ok = wait(k_full + nx * 8, ((j + 1) >> 1) & 1, B2_WAIT_SMEM_FULL);
           for (int h = 0; ok && h < 2; ++h) {
             ok = wait(o_done + h * 8, j & 1, B2_WAIT_TMEM_FULL);  // P of this block has been read: its columns may take the next scores
-            if (ok) scores(h, nx);
+            if (ok) scores(h, nx, h == 1);
           }
-          if (ok) b2::umma_commit(k_empty + nx * 8);
         }
       }
     }
