@@ -164,12 +164,11 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const uint16_t* __restric
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int m = static_cast<int>(i / vpr);
     const int v = static_cast<int>(i - static_cast<int64_t>(m) * vpr);
-    float g[8], u[8], o[8];
+    float g[8];
     unpack8(ldg_v4(x + m * ldx + v * 8), g);
-    unpack8(ldg_v4(x + m * ldx + I + v * 8), u);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = bf16_round(g[e] / (1.0f + expf(-g[e]))) * u[e];
-    stg_v4(out + static_cast<int64_t>(m) * I + v * 8, pack8(o));
+    const uint4 u = ldg_v4(x + m * ldx + I + v * 8);
+    const uint2 lo = b2::silu4({g[0], g[1], g[2], g[3]}), hi = b2::silu4({g[4], g[5], g[6], g[7]});
+    stg_v4(out + static_cast<int64_t>(m) * I + v * 8, make_uint4(b2::mul_bf16x2(lo.x, u.x), b2::mul_bf16x2(lo.y, u.y), b2::mul_bf16x2(hi.x, u.z), b2::mul_bf16x2(hi.y, u.w)));
   }
 }
 

@@ -103,14 +103,10 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return make_uint4(b2::pack_bf16(f[0], f[1]), b2::pack_bf16(f[2], f[3]), b2::pack_bf16(f[4], f[5]), b2::pack_bf16(f[6], f[7]));
 }
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-  const __nv_bfloat162 v = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
 // bf16(bf16(x * rstd) * w)
 __device__ __forceinline__ uint4 normed(const float (&x)[8], float rstd, const uint4& w) {
-  return make_uint4(mul_bf16x2(b2::pack_bf16(x[0] * rstd, x[1] * rstd), w.x), mul_bf16x2(b2::pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
-                    mul_bf16x2(b2::pack_bf16(x[4] * rstd, x[5] * rstd), w.z), mul_bf16x2(b2::pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
+  return make_uint4(b2::mul_bf16x2(b2::pack_bf16(x[0] * rstd, x[1] * rstd), w.x), b2::mul_bf16x2(b2::pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
+                    b2::mul_bf16x2(b2::pack_bf16(x[4] * rstd, x[5] * rstd), w.z), b2::mul_bf16x2(b2::pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
 }
 // token t of a staging buffer of head rows: 16 pieces of 16 bytes, piece index XORed with the token so that neither the
 // transposing stores nor the row reads meet in a bank

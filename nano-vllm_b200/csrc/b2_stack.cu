@@ -123,14 +123,10 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
   f[0] = b2::bf16_lo(v.x); f[1] = b2::bf16_hi(v.x); f[2] = b2::bf16_lo(v.y); f[3] = b2::bf16_hi(v.y);
   f[4] = b2::bf16_lo(v.z); f[5] = b2::bf16_hi(v.z); f[6] = b2::bf16_lo(v.w); f[7] = b2::bf16_hi(v.w);
 }
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-  const __nv_bfloat162 v = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
 // bf16(bf16(x * rstd) * w)
 __device__ __forceinline__ uint4 normed(const float (&x)[8], float rstd, const uint4& w) {
-  return make_uint4(mul_bf16x2(b2::pack_bf16(x[0] * rstd, x[1] * rstd), w.x), mul_bf16x2(b2::pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
-                    mul_bf16x2(b2::pack_bf16(x[4] * rstd, x[5] * rstd), w.z), mul_bf16x2(b2::pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
+  return make_uint4(b2::mul_bf16x2(b2::pack_bf16(x[0] * rstd, x[1] * rstd), w.x), b2::mul_bf16x2(b2::pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
+                    b2::mul_bf16x2(b2::pack_bf16(x[4] * rstd, x[5] * rstd), w.z), b2::mul_bf16x2(b2::pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
 }
 // exchanged words: from and to L2, where all SMs see them
 __device__ __forceinline__ uint4 ld_x4(const void* p) {
@@ -380,8 +376,8 @@ __device__ __forceinline__ void norm_project(int use) {
         if (i * 128 < span) {
           const uint2 nw = lds_v2(base + a.off_vec + (k0 + i * 128) * 2);
           sts_v2(xs + row * row_bytes(H) + (k0 + i * 128) * 2,
-                 mul_bf16x2(b2::pack_bf16(__uint_as_float(v[i].x) * rstd, __uint_as_float(v[i].y) * rstd), nw.x),
-                 mul_bf16x2(b2::pack_bf16(__uint_as_float(v[i].z) * rstd, __uint_as_float(v[i].w) * rstd), nw.y));
+                 b2::mul_bf16x2(b2::pack_bf16(__uint_as_float(v[i].x) * rstd, __uint_as_float(v[i].y) * rstd), nw.x),
+                 b2::mul_bf16x2(b2::pack_bf16(__uint_as_float(v[i].z) * rstd, __uint_as_float(v[i].w) * rstd), nw.y));
         }
     }
     __syncthreads();

@@ -107,6 +107,20 @@ def test_rmsnorm_golden(ops, golden_dir):
     assert ulp_mismatch_fraction(ops.rmsnorm(r["q"].to(DEV), r["norm_w"].to(DEV), 1e-6), r["q_normed"], 1) == 0.0
 
 
+def test_silu_of_every_gate(ops):
+    """All 65536 bf16 gates (ties, subnormals, infinities and NaN among them), in every place of a vector, times 1 and times another
+    value: the bits of the division and the exponential in fp32, rounded to bf16, then multiplied and rounded."""
+    gate = torch.arange(65536, dtype=torch.int32, device=DEV).to(torch.int16).view(torch.bfloat16)
+    act = (gate.float() / (1.0 + torch.exp(-gate.float()))).bfloat16()
+    for shift in (0, 1, 5):
+        g, a = gate.roll(shift).view(8, -1), act.roll(shift).view(8, -1)
+        for up in (1.0, -0.7109375):
+            u = torch.full_like(g, up)
+            got, want = ops.silu_and_mul(torch.cat([g, u], dim=1)), (a.float() * u.float()).bfloat16()
+            same = (got.view(torch.int16) == want.view(torch.int16)) | (got.isnan() & want.isnan())
+            assert same.all(), (g[~same][:8], got[~same][:8], want[~same][:8])
+
+
 def test_silu_and_mul(ops, golden_dir):
     d = torch.load(os.path.join(golden_dir, "col.pt"))
     for r in range(2):
