@@ -406,6 +406,10 @@ __device__ __forceinline__ void flush_rows(const GemmArgs& a, unsigned char* wbu
 // on nothing but those, so it is the same for every tensor-parallel split and can be regenerated on the host.
 // ---------------------------------------------------------------------------
 constexpr uint32_t SAMPLE_TAG = 0x53414D50u;
+// Epilogue warps of the sampler per tensor-memory quadrant: they share the quadrant's token rows.  A warp alone on its scheduler
+// had nothing to fill its latencies with (256 rows x 151936 x 1024, greedy / with temperatures: 150 / 239 us with one, 120 / 168
+// with two, 93 / 131 with four; as a plain GEMM 74).
+constexpr int SAMPLE_PARTS = 4;
 
 __host__ __device__ __forceinline__ void philox4x32_10(uint32_t (&c)[4], uint32_t k0, uint32_t k1) {
 #pragma unroll
@@ -433,43 +437,48 @@ __host__ __device__ __forceinline__ unsigned long long sample_key(uint32_t score
 
 // Scores that can still win wait here for their logarithms: a warp evaluates 32 of them at a time.
 struct SampleQueue {
-  uint4 entry[384];                           // token row, vocabulary entry, bf16-rounded logit, random bits
+  uint2 entry[160];                           // bf16 logit << 16 | token row << 8 | lane, random bits
   __align__(16) float limit[32], inv_t[32];   // of the chunk's token rows
 };
-__device__ __forceinline__ void sample_flush(const GemmArgs& a, SampleQueue* queue, int n, int lane, unsigned long long* cta_best) {
+__device__ __forceinline__ void sample_flush(const GemmArgs& a, SampleQueue* queue, int n, uint32_t vocab_id0, int lane, unsigned long long* cta_best) {
   __syncwarp();
   for (int i = lane; i < n; i += 32) {
-    const uint4 e = queue->entry[i];
-    float z = __uint_as_float(e.z);
-    if (a.temperatures != nullptr) z = z / __ldg(a.temperatures + e.x) + gumbel_from_bits(e.w);
-    atomicMax(cta_best + e.x, sample_key(__float_as_uint(z), static_cast<uint32_t>(a.vocab_offset) + e.y));
+    const uint2 e = queue->entry[i];
+    const uint32_t token = (e.x >> 8) & 255u;
+    float z = __uint_as_float(e.x & 0xffff0000u);
+    if (a.temperatures != nullptr) z = z / __ldg(a.temperatures + token) + gumbel_from_bits(e.y);
+    atomicMax(cta_best + token, sample_key(__float_as_uint(z), vocab_id0 + (e.x & 31u)));
   }
   __syncwarp();
 }
 
-// All token rows of one vocabulary entry per lane (feature-lane layout): group g of the tile's columns, tokens 8 g .. 8 g + 7,
-// comes from load(g), requested one group ahead.
+// A quarter of the token rows of one vocabulary entry per lane (feature-lane layout): group g of the tile's columns, tokens
+// 8 g .. 8 g + 7, comes from load(g), requested one group ahead; part p of SAMPLE_PARTS has the chunks p, p + SAMPLE_PARTS, ...
+// of 32 tokens.
 // Bound: the instructions per score, of which the two logarithms, the division and the exchange between the lanes were nine
 // tenths, and their fetching: unrolled over 32 tokens the code streamed from the instruction cache's outer level (577 us for 256
-// rows of 1024 features, whose weights take 48 us to read).  A score is z / T - log(-log u) with 1 - u = (c + 1/2) 2^-23 and c
-// the complement of the 23 random bits, and -log(-log u) <= -log(1 - u) <= (clz(c) - 8) log 2.  So a few integer operations
-// bound it from above, and only what reaches the best score its row has in this CTA so far is queued for the exact evaluation
-// - a handful per row (NaN included: it wins).  While a row has no score yet the bound from below takes its place: for u >= 1/2,
-// -log u <= 2 log 2 (1 - u), hence -log(-log u) >= (clz(c) - 9) log 2 - 0.3267.
+// rows of 1024 features, whose weights take 48 us to read).  A score is z / T - log(-log u) with w = 1 - u = (c + 1/2) 2^-23 and
+// c the complement of the 23 random bits, and -log(-log u) <= -log w.  A float's bits, as a number, are a chord of its binary
+// logarithm: log2 w lies 0 to 0.0861 above bits(w) 2^-23 - 127.  So a few integer operations bound the score from above (the
+// bits less their last byte, put under the exponent of 2^23), and only what reaches the best score its row has in this CTA so
+// far is queued for the exact evaluation - a handful per row (NaN included: it wins).  While a row has no score yet the bound
+// from below takes its place: for u >= 1/2, -log u <= 2 log 2 w, hence -log(-log u) >= -log w - 0.3267, 0.0597 below the chord.
 template <class Load>
-__device__ __forceinline__ void sample_feature_lanes(const GemmArgs& a, Load&& load, int feature, int lane, unsigned int call,
+__device__ __forceinline__ void sample_feature_lanes(const GemmArgs& a, Load&& load, int part, int feature, int lane, unsigned int call,
                                                      unsigned long long* cta_best, SampleQueue* queue) {
   const bool live = feature < a.N;
-  const uint32_t vocab_id = static_cast<uint32_t>(a.vocab_offset + feature);
+  const uint32_t vocab_id = static_cast<uint32_t>(a.vocab_offset + feature), vocab_id0 = vocab_id - lane;
   const float bias = (a.bias != nullptr && live) ? __uint_as_float(static_cast<uint32_t>(a.bias[feature]) << 16) : 0.f;
   const bool noisy = a.temperatures != nullptr;
   const int groups = (a.M + 7) >> 3;
+  if (part * 4 >= groups) return;
   int count = 0;
   bool fresh = false;
   float next[8];
-  load(0, next);
+  load(part * 4, next);
 #pragma unroll 1
-  for (int g = 0; g < groups; ++g) {
+  for (int g = part * 4, after; g < groups; g = after) {
+    after = (g & 3) < 3 ? g + 1 : g + 1 + (SAMPLE_PARTS - 1) * 4;
     const int j0 = (g & 3) * 8;
     if (j0 == 0) {
       // rows 8 g + l, by lane l, for all lanes: the best score here (-inf: none yet, +inf: no such row), the inverse temperature
@@ -502,49 +511,50 @@ __device__ __forceinline__ void sample_feature_lanes(const GemmArgs& a, Load&& l
       limit[4 * h] = l4.x; limit[4 * h + 1] = l4.y; limit[4 * h + 2] = l4.z; limit[4 * h + 3] = l4.w;
       it[4 * h] = t4.x; it[4 * h + 1] = t4.y; it[4 * h + 2] = t4.z; it[4 * h + 3] = t4.w;
     }
-    float z[8], upper[8], lower[8];
+    float z[8], upper[8], gap[8];
     b2::tc_wait_ld(next);
 #pragma unroll
     for (int i = 0; i < 8; ++i) z[i] = b2::bf16_round(next[i] + bias);  // the logit as the unfused path stores it
-    if (g + 1 < groups) load(g + 1, next);
+    if (after < groups) load(after, next);
+    bool may = false;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      upper[i] = lower[i] = z[i];
+      upper[i] = z[i];
       if (noisy) {
-        const uint32_t bits = r[i >> 2][i & 3];
-        const float zt = z[i] * it[i], n = static_cast<float>(__clz(~bits >> 9));
-        const float slack = fmaf(fabsf(zt), 1e-6f, 1e-3f);  // covers the roundings of both sides
-        upper[i] = zt + slack + fmaf(n, 0.6931473f, -8.f * 0.6931471f);
-        lower[i] = (bits >> 31) ? zt - slack + fmaf(n, 0.6931471f, -9.f * 0.6931473f - 0.3268f) : -INFINITY;
+        const float zt = z[i] * it[i], w = __uint_as_float((~r[i >> 2][i & 3] >> 9) | 0x3f800000u) - 0.99999994f;  // (c + 1/2) 2^-23, exactly
+        gap[i] = fmaf(__uint_as_float(__byte_perm(__float_as_uint(w), 0x4bu, 0x4321)), -0.6931472f / 32768.f, 383.f * 0.6931472f);
+        upper[i] = fmaf(fabsf(zt), 1e-6f, zt) + (gap[i] + 1e-3f);  // (a millionth and a thousandth cover the roundings of both sides)
       }
+      may |= !(upper[i] < limit[i]);
     }
     if (fresh) {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         if (limit[i] == -INFINITY) {  // (the same in all lanes)
-          const int o = __float_as_int(live ? lower[i] : -INFINITY);
+          float lower = z[i];
+          if (noisy) lower = (r[i >> 2][i & 3] >> 31) ? fmaf(fabsf(lower * it[i]), -1e-6f, lower * it[i]) + (gap[i] - 0.3878f) : -INFINITY;
+          const int o = __float_as_int(live ? lower : -INFINITY);
           const int m = __reduce_max_sync(0xffffffffu, o >= 0 ? o : o ^ 0x7fffffff);  // order-preserving as a signed integer
           limit[i] = __int_as_float(m >= 0 ? m : m ^ 0x7fffffff);
         }
     }
-    uint32_t may = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) may |= (live && !(upper[i] < limit[i]) && g * 8 + i < a.M) ? 1u << i : 0u;
-    if (__any_sync(0xffffffffu, may != 0u)) {
+    if (__any_sync(0xffffffffu, may)) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const bool in = (may >> i) & 1u;
+        const bool in = live && !(upper[i] < limit[i]) && g * 8 + i < a.M;
         const uint32_t who = __ballot_sync(0xffffffffu, in);
-        if (in) queue->entry[count + __popc(who & ((1u << lane) - 1))] = make_uint4(g * 8 + i, feature, __float_as_uint(z[i]), r[i >> 2][i & 3]);
-        count += __popc(who);
-      }
-      if (count > 128) {  // room for 8 x 32 more
-        sample_flush(a, queue, count, lane, cta_best);
-        count = 0;
+        if (who != 0u) {
+          if (in) queue->entry[count + __popc(who & ((1u << lane) - 1))] = make_uint2(__float_as_uint(z[i]) | (g * 8 + i) << 8 | lane, r[i >> 2][i & 3]);
+          count += __popc(who);
+        }
+        if ((i & 3) == 3 && count > 32) {  // room for 4 x 32 more
+          sample_flush(a, queue, count, vocab_id0, lane, cta_best);
+          count = 0;
+        }
       }
     }
   }
-  if (count > 0) sample_flush(a, queue, count, lane, cta_best);
+  if (count > 0) sample_flush(a, queue, count, vocab_id0, lane, cta_best);
 }
 
 // One 32-column chunk c of a tile leaves the registers.  Feature-lane layout (SWAP): stored at once.
@@ -885,7 +895,7 @@ struct SampleTable<EPI_SAMPLE> {
     return table;
   }
   __device__ static __forceinline__ SampleQueue* queues() {
-    __shared__ SampleQueue queue[4];
+    __shared__ SampleQueue queue[4 * SAMPLE_PARTS];
     return queue;
   }
 };
@@ -893,8 +903,11 @@ struct SampleTable<EPI_SAMPLE> {
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
+template <int EPI>
+constexpr int GEMM_THREADS = EPI == EPI_SAMPLE ? 64 + 128 * SAMPLE_PARTS : NUM_THREADS;
+
 template <int BN, bool SWAP, int EPI>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(GEMM_THREADS<EPI>, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ, const GemmArgs a) {
   using C = Cfg<BN>;
   constexpr int STAGES = C::STAGES;
@@ -931,14 +944,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
     }
     for (int i = 0; i < ACC; ++i) {
       b2::mbar_init(bar_tfull + i * 8, 1);
-      b2::mbar_init(bar_tempty + i * 8, 4);
+      b2::mbar_init(bar_tempty + i * 8, (GEMM_THREADS<EPI> - 64) / 32);
     }
     *abort_flag = 0;
     b2::mbar_fence_init();
   }
   SampleQueue* const queues = SampleTable<EPI>::queues();
   if constexpr (EPI == EPI_SAMPLE)
-    for (int t = threadIdx.x; t < 256; t += NUM_THREADS) cta_best[t] = 0ull;
+    for (int t = threadIdx.x; t < 256; t += GEMM_THREADS<EPI>) cta_best[t] = 0ull;
   if (warp == 1 && has_gemm) {
     b2::tmem_alloc(b2::smem_u32(tmem_slot), C::TMEM_COLS);
     b2::tmem_relinquish();
@@ -1049,6 +1062,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
     } else {
       // ---------------- epilogue warps ----------------
       const int q = warp & 3;  // TMEM lane quadrant this warp may read
+      const int part = (warp - 2) >> 2;  // (0 but for the sampler)
+      constexpr int PARTS = EPI == EPI_SAMPLE ? SAMPLE_PARTS : 1;
       unsigned char* wbuf = smem + STAGES * C::STAGE_BYTES + 256 + q * STAGING_BYTES_PER_WARP;  // token-row layout only
       b2::pdl_wait();
       if (is_push(EPI)) parity = *reinterpret_cast<volatile unsigned int*>(&a.dstate->rowpar_seq) & 1u;
@@ -1066,7 +1081,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
         const bool whole = (s.kb0 == 0 && s.kb1 == KB);
         if (whole) {
           if constexpr (EPI == EPI_SAMPLE) {
-            sample_feature_lanes(a, [&](int g, float (&v)[8]) { b2::tmem_ld_32x8(taddr + g * 8, v); }, p_row, lane, sample_call, cta_best, queues + q);
+            sample_feature_lanes(a, [&](int g, float (&v)[8]) { b2::tmem_ld_32x8(taddr + g * 8, v); }, part, p_row, lane, sample_call, cta_best,
+                                 queues + warp - 2);
           } else {
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
@@ -1084,11 +1100,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
           // tile's fp32 accumulation slot (vector reductions that complete in L2; nobody waits for them);
           // the contributor that arrives last at the tile's counter reads the sum once, puts the slot
           // back to zero for the next launch, and writes the output.  The slot of a split tile is indexed
-          // by its first contributor, which is unique among split tiles.
+          // by its first contributor, which is unique among split tiles.  (The sampler's warps of a quadrant share its columns
+          // and a byte each of its counter; a grid has fewer CTAs than a byte counts.)
           const int c_first = work.part.cta_of(s.tile * KB), c_last = work.part.cta_of(s.tile * KB + KB - 1);
           float* slot = a.ws + (static_cast<size_t>(c_first) * 4 + q) * (BN * 32) + lane * 4;
 #pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
+          for (int c = part; c < BN / 32; c += PARTS) {
             uint32_t r[32];
             b2::tmem_ld_32x32(taddr + c * 32, r);
             b2::tc_wait_ld();
@@ -1101,11 +1118,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
           __threadfence();
           __syncwarp();
           int old = 0;
-          if (lane == 0) old = atomicAdd(a.counters + s.tile * 4 + q, 1);
+          if (lane == 0) old = atomicAdd(a.counters + s.tile * 4 + q, static_cast<int>(1u << (part * 8)));
           old = __shfl_sync(0xffffffffu, old, 0);
+          if (PARTS > 1) old = (old >> (part * 8)) & 255;
           if (old == c_last - c_first) {
             __threadfence();
-            if (lane == 0) a.counters[s.tile * 4 + q] = 0;
+            if (PARTS > 1) {
+              if (lane == 0) atomicSub(a.counters + s.tile * 4 + q, static_cast<int>(static_cast<uint32_t>(c_last - c_first + 1) << (part * 8)));
+            } else if (lane == 0) {
+              a.counters[s.tile * 4 + q] = 0;
+            }
             if constexpr (EPI == EPI_SAMPLE) {
               sample_feature_lanes(
                   a,
@@ -1117,7 +1139,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
                       *reinterpret_cast<float4*>(p) = make_float4(0.f, 0.f, 0.f, 0.f);
                     }
                   },
-                  p_row, lane, sample_call, cta_best, queues + q);
+                  part, p_row, lane, sample_call, cta_best, queues + warp - 2);
               // (columns past the last token have only had zeros added)
             } else {
 #pragma unroll 1
@@ -1161,7 +1183,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
   if (warp == 1 && has_gemm) b2::tmem_dealloc(tmem_base, C::TMEM_COLS);
   if constexpr (EPI == EPI_SAMPLE) {
     // the CTA's best key per token row joins the launch-wide table (feature-lane layout: one token tile, row = token)
-    for (int t = threadIdx.x; t < BN; t += NUM_THREADS)
+    for (int t = threadIdx.x; t < BN; t += GEMM_THREADS<EPI>)
       if (t < a.M && cta_best[t] != 0ull) atomicMax(a.sample_keys + t, cta_best[t]);
   }
 
@@ -1777,7 +1799,7 @@ int launch_inst(const CUtensorMap& tmP, const CUtensorMap& tmQ, const GemmArgs& 
     return B2_OK;
   });
   if (crc != B2_OK) return crc;
-  B2_CUDA(b2_launch(gemm_kernel<BN, SWAP, EPI>, dim3(grid), dim3(NUM_THREADS), smem_bytes, stream, tmP, tmQ, args));
+  B2_CUDA(b2_launch(gemm_kernel<BN, SWAP, EPI>, dim3(grid), dim3(GEMM_THREADS<EPI>), smem_bytes, stream, tmP, tmQ, args));
   return B2_OK;
 }
 

@@ -78,6 +78,21 @@ def test_temperature_draws_match_oracle_noise(fresh_runtime, rows, vocab, hidden
     _check_picks(tokens, logits[::2], temps[::2], O.fused_sampler_noise(SEED, 3, idx.numel(), vocab), "row_index")
 
 
+@pytest.mark.parametrize("rows,vocab,hidden", [(31, 2056, 64), (33, 640, 1024), (96, 5000, 512), (129, 19200, 512), (225, 40000, 128)])
+def test_flat_logits_leave_the_draw_to_the_noise(fresh_runtime, rows, vocab, hidden):
+    """Every chunk of 32 rows is another warp's, in whole tiles and in tiles whose K range is cut; the bounds on the noise decide."""
+    ops, rt = fresh_runtime(vocab, hidden)
+    h, w = _case(rows, vocab, hidden, seed=rows, scale=0.05)
+    hd, wd = h.to(DEV), w.to(DEV)
+    temps = torch.linspace(0.5, 2.0, rows).to(DEV)
+    logits = ops.lm_head(hd, wd, None).clone()
+    for call in range(2):
+        tokens = ops.lm_head_sample(hd, wd, None, temps, SEED)
+        torch.cuda.synchronize()
+        _check_picks(tokens, logits, temps, O.fused_sampler_noise(SEED, call, rows, vocab), f"call {call}")
+    rt.check_status()
+
+
 def test_draw_frequencies_follow_softmax(fresh_runtime):
     vocab, hidden, rows, calls, temp = 512, 128, 64, 60, 0.7
     ops, rt = fresh_runtime(vocab, hidden, max_seqs=64)
