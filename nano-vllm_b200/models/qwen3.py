@@ -153,6 +153,8 @@ class Qwen3Model(nn.Module):
                 return None
             if (layer.input_layernorm.eps, layer.post_attention_layernorm.eps, attn.rms_norm_eps) != (self.norm.eps, self.norm.eps, first.self_attn.rms_norm_eps):
                 return None
+            if attn.attn.scale != first.self_attn.attn.scale:
+                return None
             layers.append((attn.qkv_proj.weight, attn.o_proj.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight, layer.input_layernorm.weight,
                            layer.post_attention_layernorm.weight, attn.q_norm.weight, attn.k_norm.weight, attn.attn.k_cache, attn.attn.v_cache))
         attn = first.self_attn

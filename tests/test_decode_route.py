@@ -1,0 +1,48 @@
+"""Which decode steps the model hands to the one-launch step, and what with.  The launch itself is replaced: no GPU needed."""
+import pytest
+import torch
+
+
+@pytest.fixture
+def step(pkg, monkeypatch):
+    """A small model of stock layers, and a function that runs the decision for a decode step: what ops.decode_stack was called
+    with, or None where the layers would run one by one."""
+    from nanovllm_b200 import ops
+    from nanovllm_b200.engine.model_runner import ModelConfig
+    from nanovllm_b200.models.qwen3 import Qwen3Model
+    from nanovllm_b200.utils.context import reset_context, set_context
+    model = Qwen3Model(ModelConfig(hidden_size=64, num_attention_heads=2, num_key_value_heads=1, head_dim=32, intermediate_size=64, num_hidden_layers=3, vocab_size=16,
+                                   max_position_embeddings=64))
+    for layer in model.layers:
+        layer.self_attn.attn.k_cache = layer.self_attn.attn.v_cache = torch.zeros(2, 16, 1, 32)
+    calls = []
+    monkeypatch.setattr(ops, "decode_stack", lambda *a: calls.append(a) or "normed")
+
+    def run(rows=2):
+        calls.clear()
+        ints = torch.ones(rows, dtype=torch.int32)
+        set_context(False, slot_mapping=ints, context_lens=ints, block_tables=ints.view(-1, 1))
+        try:
+            out = model._decode_in_one_launch(torch.zeros(rows, 64), torch.zeros(rows, dtype=torch.int64))
+        finally:
+            reset_context()
+        assert out == ("normed" if calls else None)
+        return calls[0] if calls else None
+
+    run.model = model
+    return run
+
+
+def test_stock_layers_go_in_one_launch(step):
+    call = step()
+    assert len(call[2]) == 3 and call[10] == 32 ** -0.5
+
+
+def test_scale_of_a_single_layer(step):
+    """The launch takes one scale of attention for all layers."""
+    attns = [layer.self_attn.attn for layer in step.model.layers]
+    attns[1].scale *= 2
+    assert step() is None
+    attns[0].scale *= 2
+    attns[2].scale *= 2
+    assert step()[10] == 2 * 32 ** -0.5
