@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.nn.modules import module as nn_module
 
 from .. import ops
 from ..layers.activation import SiluAndMul
@@ -143,6 +144,8 @@ class Qwen3Model(nn.Module):
         ctx = get_context()
         if ctx.is_prefill or ctx.context_lens is None or ctx.slot_mapping is None or ctx.block_tables is None or Attention.backend != "flash_attn":
             return None
+        if any((nn_module._global_forward_hooks, nn_module._global_forward_pre_hooks, nn_module._global_backward_hooks, nn_module._global_backward_pre_hooks)):
+            return None  # (hooks for the calls of all modules)
         first = self.layers[0]
         layers = []
         for layer in self.layers:
@@ -174,7 +177,7 @@ def _is_stock(layer: nn.Module) -> bool:
         return False
     if attn.qkv_proj.bias is not None or type(layer.input_layernorm) is not RMSNorm or type(layer.post_attention_layernorm) is not RMSNorm:
         return False
-    return not any(m._forward_hooks or m._forward_pre_hooks for m in (layer, layer.input_layernorm))
+    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (layer, layer.input_layernorm))
 
 
 class Qwen3ForCausalLM(nn.Module):

@@ -46,3 +46,27 @@ def test_scale_of_a_single_layer(step):
     attns[0].scale *= 2
     attns[2].scale *= 2
     assert step()[10] == 2 * 32 ** -0.5
+
+
+def _ignore(*_):
+    return None
+
+
+@pytest.mark.parametrize("register", ["register_module_forward_pre_hook", "register_module_forward_hook", "register_module_full_backward_pre_hook",
+                                      "register_module_full_backward_hook"])
+def test_hooks_for_all_modules(step, register):
+    handle = getattr(torch.nn.modules.module, register)(_ignore)
+    try:
+        assert step() is None
+    finally:
+        handle.remove()
+    assert step() is not None
+
+
+@pytest.mark.parametrize("register", ["register_forward_pre_hook", "register_forward_hook", "register_full_backward_pre_hook", "register_full_backward_hook"])
+@pytest.mark.parametrize("where", ["layers.1", "layers.0.input_layernorm"])
+def test_hooks_of_a_module(step, register, where):
+    handle = getattr(step.model.get_submodule(where), register)(_ignore)
+    assert step() is None
+    handle.remove()
+    assert step() is not None
