@@ -166,18 +166,30 @@ class Qwen3Model(nn.Module):
                                 attn.rotary_emb.cos_sin_cache, ctx.context_lens, ctx.slot_mapping, ctx.block_tables)
 
 
+# the methods that a step through the layers calls
+_STEP_METHODS = {cls: {name: getattr(cls, name) for name in names} for cls, names in {
+    Qwen3DecoderLayer: ("forward",), Qwen3Attention: ("attention_output",), Qwen3MLP: ("activation",), Attention: ("attend",), RMSNorm: ("forward", "rms_forward"),
+    RowParallelLinear: ("forward_fused",), MergedColumnParallelLinear: ("forward_silu_mul", "paired_weight")}.items()}
+
+
+def _unchanged(module: nn.Module, cls: type) -> bool:
+    """A module of this class itself, whose methods have not been replaced on the object or on the class."""
+    return type(module) is cls and all(name not in module.__dict__ and getattr(cls, name) is method for name, method in _STEP_METHODS[cls].items())
+
+
 def _is_stock(layer: nn.Module) -> bool:
     """A decoder layer made of this file's modules, whose calls nothing listens to."""
-    if type(layer) is not Qwen3DecoderLayer or type(layer.self_attn) is not Qwen3Attention or type(layer.mlp) is not Qwen3MLP:
+    if not _unchanged(layer, Qwen3DecoderLayer) or not _unchanged(layer.self_attn, Qwen3Attention) or not _unchanged(layer.mlp, Qwen3MLP):
         return False
     attn, mlp = layer.self_attn, layer.mlp
-    if type(attn.attn) is not Attention or type(attn.o_proj) is not RowParallelLinear or type(mlp.down_proj) is not RowParallelLinear:
+    if not _unchanged(attn.attn, Attention) or not _unchanged(attn.o_proj, RowParallelLinear) or not _unchanged(mlp.down_proj, RowParallelLinear):
         return False
-    if type(mlp.gate_up_proj) is not MergedColumnParallelLinear or not mlp.gate_up_proj.paired or attn.o_proj.bias is not None or mlp.down_proj.bias is not None:
+    if not _unchanged(mlp.gate_up_proj, MergedColumnParallelLinear) or not mlp.gate_up_proj.paired or attn.o_proj.bias is not None or mlp.down_proj.bias is not None:
         return False
-    if attn.qkv_proj.bias is not None or type(layer.input_layernorm) is not RMSNorm or type(layer.post_attention_layernorm) is not RMSNorm:
+    if attn.qkv_proj.bias is not None or not _unchanged(layer.input_layernorm, RMSNorm) or type(layer.post_attention_layernorm) is not RMSNorm:
         return False
-    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (layer, layer.input_layernorm))
+    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or m._compiled_call_impl is not None
+                   for m in (layer, layer.input_layernorm))
 
 
 class Qwen3ForCausalLM(nn.Module):

@@ -70,3 +70,29 @@ def test_hooks_of_a_module(step, register, where):
     assert step() is None
     handle.remove()
     assert step() is not None
+
+
+METHODS = [("layers.1", "forward"), ("layers.0.input_layernorm", "forward"), ("layers.0.input_layernorm", "rms_forward"), ("layers.2.self_attn", "attention_output"),
+           ("layers.2.self_attn.attn", "attend"), ("layers.1.self_attn.o_proj", "forward_fused"), ("layers.1.mlp", "activation"),
+           ("layers.1.mlp.gate_up_proj", "forward_silu_mul"), ("layers.1.mlp.gate_up_proj", "paired_weight"), ("layers.1.mlp.down_proj", "forward_fused")]
+
+
+@pytest.mark.parametrize("where,name", METHODS)
+@pytest.mark.parametrize("of", ["object", "class"])
+def test_replaced_methods(step, monkeypatch, where, name, of):
+    module = step.model.get_submodule(where)
+    method = getattr(type(module), name)
+    with monkeypatch.context() as m:
+        if of == "object":
+            module.__dict__[name] = lambda *a: method(module, *a)
+        else:
+            m.setattr(type(module), name, lambda self, *a: method(self, *a))
+        assert step() is None
+    module.__dict__.pop(name, None)
+    assert step() is not None
+
+
+@pytest.mark.parametrize("where", ["layers.1", "layers.0.input_layernorm"])
+def test_modules_compiled_in_place(step, where):
+    step.model.get_submodule(where).compile(backend="eager")
+    assert step() is None
