@@ -137,33 +137,39 @@ class Qwen3Model(nn.Module):
             normed, residual = layer(positions, normed, residual, next_norm)
         return normed
 
-
     def _decode_in_one_launch(self, embedded: torch.Tensor, positions: torch.Tensor) -> torch.Tensor | None:
         """All layers of a decode step through ops.decode_stack; None where that does not apply: the layers then run one by one.
         It computes what the stock layers compute, so every layer must be one, without hooks of its own."""
         ctx = get_context()
         if ctx.is_prefill or ctx.context_lens is None or ctx.slot_mapping is None or ctx.block_tables is None or Attention.backend != "flash_attn":
             return None
-        if any((nn_module._global_forward_hooks, nn_module._global_forward_pre_hooks, nn_module._global_backward_hooks, nn_module._global_backward_pre_hooks)):
-            return None  # (hooks for the calls of all modules)
         first = self.layers[0]
+        if not _stock_classes() or not _is_stock(first) or embedded.dim() != 2 or first.self_attn.attn.k_cache.dim() != 4:
+            return None
+        # the shape next: of a step that is not served no layers are gathered (28 of them take 300 us, and the native side checks them too)
+        attn, inter = first.self_attn, first.mlp.down_proj.weight.shape[1]
+        served = ops.decode_stack_served(embedded.shape[0], len(self.layers), embedded.shape[1], attn.num_heads, attn.num_kv_heads, attn.head_dim, inter,
+                                         attn.attn.k_cache.shape[1])
+        layers = self._stock_layers() if served else []
+        if layers is None:
+            return None
+        return ops.decode_stack(embedded, positions, layers, self.norm.weight, attn.num_heads, attn.num_kv_heads, attn.head_dim, inter, self.norm.eps,
+                                attn.rms_norm_eps, attn.attn.scale, attn.rotary_emb.cos_sin_cache, ctx.context_lens, ctx.slot_mapping, ctx.block_tables)
+
+    def _stock_layers(self) -> list[tuple] | None:
+        """What ops.decode_stack takes of every layer; None if one of them is not a stock layer or differs from the others."""
+        first = self.layers[0].self_attn
+        same = (first.rotary_emb.cos_sin_cache, self.norm.eps, self.norm.eps, first.rms_norm_eps, first.attn.scale)
         layers = []
         for layer in self.layers:
             if not _is_stock(layer):
                 return None
-            attn, mlp = layer.self_attn, layer.mlp
-            if attn.qkv_bias or attn.rotary_emb.cos_sin_cache is not first.self_attn.rotary_emb.cos_sin_cache:
+            attn, mlp, kv, in_norm, post_norm = layer.self_attn, layer.mlp, layer.self_attn.attn, layer.input_layernorm, layer.post_attention_layernorm
+            if attn.qkv_bias or attn.rotary_emb.cos_sin_cache is not same[0] or (in_norm.eps, post_norm.eps, attn.rms_norm_eps, kv.scale) != same[1:]:
                 return None
-            if (layer.input_layernorm.eps, layer.post_attention_layernorm.eps, attn.rms_norm_eps) != (self.norm.eps, self.norm.eps, first.self_attn.rms_norm_eps):
-                return None
-            if attn.attn.scale != first.self_attn.attn.scale:
-                return None
-            layers.append((attn.qkv_proj.weight, attn.o_proj.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight, layer.input_layernorm.weight,
-                           layer.post_attention_layernorm.weight, attn.q_norm.weight, attn.k_norm.weight, attn.attn.k_cache, attn.attn.v_cache))
-        attn = first.self_attn
-        return ops.decode_stack(embedded, positions, layers, self.norm.weight, attn.num_heads, attn.num_kv_heads, attn.head_dim,
-                                first.mlp.down_proj.weight.shape[1], self.norm.eps, attn.rms_norm_eps, attn.attn.scale,
-                                attn.rotary_emb.cos_sin_cache, ctx.context_lens, ctx.slot_mapping, ctx.block_tables)
+            layers.append((attn.qkv_proj.weight, attn.o_proj.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight, in_norm.weight, post_norm.weight,
+                           attn.q_norm.weight, attn.k_norm.weight, kv.k_cache, kv.v_cache))
+        return layers
 
 
 # the methods that a step through the layers calls
@@ -172,24 +178,32 @@ _STEP_METHODS = {cls: {name: getattr(cls, name) for name in names} for cls, name
     RowParallelLinear: ("forward_fused",), MergedColumnParallelLinear: ("forward_silu_mul", "paired_weight")}.items()}
 
 
-def _unchanged(module: nn.Module, cls: type) -> bool:
-    """A module of this class itself, whose methods have not been replaced on the object or on the class."""
-    return type(module) is cls and all(name not in module.__dict__ and getattr(cls, name) is method for name, method in _STEP_METHODS[cls].items())
+def _stock_classes() -> bool:
+    """Nobody has replaced a method that a step calls on its class, or listens to the calls of all modules."""
+    return not any((nn_module._global_forward_hooks, nn_module._global_forward_pre_hooks, nn_module._global_backward_hooks,
+                    nn_module._global_backward_pre_hooks)) and all(getattr(cls, name) is method for cls, methods in _STEP_METHODS.items() for name, method in methods.items())
+
+
+def _stock(module: nn.Module, cls: type) -> bool:
+    """A module of this class itself, without methods of its own."""
+    return type(module) is cls and module.__dict__.keys().isdisjoint(_STEP_METHODS[cls])
+
+
+def _listened_to(module: nn.Module) -> bool:
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks or module._compiled_call_impl is not None)
 
 
 def _is_stock(layer: nn.Module) -> bool:
     """A decoder layer made of this file's modules, whose calls nothing listens to."""
-    if not _unchanged(layer, Qwen3DecoderLayer) or not _unchanged(layer.self_attn, Qwen3Attention) or not _unchanged(layer.mlp, Qwen3MLP):
+    if not _stock(layer, Qwen3DecoderLayer) or _listened_to(layer):
         return False
-    attn, mlp = layer.self_attn, layer.mlp
-    if not _unchanged(attn.attn, Attention) or not _unchanged(attn.o_proj, RowParallelLinear) or not _unchanged(mlp.down_proj, RowParallelLinear):
+    attn, mlp, norm = layer.self_attn, layer.mlp, layer.input_layernorm
+    if not _stock(attn, Qwen3Attention) or not _stock(mlp, Qwen3MLP) or not _stock(norm, RMSNorm) or _listened_to(norm):
         return False
-    if not _unchanged(mlp.gate_up_proj, MergedColumnParallelLinear) or not mlp.gate_up_proj.paired or attn.o_proj.bias is not None or mlp.down_proj.bias is not None:
+    o_proj, gate_up, down = attn.o_proj, mlp.gate_up_proj, mlp.down_proj
+    if not _stock(attn.attn, Attention) or not _stock(o_proj, RowParallelLinear) or not _stock(down, RowParallelLinear) or not _stock(gate_up, MergedColumnParallelLinear):
         return False
-    if attn.qkv_proj.bias is not None or not _unchanged(layer.input_layernorm, RMSNorm) or type(layer.post_attention_layernorm) is not RMSNorm:
-        return False
-    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or m._compiled_call_impl is not None
-                   for m in (layer, layer.input_layernorm))
+    return gate_up.paired and o_proj.bias is None and down.bias is None and attn.qkv_proj.bias is None and type(layer.post_attention_layernorm) is RMSNorm
 
 
 class Qwen3ForCausalLM(nn.Module):

@@ -141,13 +141,18 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seql
     return _native.prefill_attention(get_runtime().handle, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, block_tables, scale)
 
 
+def decode_stack_served(rows: int, layers: int, hidden: int, nq: int, nkv: int, head_dim: int, inter: int, block_size: int) -> bool:
+    """Whether decode_stack serves a step of this shape on this runtime (see b2_decode_stack_workspace)."""
+    return _lib.b2_decode_stack_workspace(get_runtime().ctx, rows, layers, hidden, nq, nkv, head_dim, inter, block_size) > 0
+
+
 def decode_stack(x: torch.Tensor, positions: torch.Tensor, layers: list[tuple], final_norm: torch.Tensor, nq: int, nkv: int, head_dim: int, inter: int,
                  eps: float, qk_eps: float, scale: float, cos_sin: torch.Tensor, context_lens: torch.Tensor, slot_mapping: torch.Tensor,
                  block_tables: torch.Tensor) -> torch.Tensor | None:
     """All decoder layers of a decode step in one launch: x [rows, hidden] the embedded tokens, layers a list of (qkv_w, o_w,
     gate_up_w with paired rows, down_w, in_norm, post_norm, q_norm, k_norm, k_cache, v_cache).  Returns the final norm's output.
-    None when the kernel does not serve the call (more than 16 rows, several ranks, a layer that does not fit the SMs' shared
-    memory, a layout it cannot address); rows after the last one with a context come back as zeros."""
+    None when the kernel does not serve the call (a shape that decode_stack_served declines, no layers, a layout it cannot
+    address); rows after the last one with a context come back as zeros."""
     return _native.decode_stack(get_runtime().handle, x, positions, layers, final_norm, nq, nkv, head_dim, inter, eps, qk_eps, scale, cos_sin,
                                 context_lens, slot_mapping, block_tables)
 

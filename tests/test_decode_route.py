@@ -16,7 +16,8 @@ def step(pkg, monkeypatch):
     for layer in model.layers:
         layer.self_attn.attn.k_cache = layer.self_attn.attn.v_cache = torch.zeros(2, 16, 1, 32)
     calls = []
-    monkeypatch.setattr(ops, "decode_stack", lambda *a: calls.append(a) or "normed")
+    monkeypatch.setattr(ops, "decode_stack", lambda *a: calls.append(a) or ("normed" if a[2] else None))
+    monkeypatch.setattr(ops, "decode_stack_served", lambda rows, *shape: shape == (3, 64, 2, 1, 32, 64, 16) and rows <= 16, raising=False)
 
     def run(rows=2):
         calls.clear()
@@ -26,8 +27,8 @@ def step(pkg, monkeypatch):
             out = model._decode_in_one_launch(torch.zeros(rows, 64), torch.zeros(rows, dtype=torch.int64))
         finally:
             reset_context()
-        assert out == ("normed" if calls else None)
-        return calls[0] if calls else None
+        assert (out == "normed") == (len(calls) == 1 and len(calls[0][2]) > 0)
+        return None if out is None else calls[0]
 
     run.model = model
     return run
@@ -46,6 +47,20 @@ def test_scale_of_a_single_layer(step):
     attns[0].scale *= 2
     attns[2].scale *= 2
     assert step()[10] == 2 * 32 ** -0.5
+
+
+def test_nothing_is_gathered_for_a_step_that_is_not_served(step, monkeypatch):
+    from nanovllm_b200.models import qwen3
+    asked = []
+    stock = qwen3._is_stock
+    monkeypatch.setattr(qwen3, "_is_stock", lambda layer: asked.append(layer) or stock(layer))
+    assert step(17) is None and len(asked) <= 1
+    assert step(16) is not None and len(asked) > 3
+
+
+def test_first_layer_of_another_kind(step):
+    step.model.layers[0] = torch.nn.Identity()
+    assert step() is None
 
 
 def _ignore(*_):
