@@ -672,18 +672,17 @@ __device__ __forceinline__ void combine(const Place& t, const Exchange& x, int i
       float mx = m;
 #pragma unroll
       for (int k = 0; k < BATCH; ++k) mx = k0 + k <= parts ? fmaxf(mx, __uint_as_float(qm[k])) : mx;
-      const float keep = exp2f(m - mx);  // (a part has at least one token: its maximum is finite)
+      const float keep = exp2f(m - mx);  // (a part has at least one token: its maximum is finite, or its sum NaN)
       l *= keep;
 #pragma unroll
       for (int e = 0; e < 8; ++e) o[e] *= keep;
 #pragma unroll
-      for (int k = 0; k < BATCH; ++k) {
-        const float by = k0 + k <= parts ? exp2f(__uint_as_float(qm[k]) - mx) : 0.f;
-        if (by > 0.f) {
+      for (int k = 0; k < BATCH; ++k)
+        if (k0 + k <= parts) {  // (with whatever weight: what is NaN in a part is NaN in the result)
+          const float by = exp2f(__uint_as_float(qm[k]) - mx);
           l += by * __uint_as_float(ql[k]);
           add(by, p[k], q[k]);
         }
-      }
       m = mx;
     }
   }

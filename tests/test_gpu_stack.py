@@ -280,3 +280,38 @@ def test_captured_step_serves_later_batches(pkg):
         del graph
     finally:
         runner.exit()
+
+
+@pytest.mark.parametrize("kind", ["inf", "nan"])
+def test_scores_that_are_no_numbers(pkg, monkeypatch, kind):
+    """A context that many CTAs share, with an infinite key in the last of its parts, or with one part (here of 14 groups of 16 tokens)
+    whose keys are all NaN: the row comes out as NaN, as layer by layer, and the row beside it is untouched."""
+    from nanovllm_b200.models import qwen3
+    from nanovllm_b200.utils.context import reset_context, set_context
+    runner = _runner(16, 8, 3072)
+    try:
+        _weights(runner)
+        lens = [2000, 1900]
+        tables, slots = _batch(lens, 256, 64)
+        for plane in runner.kv_cache:
+            plane.normal_(generator=torch.Generator(device="cuda").manual_seed(5))
+        keys = runner.kv_cache[0, 0].view(-1, 8, 128)
+        for token in [1900] if kind == "inf" else range(5 * 14 * 16, 6 * 14 * 16):
+            keys[tables[0][token // 256] * 256 + token % 256, 0, :1 if kind == "inf" else 128] = float(kind)
+
+        def run():
+            set_context(False, slot_mapping=torch.tensor(slots, dtype=torch.int32, device="cuda"), context_lens=torch.tensor(lens, dtype=torch.int32, device="cuda"),
+                        block_tables=torch.tensor(tables, dtype=torch.int32, device="cuda"))
+            with torch.inference_mode():
+                out = runner.model(torch.tensor([1, 2], device="cuda"), torch.tensor(lens, device="cuda") - 1)
+            reset_context()
+            return out.float()
+
+        got = run()
+        monkeypatch.setattr(qwen3, "_is_stock", lambda layer: False)
+        layers = run()
+        runner.runtime.check_status()
+        assert layers[0].isnan().all() and got[0].isnan().all()
+        assert (got[1] - layers[1]).norm() <= 2 ** -6 * layers[1].norm()
+    finally:
+        runner.exit()
