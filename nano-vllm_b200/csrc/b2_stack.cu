@@ -18,9 +18,14 @@
 // buffer, keeps its own running maximum, and the parts of a (sequence, head) meet in shared memory, or in L2 where they span CTAs.
 //
 // Buffers between phases exist three times; layer l uses number l % 3.  Whoever writes a word of one also sets its counterpart of the
-// layer before back to all ones (nobody can be in this phase before every CTA has finished that layer's), which is used again two layers
-// on.  A fence in between, once a layer and in the shadow of the down projection's wait, orders the two: whoever looks there has read what was
-// written after the fence.  No result is all ones: additions, conversions and products make canonical NaNs only.
+// layer before back to all ones; that buffer is used again two layers on.  Nobody still needs the counterpart: a CTA stores in a phase
+// once it has read what every CTA stored after it had finished the layer before, and a store waits for the loads that it depends on.
+// Nobody sees it as it was before it was set back: ahead of the down projection the threads of a CTA meet, and each passes a fence.
+// What they store from then on is a release of all that the CTA has set back so far; the threads of other CTAs that read it pass
+// their fence of the next layer, which makes an acquire of it, for their whole CTA past the barriers that follow; and the layer after that is the
+// first to look at those buffers again.  (Fences of each store and load would say the same and cost a round trip to L2 in every phase; this
+// one is once a layer, in the shadow of the down projection's wait.)  Within a layer nothing is ordered but a word's own 32 bits: it
+// says itself whether it is there.  No result is all ones: additions, conversions and products make canonical NaNs only.
 //
 // Every CTA waits for all others, so the launch is cooperative: all of them are resident.  Every wait has a limit.
 #include <algorithm>
@@ -450,7 +455,10 @@ __device__ __forceinline__ void add_project(int use) {
   wait_weights(&sh.bar_b, use & 1);
 #pragma unroll
   for (int i = 0; i < MAX_KB; ++i) load_fragments(w[i], b2::smem_u32(smem) + a.off_b + min(t.g, R - 1) * (K * 2) + min(i, batches - 1) * 2048 + t.warp * (KB * 64) + t.c * 16, min(t.g, R - 1));
-  if (down) __threadfence();  // (see the exchange buffers)
+  if (down) {  // the order of what is set back and used again (see the buffers between phases)
+    __syncthreads();
+    __threadfence();
+  }
   int turn = 0;
 #pragma unroll 1
   for (int t0 = 0; t0 < rows; t0 += TILE, turn ^= 1) {
