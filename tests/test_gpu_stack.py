@@ -36,7 +36,7 @@ def _weights(runner):
             p.data.normal_(0, 1, generator=g)
 
 
-def _exact(runner, ids, pos, lens, tables, slots):
+def _exact(runner, ids, pos, lens, tables, slots, qk_norms=True):
     """The same step in float64, on copies of the caches."""
     c = runner.config
     d, hd, nq, nkv = torch.float64, c.head_dim, c.num_attention_heads, c.num_key_value_heads
@@ -59,7 +59,7 @@ def _exact(runner, ids, pos, lens, tables, slots):
         at, mlp = layer.self_attn, layer.mlp
         qkv = (norm(h, layer.input_layernorm) @ at.qkv_proj.weight.to(d).t()).view(n, nq + 2 * nkv, hd)
         q, k, v = qkv.split([nq, nkv, nkv], 1)
-        q, k = rope(norm(q, at.q_norm)), rope(norm(k, at.k_norm))
+        q, k = (rope(norm(q, at.q_norm)), rope(norm(k, at.k_norm))) if qk_norms else (rope(q), rope(k))
         kc, vc = at.attn.k_cache.to(d).view(-1, nkv, hd), at.attn.v_cache.to(d).view(-1, nkv, hd)
         for i, s in enumerate(slots):
             if s >= 0:
@@ -80,10 +80,12 @@ def _exact(runner, ids, pos, lens, tables, slots):
     return norm(h, model.norm), new
 
 
-def _compare(runner, monkeypatch, lens, tables, slots):
+def _compare(runner, monkeypatch, lens, tables, slots, qk_norms=True):
     from nanovllm_b200 import ops
+    from nanovllm_b200.layers.attention import Attention
     from nanovllm_b200.models import qwen3
-    from nanovllm_b200.utils.context import reset_context, set_context
+    from nanovllm_b200.utils.context import get_context, reset_context, set_context
+    model = runner.model.model
     n = len(lens)
     g = torch.Generator(device="cuda").manual_seed(sum(lens))
     for plane in runner.kv_cache:
@@ -94,13 +96,19 @@ def _compare(runner, monkeypatch, lens, tables, slots):
     pos = torch.tensor([max(0, x - 1) for x in lens], device="cuda")
     width = max(len(t) for t in tables)
     rows = torch.tensor([t + [-1] * (width - len(t)) for t in tables], dtype=torch.int32, device="cuda")
-    exact, _ = _exact(runner, ids, pos, lens, tables, slots)
+    exact, _ = _exact(runner, ids, pos, lens, tables, slots, qk_norms)
 
-    def run():
+    def stack_without_qk_norms():  # (no model has neither these norms nor a bias: the call itself)
+        at, ctx = model.layers[0].self_attn, get_context()
+        return ops.decode_stack(model.embed_tokens(ids), pos, [(*w[:6], None, None, *w[8:]) for w in model._stock_layers()], model.norm.weight, at.num_heads,
+                                at.num_kv_heads, at.head_dim, runner.config.intermediate_size, model.norm.eps, at.rms_norm_eps, at.attn.scale,
+                                at.rotary_emb.cos_sin_cache, ctx.context_lens, ctx.slot_mapping, ctx.block_tables)
+
+    def run(forward):
         set_context(False, slot_mapping=torch.tensor(slots, dtype=torch.int32, device="cuda"), context_lens=torch.tensor(lens, dtype=torch.int32, device="cuda"),
                     block_tables=rows)
         runner.kv_cache.copy_(cache)
-        out = runner.model(ids, pos)
+        out = forward()
         reset_context()
         return out, runner.kv_cache.clone()
 
@@ -108,11 +116,16 @@ def _compare(runner, monkeypatch, lens, tables, slots):
     stack = ops.decode_stack
     monkeypatch.setattr(ops, "decode_stack", lambda *a: calls.append(stack(*a)) or calls[-1])
     with torch.inference_mode():
-        got, kv = run()
-        again, kv_again = run()
+        launch = (lambda: runner.model(ids, pos)) if qk_norms else stack_without_qk_norms
+        got, kv = run(launch)
+        again, kv_again = run(launch)
         assert len(calls) == 2 and calls[0] is not None
         monkeypatch.setattr(qwen3, "_is_stock", lambda layer: False)
-        layers, kv_layers = run()
+        if runner.block_size % 64 != 0:
+            monkeypatch.setattr(Attention, "backend", "sdpa")  # (the only attention of the layers that takes such blocks)
+        for layer in model.layers:
+            monkeypatch.setattr(layer.self_attn, "qkv_bias", not qk_norms)  # (the layers leave the norms out of what would have a bias)
+        layers, kv_layers = run(lambda: runner.model(ids, pos))
     runner.runtime.check_status()
     live = max((i + 1 for i, x in enumerate(lens) if x > 0), default=0)
     assert not got[live:].any()
@@ -173,12 +186,27 @@ def test_shapes(pkg, monkeypatch, shape):
         runner.exit()
 
 
-def test_small_blocks(pkg, monkeypatch):
-    runner = _runner(16, 8, 3072, block_size=64, blocks=200)
+@pytest.mark.parametrize("block_size", [16, 32, 64])
+def test_small_blocks(pkg, monkeypatch, block_size):
+    runner = _runner(16, 8, 3072, block_size=block_size, blocks=200)
     try:
         _weights(runner)
         lens = [1, 64, 65, 500, 128, 63]
-        _compare(runner, monkeypatch, lens, *_batch(lens, 64, 200))
+        _compare(runner, monkeypatch, lens, *_batch(lens, block_size, 200))
+    finally:
+        runner.exit()
+
+
+def test_without_head_norms(pkg, monkeypatch):
+    runner = _runner(16, 8, 3072)
+    try:
+        _weights(runner)
+        lens = [1, 200, 77, 1030, 16, 512, 5, 300, 31, 90]
+        tables, slots = _batch(lens, 256, 64)
+        _compare(runner, monkeypatch, lens, tables, slots, qk_norms=False)
+        monkeypatch.undo()
+        slots[1] = -1  # (all new rows stored ahead)
+        _compare(runner, monkeypatch, lens, tables, slots, qk_norms=False)
     finally:
         runner.exit()
 
