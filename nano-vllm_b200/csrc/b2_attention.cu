@@ -58,25 +58,6 @@ struct AttnArgs {
   float scale_log2;  // softmax scale * log2(e)
 };
 
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-// rows 8..15 of A are zero: only the first two accumulators carry data
-__device__ __forceinline__ void mma_rows8(float& c0, float& c1, uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  asm("{\n\t.reg .f32 d2, d3;\n\t"
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, d2, d3}, {%2, %3, %4, %3}, {%5, %6}, {%0, %1, %7, %7};\n\t}"
-      : "+f"(c0), "+f"(c1)
-      : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
-}
-// 2^x; results below the normal range are as good as zero here
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ void consumers_meet() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // The tiles [pos, end) of a CTA as segments that lie inside one (sequence, head).
@@ -268,9 +249,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           uint32_t kf[4];
-          ldmatrix_x4(kf, k_row + (k >> 2) * ATT_HALF_BYTES + ((((k & 3) * 2 + k_chunk) ^ (k_tok & 7)) << 4));
-          mma_rows8(s[0][0], s[0][1], qf[k][0], qf[k][1], kf[0], kf[1]);
-          mma_rows8(s[1][0], s[1][1], qf[k][0], qf[k][1], kf[2], kf[3]);
+          b2::ldmatrix_x4(kf, k_row + (k >> 2) * ATT_HALF_BYTES + ((((k & 3) * 2 + k_chunk) ^ (k_tok & 7)) << 4));
+          b2::mma_rows8(s[0][0], s[0][1], qf[k][0], qf[k][1], kf[0], kf[1]);
+          b2::mma_rows8(s[1][0], s[1][1], qf[k][0], qf[k][1], kf[2], kf[3]);
         }
         float mx = m;
 #pragma unroll
@@ -297,7 +278,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            p[i][e] = ex2(s[i][e] - m);
+            p[i][e] = b2::ex2(s[i][e] - m);
             l += p[i][e];
           }
         const uint32_t p0 = b2::pack_bf16(p[0][0], p[0][1]), p1 = b2::pack_bf16(p[1][0], p[1][1]);
@@ -311,9 +292,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           uint32_t vf[4];
-          ldmatrix_x4_trans(vf, v_row + (j >> 2) * ATT_HALF_BYTES + ((((j & 3) * 2 + v_chunk) ^ (v_tok & 7)) << 4));
-          mma_rows8(o[2 * j][0], o[2 * j][1], p0, p1, vf[0] & keep[0], vf[1] & keep[1]);
-          mma_rows8(o[2 * j + 1][0], o[2 * j + 1][1], p0, p1, vf[2] & keep[0], vf[3] & keep[1]);
+          b2::ldmatrix_x4_trans(vf, v_row + (j >> 2) * ATT_HALF_BYTES + ((((j & 3) * 2 + v_chunk) ^ (v_tok & 7)) << 4));
+          b2::mma_rows8(o[2 * j][0], o[2 * j][1], p0, p1, vf[0] & keep[0], vf[1] & keep[1]);
+          b2::mma_rows8(o[2 * j + 1][0], o[2 * j + 1][1], p0, p1, vf[2] & keep[0], vf[3] & keep[1]);
         }
       }
       __syncwarp();
@@ -703,7 +684,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         b2::tc_wait_ld();
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
-          float x = ex2(fmaf(__uint_as_float(r[e]), a.scale_log2, -ref)), y = ex2(fmaf(__uint_as_float(r[e + 1]), a.scale_log2, -ref));
+          float x = b2::ex2(fmaf(__uint_as_float(r[e]), a.scale_log2, -ref)), y = b2::ex2(fmaf(__uint_as_float(r[e + 1]), a.scale_log2, -ref));
           if (masked) {
             if (c * 32 + e > last) x = 0.f;
             if (c * 32 + e + 1 > last) y = 0.f;

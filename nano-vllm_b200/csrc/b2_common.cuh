@@ -407,6 +407,39 @@ __device__ __forceinline__ uint2 silu_mul_pairs(const uint4& w) {
   return make_uint2(mul_bf16x2(a.x, __byte_perm(w.x, w.y, 0x7632)), mul_bf16x2(a.y, __byte_perm(w.z, w.w, 0x7632)));
 }
 
+// ---- pieces that several kernels share -------------------------------------------
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  f[0] = bf16_lo(v.x); f[1] = bf16_hi(v.x); f[2] = bf16_lo(v.y); f[3] = bf16_hi(v.y);
+  f[4] = bf16_lo(v.z); f[5] = bf16_hi(v.z); f[6] = bf16_lo(v.w); f[7] = bf16_hi(v.w);
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+}
+// bf16(bf16(x * rstd) * w)
+__device__ __forceinline__ uint4 normed(const float (&x)[8], float rstd, const uint4& w) {
+  return make_uint4(mul_bf16x2(pack_bf16(x[0] * rstd, x[1] * rstd), w.x), mul_bf16x2(pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
+                    mul_bf16x2(pack_bf16(x[4] * rstd, x[5] * rstd), w.z), mul_bf16x2(pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// rows 8..15 of A are zero: only the first two accumulators carry data
+__device__ __forceinline__ void mma_rows8(float& c0, float& c1, uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  asm("{\n\t.reg .f32 d2, d3;\n\t"
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, d2, d3}, {%2, %3, %4, %3}, {%5, %6}, {%0, %1, %7, %7};\n\t}"
+      : "+f"(c0), "+f"(c1)
+      : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
+}
+// 2^x; results below the normal range are as good as zero here
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // replace a -0.0 half (the sentinel) by +0.0 in a packed pair
 __device__ __forceinline__ uint32_t scrub_sentinel(uint32_t w) {
   if ((w & 0xFFFFu) == B2_SENTINEL16) w &= 0xFFFF0000u;

@@ -96,18 +96,6 @@ __device__ __forceinline__ void quad_meets(int part) {
   if (part == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
   else asm volatile("bar.sync 2, 128;" ::: "memory");
 }
-__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
-  f[0] = b2::bf16_lo(v.x); f[1] = b2::bf16_hi(v.x); f[2] = b2::bf16_lo(v.y); f[3] = b2::bf16_hi(v.y);
-  f[4] = b2::bf16_lo(v.z); f[5] = b2::bf16_hi(v.z); f[6] = b2::bf16_lo(v.w); f[7] = b2::bf16_hi(v.w);
-}
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-  return make_uint4(b2::pack_bf16(f[0], f[1]), b2::pack_bf16(f[2], f[3]), b2::pack_bf16(f[4], f[5]), b2::pack_bf16(f[6], f[7]));
-}
-// bf16(bf16(x * rstd) * w)
-__device__ __forceinline__ uint4 normed(const float (&x)[8], float rstd, const uint4& w) {
-  return make_uint4(b2::mul_bf16x2(b2::pack_bf16(x[0] * rstd, x[1] * rstd), w.x), b2::mul_bf16x2(b2::pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
-                    b2::mul_bf16x2(b2::pack_bf16(x[4] * rstd, x[5] * rstd), w.z), b2::mul_bf16x2(b2::pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
-}
 // token t of a staging buffer of head rows: 16 pieces of 16 bytes, piece index XORed with the token so that neither the
 // transposing stores nor the row reads meet in a bank
 __device__ __forceinline__ uint32_t staged(int token, int piece) { return token * (FM * 2) + ((piece ^ (token & 7)) << 4); }
@@ -604,8 +592,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           uint4 lo = *reinterpret_cast<const uint4*>(stg + staged(lt, pc)), hi = *reinterpret_cast<const uint4*>(stg + staged(lt, 8 + pc));
           if (rotated) {
             float x1[8], x2[8];
-            unpack8(lo, x1);
-            unpack8(hi, x2);
+            b2::unpack8(lo, x1);
+            b2::unpack8(hi, x2);
             if (norm != nullptr) {
               float ss[4];
 #pragma unroll
@@ -616,10 +604,10 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 for (int k = 0; k < 4; ++k) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
               const float rstd = rsqrtf(((ss[0] + ss[2]) + (ss[1] + ss[3])) / 128.0f + a.qk_eps);
               // (a product of two bf16 values has one rounding to bf16 either way)
-              lo = normed(x1, rstd, nw1);
-              hi = normed(x2, rstd, nw2);
-              unpack8(lo, x1);
-              unpack8(hi, x2);
+              lo = b2::normed(x1, rstd, nw1);
+              hi = b2::normed(x2, rstd, nw2);
+              b2::unpack8(lo, x1);
+              b2::unpack8(hi, x2);
             }
             const float* c = reinterpret_cast<const float*>(factors);
             float y1[8], y2[8];
@@ -628,8 +616,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
               y1[e] = __fsub_rn(__fmul_rn(x1[e], c[e]), __fmul_rn(x2[e], c[8 + e]));
               y2[e] = __fadd_rn(__fmul_rn(x2[e], c[e]), __fmul_rn(x1[e], c[8 + e]));
             }
-            lo = pack8(y1);
-            hi = pack8(y2);
+            lo = b2::pack8(y1);
+            hi = b2::pack8(y2);
           }
           const int to_slot = cache != nullptr ? slot : -1;
           ahead((g - g0 + (i0 == 0 ? 0 : STEP)) * 8 + (i0 ^ 16) + qw * 4 + row4);

@@ -85,16 +85,6 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// rows 8..15 of A are zero: only the first two accumulators carry data
-__device__ __forceinline__ void mma_rows8(float (&d)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  asm("{\n\t.reg .f32 d2, d3;\n\t"
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, d2, d3}, {%2, %3, %4, %3}, {%5, %6}, {%0, %1, %7, %7};\n\t}"
-      : "+f"(d[0]), "+f"(d[1])
-      : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
 __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
@@ -118,21 +108,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(b2::kEvictFirst) : "memory");
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-// 2^x; results below the normal range are as good as zero here
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
-  f[0] = b2::bf16_lo(v.x); f[1] = b2::bf16_hi(v.x); f[2] = b2::bf16_lo(v.y); f[3] = b2::bf16_hi(v.y);
-  f[4] = b2::bf16_lo(v.z); f[5] = b2::bf16_hi(v.z); f[6] = b2::bf16_lo(v.w); f[7] = b2::bf16_hi(v.w);
-}
-// bf16(bf16(x * rstd) * w)
-__device__ __forceinline__ uint4 normed(const float (&x)[8], float rstd, const uint4& w) {
-  return make_uint4(b2::mul_bf16x2(b2::pack_bf16(x[0] * rstd, x[1] * rstd), w.x), b2::mul_bf16x2(b2::pack_bf16(x[2] * rstd, x[3] * rstd), w.y),
-                    b2::mul_bf16x2(b2::pack_bf16(x[4] * rstd, x[5] * rstd), w.z), b2::mul_bf16x2(b2::pack_bf16(x[6] * rstd, x[7] * rstd), w.w));
-}
 // exchanged words: from and to L2, where all SMs see them
 __device__ __forceinline__ uint4 ld_x4(const void* p) {
   uint4 v;
@@ -522,15 +497,15 @@ __device__ __forceinline__ void finish_head(uint4 (&v)[4], const uint16_t* norm,
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float x[8];
-      unpack8(v[j], x);
+      b2::unpack8(v[j], x);
       ss += ((x[0] * x[0] + x[1] * x[1]) + (x[2] * x[2] + x[3] * x[3])) + ((x[4] * x[4] + x[5] * x[5]) + (x[6] * x[6] + x[7] * x[7]));
     }
     const float rstd = rsqrtf(quad_sum(ss) / static_cast<float>(HD) + eps);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float x[8];
-      unpack8(v[j], x);
-      v[j] = normed(x, rstd, *reinterpret_cast<const uint4*>(norm + j * 32 + c * 8));
+      b2::unpack8(v[j], x);
+      v[j] = b2::normed(x, rstd, *reinterpret_cast<const uint4*>(norm + j * 32 + c * 8));
     }
   }
 #pragma unroll
@@ -774,8 +749,8 @@ __device__ __forceinline__ void attention(int l_no) {
         for (int j = 0; j < 4; ++j)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            mma_rows8(s[h], qf[j].x, qf[j].y, kf[h][j].x, kf[h][j].y);
-            mma_rows8(s2[h], qf[j].z, qf[j].w, kf[h][j].z, kf[h][j].w);
+            b2::mma_rows8(s[h][0], s[h][1], qf[j].x, qf[j].y, kf[h][j].x, kf[h][j].y);
+            b2::mma_rows8(s2[h][0], s2[h][1], qf[j].z, qf[j].w, kf[h][j].z, kf[h][j].w);
           }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -868,7 +843,7 @@ __device__ __forceinline__ void attention(int l_no) {
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          p[h][e] = ex2(s[h][e] - m);
+          p[h][e] = b2::ex2(s[h][e] - m);
           l += p[h][e];
         }
       const uint32_t p0 = b2::pack_bf16(p[0][0], p[0][1]), p1 = b2::pack_bf16(p[1][0], p[1][1]), v_group = v_smem + (grp & 1) * V_BYTES;
@@ -882,9 +857,9 @@ __device__ __forceinline__ void attention(int l_no) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         uint32_t vf[4];
-        ldmatrix_x4_trans(vf, v_group + v_tok * (HD * 2) + (((j * 2 + v_chunk) ^ (v_tok & 7)) << 4));
-        mma_rows8(o[2 * j], p0, p1, vf[0], vf[1]);
-        mma_rows8(o[2 * j + 1], p0, p1, vf[2], vf[3]);
+        b2::ldmatrix_x4_trans(vf, v_group + v_tok * (HD * 2) + (((j * 2 + v_chunk) ^ (v_tok & 7)) << 4));
+        b2::mma_rows8(o[2 * j][0], o[2 * j][1], p0, p1, vf[0], vf[1]);
+        b2::mma_rows8(o[2 * j + 1][0], o[2 * j + 1][1], p0, p1, vf[2], vf[3]);
       }
       __syncwarp();
     }
@@ -1084,7 +1059,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       const float rstd = rsqrtf(ss / static_cast<float>(H) + a.eps);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(out + j * 256) = normed(x[j], rstd, __ldg(reinterpret_cast<const uint4*>(a.final_norm + j * 256 + t.lane * 8)));
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(out + j * 256) = b2::normed(x[j], rstd, __ldg(reinterpret_cast<const uint4*>(a.final_norm + j * 256 + t.lane * 8)));
     }
     __syncthreads();
     if (sh.abort != 0) {
