@@ -20,6 +20,9 @@ cases:
   store_kvcache   paged-KV scatter, 16384 tokens x D=1024
   add_rmsnorm     residual add + RMSNorm, 16384 x 4096
   embed           embedding lookup, 16384 ids into a [151936, 4096] table (one rank)
+  decode_stack    all 28 layers of a Qwen3-0.6B decode step in one launch, one sequence of 300 tokens (0.9 GB of weights)
+  decode_stack_16 the same with 16 sequences of 300 tokens
+  sampler         LM head fused with the sampler, 256 rows x 151936 x 1024 with temperatures
 """
 from __future__ import annotations
 
@@ -47,7 +50,7 @@ def main():
     os.environ.setdefault("MASTER_PORT", "29579")
     torch.cuda.set_device(0)
     dist.init_process_group("gloo", rank=0, world_size=1)
-    init_runtime(max_tokens=16384, hidden=5120, oneshot_tokens=1024)
+    init_runtime(max_tokens=16384, hidden=5120, oneshot_tokens=1024, vocab=151936 if a.case == "sampler" else 0, max_seqs=256 if a.case == "sampler" else 0)
     dev = "cuda:0"
     g = torch.Generator(device=dev).manual_seed(0)
 
@@ -108,6 +111,26 @@ def main():
         w = rnd(151936, 4096)
         ids = [torch.randint(0, 151936, (16384,), device=dev, generator=g) for _ in range(2)]
         call = lambda i: ops.embed(ids[i % 2], w, 0, 151936, 1)
+    elif a.case in ("decode_stack", "decode_stack_16"):
+        rows, context, nq, nkv, h, inter = 16 if a.case.endswith("16") else 1, 300, 16, 8, 1024, 3072
+        blocks = -(-context // 256)
+
+        def layer():
+            kv = [rnd(rows * blocks, 256, nkv, 128) for _ in range(2)]
+            return (rnd((nq + 2 * nkv) * 128, h, scale=0.02), rnd(h, nq * 128, scale=0.02), rnd(2 * inter, h, scale=0.02), rnd(h, inter, scale=0.02), rnd(h), rnd(h),
+                    rnd(128), rnd(128), *kv)
+
+        layers, x, norm = [layer() for _ in range(28)], rnd(rows, h), rnd(h)
+        cos_sin = torch.randn(context, 128, device=dev, generator=g)
+        ints = lambda values: torch.tensor(values, dtype=torch.int32, device=dev)
+        tables, lens = ints([[i * blocks + j for j in range(blocks)] for i in range(rows)]), ints([context] * rows)
+        slots, pos = ints([(i * blocks + blocks - 1) * 256 + (context - 1) % 256 for i in range(rows)]), torch.full((rows,), context - 1, device=dev)
+
+        def call(i):
+            assert ops.decode_stack(x, pos, layers, norm, nq, nkv, 128, inter, 1e-6, 1e-6, 128 ** -0.5, cos_sin, lens, slots, tables) is not None
+    elif a.case == "sampler":
+        x, w, temps = rnd(256, 1024), rnd(151936, 1024, scale=0.02), torch.full((256,), 0.6, device=dev)
+        call = lambda i: ops.lm_head_sample(x, w, None, temps, 5)
     else:
         raise SystemExit(f"unknown case {a.case}")
     with torch.inference_mode():
