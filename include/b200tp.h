@@ -422,7 +422,8 @@ int b2_paged_attention_supported(int n_seqs, int nq, int nkv, int head_dim, int 
  * Partial sums, norms' inputs and the residual's sums are fp32.  The launch is cooperative (one CTA per SM).
  * b2_decode_stack_workspace: bytes of device memory a call needs (16-byte aligned, contents irrelevant), or 0 where the
  * shape is not served: one rank, head_dim 128, at most two query heads per KV head, at most 16 rows, blocks of a power of two
- * of at least 16 tokens, 1024 hidden features, nq * 128 and inter multiples of 1024 up to 3072: a layer that fits the SMs' shared memory. */
+ * of at least 16 tokens, exactly 1024 hidden features, nq * 128 and inter multiples of 1024 up to 3072 and small enough for a layer to fit
+ * the SMs' shared memory. */
 typedef struct b2_stack_layer {
   const void *qkv_w, *o_w, *gate_up_w, *down_w, *in_norm, *post_norm, *q_norm, *k_norm;
   void *k_cache, *v_cache; /* [num_blocks][block_size][nkv][head_dim] */

@@ -408,7 +408,7 @@ __device__ __forceinline__ void flush_rows(const GemmArgs& a, unsigned char* wbu
 constexpr uint32_t SAMPLE_TAG = 0x53414D50u;
 // Epilogue warps of the sampler per tensor-memory quadrant: they share the quadrant's token rows.  A warp alone on its scheduler
 // had nothing to fill its latencies with (256 rows x 151936 x 1024, greedy / with temperatures: 150 / 239 us with one, 120 / 168
-// with two, 93 / 131 with four; as a plain GEMM 74).
+// with two, 93 / 131 with four on rows with a clear winner, 113 / 146 on random ones; as a plain GEMM 75).
 constexpr int SAMPLE_PARTS = 4;
 
 __host__ __device__ __forceinline__ void philox4x32_10(uint32_t (&c)[4], uint32_t k0, uint32_t k1) {

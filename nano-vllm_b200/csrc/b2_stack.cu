@@ -1,14 +1,15 @@
-// All decoder layers of one decode step in one launch, for models whose layer fits the SMs' shared memory.
+// All decoder layers of one decode step in one launch, for models of 1024 hidden features whose layer fits the SMs' shared memory.
 //
-// A layer of a small model is 30 MB of weights: 5 us of HBM time on the whole chip.  As five launches it took 31 us (Qwen3-0.6B, one
-// sequence): every launch waits for the one before it, sets up, has its first bytes travel and combines its split sums, and none of
+// A layer of a small model is 30 MB of weights: 5 us of HBM time on the whole chip.  As five launches it takes 29 us (Qwen3-0.6B, one
+// sequence of 300 tokens), here 17: every launch waits for the one before it, sets up, has its first bytes travel and combines its split sums, and none of
 // that overlaps.  Here one CTA per SM stays for the whole step:
 //   - every projection's output rows are dealt to the CTAs, whole rows: a CTA owns the same few rows with all of K in every layer, so
 //     no sum crosses an SM, and its share of a layer (28 + 7 + 44 + 7 rows of Qwen3-0.6B) is brought in by bulk copies one phase and
 //     more before it is used: the weights stream through the waits between the phases;
 //   - what a phase hands to the next one is its own flag: a word that is all ones has not been written yet, and a reader takes its
-//     fragments again until none is.  That is one trip through L2 (2250 clocks from the first store to the last CTA's having read
-//     everything); a barrier of all CTAs with its fence, count and polls took 4400 before the reads could start;
+//     fragments again until none is.  All to all, 4 KB among 148 CTAs, that is 1420 clocks a turn, with a barrier in between (fence,
+//     count, polls, then the reads) 3200.  Polls that begin at once stand in the stores' way: 3600 to 4400.  (Of a probe that does nothing else;
+//     here the fragments of the weights come first where a phase can begin with them.)
 //   - 8 warps split K: a warp multiplies its slice of the weights' rows (the 16 rows of an mma.sync) with its slice of 8 tokens (a lane
 //     takes 8 neighbouring elements of a row; which k of the instruction they stand for does not matter as long as both operands agree),
 //     and the 8 partial sums meet in shared memory.  tcgen05 would want 128 rows of weights in a tile: with 7 to 44 rows
@@ -37,7 +38,7 @@
 namespace {
 
 constexpr int WARPS = 8, THREADS = WARPS * 32;
-constexpr int H = 1024;               // hidden features
+constexpr int H = 1024;               // hidden features: the fragments' arrays and the norms' shares are laid out for this one size
 constexpr int KN = H / (WARPS * 32);  // k steps (of 32) of a warp in the projections of the norms' outputs
 constexpr int MT = 3;                 // and 16-row groups of a CTA's weights, at most
 constexpr int KB = 1024 / (WARPS * 32), MAX_KB = 3;  // o, down: k steps for every 1024 input features, and of those at most
@@ -166,8 +167,8 @@ __host__ __device__ __forceinline__ Deal deal_groups(const int* first, int rows,
   return d;
 }
 
-// What a CTA keeps in shared memory in front of its buffers.  The phases are functions of their own that find everything here: inlined into
-// one loop, what the compiler keeps of all of them at a time pushed their fragments out of the registers (1100 bytes of spills).
+// What a CTA keeps in shared memory in front of its buffers.  The phases are inlined into one loop, whose fragments need all registers
+// there are (255 a thread, 24 bytes of spills); they find everything else here, and nothing but the loop's counter lives on from one to the next.
 struct Shared {
   Args args;
   uint64_t bar_a, bar_b;  // weight buffers filled
@@ -1076,15 +1077,16 @@ struct Layout {
   uint32_t off_a, off_vec, off_b, off_s, off_x, off_small, off_own, smem;
   size_t words, sum_o, sum_d, qkv, attn, act, parts, bytes;  // offsets in the workspace
 };
-// The rule of what is served: the CTAs' shares of a layer have to fit shared memory one projection ahead, and the fragments'
-// arrays above.  With 148 SMs that is up to 1024 hidden and 3072 MLP features (Qwen3-0.6B); larger layers stream for longer than
-// their launches' overheads and stay on the kernels of the single projections.  Rows: tiles of 8 follow one another, and every CTA normalises
-// and takes in all of them.  The 28 layers of Qwen3-0.6B in a graph, us, this launch against one launch per projection:
+// The rule of what is served.  Hidden size: H alone (see there); a smaller one would fit and is left to the layers, as no model here has one.
+// q and MLP widths: the CTAs' shares of a layer have to fit shared memory one projection ahead, and the fragments' arrays above: with
+// 148 SMs up to 3072 (Qwen3-0.6B).  Larger layers stream for longer than their launches' overheads and stay on the kernels of the single
+// projections.  Rows: tiles of 8 follow one another, and every CTA normalises and takes in all of them.  The 28 layers of
+// Qwen3-0.6B in a graph, us, this launch against one launch per projection (the last column with kernels of an earlier state on both sides):
 //   context       1 row        8 rows       16 rows       32 rows
-//   40          391 / 806     496 / 840    725 / 884    1196 / 935
-//   300         462 / 856     618 / 909    837 / 968    1490 / 1055
-//   1200        538 / 976     840 / 1172  1198 / 1340   2229 / 1537
-//   4000        688 / 1114   1256 / 1505  2014 / 2086
+//   40          409 / 758     494 / 793    707 / 833    1196 / 935
+//   300         472 / 804     637 / 865    843 / 921    1490 / 1055
+//   1200        537 / 918     849 / 1104  1204 / 1294   2229 / 1537
+//   4000        685 / 1074   1266 / 1473  2025 / 2030
 bool layout_of(int rows, int hidden, int nq, int nkv, int I, int G, Layout* p) {
   const int Q = nq * HD, N = (nq + 2 * nkv) * HD;
   if (rows < 1 || rows > MAX_ROWS || nkv < 1 || nq % nkv != 0 || nq / nkv > MAX_GROUP || G < 1) return false;
