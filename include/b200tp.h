@@ -416,8 +416,8 @@ int b2_paged_attention_supported(int n_seqs, int nq, int nkv, int head_dim, int 
  * What the calls of a layer compute, for all layers: norm, qkv projection with q/k head norm, rotation and cache scatter,
  * attention over the paged cache, o projection + residual, norm, gate/up + SiLU * mul, down projection + residual
  * (nanovllm/models/qwen3.py:146-159), and the norm after the last one.  x [rows][hidden] bf16: the embedded tokens;
- * positions int64, context_lens / slot_mapping int32 [rows], block_tables as for b2_paged_attention_decode; out
- * [rows][hidden].  Rows after the last one with a context are padding: their output is zero and nothing is stored for them.
+ * positions int64, cos_sin on a 16-byte boundary, context_lens / slot_mapping int32 [rows], block_tables as for
+ * b2_paged_attention_decode; out [rows][hidden].  Rows after the last one with a context are padding: their output is zero and nothing is stored for them.
  * Weights are [out][in] contiguous, gate and up rows interleaved; q_norm and k_norm may be null together.
  * Partial sums, norms' inputs and the residual's sums are fp32.  The launch is cooperative (one CTA per SM).
  * b2_decode_stack_workspace: bytes of device memory a call needs (16-byte aligned, contents irrelevant), or 0 where the

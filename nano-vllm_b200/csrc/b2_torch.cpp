@@ -448,7 +448,7 @@ PyObject* decode_stack(Args a) {
     layers[i] = {ptr(w[0]), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(w[4]), ptr(w[5]), ptr(w[6]), ptr(w[7]), ptr(w[8]), ptr(w[9])};
   }
   if (n == 0 || blocks == 0 || !plain(x, x, {n, h}) || !plain(final_norm, x, {h}) || !table_layout(tables) || tables.scalar_type() != at::kInt || !cs.is_contiguous() ||
-      cs.scalar_type() != at::kFloat || cs.size(-1) != hd || pos.scalar_type() != at::kLong || !pos.is_contiguous() || pos.numel() != n)
+      cs.scalar_type() != at::kFloat || cs.size(-1) != hd || !on_16_bytes(cs) || pos.scalar_type() != at::kLong || !pos.is_contiguous() || pos.numel() != n)
     Py_RETURN_NONE;
   const int64_t bytes = b2_decode_stack_workspace(ctx, n, n_layers, h, nq, nkv, hd, inter, bs);
   if (bytes == 0) Py_RETURN_NONE;

@@ -345,3 +345,35 @@ def test_scores_that_are_no_numbers(pkg, monkeypatch, kind):
         assert (got[1] - layers[1]).norm() <= 2 ** -6 * layers[1].norm()
     finally:
         runner.exit()
+
+
+def test_rotary_table_off_16_bytes(pkg, monkeypatch):
+    """The layers read the rotary factors one by one for so few rows; the launch takes four at a time and leaves such a table to them."""
+    from nanovllm_b200.models import qwen3
+    from nanovllm_b200.utils.context import reset_context, set_context
+    runner = _runner(16, 8, 3072)
+    rotary = runner.model.model.layers[0].self_attn.rotary_emb
+    table = rotary.cos_sin_cache
+    try:
+        _weights(runner)
+        lens = [5, 40]
+        tables, slots = _batch(lens, 256, 64)
+
+        def run():
+            set_context(False, slot_mapping=torch.tensor(slots, dtype=torch.int32, device="cuda"), context_lens=torch.tensor(lens, dtype=torch.int32, device="cuda"),
+                        block_tables=torch.tensor(tables, dtype=torch.int32, device="cuda"))
+            runner.kv_cache.zero_()
+            with torch.inference_mode():
+                out = runner.model(torch.tensor([1, 2], device="cuda"), torch.tensor(lens, device="cuda") - 1)
+            reset_context()
+            return out
+
+        with torch.no_grad():
+            rotary.cos_sin_cache = torch.empty(table.numel() + 1, device="cuda")[1:].view(table.shape).copy_(table)
+        got = run()
+        rotary.cos_sin_cache = table
+        monkeypatch.setattr(qwen3, "_is_stock", lambda layer: False)
+        assert torch.equal(got, run())
+    finally:
+        rotary.cos_sin_cache = table
+        runner.exit()
