@@ -454,7 +454,8 @@ PyObject* decode_stack(Args a) {
   if (bytes == 0) Py_RETURN_NONE;
   on_current_gpu(x, "decode input");
   int32_vector(lens, n, "context_lens");
-  int32_vector(slots, n, "slot_mapping");
+  if (slots.numel() < n) raise(PyExc_ValueError, "slot_mapping: %lld slots for %lld rows", (long long)slots.numel(), (long long)n);
+  expect(slots.scalar_type() == at::kInt && slots.is_contiguous(), "slot_mapping must be contiguous int32");  // (its first n, as the layers)
   block_table_rows(tables, n);
   for (const at::Tensor* t : {&pos, &cs, &lens, &slots, &tables}) same_device(*t, x, "an operand of the decode step");
   const at::Tensor out = empty_rows(n, h, x), ws = at::detail::empty_cuda({bytes}, at::kByte, x.device(), std::nullopt);

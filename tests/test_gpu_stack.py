@@ -377,3 +377,33 @@ def test_rotary_table_off_16_bytes(pkg, monkeypatch):
     finally:
         rotary.cos_sin_cache = table
         runner.exit()
+
+
+def test_slot_mapping_longer_than_the_batch(pkg, monkeypatch):
+    """The layers read as many slots as there are rows (a buffer kept for the largest batch will do), and so does the launch; fewer are refused."""
+    from nanovllm_b200.models import qwen3
+    from nanovllm_b200.utils.context import reset_context, set_context
+    runner = _runner(16, 8, 3072)
+    try:
+        _weights(runner)
+        lens = [5, 40]
+        tables, slots = _batch(lens, 256, 64)
+
+        def run(slots):
+            set_context(False, slot_mapping=torch.tensor(slots, dtype=torch.int32, device="cuda"), context_lens=torch.tensor(lens, dtype=torch.int32, device="cuda"),
+                        block_tables=torch.tensor(tables, dtype=torch.int32, device="cuda"))
+            runner.kv_cache.zero_()
+            try:
+                with torch.inference_mode():
+                    return runner.model(torch.tensor([1, 2], device="cuda"), torch.tensor(lens, device="cuda") - 1), runner.kv_cache.clone()
+            finally:
+                reset_context()
+
+        for a, b in zip(run(slots), run(slots + [3, 4, 5])):
+            assert torch.equal(a, b)
+        with pytest.raises(ValueError):
+            run(slots[:1])
+        monkeypatch.setattr(qwen3, "_is_stock", lambda layer: False)
+        run(slots + [3, 4, 5])
+    finally:
+        runner.exit()
