@@ -17,7 +17,7 @@ def step(pkg, monkeypatch):
         layer.self_attn.attn.k_cache = layer.self_attn.attn.v_cache = torch.zeros(2, 16, 1, 32)
     calls = []
     monkeypatch.setattr(ops, "decode_stack", lambda *a: calls.append(a) or ("normed" if a[2] else None))
-    monkeypatch.setattr(ops, "decode_stack_served", lambda rows, *shape: shape == (3, 64, 2, 1, 32, 64, 16) and rows <= 16, raising=False)
+    monkeypatch.setattr(ops, "decode_stack_served", lambda rows, *shape: shape == (3, 64, 2, 1, 32, 64, 16) and rows <= 16)
 
     def run(rows=2):
         calls.clear()
