@@ -404,8 +404,8 @@ int b2_rope(const void* q, int64_t ldq, const void* k, int64_t ldk, int M, int n
  * are read on the device, so a captured call serves any later batch of the same size; they are read while earlier
  * b2_* kernels of the stream may still be running, so they must not be results of one, b2_advance_decode excepted.
  * Calls of one context must be stream-ordered: they share its workspace for partial results.
- * b2_paged_attention_supported says (1 / 0) whether the shape is served: head_dim 128, one or
- * two query heads per KV head, blocks of a multiple of 64 tokens, at most 1024 sequences. */
+ * b2_paged_attention_supported says (1 / 0) whether the shape is served: head_dim 128, blocks of a
+ * multiple of 64 tokens, at most 1024 sequences, one or two query heads per KV head, or up to eight where n_seqs * nkv >= 128. */
 int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
                               int num_blocks, int block_size, const int32_t* block_tables, int64_t bt_stride, int bt_width,
                               const int32_t* context_lens, int n_seqs, int nq, int nkv, int head_dim, float scale,

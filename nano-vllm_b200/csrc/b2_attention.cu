@@ -1,6 +1,7 @@
 // Attention with grouped-query heads: decode (one new query token per sequence over the paged KV cache) and causal prefill.
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 
 #include "b2_common.cuh"
 
@@ -28,12 +29,7 @@ namespace {
 constexpr int ATT_WARPS = 4, ATT_THREADS = (ATT_WARPS + 1) * 32;  // the last warp is the producer
 constexpr int ATT_TILE = 64;          // tokens per tile
 constexpr int ATT_HD = 128;           // head dimension
-// Query heads per KV head: one and two are served.  Not because more would be slower or less exact - with room for them the
-// kernel took 53 us against flash-attn's 71 at 64 contexts of 1056 tokens and 4 heads, and its relative error against float64 is
-// the smaller one: 2.12e-3 against 2.23e-3 for 4 and for 8 heads, 1.69e-3 against 1.77e-3 where scores have standard deviation 3
-// (the output's own rounding is 1.66e-3 of each; with 2 heads 2.10e-3 against 2.23e-3) - but because the two round differently,
-// which over the 36 layers of a 4096-wide model grows to 3 % of the hidden state: the models with wider groups keep the results
-// they had.
+// Query heads per KV head.  (Wider groups: paged_decode_wide_kernel below.)
 constexpr int ATT_MAX_GROUP = 2;
 constexpr int ATT_CTAS_PER_SM = 2;
 constexpr int ATT_STAGES = 3;
@@ -55,6 +51,7 @@ struct AttnArgs {
   int* counters;   // [sequences * KV heads], zero between launches
   B2Status* status;
   int bt_width, block_size, num_blocks, n_seqs, nkv, group;
+  int stages;  // wide groups: tiles of the ring
   float scale_log2;  // softmax scale * log2(e)
 };
 
@@ -443,6 +440,233 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 }
 
 // ---------------------------------------------------------------------------
+// paged_decode_wide_kernel
+//
+// Decode attention with 3 to 8 query heads per KV head.  Bound: HBM, as above.
+//
+// The models with wide groups are deep and wide enough that another rounding of the probabilities grows to 3 % of their hidden
+// state, and so this kernel fixes what each probability is rounded against: a context is walked from its end in blocks of 128
+// tokens, each rounded to bf16 against the maximum of that block and those walked before, and every output element is one unbroken
+// chain of tensor-core sums.  That leaves one CTA per (sequence, KV head) and shares its work out inside it: for the scores a
+// warp takes 16 tokens of each tile of 64, the maxima meet in shared memory, and for the product a warp takes 32 of the 128
+// dimensions and all tokens, with the probabilities from shared memory; every thread adds up the columns of its fragments in
+// their order.  On random data the results are flash-attn's but for 0 to 3 elements in a million.
+//
+// 64 contexts of 1056 tokens, 32 / 8 heads: 66.7 us in flash-attn, 45.2 here (6.1 TB/s); 96 of 70..700 47.0 and 28.8, 32 of 1056
+// 34.9 and 26.1.  Narrow groups take this kernel too from three pairs of (sequence, KV head) per SM on, where nothing has to be cut to fill
+// the chip and the other kernel's parts cost more than the even share saves: 256 contexts of 100..1024 tokens, 16 / 8 heads, 97.6 -> 90.8 us,
+// 128 of them 53.5 -> 48.4, 512 of 30..270 67.7 -> 55.8, 64 of 1056 49.1 -> 45.0; 37 of 40..700 (296 pairs) would go from 13.6 to 14.6.
+//
+// Four CTAs per SM with a ring of three 16 KB tiles (64 tokens of K or of V) each, or fewer with longer rings where there are no
+// more to be had: 190 KB per SM in flight.
+// ---------------------------------------------------------------------------
+constexpr int WD_MAX_GROUP = 8;
+constexpr int WD_MAX_STAGES = 6;
+constexpr int WD_CTAS_PER_SM = 4;
+constexpr int WD_BLOCK = 2 * ATT_TILE;                    // tokens that share a maximum
+constexpr int WD_STAGE_BYTES = 2 * ATT_HALF_BYTES;        // dimensions 0..63, 64..127
+constexpr int WD_P_PITCH = WD_BLOCK + 8;                  // floats: rows start 8 banks apart, so that the 8-byte accesses of half a warp meet in none
+// Wide groups, from this many (sequence, KV head) pairs on: 16 contexts of 1056 tokens and 8 KV heads 38.9 us in the library, 19.5 here
+// (of 100..3000 tokens 59 and 42).  Fewer would be faster here too (8 contexts 35 and 19), but long contexts are then cut into parts in the
+// library, each rounded for itself, and a context of one CTA walks at 36 GB/s however long it is.
+constexpr int WD_MIN_ITEMS = 128;
+constexpr uint32_t wide_smem(int stages) { return 1024 + stages * WD_STAGE_BYTES; }
+static_assert(2 * (wide_smem(WD_MAX_STAGES) + 5 * 1024) <= 228 * 1024 && 3 * (wide_smem(4) + 5 * 1024) <= 228 * 1024 && 4 * (wide_smem(3) + 5 * 1024) <= 228 * 1024, "CTAs per SM (5 KB: static, reserved)");
+
+__global__ void __launch_bounds__(ATT_THREADS, WD_CTAS_PER_SM)
+paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmK16,
+                         const __grid_constant__ CUtensorMap tmV16, const AttnArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  __shared__ __align__(16) float s_p[WD_MAX_GROUP][WD_P_PITCH];
+  __shared__ float s_m[ATT_WARPS][WD_MAX_GROUP];
+  __shared__ __align__(8) uint64_t s_bars[2 * WD_MAX_STAGES];
+  __shared__ int s_abort;
+  volatile int* abort_flag = &s_abort;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t ring = b2::smem_u32(smem), bar_full = b2::smem_u32(s_bars), bar_empty = bar_full + WD_MAX_STAGES * 8;
+  if (threadIdx.x == 0) {
+    b2::tma_prefetch_desc(&tmK);
+    b2::tma_prefetch_desc(&tmV);
+    for (int i = 0; i < a.stages; ++i) {
+      b2::mbar_init(bar_full + i * 8, 1);
+      b2::mbar_init(bar_empty + i * 8, ATT_WARPS);
+    }
+    s_abort = 0;
+    b2::mbar_fence_init();
+  }
+  __syncthreads();
+  b2::pdl_launch_dependents();
+  const int b = blockIdx.x / a.nkv, head = blockIdx.x - b * a.nkv;
+  const int len = max(0, min(__ldg(a.lens + b), a.bt_width * a.block_size));
+  const int blocks = (len + WD_BLOCK - 1) / WD_BLOCK;
+  uint16_t* out = a.out + static_cast<int64_t>(blockIdx.x) * a.group * ATT_HD;
+  int stage = 0;
+  uint32_t phase = 0;
+
+  if (warp == ATT_WARPS) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0 && blocks > 0) {
+      const int32_t* table = a.tables + static_cast<int64_t>(b) * a.bt_stride;
+      const int x = head * ATT_HD;
+      bool ok = true;
+      b2::pdl_wait();
+      for (int j = blocks - 1; ok && j >= 0; --j) {
+        int y[2];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const int tok = min(j * WD_BLOCK + t * ATT_TILE, len - 1), no = tok / a.block_size;
+          y[t] = min(max(0, __ldg(table + no)), a.num_blocks - 1) * a.block_size + tok - no * a.block_size;  // inside the cache whatever the table holds
+        }
+        for (int i = 0; ok && i < 4; ++i) {  // K, K, V, V
+          const int left = len - j * WD_BLOCK - (i & 1) * ATT_TILE;
+          if (left <= 0) continue;
+          ok = b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, 1000000000ull, B2_WAIT_SMEM_EMPTY);
+          if (!ok) break;
+          const uint32_t fb = bar_full + stage * 8, dst = ring + stage * WD_STAGE_BYTES;
+          const int row = (i & 1) ? y[1] : y[0];
+          if (left >= ATT_TILE) {
+            const CUtensorMap* m = i < 2 ? &tmK : &tmV;
+            b2::mbar_arrive_expect_tx(fb, WD_STAGE_BYTES);
+            b2::tma_load_2d(dst, m, fb, x, row, b2::kEvictFirst);
+            b2::tma_load_2d(dst + ATT_HALF_BYTES, m, fb, x + 64, row, b2::kEvictFirst);
+          } else {
+            const CUtensorMap* m = i < 2 ? &tmK16 : &tmV16;
+            const int groups = (left + 15) >> 4;
+            b2::mbar_arrive_expect_tx(fb, groups * (WD_STAGE_BYTES / 4));
+            for (int r = 0; r < groups; ++r) {
+              b2::tma_load_2d(dst + r * 16 * 128, m, fb, x, row + r * 16, b2::kEvictFirst);
+              b2::tma_load_2d(dst + r * 16 * 128 + ATT_HALF_BYTES, m, fb, x + 64, row + r * 16, b2::kEvictFirst);
+            }
+          }
+          if (++stage == a.stages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+    return;
+  }
+
+  // ---------------- consumers ----------------
+  const int g = lane >> 2, c = lane & 3;  // row (query head of the group) and column pair of the fragments
+  const int k_tok = ((lane >> 4) << 3) + (lane & 7), k_chunk = (lane >> 3) & 1;
+  const int v_tok = (((lane >> 3) & 1) << 3) + (lane & 7), v_chunk = lane >> 4;
+  b2::pdl_wait();
+  uint32_t qf[8][2];
+  {
+    const uint16_t* qrow = a.q + static_cast<int64_t>(b) * a.q_stride + (head * a.group + g) * ATT_HD;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) qf[k][i] = g < a.group ? *reinterpret_cast<const uint32_t*>(qrow + k * 16 + i * 8 + c * 2) : 0u;
+  }
+  float o[4][2] = {};  // this warp's 32 dimensions
+  float m = -INFINITY, l = 0.f;
+  // (A wait that runs out leaves its flag, the waits after it end at once, and the walk goes on to its end: every warp meets every barrier.)
+  auto landed = [&]() { b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, 1000000000ull, B2_WAIT_SMEM_FULL); };
+  auto release = [&]() {
+    __syncwarp();
+    if (lane == 0) b2::mbar_arrive(bar_empty + stage * 8);
+    if (++stage == a.stages) { stage = 0; phase ^= 1; }
+  };
+  for (int j = blocks - 1; j >= 0; --j) {
+    const int there = min(WD_BLOCK, len - j * WD_BLOCK);  // tokens of the block that exist
+    float s[2][2][2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      s[t][0][0] = s[t][0][1] = s[t][1][0] = s[t][1][1] = 0.f;
+      const int left = there - t * ATT_TILE - warp * 16;
+      if (there > t * ATT_TILE) {
+        landed();
+        if (left > 0) {
+          const uint32_t k_row = ring + stage * WD_STAGE_BYTES + (warp * 16 + k_tok) * 128;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            uint32_t kf[4];
+            b2::ldmatrix_x4(kf, k_row + (k >> 2) * ATT_HALF_BYTES + ((((k & 3) * 2 + k_chunk) ^ (k_tok & 7)) << 4));
+            b2::mma_rows8(s[t][0][0], s[t][0][1], qf[k][0], qf[k][1], kf[0], kf[1]);
+            b2::mma_rows8(s[t][1][0], s[t][1][1], qf[k][0], qf[k][1], kf[2], kf[3]);
+          }
+        }
+        release();
+      }
+      if (left < 16) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (i * 8 + c * 2 + e >= left) s[t][i][e] = -INFINITY;
+      }
+    }
+    float mx = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, s[i >> 2][(i >> 1) & 1][i & 1]);
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    if (c == 0) s_m[warp][g] = mx;
+    consumers_meet();
+    mx = fmaxf(fmaxf(fmaxf(s_m[0][g], s_m[1][g]), fmaxf(s_m[2][g], s_m[3][g])), m);
+    const float f = mx == m ? 1.f : b2::ex2((m - mx) * a.scale_log2);
+    const float ref = mx == -INFINITY ? 0.f : mx * a.scale_log2;
+    m = mx;
+    l *= f;
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        *reinterpret_cast<float2*>(&s_p[g][t * ATT_TILE + warp * 16 + i * 8 + c * 2]) =
+            make_float2(b2::ex2(fmaf(s[t][i][0], a.scale_log2, -ref)), b2::ex2(fmaf(s[t][i][1], a.scale_log2, -ref)));
+    consumers_meet();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      o[i][0] *= f;
+      o[i][1] *= f;
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (there <= t * ATT_TILE) break;
+      landed();
+      const uint32_t v_row = ring + stage * WD_STAGE_BYTES + (warp >> 1) * ATT_HALF_BYTES + v_tok * 128;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int left = there - t * ATT_TILE - k * 16;
+        if (left <= 0) break;
+        const float* pr = &s_p[g][t * ATT_TILE + k * 16 + c * 2];
+        const float2 x = *reinterpret_cast<const float2*>(pr), y = *reinterpret_cast<const float2*>(pr + 8);
+        l = l + x.x + x.y + y.x + y.y;  // (every warp reads all of them: each holds the whole sum)
+        const uint32_t p0 = b2::pack_bf16(x.x, x.y), p1 = b2::pack_bf16(y.x, y.y);
+        // rows past the context's end may hold anything: they count as zero
+        uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
+        if (left < 16) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) keep[i] = (i * 8 + c * 2 < left ? 0xffffu : 0u) | (i * 8 + c * 2 + 1 < left ? 0xffff0000u : 0u);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          uint32_t vf[4];
+          b2::ldmatrix_x4_trans(vf, v_row + k * 16 * 128 + (((((warp & 1) * 2 + i) * 2 + v_chunk) ^ (v_tok & 7)) << 4));
+          b2::mma_rows8(o[2 * i][0], o[2 * i][1], p0, p1, vf[0] & keep[0], vf[1] & keep[1]);
+          b2::mma_rows8(o[2 * i + 1][0], o[2 * i + 1][1], p0, p1, vf[2] & keep[0], vf[3] & keep[1]);
+        }
+      }
+      release();
+    }
+  }
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  if (g < a.group) {
+    const float inv = l > 0.f ? __fdividef(1.f, l) : 0.f;  // (no context: zeros)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<uint32_t*>(out + g * ATT_HD + warp * 32 + i * 8 + c * 2) = b2::pack_bf16(o[i][0] * inv, o[i][1] * inv);
+  }
+  const int aborted = *abort_flag;
+  if (aborted) {
+    for (int i = 0; i < 100; ++i) __nanosleep(2000);  // copies in flight land before the CTA leaves
+    if (threadIdx.x == 0) b2::report_timeout(a.status, aborted);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // prefill_attention_kernel
 //
 // Causal attention of many query tokens per sequence over keys and values in rows of a matrix (the qkv output) or in the paged
@@ -757,6 +981,9 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   if (warp == 1) b2::tmem_dealloc(tmem, 512);
 }
 
+// softmax scale * log2(e); masked scores are -inf, and -inf times zero is none
+float scale_for_exp2(float scale) { return scale == 0.f ? FLT_MIN : scale * 1.4426950408889634f; }
+
 constexpr size_t ATT_SMEM_LIMIT = 113 * 1024;  // two CTAs per SM (228 KB, 1 KB of it reserved per CTA)
 constexpr size_t attention_smem(int n_seqs, int group) {
   return 1024 + ATT_STAGES * ATT_STAGE_BYTES + static_cast<size_t>(ATT_WARPS) * group * ATT_HD * sizeof(float) + (2 * static_cast<size_t>(n_seqs) + 1) * sizeof(int);
@@ -771,6 +998,7 @@ int configure_once() {
   if (dev < 0 || dev >= 64) return b2::set_error(B2_ERR_UNSUPPORTED, "device ordinal %d not supported", dev);
   if (!done[dev].load(std::memory_order_acquire)) {
     B2_CUDA(cudaFuncSetAttribute(paged_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM_LIMIT));
+    B2_CUDA(cudaFuncSetAttribute(paged_decode_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem(WD_MAX_STAGES)));
     B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     done[dev].store(true, std::memory_order_release);
   }
@@ -782,8 +1010,8 @@ int configure_once() {
 extern "C" {
 
 int b2_paged_attention_supported(int n_seqs, int nq, int nkv, int head_dim, int block_size) {
-  return n_seqs > 0 && n_seqs <= ATT_MAX_SEQS && nkv > 0 && nq % nkv == 0 && nq / nkv <= ATT_MAX_GROUP && head_dim == ATT_HD && block_size % ATT_TILE == 0 &&
-         n_seqs <= B2_ATTN_MAX_ITEMS / nkv;
+  return n_seqs > 0 && n_seqs <= ATT_MAX_SEQS && nkv > 0 && nq % nkv == 0 && nq / nkv <= WD_MAX_GROUP && head_dim == ATT_HD && block_size % ATT_TILE == 0 &&
+         n_seqs <= B2_ATTN_MAX_ITEMS / nkv && (nq / nkv <= ATT_MAX_GROUP || n_seqs * nkv >= WD_MIN_ITEMS);
 }
 
 int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k_cache, const void* v_cache, int num_blocks, int block_size,
@@ -809,7 +1037,7 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   a.n_seqs = n_seqs;
   a.nkv = nkv;
   a.group = nq / nkv;
-  a.scale_log2 = scale * 1.4426950408889634f;
+  a.scale_log2 = scale_for_exp2(scale);
   a.out = static_cast<uint16_t*>(out);
   a.ws = ctx->attn_ws;
   a.counters = ctx->attn_counters;
@@ -821,9 +1049,15 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   }
   const int64_t most = static_cast<int64_t>(n_seqs) * nkv * ((static_cast<int64_t>(bt_width) * block_size + ATT_TILE - 1) / ATT_TILE);
   const int grid = static_cast<int>(std::min<int64_t>(most, static_cast<int64_t>(ctx->num_sms) * ATT_CTAS_PER_SM));
-  const size_t smem = attention_smem(n_seqs, a.group);
   const int crc = configure_once();
   if (crc != B2_OK) return crc;
+  const int items = n_seqs * nkv;
+  if (a.group > ATT_MAX_GROUP || (items >= 3 * ctx->num_sms && scale >= 0.f)) {  // (it takes the largest score for the maximum, whatever the scale)
+    a.stages = items <= 2 * ctx->num_sms ? WD_MAX_STAGES : items <= 3 * ctx->num_sms ? 4 : 3;
+    B2_CUDA(b2_launch(paged_decode_wide_kernel, dim3(items), dim3(ATT_THREADS), wide_smem(a.stages), static_cast<cudaStream_t>(stream), maps[0], maps[1], maps[2], maps[3], a));
+    return B2_OK;
+  }
+  const size_t smem = attention_smem(n_seqs, a.group);
   B2_CUDA(b2_launch(paged_decode_kernel, dim3(grid), dim3(ATT_THREADS), smem, static_cast<cudaStream_t>(stream), maps[0], maps[1], maps[2], maps[3], a));
   return B2_OK;
 }

@@ -128,7 +128,7 @@ def embed(ids: torch.Tensor, w: torch.Tensor, vocab_start: int, vocab_end: int, 
 def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, context_lens: torch.Tensor, block_tables: torch.Tensor,
                     scale: float) -> torch.Tensor | None:
     """Decode attention: one query token per sequence, q [n, nq, head_dim], over the paged cache.  None when the
-    kernel does not serve the call (head_dim other than 128, more than 2 query heads per KV head, a layout it cannot address);
+    kernel does not serve the call (head_dim other than 128, more than 2 query heads per KV head in a small batch, a layout it cannot address);
     operands that do not fit each other, or are not on one GPU, raise."""
     return _native.paged_attention(get_runtime().handle, q, k_cache, v_cache, context_lens, block_tables, scale)
 
