@@ -444,8 +444,8 @@ int b2_decode_stack(b2_ctx* ctx, const b2_stack_layer* layers, int n_layers, con
  * sequence b's keys in rows cu_k[b] .. ; else k and v are the caches, kv_rows = blocks * block_size slots, and
  * block_tables (bt_width columns, row stride bt_stride) says where.  max_q: the most query rows of a sequence.
  * out [tokens, nq, head_dim] contiguous.  fp32 scores and sums, probabilities rounded to bf16 for the second product.
- * b2_prefill_attention_supported says (1 / 0) whether the shape is served: head_dim 128, two query heads per KV head, blocks
- * of a multiple of 128 tokens (block_size 0: no block table). */
+ * b2_prefill_attention_supported says (1 / 0) whether the shape is served: head_dim 128, an even number of query heads per KV
+ * head, blocks of a multiple of 128 tokens (block_size 0: no block table). */
 int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, int64_t kv_rows,
                          const int32_t* block_tables, int64_t bt_stride, int bt_width, int block_size, const int32_t* cu_q,
                          const int32_t* cu_k, int n_seqs, int max_q, int tokens, int nq, int nkv, int head_dim, float scale,

@@ -670,28 +670,40 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 // prefill_attention_kernel
 //
 // Causal attention of many query tokens per sequence over keys and values in rows of a matrix (the qkv output) or in the paged
-// cache.  Bound: the exponentials and the tensor pipe, which take about the same time per block (16 exponentials and 4096
-// multiply-adds per clock and SM); one sequence of 8192 tokens, 16 heads, 458 us = 601 TFLOP/s.
+// cache.  Bound: the tensor pipe and what feeds it.  A block of 64 keys takes both heads' scores 768 clocks (Q is read again for
+// every 64 columns: 48 KB of shared memory per head), their products 512 and their exponentials 1024 of the units that run beside
+// those; the walk does a block in about 1900, and in 1800 with the softmax left out.  One sequence of 8192 tokens, 16 heads, 458 -> 246 us
+// (1120 TFLOP/s); eight of 2048 244 -> 168; four of 1024, 32 / 8 heads, 131 us in flash-attn, 57 here.
 //
-// A CTA takes 128 query tokens of one sequence for the two heads that share a KV head: both heads' scores come from the same
-// K block, and while the tensor cores work for one head, four warps turn the other's scores into probabilities.
-//   warp 0      TMA: Q of both heads once, then K and V blocks of 128 tokens, two of each in flight
-//   warp 1      tcgen05.mma: S = Q K^T (128 x 128, fp32, tensor memory), O += P V with P read from tensor memory
-//   warps 2..9  one thread per query row and head: running maximum and sum, P = exp2(...) rounded to bf16 over S
-// Tensor memory: S of the two heads, then O of the two heads, 128 columns each.  O is rescaled whenever a row's maximum grows, so
-// that the largest probability is exactly 1.  (Rescaling only past a growth of 2^8 rounds it: against float64, scores of standard
-// deviation 3, 2048 tokens, the error was 2.13e-3 where flash-attn's is 1.76e-3, and is 1.77e-3 now; of that the output's own
-// rounding is 1.66e-3.  8192 tokens x 16 heads took 478 us instead of 446; 458 since the TMA and MMA warps walk whole, see b2_gemm_tile.cu.)
+// A CTA takes 128 query tokens of one sequence for two heads that share a KV head, and walks the keys from the tile's diagonal
+// down in blocks of 64:
+//   warp 0        TMA: Q of both heads once, then K and V blocks, four of each in flight
+//   warps 1, 2    tcgen05.mma of a head each: S = Q K^T (128 x 64, fp32, tensor memory), O += P V with P read from tensor memory
+//   warps 4..11   one thread per query row and head: running maximum and sum, P = exp2(...) rounded to bf16 over S
+//   warps 12..15  O is rescaled where a row's maximum has grown, while the softmax warps are at their exponentials
+// Tensor memory: two S of 64 columns per head, then O of the two heads, 128 columns each.  With two S the scores of the next
+// block are there before this one's are done with: a head's warp issues P V (block j), then Q K^T (block j + 2) into the columns
+// that P is read from, and needs no wait between the two, as they execute in the order of issue.  (With one S of 128 keys per head
+// and one warp for both, the heads ran in step: 7700 clocks per 128 keys.  One warp for both, here: 275 us instead of 246; values that are
+// the same in all lanes but not in a form that shows it, b2::uniform: 346.)
+//
+// Every probability is rounded to bf16 against the maximum of its block and those walked before, as in flash-attn, whose results
+// these are, bit for bit on random data.  Over a block table that library takes blocks of 128 tokens; PAIRS does the same: two blocks share the
+// maximum of both, the lower one goes first.  Narrow groups do without: 28 layers of a 1024-wide model move by 0.5 %.
+//
+// O is rescaled whenever a row's maximum grows, so that the largest probability so far is exactly 1 (rescaling only past a growth of
+// 2^8 rounds it: 2.13e-3 from float64 where scores have standard deviation 3, against 1.76e-3).
 // ---------------------------------------------------------------------------
-constexpr int PF_ROWS = 128, PF_KEYS = 128, PF_THREADS = 320;
-constexpr uint32_t PF_TILE = 128 * 128 * 2;                     // 128 rows of 128 bf16, as two 64-wide swizzled halves
-constexpr uint32_t PF_SMEM = 1024 + 2 * PF_TILE + 4 * PF_TILE;  // alignment, Q, two K and two V blocks
+constexpr int PF_ROWS = 128, PF_KEYS = 64, PF_THREADS = 512, PF_STAGES = 4;
+constexpr uint32_t PF_Q = 128 * 128 * 2;        // 128 rows of 128 bf16, as two 64-wide swizzled halves
+constexpr uint32_t PF_KV = PF_KEYS * 128 * 2;   // a block of keys or of values, the same way
+constexpr uint32_t PF_SMEM = 1024 + 2 * PF_Q + 2 * PF_STAGES * PF_KV;
 constexpr uint64_t PF_LIMIT_NS = 1000000000ull;
 
 struct PrefillArgs {
   const int32_t *cu_q, *cu_k, *tables;  // tables: null = keys and values are rows cu_k[b] .. of the matrices
   int64_t bt_stride;
-  int bt_width, block_size, kv_rows, nq;
+  int bt_width, block_size, kv_rows, nq, group;
   uint16_t* out;
   float scale_log2;
   B2Status* status;
@@ -705,47 +717,65 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t d, uint32_t a_tmem, uint64
       ::"r"(d), "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]),
       "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// tcgen05.wait::ld, before which nothing reads the 64 columns
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[2][32]) {
+  b2::tc_wait_ld();
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 32; i += 8)
+      asm volatile("" : "+r"(r[h][i]), "+r"(r[h][i + 1]), "+r"(r[h][i + 2]), "+r"(r[h][i + 3]), "+r"(r[h][i + 4]), "+r"(r[h][i + 5]), "+r"(r[h][i + 6]), "+r"(r[h][i + 7]));
+}
+// two products and sums in one instruction, each rounded as fmaf rounds it
+__device__ __forceinline__ uint64_t pair_of(float x, float y) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(x), "f"(y));
+  return p;
+}
+__device__ __forceinline__ void fma_pair(float& x, float& y, uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(d));
+}
 // V as the second operand, [tokens][dimensions] with the dimensions contiguous: MN-major, 128-byte swizzle.  8 tokens are 1024
-// bytes apart (stride offset), the two halves of 64 dimensions PF_TILE / 2 (leading offset).
+// bytes apart (stride offset), the two halves of 64 dimensions PF_KV / 2 (leading offset).
 __device__ __forceinline__ uint64_t umma_smem_desc_mn(uint32_t addr) {
-  return static_cast<uint64_t>((addr & 0x3FFFF) >> 4) | (static_cast<uint64_t>((PF_TILE / 2) >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+  return static_cast<uint64_t>((addr & 0x3FFFF) >> 4) | (static_cast<uint64_t>((PF_KV / 2) >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
          (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
 }
 
+template <bool PAIRS>
 __global__ void __launch_bounds__(PF_THREADS, 1)
 prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const PrefillArgs a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const uint32_t s_q = b2::smem_u32(smem), s_k = s_q + 2 * PF_TILE, s_v = s_k + 2 * PF_TILE;
-  __shared__ __align__(8) uint64_t s_bars[15];
+  const uint32_t s_q = b2::smem_u32(smem), s_k = s_q + 2 * PF_Q, s_v = s_k + PF_STAGES * PF_KV;
+  __shared__ __align__(8) uint64_t s_bars[1 + 4 * PF_STAGES + 4 + 4 + 16 + 2 + 2];
+  __shared__ float s_factor[2][2][PF_ROWS];  // [head][block & 1][row]: what O is multiplied by before the block's product
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   volatile int* abort_flag = &s_abort;
   const uint32_t bars = b2::smem_u32(s_bars);
-  const uint32_t q_full = bars, k_full = bars + 8, k_empty = bars + 24, v_full = bars + 40, v_empty = bars + 56, s_full = bars + 72, p_full = bars + 88,
-                 o_done = bars + 104;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t q_full = bars, k_full = bars + 8, k_empty = k_full + PF_STAGES * 8, v_full = k_empty + PF_STAGES * 8, v_empty = v_full + PF_STAGES * 8;
+  // [head][block & 1], and for the factors one per warp beside those; o_done: the product of a block, o_final: of the last one
+  const uint32_t s_full = v_empty + PF_STAGES * 8, p_full = s_full + 4 * 8, f_full = p_full + 4 * 8, o_done = f_full + 16 * 8, o_final = o_done + 2 * 8;
+  const int warp = b2::uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     b2::tma_prefetch_desc(&tmQ);
     b2::tma_prefetch_desc(&tmK);
     b2::tma_prefetch_desc(&tmV);
     b2::mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      b2::mbar_init(k_full + i * 8, 1);
-      b2::mbar_init(k_empty + i * 8, 1);
-      b2::mbar_init(v_full + i * 8, 1);
-      b2::mbar_init(v_empty + i * 8, 1);
-      b2::mbar_init(s_full + i * 8, 1);
-      b2::mbar_init(p_full + i * 8, 4);
-      b2::mbar_init(o_done + i * 8, 1);
-    }
+    for (int i = 0; i < 4 * PF_STAGES; ++i) b2::mbar_init(k_full + i * 8, (i / PF_STAGES) & 1 ? 2 : 1);  // (a block is free when both heads are done with it)
+    for (int i = 0; i < 4; ++i) b2::mbar_init(s_full + i * 8, 1);
+    for (int i = 0; i < 4; ++i) b2::mbar_init(p_full + i * 8, 8);
+    for (int i = 0; i < 16 + 4; ++i) b2::mbar_init(f_full + i * 8, 1);
     s_abort = 0;
     b2::mbar_fence_init();
   }
@@ -756,202 +786,194 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   b2::tc_fence_before();
   __syncthreads();
   b2::tc_fence_after();
-  const uint32_t tmem = s_tmem;
+  const uint32_t tmem = b2::uniform(s_tmem);
   b2::pdl_launch_dependents();
   b2::pdl_wait();
 
   // sequence, pair of heads, tile of 128 query tokens (the long rows of the causal triangle first)
-  const int b = blockIdx.z, kv_head = blockIdx.y, head = kv_head * 2;
-  const int q0 = __ldg(a.cu_q + b), q_len = __ldg(a.cu_q + b + 1) - q0;
-  const int k0 = __ldg(a.cu_k + b), kv_len = __ldg(a.cu_k + b + 1) - k0;
-  const int t0 = (gridDim.x - 1 - blockIdx.x) * PF_ROWS;
+  const int b = blockIdx.y, head = blockIdx.x * 2, kv_head = head / a.group;
+  const int q0 = b2::uniform(__ldg(a.cu_q + b)), q_len = b2::uniform(__ldg(a.cu_q + b + 1)) - q0;
+  const int k0 = b2::uniform(__ldg(a.cu_k + b)), kv_len = b2::uniform(__ldg(a.cu_k + b + 1)) - k0;
+  const int t0 = (gridDim.z - 1 - blockIdx.z) * PF_ROWS;
   const int shift = kv_len - q_len;  // position of the first query token
-  const int n = t0 < q_len && kv_len > 0 ? max(1, (min(kv_len, shift + min(q_len, t0 + PF_ROWS)) + PF_KEYS - 1) / PF_KEYS) : 0;  // key blocks
+  const int n = kv_len > 0 ? max(1, (min(kv_len, shift + min(q_len, t0 + PF_ROWS)) + PF_KEYS - 1) / PF_KEYS) : 0;  // key blocks
+  if (t0 >= q_len || n == 0) {
+    // queries of a sequence without keys: nothing to attend to
+    for (int i = threadIdx.x; i < min(PF_ROWS, q_len - t0) * 32; i += PF_THREADS)
+      *reinterpret_cast<uint4*>(a.out + (static_cast<int64_t>(q0 + t0 + (i >> 5)) * a.nq + head) * 128 + (i & 31) * 8) = make_uint4(0, 0, 0, 0);
+    if (warp == 1) b2::tmem_dealloc(tmem, 512);
+    return;
+  }
+  auto all_wait = [&](uint32_t bar, uint32_t phase, int code) {
+    return __all_sync(0xffffffffu, b2::mbar_wait(bar, phase, abort_flag, PF_LIMIT_NS, code)) != 0;
+  };
+  // block j of the walk in the order of the keys (its scores are in buffer j & 1 of its head)
+  const int odd = PAIRS ? n & 1 : 0;
+  auto block_of = [&](int j) { return !PAIRS || j < odd ? n - 1 - j : n - odd - 2 - ((j - odd) & ~1) + ((j - odd) & 1); };
 
   if (warp == 0) {
     // (the whole warp walks and one thread issues, here and in the next warp: operands then stay in uniform registers)
-    if (n > 0) {
+    if (b2::elect_one()) {
+      b2::mbar_arrive_expect_tx(q_full, 2 * PF_Q);
+      for (int h = 0; h < 2; ++h)
+        for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_q + h * PF_Q + i * (PF_Q / 2), &tmQ, q_full, (head + h) * 128 + i * 64, q0 + t0, b2::kEvictFirst);
+    }
+    __syncwarp();
+    const int x = kv_head * 128;
+    auto load = [&](int j, const CUtensorMap* map, uint32_t full, uint32_t empty, uint32_t dst) {
+      const int st = j & (PF_STAGES - 1), tok = block_of(j) * PF_KEYS;
+      int y = k0 + tok;
+      if (a.tables != nullptr) {
+        const int blk = tok / a.block_size;
+        y = max(0, __ldg(a.tables + static_cast<int64_t>(b) * a.bt_stride + min(blk, a.bt_width - 1))) * a.block_size + tok - blk * a.block_size;
+        y = min(y, a.kv_rows - 1);  // (a bad table entry must not lead outside the cache)
+      }
+      if (!all_wait(empty + st * 8, ((j / PF_STAGES) & 1) ^ 1, B2_WAIT_SMEM_EMPTY)) return false;
       if (b2::elect_one()) {
-        b2::mbar_arrive_expect_tx(q_full, 2 * PF_TILE);
-        for (int h = 0; h < 2; ++h)
-          for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_q + h * PF_TILE + i * (PF_TILE / 2), &tmQ, q_full, (head + h) * 128 + i * 64, q0 + t0, b2::kEvictFirst);
+        b2::mbar_arrive_expect_tx(full + st * 8, PF_KV);
+        for (int i = 0; i < 2; ++i) b2::tma_load_2d(dst + st * PF_KV + i * (PF_KV / 2), map, full + st * 8, x + i * 64, y, b2::kEvictLast);
       }
       __syncwarp();
-      const int x = kv_head * 128;
-      auto free = [&](uint32_t bar, uint32_t phase) { return __all_sync(0xffffffffu, b2::mbar_wait(bar, phase, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_EMPTY)) != 0; };
-      for (int j = 0; j < n; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = ((j >> 1) & 1) ^ 1;
-        int y = k0 + j * PF_KEYS;
-        if (a.tables != nullptr) {
-          const int tok = j * PF_KEYS, blk = tok / a.block_size;
-          y = max(0, __ldg(a.tables + static_cast<int64_t>(b) * a.bt_stride + min(blk, a.bt_width - 1))) * a.block_size + tok - blk * a.block_size;
-          y = min(y, a.kv_rows - 1);  // (a bad table entry must not lead outside the cache)
-        }
-        if (!free(k_empty + st * 8, ph)) break;
-        if (b2::elect_one()) {
-          b2::mbar_arrive_expect_tx(k_full + st * 8, PF_TILE);
-          for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_k + st * PF_TILE + i * (PF_TILE / 2), &tmK, k_full + st * 8, x + i * 64, y, b2::kEvictLast);
-        }
-        __syncwarp();
-        if (!free(v_empty + st * 8, ph)) break;
-        if (b2::elect_one()) {
-          b2::mbar_arrive_expect_tx(v_full + st * 8, PF_TILE);
-          for (int i = 0; i < 2; ++i) b2::tma_load_2d(s_v + st * PF_TILE + i * (PF_TILE / 2), &tmV, v_full + st * 8, x + i * 64, y, b2::kEvictLast);
-        }
-        __syncwarp();
-      }
+      return true;
+    };
+    // in the order of use: K of two blocks, then V of a block and K of the one after the next
+    bool ok = load(0, &tmK, k_full, k_empty, s_k);
+    if (n > 1) ok = ok && load(1, &tmK, k_full, k_empty, s_k);
+    for (int j = 0; ok && j < n; ++j) {
+      ok = load(j, &tmV, v_full, v_empty, s_v);
+      if (j + 2 < n) ok = ok && load(j + 2, &tmK, k_full, k_empty, s_k);
     }
-  } else if (warp == 1) {
-    if (n > 0) {
-      constexpr uint32_t idesc_s = b2::umma_idesc_bf16(PF_KEYS);
-      constexpr uint32_t idesc_o = b2::umma_idesc_bf16(128) | (1u << 16);  // second operand MN-major
-      auto wait = [&](uint32_t bar, uint32_t phase, int code) {
-        const bool ok = __all_sync(0xffffffffu, b2::mbar_wait(bar, phase, abort_flag, PF_LIMIT_NS, code)) != 0;
-        b2::tc_fence_after();
-        return ok;
-      };
-      auto scores = [&](int h, int st, bool last_of_block) {
-        if (b2::elect_one()) {
+  } else if (warp <= 2) {
+    const int h = warp - 1;
+    constexpr uint32_t idesc_s = b2::umma_idesc_bf16(PF_KEYS);
+    constexpr uint32_t idesc_o = b2::umma_idesc_bf16(128) | (1u << 16);  // second operand MN-major
+    const uint64_t desc_q = b2::umma_smem_desc(s_q + h * PF_Q), desc_k = b2::umma_smem_desc(s_k), desc_v = umma_smem_desc_mn(s_v);  // (addresses in 16 bytes)
+    auto wait = [&](uint32_t bar, uint32_t phase, int code) {
+      const bool ok = all_wait(bar, phase, code);
+      b2::tc_fence_after();
+      return ok;
+    };
+    auto scores = [&](int j) {
+      const int st = j & (PF_STAGES - 1), buf = h * 2 + (j & 1);
+      const bool ok = wait(k_full + st * 8, (j / PF_STAGES) & 1, B2_WAIT_SMEM_FULL);
+      if (ok && b2::elect_one()) {
+        const uint64_t dk = desc_k + st * (PF_KV >> 4);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            b2::umma_bf16(tmem + h * 128, b2::umma_smem_desc(s_q + h * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3),
-                          b2::umma_smem_desc(s_k + st * PF_TILE + (k >> 2) * (PF_TILE / 2)) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
-          b2::umma_commit(s_full + h * 8);
-          if (last_of_block) b2::umma_commit(k_empty + st * 8);
-        }
-        __syncwarp();
-      };
-      bool ok = wait(q_full, 0, B2_WAIT_SMEM_FULL) && wait(k_full, 0, B2_WAIT_SMEM_FULL);
-      if (ok) {
-        scores(0, 0, false);
-        scores(1, 0, true);
+        for (int k = 0; k < 8; ++k)
+          b2::umma_bf16(tmem + buf * PF_KEYS, desc_q + (k >> 2) * (PF_Q >> 5) + 2 * (k & 3), dk + (k >> 2) * (PF_KV >> 5) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
+        b2::umma_commit(s_full + buf * 8);
+        b2::umma_commit(k_empty + st * 8);
       }
-      for (int j = 0; ok && j < n; ++j) {
-        const int st = j & 1, nx = (j + 1) & 1;
-        ok = wait(v_full + st * 8, (j >> 1) & 1, B2_WAIT_SMEM_FULL);
-        for (int h = 0; ok && h < 2; ++h) {
-          ok = wait(p_full + h * 8, j & 1, B2_WAIT_TMEM_EMPTY);
-          if (!ok) break;
-          if (b2::elect_one()) {
+      __syncwarp();
+      return ok;
+    };
+    bool ok = wait(q_full, 0, B2_WAIT_SMEM_FULL) && scores(0);
+    if (n > 1) ok = ok && scores(1);
+    for (int j = 0; ok && j < n; ++j) {
+      const int st = j & (PF_STAGES - 1), buf = h * 2 + (j & 1);
+      ok = wait(v_full + st * 8, (j / PF_STAGES) & 1, B2_WAIT_SMEM_FULL) && wait(p_full + buf * 8, (j >> 1) & 1, B2_WAIT_TMEM_EMPTY);
+      if (!ok) break;
+      if (b2::elect_one()) {
+        const uint64_t dv = desc_v + st * (PF_KV >> 4);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)  // 16 tokens: 8 columns of P, 2048 bytes of V
-              umma_bf16_ts(tmem + 256 + h * 128, tmem + h * 128 + k * 8, umma_smem_desc_mn(s_v + st * PF_TILE + k * 2048), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-            b2::umma_commit(o_done + h * 8);
-            if (h == 1) b2::umma_commit(v_empty + st * 8);
-          }
-          __syncwarp();
-        }
-        if (!ok) break;
-        if (j + 1 < n) {
-          ok = wait(k_full + nx * 8, ((j + 1) >> 1) & 1, B2_WAIT_SMEM_FULL);
-          for (int h = 0; ok && h < 2; ++h) {
-            ok = wait(o_done + h * 8, j & 1, B2_WAIT_TMEM_FULL);  // P of this block has been read: its columns may take the next scores
-            if (ok) scores(h, nx, h == 1);
-          }
-        }
+        for (int k = 0; k < PF_KEYS / 16; ++k)  // 16 tokens: 8 columns of P, 2048 bytes of V
+          umma_bf16_ts(tmem + 256 + h * 128, tmem + buf * PF_KEYS + k * 8, dv + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+        b2::umma_commit(o_done + h * 8);
+        b2::umma_commit(v_empty + st * 8);
+        if (j == n - 1) b2::umma_commit(o_final + h * 8);
       }
+      __syncwarp();
+      if (j + 2 < n) ok = scores(j + 2);  // into the columns that P of this block is read from, after it
     }
-  } else if (n > 0) {
-    const int h = warp >= 6 ? 1 : 0, q = warp & 3, row = q * 32 + lane;
+  } else if (warp >= 4 && warp < 12) {
+    const int h = (warp >> 2) - 1, q = warp & 3, row = q * 32 + lane;
     const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
-    const uint32_t t_s = tmem + h * 128 + lanes, t_o = tmem + 256 + h * 128 + lanes;
     const int pos = shift + t0 + row;  // the last key this row sees
-    float m = -INFINITY, l = 0.f;      // the row's maximum, in units of scores, and its sum
+    float m = -INFINITY;               // the row's maximum, in units of scores
+    float l[4] = {};                   // its sum, of columns 2 i and 2 i + 1 of every eight
+    const uint64_t scale2 = pair_of(a.scale_log2, a.scale_log2);
     bool ok = true;
     for (int j = 0; ok && j < n; ++j) {
-      ok = b2::mbar_wait(s_full + h * 8, j & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_TMEM_FULL);
-      b2::tc_fence_after();
-      const int last = min(pos, kv_len - 1) - j * PF_KEYS;  // keys 0 .. last of the block count
-      const bool masked = __any_sync(0xffffffffu, last < PF_KEYS - 1);
-      float mx = -INFINITY;
+      const int buf = h * 2 + (j & 1);
+      const uint32_t t_s = tmem + buf * PF_KEYS + lanes;
+      // this block's scores, and without those that the row does not see
+      uint32_t r[2][32];
+      auto fetch = [&](int i) {
+        const uint32_t at = tmem + (h * 2 + (i & 1)) * PF_KEYS + lanes;
+        ok = all_wait(s_full + (h * 2 + (i & 1)) * 8, (i >> 1) & 1, B2_WAIT_TMEM_FULL);
+        b2::tc_fence_after();
+        b2::tmem_ld_32x32(at, r[0]);
+        b2::tmem_ld_32x32(at + 32, r[1]);
+        tc_wait_ld(r);
+        const int last = min(pos, kv_len - 1) - block_of(i) * PF_KEYS;  // keys 0 .. last of the block count
+        if (__any_sync(0xffffffffu, last < PF_KEYS - 1)) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        b2::tmem_ld_32x32(t_s + c * 32, r);
-        b2::tc_wait_ld();
-        if (masked) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) mx = fmaxf(mx, c * 32 + e <= last ? __uint_as_float(r[e]) : -INFINITY);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(r[e]));
+          for (int e = 0; e < 64; ++e)
+            if (e > last) r[e >> 5][e & 31] = 0xff800000u;  // -inf
         }
+      };
+      float mx[4] = {m, m, m, m};
+      auto maxima = [&]() {
+#pragma unroll
+        for (int e = 0; e < 64; e += 4)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], __uint_as_float(r[e >> 5][(e & 31) + i]));
+      };
+      if (PAIRS && j >= odd && ((j - odd) & 1) == 0) {  // the second of a pair is seen first for its maximum
+        fetch(j + 1);
+        maxima();
       }
-      const bool grow = mx > m;
-      if (__any_sync(0xffffffffu, grow)) {
-        const float f = grow ? (m == -INFINITY ? 0.f : exp2f((m - mx) * a.scale_log2)) : 1.f;
-        if (grow) m = mx;
-        l *= f;
-        if (j > 0) {  // (the previous block's product is complete: its scores' successor has been computed after it)
-#pragma unroll
-          for (int c = 0; c < 4; c += 2) {
-            uint32_t r[2][32];
-            b2::tmem_ld_32x32(t_o + c * 32, r[0]);
-            b2::tmem_ld_32x32(t_o + c * 32 + 32, r[1]);
-            b2::tc_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t w[16];
-#pragma unroll
-              for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(__uint_as_float(r[i >> 1][(i & 1) * 16 + e]) * f);
-              tmem_st_32x16(t_o + c * 32 + i * 16, w);
-            }
-          }
-        }
-      }
+      fetch(j);
+      if (!PAIRS || j < odd || ((j - odd) & 1) == 0) maxima();
+      const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      const float f = top > m ? b2::ex2((m - top) * a.scale_log2) : 1.f;
+      m = top;
+      s_factor[h][j & 1][row] = f;
+      __syncwarp();
+      if (lane == 0) b2::mbar_arrive(f_full + (buf * 4 + q) * 8);
       const float ref = m == -INFINITY ? 0.f : m * a.scale_log2;
+      const uint64_t ref2 = pair_of(-ref, -ref);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32], p[16];
-        b2::tmem_ld_32x32(t_s + c * 32, r);
-        b2::tc_wait_ld();
+      for (int i = 0; i < 4; ++i) l[i] *= f;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t p[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
-          float x = b2::ex2(fmaf(__uint_as_float(r[e]), a.scale_log2, -ref)), y = b2::ex2(fmaf(__uint_as_float(r[e + 1]), a.scale_log2, -ref));
-          if (masked) {
-            if (c * 32 + e > last) x = 0.f;
-            if (c * 32 + e + 1 > last) y = 0.f;
-          }
-          l += x + y;
+          float x, y;
+          fma_pair(x, y, pair_of(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1])), scale2, ref2);
+          x = b2::ex2(x);
+          y = b2::ex2(y);
+          l[(e >> 1) & 3] = l[(e >> 1) & 3] + x + y;
           p[e >> 1] = b2::pack_bf16(x, y);
         }
-        tmem_st_32x16(t_s + c * 16, p);  // columns this row has read already
-      }
-      if (h == 0 && (j + 1) * PF_KEYS > kv_len) {
-        // Rows past the sequence's last key count as zero: in the cache they may hold anything, in a matrix they are the next
-        // sequence's, and a probability of zero times Inf or NaN is NaN.
-        ok = b2::mbar_wait(v_full + (j & 1) * 8, (j >> 1) & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_SMEM_FULL) && ok;
-        if (j * PF_KEYS + row >= kv_len) {
-          unsigned char* v = smem + (s_v - s_q) + (j & 1) * PF_TILE + row * 128;
-#pragma unroll
-          for (int i = 0; i < 16; ++i)  // (another piece of every row of eight, so that they do not meet in a bank)
-            *reinterpret_cast<uint4*>(v + (i >> 3) * (PF_TILE / 2) + ((i ^ row) & 7) * 16) = make_uint4(0, 0, 0, 0);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tmem_st_32x16(t_s + c * 16, p);  // (this row has read its columns)
       }
       tc_wait_st();
       b2::tc_fence_before();
       __syncwarp();
-      if (lane == 0) b2::mbar_arrive(p_full + h * 8);
+      if (lane == 0) b2::mbar_arrive(p_full + buf * 8);
     }
-    ok = b2::mbar_wait(o_done + h * 8, (n - 1) & 1, abort_flag, PF_LIMIT_NS, B2_WAIT_TMEM_FULL) && ok;
+    ok = all_wait(o_final + h * 8, 0, B2_WAIT_TMEM_FULL) && ok;
     b2::tc_fence_after();
     if (ok && !*abort_flag) {
       // rows leave through this head's part of the Q buffer (its last product is complete): whole 256-byte rows
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      unsigned char* mine = smem + h * PF_TILE + q * 32 * 256;
+      const float sum = (l[0] + l[2]) + (l[1] + l[3]), inv = sum > 0.f ? __fdividef(1.f, sum) : 0.f;
+      const uint32_t t_o = tmem + 256 + h * 128 + lanes;
+      unsigned char* mine = smem + h * PF_Q + q * 32 * 256;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        b2::tmem_ld_32x32(t_o + c * 32, r);
-        b2::tc_wait_ld();
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r[2][32];
+        b2::tmem_ld_32x32(t_o + c * 64, r[0]);
+        b2::tmem_ld_32x32(t_o + c * 64 + 32, r[1]);
+        tc_wait_ld(r);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
+        for (int g = 0; g < 8; ++g) {
           uint32_t w[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) w[e] = b2::pack_bf16(__uint_as_float(r[g * 8 + 2 * e]) * inv, __uint_as_float(r[g * 8 + 2 * e + 1]) * inv);
-          const int piece = c * 4 + g;
+          for (int e = 0; e < 4; ++e)
+            w[e] = b2::pack_bf16(__uint_as_float(r[g >> 2][(g & 3) * 8 + 2 * e]) * inv, __uint_as_float(r[g >> 2][(g & 3) * 8 + 2 * e + 1]) * inv);
+          const int piece = c * 8 + g;
           *reinterpret_cast<uint4*>(mine + lane * 256 + ((piece ^ (lane & 15)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
@@ -964,9 +986,50 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
               *reinterpret_cast<const uint4*>(mine + r * 256 + ((piece ^ (r & 15)) << 4));
       }
     }
-  } else if (t0 < q_len) {  // queries of a sequence without keys: nothing to attend to
-    for (int i = threadIdx.x - 64; i < min(PF_ROWS, q_len - t0) * 32; i += PF_THREADS - 64)
-      *reinterpret_cast<uint4*>(a.out + (static_cast<int64_t>(q0 + t0 + (i >> 5)) * a.nq + head) * 128 + (i & 31) * 8) = make_uint4(0, 0, 0, 0);
+  } else if (warp >= 12) {
+    const int q = warp & 3, row = q * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
+    bool ok = true;
+    const int at = PAIRS && n > 1 ? 1 - odd : 0;  // where in the walk the last block of the keys is
+    if (n * PF_KEYS > kv_len) {
+      // Rows past the sequence's last key count as zero: in the cache they may hold anything, in a matrix they are the next
+      // sequence's, and a probability of zero times Inf or NaN is NaN.
+      ok = all_wait(v_full + at * 8, 0, B2_WAIT_SMEM_FULL);
+      const int key = row & 63;
+      if ((n - 1) * PF_KEYS + key >= kv_len) {
+        unsigned char* v = smem + (s_v - s_q) + at * PF_KV + (row >> 6) * (PF_KV / 2) + key * 128;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)  // (another piece of every row of eight, so that they do not meet in a bank)
+          *reinterpret_cast<uint4*>(v + ((i ^ key) & 7) * 16) = make_uint4(0, 0, 0, 0);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    for (int j = 0; ok && j < n; ++j)
+      for (int h = 0; ok && h < 2; ++h) {
+        const int buf = h * 2 + (j & 1);
+        ok = all_wait(f_full + (buf * 4 + q) * 8, (j >> 1) & 1, B2_WAIT_TMEM_FULL);
+        const float f = s_factor[h][j & 1][row];
+        if (ok && j > 0) ok = all_wait(o_done + h * 8, (j - 1) & 1, B2_WAIT_TMEM_FULL);  // (every phase is seen: none is taken for the one before)
+        if (ok && j > 0 && __any_sync(0xffffffffu, f != 1.f)) {
+          b2::tc_fence_after();
+          const uint32_t t_o = tmem + 256 + h * 128 + lanes;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t r[2][32];
+            b2::tmem_ld_32x32(t_o + c * 64, r[0]);
+            b2::tmem_ld_32x32(t_o + c * 64 + 32, r[1]);
+            tc_wait_ld(r);
+#pragma unroll
+            for (int e = 0; e < 64; ++e) r[e >> 5][e & 31] = __float_as_uint(__uint_as_float(r[e >> 5][e & 31]) * f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) tmem_st_32x16(t_o + c * 64 + i * 16, &r[i >> 1][(i & 1) * 16]);
+          }
+          tc_wait_st();
+          b2::tc_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) b2::mbar_arrive(p_full + buf * 8);
+      }
   }
 
   __syncwarp();
@@ -999,7 +1062,8 @@ int configure_once() {
   if (!done[dev].load(std::memory_order_acquire)) {
     B2_CUDA(cudaFuncSetAttribute(paged_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM_LIMIT));
     B2_CUDA(cudaFuncSetAttribute(paged_decode_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem(WD_MAX_STAGES)));
-    B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
+    B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
+    B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     done[dev].store(true, std::memory_order_release);
   }
   return B2_OK;
@@ -1062,12 +1126,9 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   return B2_OK;
 }
 
-// Exactly two query heads per KV head: a CTA's two tiles of scores are theirs.  Any number of tokens, though alone on the GPU
-// calls of a few are slower than flash-attn's (16 tokens 6.9 and 4.8 us; 32 sequences of one token over 768 cached 54 and 38): prefill steps are issued
-// eagerly, and the library's Python entry takes the host longer than that.  Whole steps of the 0.6B model, own and library:
-// one prompt of 16 tokens 1.52 and 2.67 ms, 32 of up to 16 tokens over 768 cached 3.82 and 3.86, 16 of up to 4 tokens 2.19 and 2.75.
+// An even number of query heads per KV head: a CTA's two tiles of scores are those of two heads with the same keys.
 int b2_prefill_attention_supported(int nq, int nkv, int head_dim, int block_size) {
-  return nkv > 0 && nq == 2 * nkv && head_dim == 128 && (block_size <= 0 || block_size % PF_KEYS == 0);
+  return nkv > 0 && nq > 0 && nq % (2 * nkv) == 0 && nq <= 65534 && head_dim == 128 && (block_size <= 0 || block_size % 128 == 0);
 }
 
 int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, int64_t kv_rows,
@@ -1097,9 +1158,11 @@ int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const voi
   a.kv_rows = static_cast<int>(kv_rows);
   a.nq = nq;
   a.out = static_cast<uint16_t*>(out);
-  a.scale_log2 = scale * 1.4426950408889634f;
+  a.scale_log2 = scale_for_exp2(scale);
   a.status = ctx->status_dev;
-  B2_CUDA(b2_launch(prefill_attention_kernel, dim3((max_q + PF_ROWS - 1) / PF_ROWS, nkv, n_seqs), dim3(PF_THREADS), PF_SMEM, static_cast<cudaStream_t>(stream),
+  a.group = nq / nkv;
+  const auto kernel = block_tables != nullptr && a.group > 2 ? prefill_attention_kernel<true> : prefill_attention_kernel<false>;
+  B2_CUDA(b2_launch(kernel, dim3(nq / 2, n_seqs, (max_q + PF_ROWS - 1) / PF_ROWS), dim3(PF_THREADS), PF_SMEM, static_cast<cudaStream_t>(stream),
                     tmQ, tmK, tmV, a));
   return B2_OK;
 }

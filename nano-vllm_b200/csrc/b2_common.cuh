@@ -123,6 +123,11 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, float x, float y, f
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
+// A value that all lanes of the warp hold, in a form that shows it: the compiler keeps what is computed from it, and loops that it bounds,
+// in the uniform registers from which TMA and tcgen05 instructions take their operands.
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 // True in one thread of a converged warp.  Tensor-core instructions take their operands from uniform registers, which the compiler only
 // keeps values in while the whole warp runs the code: a role's loop is run by all its lanes, and this thread issues.
 __device__ __forceinline__ bool elect_one() {

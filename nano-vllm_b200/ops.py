@@ -136,8 +136,8 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
 def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.Tensor, max_seqlen_q: int,
                       block_tables: torch.Tensor | None, scale: float) -> torch.Tensor | None:
     """Causal attention of q [tokens, nq, head_dim] over k, v [tokens, nkv, head_dim], or over the paged caches when
-    block_tables is given.  None when the kernel does not serve the call (it takes head_dim 128, two query heads per
-    KV head, forward only); operands that do not fit each other, or are not on one GPU, raise."""
+    block_tables is given.  None when the kernel does not serve the call (it takes head_dim 128, an even number of
+    query heads per KV head, forward only); operands that do not fit each other, or are not on one GPU, raise."""
     return _native.prefill_attention(get_runtime().handle, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, block_tables, scale)
 
 

@@ -69,6 +69,20 @@ def test_layouts_of_the_general_path_are_declined(pkg, kind, name, other):
     assert call(kind, args) is None
 
 
+@pytest.mark.parametrize("n_seqs,each,nq,served", [(75, 4, 8, False), (74, 4, 8, True), (75, 95, 8, False), (75, 96, 8, True), (75, 4, 4, True), (300, 1, 2, False), (8, 1, 8, True)])
+def test_many_short_prompts_of_wide_groups_are_declined(pkg, n_seqs, each, nq, served):
+    """Four heads per KV head and more, over 296 tiles of which most rows would be empty; odd groups are never served."""
+    nkv = 2
+    kv = [torch.zeros(n_seqs * each, nkv, 128, dtype=torch.bfloat16) for _ in range(2)]
+    cu = torch.arange(0, n_seqs * each + 1, each, dtype=torch.int32)
+    args = dict(q=torch.zeros(n_seqs * each, nq, 128, dtype=torch.bfloat16), k=kv[0], v=kv[1], cu_q=cu, cu_k=cu.clone(), max_q=each, block_tables=None)
+    if served:
+        with pytest.raises(TypeError, match="GPU"):  # (host tensors)
+            call("prefill", args)
+    else:
+        assert call("prefill", args) is None
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind,name", [("paged", x) for x in ("k_cache", "v_cache", "context_lens", "block_tables")] +
                          [("prefix", x) for x in ("k", "v", "cu_q", "cu_k", "block_tables")])

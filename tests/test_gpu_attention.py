@@ -70,15 +70,16 @@ def test_paged_attention_declines_other_shapes(rt):
     assert ops.paged_attention(torch.zeros(1, 3, 128, dtype=torch.bfloat16, device=DEV), kc, kc, lens, tables, 1.0) is None
 
 
-# (new tokens, cached tokens) per sequence: edges of the 128-token tiles and key blocks, a prefix, several blocks, one token
-PREFILL = [([(1, 0)], False), ([(127, 0), (128, 0), (129, 0)], False), ([(117, 0)], False), ([(300, 0), (5, 0), (1000, 0)], False),
+# (new tokens, cached tokens) per sequence: edges of the 128-token tiles and the 64-token key blocks, a prefix, several blocks, one token
+PREFILL = [([(1, 0)], False), ([(63, 0), (64, 0), (65, 0), (191, 0), (193, 0)], False), ([(64, 64), (63, 1), (65, 63)], True), ([(127, 0), (128, 0), (129, 0)], False), ([(117, 0)], False), ([(300, 0), (5, 0), (1000, 0)], False),
            ([(100, 512), (130, 256), (1, 255), (256, 1)], True), ([(900, 1100)], True)]
 
 
+@pytest.mark.parametrize("nq,nkv", [(16, 8), (8, 2), (8, 1)])
 @pytest.mark.parametrize("seqs,paged", PREFILL)
-def test_prefill_attention_against_fp32(rt, seqs, paged):
+def test_prefill_attention_against_fp32(rt, seqs, paged, nq, nkv):
     from nanovllm_b200 import ops
-    nq, nkv, hd, bs, scale = 16, 8, 128, 256, 128 ** -0.5
+    hd, bs, scale = 128, 256, 128 ** -0.5
     g = torch.Generator().manual_seed(sum(a + b for a, b in seqs))
     tokens = sum(a for a, _ in seqs)
     qkv = torch.randn(tokens, (nq + 2 * nkv) * hd, generator=g).bfloat16()
