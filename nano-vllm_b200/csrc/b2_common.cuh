@@ -124,7 +124,9 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, float x, float y, f
 }
 
 // A value that all lanes of the warp hold, in a form that shows it: the compiler keeps what is computed from it, and loops that it bounds,
-// in the uniform registers from which TMA and tcgen05 instructions take their operands.
+// in the uniform registers from which TMA and tcgen05 instructions take their operands.  (The warp's number, the tensor memory's address, a CTA's
+// rank: feature-lane GEMMs of up to 64 tokens 1-8 % - 37 x 10240 x 5120 28.9 -> 25.6 us, 64 x 24576 x 4096 with SiLU 42.8 -> 41.2 -,
+// prefill attention 346 -> 285 us at 8192 tokens.  Not in gemm_tile_kernel: its epilogue then spills, and it was 0.4 us slower.)
 __device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 __device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
 

@@ -927,7 +927,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
   unsigned long long* const cta_best = SampleTable<EPI>::get();
   unsigned int sample_call = 0;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = b2::uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int cta = blockIdx.x;
   const int KB = a.kblocks;
   const int tiles = a.tilesP * a.tilesQ;
@@ -959,7 +959,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUt
   b2::tc_fence_before();
   __syncthreads();
   b2::tc_fence_after();
-  const uint32_t tmem_base = has_gemm ? *tmem_slot : 0;
+  const uint32_t tmem_base = has_gemm ? b2::uniform(*tmem_slot) : 0;
   // The next kernel in the stream may start its own set-up from now on - unless this launch is a fused row-parallel
   // call: its CTAs later wait for rows that other CTAs of the same grid (and of the peers' grids) produce, so the
   // dependents are released only once every CTA has delivered its part (fused_tail), when nothing of this grid
@@ -1249,9 +1249,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
   unsigned char* red_buf = smem + STAGES * C::STAGE_BYTES + 256;
   __shared__ float red[NUM_THREADS / 32];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int S = static_cast<int>(b2::cluster_nctarank());
-  const int crank = static_cast<int>(b2::cluster_ctarank());
+  const int warp = b2::uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  const int S = b2::uniform(static_cast<int>(b2::cluster_nctarank()));
+  const int crank = b2::uniform(static_cast<int>(b2::cluster_ctarank()));
   // the output tile of this cluster: features [tile * 128, +128) of the tokens [tok0, tok0 + BN); the token tiles of one
   // feature tile belong to consecutive clusters, so that its weight tiles are read from DRAM once and from L2 after that
   const int ct = blockIdx.x / S;
@@ -1284,7 +1284,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
   b2::tc_fence_before();
   __syncthreads();
   b2::tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = b2::uniform(*tmem_slot);
   if (threadIdx.x == 0 && !is_push(EPI)) b2::pdl_launch_dependents();
   if (threadIdx.x == 0) stamp(a, 0);
   unsigned int parity = 0;
