@@ -2,7 +2,7 @@
 // on interleaved pairs, the head work of the qkv projection).
 //
 // One CTA pair (tcgen05.mma.cta_group::2) computes a tile of 256 features x bn tokens, bn <= 256 in steps of 32 chosen per
-// problem.  Weights fill the 256-row side, so a batch of any size wastes at most 31 token columns; each CTA of the pair stages
+// problem (16 for whole tiles).  Weights fill the 256-row side, so a batch of any size wastes at most 31 token columns a tile; each CTA of the pair stages
 // its own 128 weight rows and half of the tokens, which both tensor cores read.  Two instances:
 //   MULTI   more tiles than SM pairs, or a long ring: one CTA per SM, the pair walks its tiles with two accumulators in
 //           tensor memory, so that 8 epilogue warps store a tile under the next one's MMAs (with 2 CTAs per SM and one tile
@@ -456,7 +456,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(sums + g * 256 + i * 128) = make_float4(0.f, 0.f, 0.f, 0.f);
-      } else if (g1 - g >= 4) {
+      } else if (MULTI || g1 - g >= 4) {  // (a whole tile's columns are allocated in powers of two from 32)
         tmem_ld_16x256_x4(taddr + g * 8, acc[0]);
         tmem_ld_16x256_x4(taddr + (16u << 16) + g * 8, acc[1]);
       } else {  // (never past the columns that are allocated)
@@ -789,7 +789,9 @@ int launch_tile_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int
   a.M = M;
   a.N = N;
   a.kblocks = p.kblocks;
-  a.bn = p.bn;
+  // Whole tiles are as narrow as the tokens let them be in steps of 16 columns, the least step of a pair's tcgen05.mma: 777 tokens are 4 x 208
+  // and not the plan's 4 x 224.  An output's sum over K is the same; where K is cut, widths decide where, and stay.
+  a.bn = p.split == 1 && p.ranged == 0 ? ((M + p.tiles_t - 1) / p.tiles_t + 15) / 16 * 16 : p.bn;
   a.stages = p.stages;
   a.split = p.split;
   a.rounds = p.rounds;
@@ -818,7 +820,7 @@ int launch_tile_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int
   CUtensorMap tmW, tmX;
   rc = encode_tmap_2d(&tmW, W, K, N, ldw, BK, FM);
   if (rc != B2_OK) return rc;
-  rc = encode_tmap_2d(&tmX, A, K, M, lda, BK, p.bn / 2);
+  rc = encode_tmap_2d(&tmX, A, K, M, lda, BK, a.bn / 2);
   if (rc != B2_OK) return rc;
   if (p.multi)
     B2_CUDA(b2_launch_cluster(gemm_tile_kernel<true>, dim3(p.grid), dim3(Shape<true>::THREADS), p.smem, stream, 2u, tmW, tmX, a));

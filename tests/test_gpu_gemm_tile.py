@@ -105,3 +105,28 @@ def test_qkv_with_operands_off_the_16_byte_grid(rt, m):
     rt.check_status()
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m", [513, 530, 565, 777, 1041])
+def test_rows_are_the_same_whatever_the_width_of_the_tile(rt, m):
+    """From 512 tokens on K is not cut, so a row's results are the same bits in a batch whose tiles are another number of columns wide
+    (here 16 past a multiple of 32: 176, 144, 208; the whole batch 256 or 192), with each of the epilogues."""
+    from nanovllm_b200 import ops
+    nq, nkv, hd, k, full = 8, 4, 128, 512, 1536
+    g = torch.Generator(device=DEV).manual_seed(m)
+    x = torch.empty(full, k, device=DEV).normal_(generator=g).bfloat16()
+    w = torch.empty((nq + 2 * nkv) * hd, k, device=DEV).normal_(0, 0.05, generator=g).bfloat16()
+    qw, kw = ((torch.rand(hd, device=DEV, generator=g) + 0.5).bfloat16() for _ in range(2))
+    pos = torch.randint(0, 2048, (full,), device=DEV, generator=g)
+    table, slots = O.rope_cache(hd, 2048, 1e6).to(DEV), torch.arange(full, device=DEV, dtype=torch.int32)
+
+    def run(n):
+        kc, vc = (torch.zeros(full // 256, 256, nkv, hd, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        qkv = ops.qkv_fused(x[:n], w, None, nq, nkv, hd, qw, kw, 1e-6, pos[:n], table, kc, vc, slots[:n])
+        return [ops.gemm(x[:n], w)[:m], ops.gemm_silu_mul(x[:n], w)[:m], qkv[:m]] + [c.view(full, -1)[:m] for c in (kc, vc)]
+
+    part, whole = run(m), run(full)
+    torch.cuda.synchronize()
+    rt.check_status()
+    for a, b in zip(part, whole):
+        assert torch.equal(a, b)
