@@ -453,27 +453,30 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 // their order.  On random data the results are flash-attn's but for 0 to 3 elements in a million.
 //
 // 64 contexts of 1056 tokens, 32 / 8 heads: 66.7 us in flash-attn, 45.2 here (6.1 TB/s); 96 of 70..700 47.0 and 28.8, 32 of 1056
-// 34.9 and 26.1.  Narrow groups take this kernel too from three pairs of (sequence, KV head) per SM on, where nothing has to be cut to fill
+// 34.9 and 23.7.  Narrow groups take this kernel too from three pairs of (sequence, KV head) per SM on, where nothing has to be cut to fill
 // the chip and the other kernel's parts cost more than the even share saves: 256 contexts of 100..1024 tokens, 16 / 8 heads, 97.6 -> 90.8 us,
-// 128 of them 53.5 -> 48.4, 512 of 30..270 67.7 -> 55.8, 64 of 1056 49.1 -> 45.0; 37 of 40..700 (296 pairs) would go from 13.6 to 14.6.
+// 128 of them 53.5 -> 48.4, 512 of 30..270 67.7 -> 55.8, 64 of 1056 49.1 -> 45.0; 37 of 40..700 (296 pairs) would go from 13.6 to 14.1.
 //
 // Four CTAs per SM with a ring of three 16 KB tiles (64 tokens of K or of V) each, or fewer with longer rings where there are no
-// more to be had: 190 KB per SM in flight.
+// more to be had: 190 KB per SM in flight.  With no more than two CTAs for an SM (FEW) a block's product runs side by side with the next
+// block's scores: nothing else fills the gaps in a warp's chains of eight tensor-core sums.  A block takes 1.0 us instead of 1.8: 16 contexts
+// of 1056 tokens 19.5 -> 13.4 us (16.1 by the producer's whole warp and the longer ring alone), of 100..3000 42 -> 26, 32 of 1056 26.1 -> 23.7.
 // ---------------------------------------------------------------------------
 constexpr int WD_MAX_GROUP = 8;
-constexpr int WD_MAX_STAGES = 6;
+constexpr int WD_MAX_STAGES = 12;
 constexpr int WD_CTAS_PER_SM = 4;
 constexpr int WD_BLOCK = 2 * ATT_TILE;                    // tokens that share a maximum
 constexpr int WD_STAGE_BYTES = 2 * ATT_HALF_BYTES;        // dimensions 0..63, 64..127
 constexpr int WD_P_PITCH = WD_BLOCK + 8;                  // floats: rows start 8 banks apart, so that the 8-byte accesses of half a warp meet in none
-// Wide groups, from this many (sequence, KV head) pairs on: 16 contexts of 1056 tokens and 8 KV heads 38.9 us in the library, 19.5 here
-// (of 100..3000 tokens 59 and 42).  Fewer would be faster here too (8 contexts 35 and 19), but long contexts are then cut into parts in the
-// library, each rounded for itself, and a context of one CTA walks at 36 GB/s however long it is.
+// Wide groups, from this many (sequence, KV head) pairs on: 16 contexts of 1056 tokens and 8 KV heads 38.8 us in the library, 13.4 here
+// (of 100..3000 tokens 59 and 26).  Fewer would be faster here too (8 contexts 36 and 11), but long contexts are then cut into parts in the
+// library, each rounded for itself, and a context of one CTA walks at 65 GB/s however long it is (8 of 4000 tokens: 37 and 33).
 constexpr int WD_MIN_ITEMS = 128;
 constexpr uint32_t wide_smem(int stages) { return 1024 + stages * WD_STAGE_BYTES; }
-static_assert(2 * (wide_smem(WD_MAX_STAGES) + 5 * 1024) <= 228 * 1024 && 3 * (wide_smem(4) + 5 * 1024) <= 228 * 1024 && 4 * (wide_smem(3) + 5 * 1024) <= 228 * 1024, "CTAs per SM (5 KB: static, reserved)");
+static_assert(wide_smem(WD_MAX_STAGES) + 6 * 1024 <= 228 * 1024 && 2 * (wide_smem(6) + 6 * 1024) <= 228 * 1024 && 3 * (wide_smem(4) + 6 * 1024) <= 228 * 1024 && 4 * (wide_smem(3) + 6 * 1024) <= 228 * 1024, "CTAs per SM (6 KB: static, reserved)");
 
-__global__ void __launch_bounds__(ATT_THREADS, WD_CTAS_PER_SM)
+template <bool FEW>
+__global__ void __launch_bounds__(ATT_THREADS, FEW ? 2 : WD_CTAS_PER_SM)
 paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmK16,
                          const __grid_constant__ CUtensorMap tmV16, const AttnArgs a) {
   extern __shared__ unsigned char smem_raw[];
@@ -498,33 +501,34 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   __syncthreads();
   b2::pdl_launch_dependents();
   const int b = blockIdx.x / a.nkv, head = blockIdx.x - b * a.nkv;
-  const int len = max(0, min(__ldg(a.lens + b), a.bt_width * a.block_size));
+  const int len = b2::uniform(max(0, min(__ldg(a.lens + b), a.bt_width * a.block_size)));
   const int blocks = (len + WD_BLOCK - 1) / WD_BLOCK;
   uint16_t* out = a.out + static_cast<int64_t>(blockIdx.x) * a.group * ATT_HD;
   int stage = 0;
   uint32_t phase = 0;
 
-  if (warp == ATT_WARPS) {
-    // ---------------- TMA producer ----------------
-    if (lane == 0 && blocks > 0) {
-      const int32_t* table = a.tables + static_cast<int64_t>(b) * a.bt_stride;
-      const int x = head * ATT_HD;
-      bool ok = true;
-      b2::pdl_wait();
-      for (int j = blocks - 1; ok && j >= 0; --j) {
-        int y[2];
+  if (b2::uniform(warp) == ATT_WARPS) {  // (uniform for everyone, it costs the other warps registers that they spill)
+    // ---------------- TMA producer: the whole warp walks, one thread issues (see b2_gemm_tile.cu) ----------------
+    const int32_t* table = a.tables + static_cast<int64_t>(b) * a.bt_stride;
+    const int x = head * ATT_HD;
+    bool ok = true;
+    b2::pdl_wait();
+    for (int j = blocks - 1; ok && j >= 0; --j) {
+      int y[2];
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const int tok = min(j * WD_BLOCK + t * ATT_TILE, len - 1), no = tok / a.block_size;
-          y[t] = min(max(0, __ldg(table + no)), a.num_blocks - 1) * a.block_size + tok - no * a.block_size;  // inside the cache whatever the table holds
-        }
-        for (int i = 0; ok && i < 4; ++i) {  // K, K, V, V
-          const int left = len - j * WD_BLOCK - (i & 1) * ATT_TILE;
-          if (left <= 0) continue;
-          ok = b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, 1000000000ull, B2_WAIT_SMEM_EMPTY);
-          if (!ok) break;
-          const uint32_t fb = bar_full + stage * 8, dst = ring + stage * WD_STAGE_BYTES;
-          const int row = (i & 1) ? y[1] : y[0];
+      for (int t = 0; t < 2; ++t) {
+        const int tok = max(0, min(j * WD_BLOCK + t * ATT_TILE, len - 1)), no = tok / a.block_size;
+        y[t] = b2::uniform(min(max(0, __ldg(table + no)), a.num_blocks - 1)) * a.block_size + tok - no * a.block_size;  // inside the cache whatever the table holds
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // K, K, V, V
+        const int left = len - j * WD_BLOCK - (i & 1) * ATT_TILE;
+        if (left <= 0) continue;
+        ok = __all_sync(0xffffffffu, b2::mbar_wait(bar_empty + stage * 8, phase ^ 1, abort_flag, 1000000000ull, B2_WAIT_SMEM_EMPTY)) != 0;
+        if (!ok) break;
+        const uint32_t fb = bar_full + stage * 8, dst = ring + stage * WD_STAGE_BYTES;
+        const int row = y[i & 1];
+        if (b2::elect_one()) {
           if (left >= ATT_TILE) {
             const CUtensorMap* m = i < 2 ? &tmK : &tmV;
             b2::mbar_arrive_expect_tx(fb, WD_STAGE_BYTES);
@@ -539,8 +543,9 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
               b2::tma_load_2d(dst + r * 16 * 128 + ATT_HALF_BYTES, m, fb, x + 64, row + r * 16, b2::kEvictFirst);
             }
           }
-          if (++stage == a.stages) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == a.stages) { stage = 0; phase ^= 1; }
       }
     }
     return;
@@ -563,14 +568,41 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   float m = -INFINITY, l = 0.f;
   // (A wait that runs out leaves its flag, the waits after it end at once, and the walk goes on to its end: every warp meets every barrier.)
   auto landed = [&]() { b2::mbar_wait(bar_full + stage * 8, phase, abort_flag, 1000000000ull, B2_WAIT_SMEM_FULL); };
-  auto release = [&]() {
-    __syncwarp();
-    if (lane == 0) b2::mbar_arrive(bar_empty + stage * 8);
+  auto advance = [&]() {
+    const int was = stage;
     if (++stage == a.stages) { stage = 0; phase ^= 1; }
+    return was;
   };
-  for (int j = blocks - 1; j >= 0; --j) {
-    const int there = min(WD_BLOCK, len - j * WD_BLOCK);  // tokens of the block that exist
-    float s[2][2][2];
+  auto release = [&](int st) {
+    __syncwarp();
+    if (lane == 0) b2::mbar_arrive(bar_empty + st * 8);
+  };
+  auto k_row = [&]() { return ring + stage * WD_STAGE_BYTES + (warp * 16 + k_tok) * 128; };
+  auto v_row = [&]() { return ring + stage * WD_STAGE_BYTES + (warp >> 1) * ATT_HALF_BYTES + v_tok * 128; };
+  // 16 dimensions of the scores of this warp's 16 tokens of a tile
+  auto keys = [&](uint32_t row, int k, float (&d)[2][2]) {
+    uint32_t kf[4];
+    b2::ldmatrix_x4(kf, row + (k >> 2) * ATT_HALF_BYTES + ((((k & 3) * 2 + k_chunk) ^ (k_tok & 7)) << 4));
+    b2::mma_rows8(d[0][0], d[0][1], qf[k][0], qf[k][1], kf[0], kf[1]);
+    b2::mma_rows8(d[1][0], d[1][1], qf[k][0], qf[k][1], kf[2], kf[3]);
+  };
+  // 16 tokens of the product: the probabilities' fragments, their sum (every warp reads all of them: each holds the whole sum), the values;
+  // rows past the context's end may hold anything and count as zero
+  auto values = [&](uint32_t row, int t, int k, uint32_t keep0, uint32_t keep1) {
+    const float* pr = &s_p[g][t * ATT_TILE + k * 16 + c * 2];
+    const float2 x = *reinterpret_cast<const float2*>(pr), y = *reinterpret_cast<const float2*>(pr + 8);
+    l = l + x.x + x.y + y.x + y.y;
+    const uint32_t p0 = b2::pack_bf16(x.x, x.y), p1 = b2::pack_bf16(y.x, y.y);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint32_t vf[4];
+      b2::ldmatrix_x4_trans(vf, row + k * 16 * 128 + (((((warp & 1) * 2 + i) * 2 + v_chunk) ^ (v_tok & 7)) << 4));
+      b2::mma_rows8(o[2 * i][0], o[2 * i][1], p0, p1, vf[0] & keep0, vf[1] & keep1);
+      b2::mma_rows8(o[2 * i + 1][0], o[2 * i + 1][1], p0, p1, vf[2] & keep0, vf[3] & keep1);
+    }
+  };
+  float s[2][2][2];  // scores of this warp's tokens
+  auto scores = [&](int there) {
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       s[t][0][0] = s[t][0][1] = s[t][1][0] = s[t][1][1] = 0.f;
@@ -578,16 +610,11 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       if (there > t * ATT_TILE) {
         landed();
         if (left > 0) {
-          const uint32_t k_row = ring + stage * WD_STAGE_BYTES + (warp * 16 + k_tok) * 128;
+          const uint32_t row = k_row();
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            uint32_t kf[4];
-            b2::ldmatrix_x4(kf, k_row + (k >> 2) * ATT_HALF_BYTES + ((((k & 3) * 2 + k_chunk) ^ (k_tok & 7)) << 4));
-            b2::mma_rows8(s[t][0][0], s[t][0][1], qf[k][0], qf[k][1], kf[0], kf[1]);
-            b2::mma_rows8(s[t][1][0], s[t][1][1], qf[k][0], qf[k][1], kf[2], kf[3]);
-          }
+          for (int k = 0; k < 8; ++k) keys(row, k, s[t]);
         }
-        release();
+        release(advance());
       }
       if (left < 16) {
 #pragma unroll
@@ -597,6 +624,11 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
             if (i * 8 + c * 2 + e >= left) s[t][i][e] = -INFINITY;
       }
     }
+  };
+  if (FEW && blocks > 0) scores(len - (blocks - 1) * WD_BLOCK);
+  for (int j = blocks - 1; j >= 0; --j) {
+    const int there = min(WD_BLOCK, len - j * WD_BLOCK);  // tokens of the block that exist
+    if (!FEW) scores(there);
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < 8; ++i) mx = fmaxf(mx, s[i >> 2][(i >> 1) & 1][i & 1]);
@@ -621,35 +653,48 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       o[i][0] *= f;
       o[i][1] *= f;
     }
+    if (FEW && j > 0 && there == WD_BLOCK) {
+      // this block's product and the next one's scores side by side: four and four chains, of which a warp alone fills the gaps of neither
+      uint32_t vr[2], kr[2];
+      int from[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i < 2) vr[i] = v_row();
+        else kr[i - 2] = k_row();
+        landed();
+        from[i] = advance();
+      }
+#pragma unroll
+      for (int t = 0; t < 2; ++t) s[t][0][0] = s[t][0][1] = s[t][1][0] = s[t][1][1] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        keys(kr[0], k, s[0]);
+        keys(kr[1], k, s[1]);
+        values(vr[k >> 2], k >> 2, k & 3, 0xffffffffu, 0xffffffffu);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) release(from[i]);
+      continue;
+    }
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       if (there <= t * ATT_TILE) break;
+      const uint32_t row = v_row();
       landed();
-      const uint32_t v_row = ring + stage * WD_STAGE_BYTES + (warp >> 1) * ATT_HALF_BYTES + v_tok * 128;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int left = there - t * ATT_TILE - k * 16;
         if (left <= 0) break;
-        const float* pr = &s_p[g][t * ATT_TILE + k * 16 + c * 2];
-        const float2 x = *reinterpret_cast<const float2*>(pr), y = *reinterpret_cast<const float2*>(pr + 8);
-        l = l + x.x + x.y + y.x + y.y;  // (every warp reads all of them: each holds the whole sum)
-        const uint32_t p0 = b2::pack_bf16(x.x, x.y), p1 = b2::pack_bf16(y.x, y.y);
-        // rows past the context's end may hold anything: they count as zero
         uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
         if (left < 16) {
 #pragma unroll
           for (int i = 0; i < 2; ++i) keep[i] = (i * 8 + c * 2 < left ? 0xffffu : 0u) | (i * 8 + c * 2 + 1 < left ? 0xffff0000u : 0u);
         }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          uint32_t vf[4];
-          b2::ldmatrix_x4_trans(vf, v_row + k * 16 * 128 + (((((warp & 1) * 2 + i) * 2 + v_chunk) ^ (v_tok & 7)) << 4));
-          b2::mma_rows8(o[2 * i][0], o[2 * i][1], p0, p1, vf[0] & keep[0], vf[1] & keep[1]);
-          b2::mma_rows8(o[2 * i + 1][0], o[2 * i + 1][1], p0, p1, vf[2] & keep[0], vf[3] & keep[1]);
-        }
+        values(row, t, k, keep[0], keep[1]);
       }
-      release();
+      release(advance());
     }
+    if (FEW && j > 0) scores(WD_BLOCK);
   }
   l += __shfl_xor_sync(0xffffffffu, l, 2);
   l += __shfl_xor_sync(0xffffffffu, l, 1);
@@ -1061,7 +1106,8 @@ int configure_once() {
   if (dev < 0 || dev >= 64) return b2::set_error(B2_ERR_UNSUPPORTED, "device ordinal %d not supported", dev);
   if (!done[dev].load(std::memory_order_acquire)) {
     B2_CUDA(cudaFuncSetAttribute(paged_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM_LIMIT));
-    B2_CUDA(cudaFuncSetAttribute(paged_decode_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem(WD_MAX_STAGES)));
+    B2_CUDA(cudaFuncSetAttribute(paged_decode_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem(4)));
+    B2_CUDA(cudaFuncSetAttribute(paged_decode_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem(WD_MAX_STAGES)));
     B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     B2_CUDA(cudaFuncSetAttribute(prefill_attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     done[dev].store(true, std::memory_order_release);
@@ -1117,8 +1163,10 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   if (crc != B2_OK) return crc;
   const int items = n_seqs * nkv;
   if (a.group > ATT_MAX_GROUP || (items >= 3 * ctx->num_sms && scale >= 0.f)) {  // (it takes the largest score for the maximum, whatever the scale)
-    a.stages = items <= 2 * ctx->num_sms ? WD_MAX_STAGES : items <= 3 * ctx->num_sms ? 4 : 3;
-    B2_CUDA(b2_launch(paged_decode_wide_kernel, dim3(items), dim3(ATT_THREADS), wide_smem(a.stages), static_cast<cudaStream_t>(stream), maps[0], maps[1], maps[2], maps[3], a));
+    const bool few = items <= 2 * ctx->num_sms;
+    a.stages = items <= ctx->num_sms ? WD_MAX_STAGES : few ? 6 : items <= 3 * ctx->num_sms ? 4 : 3;
+    const auto kernel = few ? paged_decode_wide_kernel<true> : paged_decode_wide_kernel<false>;
+    B2_CUDA(b2_launch(kernel, dim3(items), dim3(ATT_THREADS), wide_smem(a.stages), static_cast<cudaStream_t>(stream), maps[0], maps[1], maps[2], maps[3], a));
     return B2_OK;
   }
   const size_t smem = attention_smem(n_seqs, a.group);

@@ -27,9 +27,10 @@ CASES = [((1,), 16, 8), ((63, 64, 65, 0, 15, 16, 17), 16, 8), ((255, 256, 257, 0
          (tuple(range(40, 706, 18)) + (0,) * 11, 16, 8), ((0, 300, 0, 0, 900, 0), 16, 8), ((0, 0), 16, 8), ((700,) * 60 + (0,) * 4, 8, 8)]
 
 # wide groups, where there are enough (sequence, KV head) pairs: edges of the 16-row groups, the tiles of 64 and the blocks of 128 tokens, of a
-# cache block, rows without a context, three, four, seven and eight query heads per KV head, the fewest pairs that are served
+# cache block, rows without a context, three, four, seven and eight query heads per KV head, the fewest pairs that are served (one CTA per SM), two
 WIDE = [((0, 1, 15, 16, 17, 63, 64, 65, 79, 80, 81, 127, 128, 129, 191, 192, 193, 255, 256, 257, 0, 383, 384, 385, 511, 512, 513, 700, 1200, 0), 32, 8),
-        (tuple(range(1, 900, 29)), 64, 8), (tuple(range(40, 520, 6)), 9, 3), (tuple(range(3, 1000, 16)) + (0,) * 3, 28, 4), ((257,) * 128, 4, 1)]
+        (tuple(range(1, 900, 29)), 64, 8), (tuple(range(40, 520, 6)), 9, 3), (tuple(range(3, 1000, 16)) + (0,) * 3, 28, 4), ((257,) * 128, 4, 1),
+        (tuple(range(1, 700, 14)), 32, 8), (tuple(range(1, 480, 8)), 64, 8)]  # and three and four CTAs per SM
 
 
 @pytest.mark.parametrize("lens,nq,nkv", CASES + WIDE)
