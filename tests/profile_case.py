@@ -14,6 +14,8 @@ cases:
   qkv_prefill     qkv projection M=2048, N=4096, K=1024 with the head work in its epilogue (Qwen3-0.6B prefill), 24 weight copies
   silu_mid        gate/up + SiLU*mul, M=256, N=24576, K=4096, 2 weight copies
   attn_decode     decode attention, 64 contexts of 300..1371 tokens, 16 query / 8 KV heads, paged cache in shuffled blocks
+  attn_decode_few the same with the first 24 of them
+  attn_decode_wide the same with the first 24 of them and 32 query heads
   attn_prefill    causal prefill attention, 8 sequences of 2048 tokens, 16 query / 8 KV heads
   rowpar_decode   fused row-parallel launch, M=64, N=4096, Kr=12288 (Qwen3-8B down_proj at TP=1)
   rowpar_prefill  fused row-parallel launch, M=1024, N=5120, Kr=1024
@@ -78,14 +80,14 @@ def main():
         vc = torch.zeros_like(kc)
         slots = torch.randperm(16 * 256, device=dev)[:m].to(torch.int32)
         call = lambda j: ops.qkv_fused(x, ws[j % copies], None, nq, nkv, 128, qw, kw, 1e-6, pos, cos_sin, kc, vc, slots)
-    elif a.case == "attn_decode":
-        lens = [300 + 17 * i for i in range(64)]
+    elif a.case.startswith("attn_decode"):
+        lens = [300 + 17 * i for i in range(64 if a.case == "attn_decode" else 24)]
         need = [-(-n // 256) for n in lens]
         order = torch.randperm(sum(need), device=dev, generator=g).to(torch.int32)
-        tables = torch.zeros(64, max(need), dtype=torch.int32, device=dev)
+        tables = torch.zeros(len(lens), max(need), dtype=torch.int32, device=dev)
         for i, n in enumerate(need):
             tables[i, :n] = order[sum(need[:i]):sum(need[:i]) + n]
-        kc, vc, q = rnd(sum(need), 256, 8, 128), rnd(sum(need), 256, 8, 128), rnd(64, 16, 128)
+        kc, vc, q = rnd(sum(need), 256, 8, 128), rnd(sum(need), 256, 8, 128), rnd(len(lens), 32 if a.case == "attn_decode_wide" else 16, 128)
         context_lens = torch.tensor(lens, dtype=torch.int32, device=dev)
         call = lambda i: ops.paged_attention(q, kc, vc, context_lens, tables, 128 ** -0.5)
     elif a.case == "attn_prefill":
