@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
+#include <cmath>
 
 #include "b2_common.cuh"
 
@@ -52,7 +53,8 @@ struct AttnArgs {
   B2Status* status;
   int bt_width, block_size, num_blocks, n_seqs, nkv, group;
   int stages;  // wide groups: tiles of the ring
-  float scale_log2;  // softmax scale * log2(e)
+  uint32_t flip;     // wide groups: the sign bits of a pair of bf16 where the scale is negative
+  float scale_log2;  // softmax scale * log2(e); wide groups: its size
 };
 
 __device__ __forceinline__ void consumers_meet() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
@@ -562,7 +564,7 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 #pragma unroll
     for (int k = 0; k < 8; ++k)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) qf[k][i] = g < a.group ? *reinterpret_cast<const uint32_t*>(qrow + k * 16 + i * 8 + c * 2) : 0u;
+      for (int i = 0; i < 2; ++i) qf[k][i] = g < a.group ? *reinterpret_cast<const uint32_t*>(qrow + k * 16 + i * 8 + c * 2) ^ a.flip : 0u;
   }
   float o[4][2] = {};  // this warp's 32 dimensions
   float m = -INFINITY, l = 0.f;
@@ -750,7 +752,8 @@ struct PrefillArgs {
   int64_t bt_stride;
   int bt_width, block_size, kv_rows, nq, group;
   uint16_t* out;
-  float scale_log2;
+  uint32_t negate;   // the instruction descriptor's bit that negates Q, where the scale is negative
+  float scale_log2;  // size of softmax scale * log2(e)
   B2Status* status;
 };
 
@@ -890,7 +893,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     }
   } else if (warp <= 2) {
     const int h = warp - 1;
-    constexpr uint32_t idesc_s = b2::umma_idesc_bf16(PF_KEYS);
+    const uint32_t idesc_s = b2::umma_idesc_bf16(PF_KEYS) | a.negate;
     constexpr uint32_t idesc_o = b2::umma_idesc_bf16(128) | (1u << 16);  // second operand MN-major
     const uint64_t desc_q = b2::umma_smem_desc(s_q + h * PF_Q), desc_k = b2::umma_smem_desc(s_k), desc_v = umma_smem_desc_mn(s_v);  // (addresses in 16 bytes)
     auto wait = [&](uint32_t bar, uint32_t phase, int code) {
@@ -1089,8 +1092,9 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   if (warp == 1) b2::tmem_dealloc(tmem, 512);
 }
 
-// softmax scale * log2(e); masked scores are -inf, and -inf times zero is none
-float scale_for_exp2(float scale) { return scale == 0.f ? FLT_MIN : scale * 1.4426950408889634f; }
+// Softmax scale * log2(e) for kernels that mask and compare scores before they scale them: its size - masked scores are -inf, and -inf times
+// zero is none -, with the query negated in a negative one's place, which changes no product but for its sign.
+float scale_size(float scale) { return std::max(fabsf(scale * 1.4426950408889634f), FLT_MIN); }
 
 constexpr size_t ATT_SMEM_LIMIT = 113 * 1024;  // two CTAs per SM (228 KB, 1 KB of it reserved per CTA)
 constexpr size_t attention_smem(int n_seqs, int group) {
@@ -1147,7 +1151,7 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   a.n_seqs = n_seqs;
   a.nkv = nkv;
   a.group = nq / nkv;
-  a.scale_log2 = scale_for_exp2(scale);
+  a.scale_log2 = scale * 1.4426950408889634f;
   a.out = static_cast<uint16_t*>(out);
   a.ws = ctx->attn_ws;
   a.counters = ctx->attn_counters;
@@ -1162,8 +1166,10 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   const int crc = configure_once();
   if (crc != B2_OK) return crc;
   const int items = n_seqs * nkv;
-  if (a.group > ATT_MAX_GROUP || (items >= 3 * ctx->num_sms && scale >= 0.f)) {  // (it takes the largest score for the maximum, whatever the scale)
+  if (a.group > ATT_MAX_GROUP || items >= 3 * ctx->num_sms) {
     const bool few = items <= 2 * ctx->num_sms;
+    a.flip = scale < 0.f ? 0x80008000u : 0u;
+    a.scale_log2 = scale_size(scale);
     a.stages = items <= ctx->num_sms ? WD_MAX_STAGES : few ? 6 : items <= 3 * ctx->num_sms ? 4 : 3;
     const auto kernel = few ? paged_decode_wide_kernel<true> : paged_decode_wide_kernel<false>;
     B2_CUDA(b2_launch(kernel, dim3(items), dim3(ATT_THREADS), wide_smem(a.stages), static_cast<cudaStream_t>(stream), maps[0], maps[1], maps[2], maps[3], a));
@@ -1206,7 +1212,8 @@ int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const voi
   a.kv_rows = static_cast<int>(kv_rows);
   a.nq = nq;
   a.out = static_cast<uint16_t*>(out);
-  a.scale_log2 = scale_for_exp2(scale);
+  a.negate = scale < 0.f ? b2::kUmmaNegateA : 0u;
+  a.scale_log2 = scale_size(scale);
   a.status = ctx->status_dev;
   a.group = nq / nkv;
   const auto kernel = block_tables != nullptr && a.group > 2 ? prefill_attention_kernel<true> : prefill_attention_kernel<false>;

@@ -362,6 +362,9 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int n) {
          | (static_cast<uint32_t>(128 >> 4) << 24); // M / 16
 }
 
+// added to a descriptor: the first operand is negated
+constexpr uint32_t kUmmaNegateA = 1u << 13;
+
 // The same for a CTA pair: M = 256 (128 rows per CTA), N = n.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_pair(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);

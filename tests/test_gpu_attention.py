@@ -202,3 +202,62 @@ def test_prefill_of_a_sequence_without_keys_is_zero(rt):
     torch.cuda.synchronize()
     rt.check_status()
     assert (got[5:205] == 0).all() and (got[:5] != 0).any() and (got[205:] != 0).any()
+
+
+def paged_cache(total, nkv, g, bs=256):
+    """Keys and values of sequences of so many tokens, in shuffled cache blocks: caches, block tables, and each sequence's own rows."""
+    need = [max(1, -(-x // bs)) for x in total]
+    ids = torch.randperm(sum(need), generator=g).split(need)
+    tables = torch.zeros(len(total), max(16, max(need)), dtype=torch.int32)
+    caches = [torch.randn(sum(need), bs, nkv, 128, generator=g).bfloat16() for _ in range(2)]
+    for i, own in enumerate(ids):
+        tables[i, :need[i]] = own
+    return caches, tables, [[c[own].reshape(-1, nkv, 128)[:x] for c in caches] for own, x in zip(ids, total)]
+
+
+def exact_attention(q, k, v, scale):
+    """Causal attention of the last q.shape[0] positions in fp64: q [t, nq, hd], k, v [context, nkv, hd]."""
+    k, v = (x.double().repeat_interleave(q.shape[1] // k.shape[1], 1) for x in (k, v))
+    s = torch.einsum("qhd,khd->hqk", q.double(), k) * scale
+    t, n = q.shape[0], k.shape[0]
+    s.masked_fill_(torch.arange(n, device=q.device) > (torch.arange(t, device=q.device) + n - t).unsqueeze(1), float("-inf"))
+    return torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v)
+
+
+SCALES = [-128 ** -0.5, -0.5, 0.0, -0.0, 1e-39]
+
+
+@pytest.mark.parametrize("scale", SCALES)
+@pytest.mark.parametrize("nq,nkv,n", [(16, 8, 20), (16, 8, 60), (32, 8, 31), (32, 8, 40), (64, 8, 60)])
+def test_decode_takes_any_scale(rt, nq, nkv, n, scale):
+    """Negative scales, zero and one that no normal number holds, on either kernel and each of the wide one's forms: contexts that end
+    inside a block, where scores are masked."""
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    lens = [(1 + 37 * i) % 300 for i in range(n)]
+    caches, tables, rows = paged_cache(lens, nkv, g)
+    q = torch.randn(n, nq, 128, generator=g).bfloat16()
+    ref = torch.stack([exact_attention(q[i:i + 1], *rows[i], scale)[0].float() if lens[i] else torch.zeros(nq, 128) for i in range(n)])
+    got = ops.paged_attention(q.to(DEV), *(c.to(DEV) for c in caches), torch.tensor(lens, dtype=torch.int32, device=DEV), tables.to(DEV), scale)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(got, ref, f"decode {nq}/{nkv} heads, scale {scale}")
+
+
+@pytest.mark.parametrize("scale", SCALES)
+@pytest.mark.parametrize("nq,nkv", [(4, 2), (8, 2)])
+@pytest.mark.parametrize("paged", [False, True])
+def test_prefill_takes_any_scale(rt, paged, nq, nkv, scale):
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(nq)
+    new, old = [150, 64, 1, 200], [100, 0, 300, 56] if paged else [0] * 4
+    total = [a + b for a, b in zip(new, old)]
+    caches, tables, rows = paged_cache(total, nkv, g)
+    q = torch.randn(sum(new), nq, 128, generator=g).bfloat16()
+    ref = torch.cat([exact_attention(x, *kv, scale).float() for x, kv in zip(q.split(new), rows)])
+    cu, cu_k = (torch.tensor([0] + x).cumsum(0).to(torch.int32).to(DEV) for x in (new, total))
+    k, v = caches if paged else (torch.cat([kv[j] for kv in rows]) for j in (0, 1))
+    got = ops.prefill_attention(q.to(DEV), k.to(DEV), v.to(DEV), cu, cu_k, max(new), tables.to(DEV) if paged else None, scale)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(got, ref, f"prefill {nq}/{nkv} heads, scale {scale}")
