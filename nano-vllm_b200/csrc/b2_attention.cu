@@ -455,9 +455,10 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 // their order.  On random data the results are flash-attn's but for 0 to 3 elements in a million.
 //
 // 64 contexts of 1056 tokens, 32 / 8 heads: 66.7 us in flash-attn, 45.2 here (6.1 TB/s); 96 of 70..700 47.0 and 28.8, 32 of 1056
-// 34.9 and 23.7.  Narrow groups take this kernel too from three pairs of (sequence, KV head) per SM on, where nothing has to be cut to fill
-// the chip and the other kernel's parts cost more than the even share saves: 256 contexts of 100..1024 tokens, 16 / 8 heads, 97.6 -> 90.8 us,
-// 128 of them 53.5 -> 48.4, 512 of 30..270 67.7 -> 55.8, 64 of 1056 49.1 -> 45.0; 37 of 40..700 (296 pairs) would go from 13.6 to 14.1.
+// 34.9 and 23.7.  Not for narrow groups, although batches of about equal contexts would gain where there are three CTAs an SM and more (64 of 1056
+// tokens, 16 / 8 heads, 48.7 and 43.7 us, 512 of 30..270 68 and 54): the other kernel's warps round against maxima of their own, which is
+// nearer to float64 (2.12e-3 and 2.23e-3; 2.05e-3 and 2.18e-3 for contexts of 100..1024), and its even ranges take a long context apart, which is walked
+// alone here (63 contexts of 100 tokens and one of 4000 15.6 and 57.7 us, one of 32000 34 and 418).
 //
 // Four CTAs per SM with a ring of three 16 KB tiles (64 tokens of K or of V) each, or fewer with longer rings where there are no
 // more to be had: 190 KB per SM in flight.  With no more than two CTAs for an SM (FEW) a block's product runs side by side with the next
@@ -1166,7 +1167,7 @@ int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, cons
   const int crc = configure_once();
   if (crc != B2_OK) return crc;
   const int items = n_seqs * nkv;
-  if (a.group > ATT_MAX_GROUP || items >= 3 * ctx->num_sms) {
+  if (a.group > ATT_MAX_GROUP) {
     const bool few = items <= 2 * ctx->num_sms;
     a.flip = scale < 0.f ? 0x80008000u : 0u;
     a.scale_log2 = scale_size(scale);
