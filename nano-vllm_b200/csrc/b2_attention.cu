@@ -471,9 +471,9 @@ constexpr int WD_CTAS_PER_SM = 4;
 constexpr int WD_BLOCK = 2 * ATT_TILE;                    // tokens that share a maximum
 constexpr int WD_STAGE_BYTES = 2 * ATT_HALF_BYTES;        // dimensions 0..63, 64..127
 constexpr int WD_P_PITCH = WD_BLOCK + 8;                  // floats: rows start 8 banks apart, so that the 8-byte accesses of half a warp meet in none
-// Wide groups, from this many (sequence, KV head) pairs on: 16 contexts of 1056 tokens and 8 KV heads 38.8 us in the library, 13.4 here
-// (of 100..3000 tokens 59 and 26).  Fewer would be faster here too (8 contexts 36 and 11), but long contexts are then cut into parts in the
-// library, each rounded for itself, and a context of one CTA walks at 65 GB/s however long it is (8 of 4000 tokens: 37 and 33).
+// The fewest (sequence, KV head) pairs that are served (16 contexts of 1056 tokens and 8 KV heads 38.8 us in the library, 13.4 here, of 100..3000 tokens
+// 59 and 26).  Up to 1.6 pairs an SM the library cuts long contexts into parts, each rounded for itself, and is a little nearer to float64; a
+// context of one CTA walks at 70 GB/s with one CTA for an SM, at 50 with two, at 40 beyond, however long it is.  Attention.attend leaves those batches to the library.
 constexpr int WD_MIN_ITEMS = 128;
 constexpr uint32_t wide_smem(int stages) { return 1024 + stages * WD_STAGE_BYTES; }
 static_assert(wide_smem(WD_MAX_STAGES) + 6 * 1024 <= 228 * 1024 && 2 * (wide_smem(6) + 6 * 1024) <= 228 * 1024 && 3 * (wide_smem(4) + 6 * 1024) <= 228 * 1024 && 4 * (wide_smem(3) + 6 * 1024) <= 228 * 1024, "CTAs per SM (6 KB: static, reserved)");

@@ -6,9 +6,12 @@ b2_store_kvcache: 16-byte vector copies, several tokens per CTA, bit-exact).
 `Attention` keeps the reference's interface (:43-75).  Decode attention runs on
 b2_paged_attention_decode and prefill attention on b2_prefill_attention; the
 shapes they do not serve stay a library call, as in the reference: flash-attn's
-paged and varlen kernels.
+paged and varlen kernels.  So do decode batches of wide groups in which that
+library cuts contexts (decode_is_cut).
 """
 from __future__ import annotations
+
+import functools
 
 import torch
 from torch import nn
@@ -57,6 +60,22 @@ def _sdpa_paged(q, k_cache, v_cache, context_lens, block_tables, scale, q_lens=N
     return torch.cat(outs)
 
 
+@functools.lru_cache(maxsize=None)
+def _sms(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+def decode_is_cut(n_seqs: int, nq: int, nkv: int, block_size: int, sms: int) -> bool:
+    """True for decode batches of three and more query heads per KV head that are the library's: below 0.8 of two (sequence, KV head) pairs
+    per SM it cuts contexts into parts, each rounded for itself and walked beside the others, where the own kernel walks a context in one
+    CTA.  Its results are nearer to float64 there (32 / 8 heads, error x 1e3: 20 contexts of 4000 tokens 2.220 and 2.271, of 100..3000 2.197
+    and 2.205, 28 of 4000 2.213 and 2.260), and one long context does not hold up the batch (19 of 100 tokens and one of 4000 35 and 46 us, of 16000
+    100 and 171), although batches of about equal contexts take longer (20 of 300 tokens 21.3 and 7.7 us, of 4000 83 and 60).  From that line on
+    the results are the same and the own kernel was the faster one in all that was tried (30 contexts of 300 tokens 20 and 9 us, 29 of 100
+    and one of 32000 552 and 359).  The library wants cache blocks of a multiple of 256 tokens."""
+    return nq > 2 * nkv and 5 * n_seqs * nkv < 8 * sms and block_size % 256 == 0
+
+
 class Attention(nn.Module):
     # "flash_attn" (own kernels, the reference's library call for what they do not serve) or "sdpa" (plain PyTorch, for tests on small
     # shapes when flash-attn cannot run)
@@ -92,7 +111,10 @@ class Attention(nn.Module):
             o = ops.prefill_attention(q, k_cache if cached else k, v_cache if cached else v, ctx.cu_seqlens_q, ctx.cu_seqlens_k, ctx.max_seqlen_q,
                                       ctx.block_tables, self.scale)
         else:
-            o = ops.paged_attention(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
+            o = None
+            n, nq, _ = q.shape
+            if flash_attn_with_kvcache is None or nq <= 2 * k_cache.shape[2] or not decode_is_cut(n, nq, k_cache.shape[2], k_cache.shape[1], _sms(q.get_device())):
+                o = ops.paged_attention(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
         if o is not None:
             return o
         if flash_attn_varlen_func is None:
