@@ -6,8 +6,8 @@ b2_store_kvcache: 16-byte vector copies, several tokens per CTA, bit-exact).
 `Attention` keeps the reference's interface (:43-75).  Decode attention runs on
 b2_paged_attention_decode and prefill attention on b2_prefill_attention; the
 shapes they do not serve stay a library call, as in the reference: flash-attn's
-paged and varlen kernels.  So do decode batches of wide groups in which that
-library cuts contexts (decode_is_cut).
+paged and varlen kernels.  So do batches of wide groups for which that library
+is the better one (decode_is_cut, prefill_is_short).
 """
 from __future__ import annotations
 
@@ -76,6 +76,16 @@ def decode_is_cut(n_seqs: int, nq: int, nkv: int, block_size: int, sms: int) -> 
     return nq > 2 * nkv and 5 * n_seqs * nkv < 8 * sms and block_size % 256 == 0
 
 
+def prefill_is_short(tokens: int, n_seqs: int, max_q: int, nq: int, nkv: int, block_size: int, sms: int) -> bool:
+    """True for prefill batches over the cache of three and more query heads per KV head that are the library's.  One new token per sequence: it
+    cuts the keys there (32 / 8 heads, 1 x 1 token over 768 cached 11 and 22 us, over 8000 23 and 166, 16 x 1 over 768 29 and 45).  Or few rows: the
+    time is one CTA's walk over the keys, which is the library's shorter one by a fifth (16 tokens over 8000 139 and 171 us, 200 over 8000 143 and
+    178, 4 x 64 over 512 0.88 of the own time) as long as its tiles of 64 rows of each head all run at once; past that the own kernel
+    was 1.05 to 2.4 times as fast (300 tokens over 512 1.17, 4 x 100 over 512 1.15)."""
+    tiles = min(n_seqs * -(-max_q // 64), tokens // 64 + n_seqs)  # at most so many
+    return nq > 2 * nkv and block_size % 256 == 0 and (max_q <= 1 or nq * tiles <= sms)
+
+
 class Attention(nn.Module):
     # "flash_attn" (own kernels, the reference's library call for what they do not serve) or "sdpa" (plain PyTorch, for tests on small
     # shapes when flash-attn cannot run)
@@ -106,15 +116,16 @@ class Attention(nn.Module):
                     return torch.cat(outs)
                 return _sdpa_paged(q, k_cache, v_cache, k_lens, ctx.block_tables, self.scale, q_lens)
             return _sdpa_paged(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
+        n, nq, nkv = q.shape[0], self.num_heads, self.num_kv_heads
+        wide, o = nq > 2 * nkv, None
         if ctx.is_prefill:
             cached = ctx.block_tables is not None  # prefix cache / chunked prefill: read K/V from the cache
-            o = ops.prefill_attention(q, k_cache if cached else k, v_cache if cached else v, ctx.cu_seqlens_q, ctx.cu_seqlens_k, ctx.max_seqlen_q,
-                                      ctx.block_tables, self.scale)
-        else:
-            o = None
-            n, nq, _ = q.shape
-            if flash_attn_with_kvcache is None or nq <= 2 * k_cache.shape[2] or not decode_is_cut(n, nq, k_cache.shape[2], k_cache.shape[1], _sms(q.get_device())):
-                o = ops.paged_attention(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
+            if not (cached and wide and flash_attn_varlen_func is not None and
+                    prefill_is_short(n, ctx.cu_seqlens_q.numel() - 1, ctx.max_seqlen_q, nq, nkv, k_cache.shape[1], _sms(q.get_device()))):
+                o = ops.prefill_attention(q, k_cache if cached else k, v_cache if cached else v, ctx.cu_seqlens_q, ctx.cu_seqlens_k, ctx.max_seqlen_q,
+                                          ctx.block_tables, self.scale)
+        elif not (wide and flash_attn_with_kvcache is not None and decode_is_cut(n, nq, nkv, k_cache.shape[1], _sms(q.get_device()))):
+            o = ops.paged_attention(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
         if o is not None:
             return o
         if flash_attn_varlen_func is None:

@@ -45,3 +45,17 @@ def test_decode(route, n, nq, nkv, block, who):
     assert route(nq, nkv, context, meta_cache(nkv, block), n) == who
     assert route(nq, nkv, context, meta_cache(nkv, block), n, library=False) == "own"
     assert route(nq, nkv, context, meta_cache(nkv, block), n, own=False) == "library"
+
+
+# wide groups over the cache: one row per sequence; up to 148 tiles of 64 rows and a head; not without a cache, not for narrow groups
+@pytest.mark.parametrize("rows,nq,nkv,cached,block,who", [
+    ([1], 32, 8, True, 256, "library"), ([1] * 40, 32, 8, True, 256, "library"), ([16], 32, 8, True, 256, "library"), ([256], 32, 8, True, 256, "library"),
+    ([257], 32, 8, True, 256, "own"), ([100] * 2, 32, 8, True, 256, "library"), ([100] * 4, 32, 8, True, 256, "own"), ([1024], 32, 8, True, 256, "own"),
+    ([250, 1], 24, 8, True, 256, "library"), ([250, 1, 1], 32, 8, True, 256, "own"), ([1], 32, 8, False, 256, "own"), ([16], 32, 8, False, 256, "own"),
+    ([1], 16, 8, True, 256, "own"), ([16], 16, 8, True, 256, "own"), ([16], 32, 8, True, 128, "own")])
+def test_prefill(route, rows, nq, nkv, cached, block, who):
+    cu = torch.tensor([0] + rows).cumsum(0).to(torch.int32)
+    context = SimpleNamespace(is_prefill=True, cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=max(rows), max_seqlen_k=max(rows),
+                              block_tables=torch.zeros(len(rows), 4, dtype=torch.int32) if cached else None)
+    assert route(nq, nkv, context, meta_cache(nkv, block), sum(rows)) == who
+    assert route(nq, nkv, context, meta_cache(nkv, block), sum(rows), library=False) == "own"
