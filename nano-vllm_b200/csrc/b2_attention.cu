@@ -731,7 +731,8 @@ paged_decode_wide_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 //   warps 12..15  O is rescaled where a row's maximum has grown, while the softmax warps are at their exponentials
 // Tensor memory: two S of 64 columns per head, then O of the two heads, 128 columns each.  With two S the scores of the next
 // block are there before this one's are done with: a head's warp issues P V (block j), then Q K^T (block j + 2) into the columns
-// that P is read from, and needs no wait between the two, as they execute in the order of issue.  (With one S of 128 keys per head
+// that P is read from.  The order of issue is promised only to products of one shape and accumulator, which these are not: the warp waits for P V
+// in between, while the other head's products run (without the wait the times were the same: 246 us at 8192 tokens, 16 heads).  (With one S of 128 keys per head
 // and one warp for both, the heads ran in step: 7700 clocks per 128 keys.  One warp for both, here: 275 us instead of 246; values that are
 // the same in all lanes but not in a form that shows it, b2::uniform: 346.)
 //
@@ -932,7 +933,8 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         if (j == n - 1) b2::umma_commit(o_final + h * 8);
       }
       __syncwarp();
-      if (j + 2 < n) ok = scores(j + 2);  // into the columns that P of this block is read from, after it
+      // into the columns that P of this block is read from, once it has been
+      if (j + 2 < n) ok = wait(o_done + h * 8, j & 1, B2_WAIT_TMEM_FULL) && scores(j + 2);
     }
   } else if (warp >= 4 && warp < 12) {
     const int h = (warp >> 2) - 1, q = warp & 3, row = q * 32 + lane;
