@@ -499,7 +499,7 @@ int b2_plan_tile_contributors(const b2_gemm_plan* plan, int tile, int* first_cta
 /* The same for the kernel of CTA pairs over tiles of 256 features x up to 256 tokens, which serves the store GEMMs
  * (b2_gemm, b2_gemm_silu_mul, b2_qkv_fused, b2_rowpar_fused on one rank) of more than 64 tokens that no cluster plan takes. */
 typedef struct b2_tile_plan {
-  int bn;               /* token columns of a tile                                                       */
+  int bn;               /* token columns of a tile by which the plan is chosen, in steps of 32           */
   int tiles_f, tiles_t; /* feature tiles, token tiles                                                    */
   int kblocks;          /* 64-wide K blocks per tile                                                     */
   int split;            /* pairs of a cluster that share a tile's K range (1: none)                      */
@@ -509,6 +509,7 @@ typedef struct b2_tile_plan {
   int rounds, ranged;   /* multi: whole tiles per pair, tiles after those that are dealt out by K blocks */
   int grid;             /* CTAs launched, two per pair                                                   */
   int out_off, bar_off, smem; /* shared memory: output staging, barriers, bytes in all                   */
+  int width;            /* token columns of a tile as launched: bn, or less in steps of 16 where no tile is split */
 } b2_tile_plan;
 /* resident_clusters: NULL (no tile is split over a cluster) or int[10]: entry [S] with half of an SM's shared memory per
  * CTA, [5 + S] with all of it = clusters of 2 S CTAs the device holds at once. */

@@ -52,7 +52,7 @@ class GemmPlan(C.Structure):
 class TilePlan(C.Structure):
     """b2_tile_plan: the same for the CTA-pair kernel of more than 64 tokens."""
     _fields_ = [(n, C.c_int) for n in ("bn", "tiles_f", "tiles_t", "kblocks", "split", "group", "stages", "multi", "rounds", "ranged", "grid",
-                                       "out_off", "bar_off", "smem")]
+                                       "out_off", "bar_off", "smem", "width")]
 
 
 _p, _i, _i64, _f = C.c_void_p, C.c_int, C.c_int64, C.c_float

@@ -732,11 +732,16 @@ int plan_tile_gemm(int M, int N, int K, int num_sms, int tile_cap, Resident&& re
         best = cost;
         const int64_t grid = multi ? (ranged > 0 ? pairs : std::min<int64_t>(tiles, pairs)) * 2 : work * 2;
         *p = TilePlan{bn, tiles_f, tiles_t, kblocks, s, std::min(tiles_t, 16), stages, multi ? 1 : 0, static_cast<int>(rounds), static_cast<int>(ranged),
-                      static_cast<int>(grid), static_cast<int>(out_off), static_cast<int>(ring), static_cast<int>(ring + SMEM_EXTRA)};
+                      static_cast<int>(grid), static_cast<int>(out_off), static_cast<int>(ring), static_cast<int>(ring + SMEM_EXTRA), bn};
       }
     }
   }
-  return best < 1e30 ? B2_OK : B2_ERR_SHAPE;
+  if (best >= 1e30) return B2_ERR_SHAPE;
+  // Whole tiles are as narrow as the tokens let them be in steps of 16 columns, the least step of a pair's tcgen05.mma: 777 tokens are 4 x 208
+  // and not 4 x 224.  An output's sum over K is the same; where K is cut, widths decide where, and stay.  (The choice is made by bn: by
+  // the true widths it would fall on other tiles, and below 512 tokens on other cuts.)
+  if (p->split == 1 && p->ranged == 0) p->width = ((M + p->tiles_t - 1) / p->tiles_t + 15) / 16 * 16;
+  return B2_OK;
 }
 
 // clusters of 2 * split CTAs resident at once, asked once per device for the two sizes of shared memory
@@ -789,9 +794,7 @@ int launch_tile_gemm(b2_ctx* ctx, const void* A, int64_t lda, const void* W, int
   a.M = M;
   a.N = N;
   a.kblocks = p.kblocks;
-  // Whole tiles are as narrow as the tokens let them be in steps of 16 columns, the least step of a pair's tcgen05.mma: 777 tokens are 4 x 208
-  // and not the plan's 4 x 224.  An output's sum over K is the same; where K is cut, widths decide where, and stay.
-  a.bn = p.split == 1 && p.ranged == 0 ? ((M + p.tiles_t - 1) / p.tiles_t + 15) / 16 * 16 : p.bn;
+  a.bn = p.width;
   a.stages = p.stages;
   a.split = p.split;
   a.rounds = p.rounds;

@@ -108,3 +108,33 @@ def test_plan_property(m, n8, k8, sms):
     rc, p = plan_of(_abi, m, n8 * 8, k8 * 8, sms=sms, resident=resident)
     assert rc == 0
     check(_abi, p, m, n8 * 8, k8 * 8, sms=sms, resident=resident)
+
+
+def check_width(p, m):
+    """The columns that are launched: the fewest in steps of 16 that as many whole tiles cover the tokens with, the plan's own where K is cut."""
+    assert 16 <= p.width <= p.bn and p.tiles_t * p.width >= m > (p.tiles_t - 1) * p.width  # (no tile without tokens)
+    if p.split == 1 and p.ranged == 0:
+        assert p.width % 16 == 0 and p.tiles_t * (p.width - 16) < m
+    else:
+        assert p.width == p.bn
+    # the last 32 columns are read whole: inside what is allocated, in powers of two, for one accumulator
+    assert -(-p.width // 32) * 32 <= max(32, 1 << (p.width - 1).bit_length())
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES + [(m, 4096, 4096) for m in (513, 530, 565, 593, 777, 1041)])
+def test_launched_width(pkg, m, n, k):
+    from nanovllm_b200 import _abi
+    rc, p = plan_of(_abi, m, n, k)
+    assert rc == 0
+    check_width(p, m)
+
+
+@settings(max_examples=150, deadline=None)
+@given(m=st.integers(65, 16384), n8=st.integers(1, 7000), k8=st.integers(1, 3200))
+def test_launched_width_property(m, n8, k8):
+    import __graft_entry__
+    __graft_entry__.load_package()
+    from nanovllm_b200 import _abi
+    rc, p = plan_of(_abi, m, n8 * 8, k8 * 8)
+    assert rc == 0
+    check_width(p, m)
