@@ -291,3 +291,152 @@ def test_decode_of_narrow_groups_rounds_against_each_warps_own_maximum(rt, n, st
         bound += (plain.double() - exact).pow(2).sum().item()
     rt.check_status()
     assert ours ** 0.5 <= 1.02 * bound ** 0.5, f"{ours ** 0.5 / bound ** 0.5:.4f} times the error"
+
+
+LIBRARY_DECODE = [((257,) * 30, 32, 8), (tuple(range(1, 1200, 18)), 32, 8), (tuple(range(70, 700, 6)), 64, 8), ((1056,) * 80, 9, 3)]
+
+
+@pytest.mark.parametrize("lens,nq,nkv", LIBRARY_DECODE)
+def test_wide_decode_is_the_librarys_result(rt, lens, nq, nkv):
+    """Where the library does not cut contexts (0.8 of two pairs per SM and more) every probability has the same fp32 value and is rounded
+    against the same maximum, and a product's sums are the same chain.  Bound: only the sum of probabilities is added up in another order; if its
+    last bit differs, by 2^-23, one in 2^15 results falls on the other side of a tie between two bf16 numbers, 2^-8 apart."""
+    flash = pytest.importorskip("flash_attn")
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(len(lens))
+    caches, tables, _ = paged_cache(lens, nkv, g)
+    q = torch.randn(len(lens), nq, 128, generator=g).bfloat16().to(DEV)
+    kc, vc, tables = (x.to(DEV) for x in (*caches, tables))
+    lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    got = ops.paged_attention(q, kc, vc, lens, tables, 128 ** -0.5)
+    ref = flash.flash_attn_with_kvcache(q.unsqueeze(1), kc, vc, cache_seqlens=lens, block_table=tables, softmax_scale=128 ** -0.5, causal=True).squeeze(1)
+    rt.check_status()
+    assert (got != ref).sum().item() <= max(4, got.numel() * 2 ** -15)
+    assert_close_bf16(got, ref.float(), "wide decode and the library")
+
+
+@pytest.mark.parametrize("nq,nkv,new,old", [(16, 8, (117, 64, 300), None), (32, 8, (500, 129, 1), None), (64, 8, (700,), None), (4, 2, (1500,), None),
+                                            (32, 8, (100, 300, 65), (512, 77, 0)), (64, 8, (900,), (700,)), (8, 1, (257, 128), (256, 3000))])
+def test_prefill_is_the_librarys_result(rt, nq, nkv, new, old):
+    """Bit for bit: over rows for any group, over a block table for groups of four and more (two heads per KV head take one maximum per 64 keys there,
+    the library one per 128)."""
+    flash = pytest.importorskip("flash_attn")
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(sum(new))
+    total = [a + b for a, b in zip(new, old or [0] * len(new))]
+    caches, tables, rows = paged_cache(total, nkv, g)
+    q = torch.randn(sum(new), nq, 128, generator=g).bfloat16().to(DEV)
+    k, v = (x.to(DEV) for x in (caches if old else (torch.cat([kv[j] for kv in rows]) for j in (0, 1))))
+    cu, cu_k = (torch.tensor([0, *x]).cumsum(0).to(torch.int32).to(DEV) for x in (new, total))
+    tables = tables.to(DEV) if old else None
+    got = ops.prefill_attention(q, k, v, cu, cu_k, max(new), tables, 128 ** -0.5)
+    ref = flash.flash_attn_varlen_func(q, k, v, max_seqlen_q=max(new), cu_seqlens_q=cu, max_seqlen_k=max(total), cu_seqlens_k=cu_k, softmax_scale=128 ** -0.5,
+                                       causal=True, block_table=tables)
+    rt.check_status()
+    assert torch.equal(got, ref)
+
+
+def trend(q, rows, slope):
+    """Dimension 0 carries scores that rise or fall along the keys, half as steep for every other query head (the scale is 128 ** -0.5)."""
+    q[..., 0] = torch.tensor([16.0, 8.0]).repeat(-(-q.shape[1] // 2))[:q.shape[1]].bfloat16()
+    for k, _ in rows:
+        k[..., 0] = (torch.arange(len(k)) * slope * 128 ** 0.5 / 16.0).unsqueeze(1).bfloat16()
+
+
+def put_back(caches, tables, rows, bs=256):
+    """The sequences' own rows into the cache again."""
+    for i, kv in enumerate(rows):
+        for cache, x in zip(caches, kv):
+            for p in range(0, len(x), bs):
+                cache[tables[i, p // bs], :len(x[p:p + bs])] = x[p:p + bs]
+
+
+# every form: narrow groups with whole items and with even ranges, on both sides of 444 pairs; wide ones with two CTAs per SM and more
+RAGGED = [0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 191, 193, 255, 256, 257, 0, 511, 513, 640]
+
+
+@pytest.mark.parametrize("slope", [0.05, -0.05])
+@pytest.mark.parametrize("nq,nkv,n,far", [(16, 8, 20, 0), (16, 8, 55, 3000), (16, 8, 56, 3000), (16, 8, 64, 0), (8, 8, 60, 1500), (32, 8, 31, 0), (32, 8, 31, 2000), (64, 8, 60, 0)])
+def test_decode_rescales_as_maxima_grow(rt, nq, nkv, n, far, slope):
+    """Scores that rise or fall along the context by 2^9 in 128 tokens: whichever end a walk starts from, one of the two has every block's
+    maximum outgrow all earlier ones.  Ragged lengths, rows without a context, one far longer than the rest."""
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    lens = [RAGGED[i % len(RAGGED)] for i in range(n)]
+    if far:
+        lens[n // 2] = far
+    caches, tables, rows = paged_cache(lens, nkv, g)
+    q = torch.randn(n, nq, 128, generator=g).bfloat16()
+    trend(q, rows, slope)
+    put_back(caches, tables, rows)
+    ref = torch.stack([exact_attention(q[i:i + 1], *rows[i], 128 ** -0.5)[0].float() if lens[i] else torch.zeros(nq, 128) for i in range(n)])
+    got = ops.paged_attention(q.to(DEV), *(c.to(DEV) for c in caches), torch.tensor(lens, dtype=torch.int32, device=DEV), tables.to(DEV), 128 ** -0.5)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(got, ref, f"decode {nq}/{nkv} heads, slope {slope}")
+
+
+@pytest.mark.parametrize("slope", [0.05, -0.05])
+@pytest.mark.parametrize("nq,nkv", [(4, 2), (8, 2), (8, 1)])
+def test_prefill_over_the_cache_rescales_as_maxima_grow(rt, nq, nkv, slope):
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(nq + nkv)
+    new, old = [300, 65, 128, 1], [200, 0, 64, 700]
+    total = [a + b for a, b in zip(new, old)]
+    caches, tables, rows = paged_cache(total, nkv, g)
+    q = torch.randn(sum(new), nq, 128, generator=g).bfloat16()
+    trend(q, rows, slope)
+    put_back(caches, tables, rows)
+    ref = torch.cat([exact_attention(x, *kv, 128 ** -0.5).float() for x, kv in zip(q.split(new), rows)])
+    cu, cu_k = (torch.tensor([0] + x).cumsum(0).to(torch.int32).to(DEV) for x in (new, total))
+    got = ops.prefill_attention(q.to(DEV), *(c.to(DEV) for c in caches), cu, cu_k, max(new), tables.to(DEV), 128 ** -0.5)
+    torch.cuda.synchronize()
+    rt.check_status()
+    assert_close_bf16(got, ref, f"prefill over the cache {nq}/{nkv} heads, slope {slope}")
+
+
+@pytest.mark.parametrize("nq,nkv,n", [(16, 8, 20), (16, 8, 60), (32, 8, 31), (32, 8, 60)])
+def test_decode_keeps_nan_in_its_sequence(rt, nq, nkv, n):
+    """A key that is NaN, or a value that is infinite, shows in its sequence's results, and in no other's."""
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    lens = [200 + 13 * i for i in range(n)]
+    caches, tables, rows = paged_cache(lens, nkv, g)
+    q = torch.randn(n, nq, 128, generator=g).bfloat16().to(DEV)
+
+    def run():
+        return ops.paged_attention(q, *(c.to(DEV) for c in caches), torch.tensor(lens, dtype=torch.int32, device=DEV), tables.to(DEV), 128 ** -0.5).cpu()
+
+    clean = run()
+    rows[3][0][70], rows[7][1][5, :, 9] = float("nan"), float("inf")
+    put_back(caches, tables, rows)
+    got = run()
+    rt.check_status()
+    others = [i for i in range(n) if i not in (3, 7)]
+    assert torch.equal(got[others], clean[others])
+    assert got[3].isnan().all() and (got[7, :, 9] == float("inf")).all()
+    rest = [d for d in range(128) if d != 9]
+    assert torch.equal(got[7][:, rest], clean[7][:, rest])
+
+
+@pytest.mark.parametrize("nq,nkv,paged", [(4, 2, False), (4, 2, True), (8, 2, False), (8, 2, True)])
+def test_prefill_keeps_nan_from_earlier_rows(rt, nq, nkv, paged):
+    """A key that is NaN shows in every row that sees it and in none before it, also where they share a block of keys."""
+    from nanovllm_b200 import ops
+    g = torch.Generator().manual_seed(3)
+    lens = [300, 140]
+    caches, tables, rows = paged_cache(lens, nkv, g)
+    q = torch.randn(sum(lens), nq, 128, generator=g).bfloat16().to(DEV)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+
+    def run():
+        k, v = caches if paged else (torch.cat([kv[j] for kv in rows]) for j in (0, 1))
+        return ops.prefill_attention(q, k.to(DEV), v.to(DEV), cu, cu, 300, tables.to(DEV) if paged else None, 128 ** -0.5).cpu()
+
+    clean = run()
+    rows[0][0][170] = float("nan")
+    put_back(caches, tables, rows)
+    got = run()
+    rt.check_status()
+    assert torch.equal(got[:170], clean[:170]) and torch.equal(got[300:], clean[300:])
+    assert got[170:300].isnan().all()
