@@ -388,9 +388,12 @@ PyObject* prefill_attention(Args a) {
       rows > (1 << 30) || cu_q.numel() > 65536 || v.strides() != k.strides() || !on_16_bytes(v))
     Py_RETURN_NONE;
   if (paged ? !k.is_contiguous() || !on_16_bytes(k) || !table_layout(tables) : !row_layout(k, nkv, hd)) Py_RETURN_NONE;
-  // Wide groups, many sequences of a few tokens: a CTA's tile of 128 rows is mostly empty and takes 5 us however few there are.  With 32 / 8 heads
-  // 32 sequences of 64 tokens 23 us in the library's kernel 20, of one token over 768 cached 88 and 39; 16 of 60 over 768 46 and 55.
-  if (nq > 2 * nkv && n < 96 * (cu_q.numel() - 1) && (cu_q.numel() - 1) * (nq / 2) > 296) Py_RETURN_NONE;
+  // Wide groups, many sequences of a few tokens: a CTA's tile of 128 rows is mostly empty and takes 5 us however few there are, so that more than two
+  // of them an SM cost more than the library's tiles of 64 rows.  Time there over time here, 300 to 2000 tiles of prompts without a cached part: of
+  // 1 token 0.2-0.9, of 16 to 64 0.88-1.02, of 80 1.2-1.4, of 96 1.19-1.35, of lengths around 96 1.2-1.4: the line is where it pays in all of them.  Up
+  // to two an SM (290 tiles) 16 to 64 tokens 1.0-1.08.  Over 768 cached tokens 1 token 0.2-0.6, 16 to 64 1.02-1.19: the line is the same for all.
+  constexpr int64_t kRows = 96, kTwoAnSm = 2 * 148;
+  if (nq > 2 * nkv && n < kRows * (cu_q.numel() - 1) && (cu_q.numel() - 1) * (nq / 2) > kTwoAnSm) Py_RETURN_NONE;
   if (c10::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) Py_RETURN_NONE;  // (forward only)
   const int64_t n_seqs = cu_q.numel() - 1, max_q = integer(a[6]);
   values_like_keys(k, v, hd);
