@@ -403,7 +403,7 @@ int b2_rope(const void* q, int64_t ldq, const void* k, int64_t ldk, int M, int n
  * fp32 scores and sums, probabilities rounded to bf16 for the second product.  Lengths and tables
  * are read on the device, so a captured call serves any later batch of the same size; they are read while earlier
  * b2_* kernels of the stream may still be running, so they must not be results of one, b2_advance_decode excepted.
- * Calls of one context must be stream-ordered: they share its workspace for partial results.
+ * Calls of one context must be stream-ordered: they share its workspace for partial results.  scale: of either sign, or zero.
  * b2_paged_attention_supported says (1 / 0) whether the shape is served: head_dim 128, blocks of a
  * multiple of 64 tokens, at most 1024 sequences, one or two query heads per KV head, or up to eight where n_seqs * nkv >= 128. */
 int b2_paged_attention_decode(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
@@ -443,7 +443,7 @@ int b2_decode_stack(b2_ctx* ctx, const b2_stack_layer* layers, int n_layers, con
  * own position.  block_tables NULL: k and v are matrices of kv_rows rows (row stride kv_stride; views of the qkv output),
  * sequence b's keys in rows cu_k[b] .. ; else k and v are the caches, kv_rows = blocks * block_size slots, and
  * block_tables (bt_width columns, row stride bt_stride) says where.  max_q: the most query rows of a sequence.
- * out [tokens, nq, head_dim] contiguous.  fp32 scores and sums, probabilities rounded to bf16 for the second product.
+ * out [tokens, nq, head_dim] contiguous.  fp32 scores and sums, probabilities rounded to bf16 for the second product.  scale: of either sign, or zero.
  * b2_prefill_attention_supported says (1 / 0) whether the shape is served: head_dim 128, an even number of query heads per KV
  * head, blocks of a multiple of 128 tokens (block_size 0: no block table). */
 int b2_prefill_attention(b2_ctx* ctx, const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, int64_t kv_rows,

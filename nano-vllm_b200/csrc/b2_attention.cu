@@ -452,7 +452,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 // chain of tensor-core sums.  That leaves one CTA per (sequence, KV head) and shares its work out inside it: for the scores a
 // warp takes 16 tokens of each tile of 64, the maxima meet in shared memory, and for the product a warp takes 32 of the 128
 // dimensions and all tokens, with the probabilities from shared memory; every thread adds up the columns of its fragments in
-// their order.  On random data the results are flash-attn's but for 0 to 3 elements in a million.
+// their order.  Where flash-attn does not cut contexts the results are its own but for 0 to 3 elements in a million of random data.
 //
 // 64 contexts of 1056 tokens, 32 / 8 heads: 66.7 us in flash-attn, 45.2 here (6.1 TB/s); 96 of 70..700 47.0 and 28.8, 32 of 1056
 // 34.9 and 23.7.  Not for narrow groups, although batches of about equal contexts would gain where there are three CTAs an SM and more (64 of 1056

@@ -15,8 +15,9 @@ cases:
   silu_mid        gate/up + SiLU*mul, M=256, N=24576, K=4096, 2 weight copies
   attn_decode     decode attention, 64 contexts of 300..1371 tokens, 16 query / 8 KV heads, paged cache in shuffled blocks
   attn_decode_few the same with the first 24 of them
-  attn_decode_wide the same with the first 24 of them and 32 query heads
+  attn_decode_wide the 64 contexts with 32 query heads
   attn_prefill    causal prefill attention, 8 sequences of 2048 tokens, 16 query / 8 KV heads
+  attn_prefill_cached 8 sequences of 1024 tokens over 512 cached ones, 32 query / 8 KV heads, paged cache in shuffled blocks
   rowpar_decode   fused row-parallel launch, M=64, N=4096, Kr=12288 (Qwen3-8B down_proj at TP=1)
   rowpar_prefill  fused row-parallel launch, M=1024, N=5120, Kr=1024
   store_kvcache   paged-KV scatter, 16384 tokens x D=1024
@@ -81,7 +82,7 @@ def main():
         slots = torch.randperm(16 * 256, device=dev)[:m].to(torch.int32)
         call = lambda j: ops.qkv_fused(x, ws[j % copies], None, nq, nkv, 128, qw, kw, 1e-6, pos, cos_sin, kc, vc, slots)
     elif a.case.startswith("attn_decode"):
-        lens = [300 + 17 * i for i in range(64 if a.case == "attn_decode" else 24)]
+        lens = [300 + 17 * i for i in range(24 if a.case == "attn_decode_few" else 64)]
         need = [-(-n // 256) for n in lens]
         order = torch.randperm(sum(need), device=dev, generator=g).to(torch.int32)
         tables = torch.zeros(len(lens), max(need), dtype=torch.int32, device=dev)
@@ -94,6 +95,11 @@ def main():
         q, k, v = rnd(16384, 16, 128), rnd(16384, 8, 128), rnd(16384, 8, 128)
         cu = torch.arange(0, 16385, 2048, dtype=torch.int32, device=dev)
         call = lambda i: ops.prefill_attention(q, k, v, cu, cu, 2048, None, 128 ** -0.5)
+    elif a.case == "attn_prefill_cached":
+        q, kc, vc = rnd(8192, 32, 128), rnd(48, 256, 8, 128), rnd(48, 256, 8, 128)
+        cu, cu_k = (torch.arange(0, 8 * n + 1, n, dtype=torch.int32, device=dev) for n in (1024, 1536))
+        tables = torch.randperm(48, device=dev, generator=g).to(torch.int32).view(8, 6)
+        call = lambda i: ops.prefill_attention(q, kc, vc, cu, cu_k, 1024, tables, 128 ** -0.5)
     elif a.case in ("rowpar_decode", "rowpar_prefill", "oproj_decode"):
         m, n, k, copies = {"rowpar_decode": (64, 4096, 12288, 4), "rowpar_prefill": (1024, 5120, 1024, 8), "oproj_decode": (64, 4096, 4096, 8)}[a.case]
         x, ws, res, nw = rnd(m, k), [rnd(n, k, scale=0.02) for _ in range(copies)], rnd(m, n), rnd(n)
