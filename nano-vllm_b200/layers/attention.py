@@ -62,7 +62,7 @@ def _sdpa_paged(q, k_cache, v_cache, context_lens, block_tables, scale, q_lens=N
 
 @functools.lru_cache(maxsize=None)
 def _sms(device: int) -> int:
-    return torch.cuda.get_device_properties(device).multi_processor_count
+    return torch.cuda.get_device_properties(device).multi_processor_count if device >= 0 else 0
 
 
 def decode_is_cut(n_seqs: int, nq: int, nkv: int, block_size: int, sms: int) -> bool:
@@ -117,14 +117,14 @@ class Attention(nn.Module):
                 return _sdpa_paged(q, k_cache, v_cache, k_lens, ctx.block_tables, self.scale, q_lens)
             return _sdpa_paged(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
         n, nq, nkv = q.shape[0], self.num_heads, self.num_kv_heads
-        wide, o = nq > 2 * nkv, None
+        sms, o = _sms(q.get_device()) if nq > 2 * nkv else 0, None  # (0: not a wide group, or tensors that the kernels refuse)
         if ctx.is_prefill:
             cached = ctx.block_tables is not None  # prefix cache / chunked prefill: read K/V from the cache
-            if not (cached and wide and flash_attn_varlen_func is not None and
-                    prefill_is_short(n, ctx.cu_seqlens_q.numel() - 1, ctx.max_seqlen_q, nq, nkv, k_cache.shape[1], _sms(q.get_device()))):
+            if not (cached and sms and flash_attn_varlen_func is not None and
+                    prefill_is_short(n, ctx.cu_seqlens_q.numel() - 1, ctx.max_seqlen_q, nq, nkv, k_cache.shape[1], sms)):
                 o = ops.prefill_attention(q, k_cache if cached else k, v_cache if cached else v, ctx.cu_seqlens_q, ctx.cu_seqlens_k, ctx.max_seqlen_q,
                                           ctx.block_tables, self.scale)
-        elif not (wide and flash_attn_with_kvcache is not None and decode_is_cut(n, nq, nkv, k_cache.shape[1], _sms(q.get_device()))):
+        elif not (sms and flash_attn_with_kvcache is not None and decode_is_cut(n, nq, nkv, k_cache.shape[1], sms)):
             o = ops.paged_attention(q, k_cache, v_cache, ctx.context_lens, ctx.block_tables, self.scale)
         if o is not None:
             return o

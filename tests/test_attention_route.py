@@ -12,13 +12,14 @@ def route(pkg, monkeypatch):
     """attend() on fakes: (own kernel serves, library present, call) -> who answered."""
     from nanovllm_b200.layers import attention as A
 
-    def attend(nq, nkv, context, cache, q_rows, own=True, library=True):
+    def attend(nq, nkv, context, cache, q_rows, own=True, library=True, on_gpu=True):
         said = []
 
         def answer(name, result):
             return lambda q, *a, **k: said.append(name) or (q if result else None)
 
-        monkeypatch.setattr(A, "_sms", lambda _: SMS)
+        if on_gpu:
+            monkeypatch.setattr(A, "_sms", lambda _: SMS)
         monkeypatch.setattr(A, "ops", SimpleNamespace(paged_attention=answer("own", own), prefill_attention=answer("own", own)))
         for f in ("flash_attn_varlen_func", "flash_attn_with_kvcache"):
             monkeypatch.setattr(A, f, answer("library", True) if library else None)
@@ -59,3 +60,11 @@ def test_prefill(route, rows, nq, nkv, cached, block, who):
                               block_tables=torch.zeros(len(rows), 4, dtype=torch.int32) if cached else None)
     assert route(nq, nkv, context, meta_cache(nkv, block), sum(rows)) == who
     assert route(nq, nkv, context, meta_cache(nkv, block), sum(rows), library=False) == "own"
+
+
+def test_tensors_off_the_gpu_are_left_to_the_own_checks(route):
+    """They are refused there, as ever: no device is asked for its SMs."""
+    cu = torch.tensor([0, 1], dtype=torch.int32)
+    for context in (SimpleNamespace(is_prefill=False, context_lens=None, block_tables=None),
+                    SimpleNamespace(is_prefill=True, cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=1, max_seqlen_k=1, block_tables=torch.zeros(1, 4))):
+        assert route(32, 8, context, meta_cache(8), 1, on_gpu=False) == "own"
